@@ -21,7 +21,7 @@
 #include <cstdint>
 
 #include "../common/df32.h"
-#include "../common/rr_math.h"
+#include "../common/rr_math_split.h"
 #include "common.cuh"
 #include "dfeval.cuh"
 #include "mixed.cuh"
@@ -56,12 +56,12 @@ __device__ bool probe_eval64(const uint32_t* code, int len, const double* K, con
         st[sp++] = tos;
         tos = K[arg];
         break;
-      case RRG_OP_SIN: tos = rr_sin(tos); break;
-      case RRG_OP_COS: tos = rr_cos(tos); break;
-      case RRG_OP_LN: tos = rr_log(tos); break;
-      case RRG_OP_EXP: tos = rr_exp(tos); break;
-      case RRG_OP_SQRT: tos = __dsqrt_rn(tos); break;
-      case RRG_OP_SQR: tos = __dmul_rn(tos, tos); break;
+      case RRG_OP_SIN:
+      case RRG_OP_COS: tos = rrs_sincos(tos, op - RRG_OP_SIN); break;
+      case RRG_OP_LN: tos = rrs_log(tos); break;
+      case RRG_OP_EXP: tos = rrs_exp(tos); break;
+      case RRG_OP_SQRT: tos = fi_sqrt(tos); break;
+      case RRG_OP_SQR: tos = fi_mul(tos, tos); break;
       case RRG_OP_EMIT:
 #pragma unroll
         for (int s = 0; s < MM; ++s)
@@ -84,14 +84,14 @@ __device__ bool probe_eval64(const uint32_t* code, int len, const double* K, con
         switch (base) {
           case RRG_ADD: tos = __dadd_rn(a, b); break;
           case RRG_SUB: tos = __dsub_rn(a, b); break;
-          case RRG_MUL: tos = __dmul_rn(a, b); break;
-          case RRG_DIV: tos = __ddiv_rn(a, b); break;
+          case RRG_MUL: tos = fi_mul(a, b); break;
+          case RRG_DIV: tos = fi_div(a, b); break;
           case RRG_POW: tos = rr_pow(a, b); break;
-          case RRG_LT: tos = a < b ? 1.0 : 0.0; break;
-          case RRG_EQ: tos = a == b ? 1.0 : 0.0; break;
-          case RRG_NE: tos = a != b ? 1.0 : 0.0; break;
-          case RRG_MIN: tos = a < b ? a : b; break;
-          default: tos = a > b ? a : b; break;
+          case RRG_LT: tos = fi_lt(a, b) ? 1.0 : 0.0; break;
+          case RRG_EQ: tos = fi_eq(a, b) ? 1.0 : 0.0; break;
+          case RRG_NE: tos = fi_eq(a, b) ? 0.0 : 1.0; break;
+          case RRG_MIN: tos = fi_lt(a, b) ? a : b; break;
+          default: tos = fi_lt(b, a) ? a : b; break;
         }
       }
     }

@@ -15,7 +15,7 @@
 #include <cfloat>
 #include <cstdint>
 
-#include "../common/rr_math.h"
+#include "../common/rr_math_split.h"
 #include "../common/rr_sum.h"
 #include "common.cuh"
 #include "plain.cuh"
@@ -28,27 +28,37 @@ namespace {
 
 constexpr int kMaxK = RRG_MAX_TERMS;
 
+// Operators of the FP64 interpreter.  Sums take the FP64 pipe, one instruction
+// each; products, quotients, roots and comparisons are formed on the integer
+// pipes (csrc/common/fp64_int.h) and the elementary functions in their split
+// forms (rr_math_split.h): the kernel is bound by the FP64 pipe (an
+// instruction holds it for 16 cycles), so what leaves it is what is saved.
+// GB300, ms of the FP64 evaluation phase with native operations / now: 2048
+// random trees at 100k rows 105.1 / 78.5, a 660-candidate local-search round
+// at 1M rows 23.2 / 17.4.  The results are the same bits.
 __device__ __forceinline__ double bin64(int base, double a, double b) {
   switch (base) {
     case RRG_ADD: return __dadd_rn(a, b);
     case RRG_SUB: return __dsub_rn(a, b);
-    case RRG_MUL: return __dmul_rn(a, b);
-    case RRG_DIV: return __ddiv_rn(a, b);
+    case RRG_MUL: return fi_mul(a, b);
+    case RRG_DIV: return fi_div(a, b);
     case RRG_POW: return rr_pow(a, b);
-    case RRG_LT: return a < b ? 1.0 : 0.0;
-    case RRG_EQ: return a == b ? 1.0 : 0.0;
-    case RRG_NE: return a != b ? 1.0 : 0.0;
-    case RRG_MIN: return a < b ? a : b;
-    case RRG_MAX: return a > b ? a : b;
+    case RRG_LT: return fi_lt(a, b) ? 1.0 : 0.0;
+    case RRG_EQ: return fi_eq(a, b) ? 1.0 : 0.0;
+    case RRG_NE: return fi_eq(a, b) ? 0.0 : 1.0;
+    case RRG_MIN: return fi_lt(a, b) ? a : b;
+    case RRG_MAX: return fi_lt(b, a) ? a : b;
     default: return __longlong_as_double(0x7ff8000000000000ll);
   }
 }
 
 // Runs the code of one candidate on `row`; factor slot s is written to
-// out[s * n_pad + row].  Spill stack in shared memory, stride blockDim.x.
-// Table programs also read columns of T (same rows, column stride n_pad).
-__device__ __forceinline__ void run_row64(const uint32_t* code, int len, const double* consts, const DevData& ds,
-                                          int64_t row, double* st, double* out, const double* T, uint32_t* status) {
+// out[s * n_pad + row], or, with ONE (a one-column program), returned instead.
+// Spill stack in shared memory, stride blockDim.x.  Table programs also read
+// columns of T (same rows, column stride n_pad).
+template <bool ONE>
+__device__ __forceinline__ double run_row64(const uint32_t* code, int len, const double* consts, const DevData& ds,
+                                            int64_t row, double* st, double* out, const double* T, uint32_t* status) {
   double tos = 0.0;
   int sp = 0;
   const int stride = blockDim.x;
@@ -60,38 +70,38 @@ __device__ __forceinline__ void run_row64(const uint32_t* code, int len, const d
       case RRG_OP_LDV: tos = ds.X64[(int64_t)arg * ds.n_pad + row]; break;
       case RRG_OP_LDC: tos = consts[arg]; break;
       case RRG_OP_PSV:
-        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return; }
+        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return tos; }
         st[sp++ * stride] = tos;
         tos = ds.X64[(int64_t)arg * ds.n_pad + row];
         break;
       case RRG_OP_PSC:
-        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return; }
+        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return tos; }
         st[sp++ * stride] = tos;
         tos = consts[arg];
         break;
-      case RRG_OP_SIN: tos = rr_sin(tos); break;
-      case RRG_OP_COS: tos = rr_cos(tos); break;
-      case RRG_OP_LN: tos = rr_log(tos); break;
-      case RRG_OP_EXP: tos = rr_exp(tos); break;
-      case RRG_OP_SQRT: tos = __dsqrt_rn(tos); break;
-      case RRG_OP_SQR: tos = __dmul_rn(tos, tos); break;
+      case RRG_OP_SIN:
+      case RRG_OP_COS: tos = rrs_sincos(tos, op - RRG_OP_SIN); break;
+      case RRG_OP_LN: tos = rrs_log(tos); break;
+      case RRG_OP_EXP: tos = rrs_exp(tos); break;
+      case RRG_OP_SQRT: tos = fi_sqrt(tos); break;
+      case RRG_OP_SQR: tos = fi_mul(tos, tos); break;
       case kOpLDT: tos = T[(int64_t)arg * ds.n_pad + row]; break;
       case kOpPST:
-        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return; }
+        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return tos; }
         st[sp++ * stride] = tos;
         tos = T[(int64_t)arg * ds.n_pad + row];
         break;
       case RRG_OP_EMIT:
-        out[(int64_t)arg * ds.n_pad + row] = tos;
+        if (!ONE) out[(int64_t)arg * ds.n_pad + row] = tos;
         sp = 0;
         break;
       default: {
         const int kk = op - RRG_OP_BIN;
-        if (kk < 0 || kk >= 8 * RRG_N_BASE) { atomicOr(status, ST_BAD_CODE); return; }
+        if (kk < 0 || kk >= 8 * RRG_N_BASE) { atomicOr(status, ST_BAD_CODE); return tos; }
         const int base = kk >> 3, src = (kk & 7) >> 1, dir = kk & 1;
         double other;
         if (src == RRG_SRC_S) {
-          if (sp <= 0) { atomicOr(status, ST_STACK); return; }
+          if (sp <= 0) { atomicOr(status, ST_STACK); return tos; }
           other = st[--sp * stride];
         } else if (src == RRG_SRC_V) {
           other = ds.X64[(int64_t)arg * ds.n_pad + row];
@@ -104,6 +114,7 @@ __device__ __forceinline__ void run_row64(const uint32_t* code, int len, const d
       }
     }
   }
+  return tos;
 }
 
 // One-column table program on rows [r0, r1) of this block, written to Ac;
@@ -115,18 +126,18 @@ __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len,
   uint32_t f = 0;
   unsigned long long mx = 0;
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-    run_row64(code, len, consts, ds, r, st, Ac, T, status);
-    const double v = Ac[r];
-    const double a = fabs(v);
-    if (v != v) {
+    const double v = run_row64<true>(code, len, consts, ds, r, st, nullptr, T, status);
+    Ac[r] = v;
+    // on the bits of |v| (non-negative doubles order as integers, NaN above)
+    const unsigned long long a = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    if (a > 0x7ff0000000000000ull) {
       f |= kCsNaN;
-    } else if (!(a <= 1.35e154)) {  // infinite, or its square overflows
+    } else if (a > 0x5ff01c2a01d98729ull) {  // above 1.35e154: infinite, or its square overflows
       f |= kCsBig;
     } else {
-      const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
-      mx = bits > mx ? bits : mx;
+      mx = a > mx ? a : mx;
     }
-    if (r >= 1 && !(a <= 1e-150)) f |= kCsTail;
+    if (r >= 1 && a > 0x20ca2fe76a3f9475ull) f |= kCsTail;  // above 1e-150, or not finite
   }
   f = __reduce_or_sync(0xffffffffu, f);
   for (int o = 16; o > 0; o >>= 1) {
@@ -191,7 +202,7 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
     return;
   }
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x)
-    run_row64(code, cd.code_len, b.consts, ds, r, st, Ac, A, status);
+    run_row64<false>(code, cd.code_len, b.consts, ds, r, st, Ac, A, status);
 }
 
 namespace {
