@@ -12,12 +12,13 @@
  * 18.1 (a native quotient 143.9), a root 43.2 (a native one 150.2).
  *
  * Methods: significands as 64-bit integers with the leading bit at bit 63.
- *   product   the 128-bit product, normalised, rounded on its upper word with
- *             the lower word as a sticky bit;
+ *   product   a lower bound of the upper product word, normalised; rounding
+ *             is decided unless it lies next to a half-way point, where the
+ *             native product runs;
  *   quotient  the divisor's 64-bit reciprocal by Newton's iteration from an
  *             FP32 reciprocal, in fixed point, biased low by a few units, so
  *             that the upper product word is a lower bound of the quotient
- *             within 9 units of 2^-64; a quotient of two 53-bit significands
+ *             within 13 units of 2^-64; a quotient of two 53-bit significands
  *             is never half-way between two others, so rounding is decided
  *             unless the bound lies just below a half-way point, where the
  *             sign of the exact remainder of the half-way point decides;
@@ -80,23 +81,85 @@ RRM_FN double fi_pack(uint64_t sign, int e, uint64_t sig53) {
   return rrm_from_bits(sign | (sig53 + ((uint64_t)(uint32_t)(e - 1) << 52)));
 }
 
+/* a lower bound of floor(a b / 2^64), at most two below it: the three upper
+ * partial products, without the carries of the lower ones */
+RRM_FN uint64_t fi_mulhi_low(uint64_t a, uint64_t b) {
+  const uint64_t x = (uint64_t)fi_hi(a) * (uint32_t)b, y = (uint64_t)(uint32_t)a * fi_hi(b);
+  return (uint64_t)fi_hi(a) * fi_hi(b) + fi_hi(x) + fi_hi(y);
+}
+
+/* Operand range of an operation with one fixed operand: its other operand's
+ * upper word ha is in range when ha * 2 - lo2 <= span2 (unsigned), i.e. its
+ * biased exponent lies in [lo, hi]; never, when lo > hi. */
+typedef struct {
+  uint32_t lo2, span2;
+} fi_range;
+RRM_FN fi_range fi_range_of(int lo, int hi) {
+  fi_range r;
+  lo = lo < 1 ? 1 : lo;
+  hi = hi > 2046 ? 2046 : hi;
+  r.lo2 = lo > hi ? 1u : (uint32_t)lo << 21; /* ha * 2 is even */
+  r.span2 = lo > hi ? 0u : ((uint32_t)(hi - lo + 1) << 21) - 1u;
+  return r;
+}
+RRM_FN int fi_in_range(fi_range r, uint32_t ha) { return ha * 2u - r.lo2 <= r.span2; }
+/* the double of a 53-bit significand (possibly 2^53) and the rest of its
+ * upper word: sign and biased exponent - 1 */
+RRM_FN double fi_join(uint64_t sig, uint32_t add) {
+  return rrm_from_bits((uint64_t)(fi_hi(sig) + add) << 32 | (uint32_t)sig);
+}
+
+/* native operations out of line: a branch to them stays a branch (inlined, the
+ * compiler runs the native product for every operand and selects) */
+#if defined(__CUDACC__)
+#define FI_SLOW static __host__ __device__ __noinline__
+#else
+#define FI_SLOW static
+#endif
+FI_SLOW double fi_slow_mul(double a, double b) { return RRM_MUL(a, b); }
+
 /* ---------------------------------------------------------------- product -- */
 RRM_FN double fi_mul(double a, double b) {
   const uint64_t ua = rrm_bits(a), ub = rrm_bits(b);
   const int ea = fi_exp(ua), eb = fi_exp(ub), e = ea + eb - 1023;
-  if (!fi_normal(ea) || !fi_normal(eb) || (uint32_t)(e - 1) >= 2045u) return RRM_MUL(a, b);
-  const uint64_t A = fi_sig(ua), B = fi_sig(ub);
-  uint64_t hi = fi_mulhi(A, B), lo = A * B; /* in [2^126, 2^128) */
-  const int big = (int)(hi >> 63);
-  if (!big) {
-    hi = (hi << 1) | (lo >> 63);
-    lo <<= 1;
+  uint64_t q = fi_mulhi_low(fi_sig(ua), fi_sig(ub)); /* in [2^62 - 2, 2^64) */
+  const int small = (int64_t)q < 0 ? 0 : 1;
+  if (small) q += q;
+  /* the product's upper bits lie in [q, q + 6); next to a half-way point, and
+   * out of the normal range, the native product (a warp in ten) */
+  const uint32_t rest = (uint32_t)q & 0x7ffu;
+  if (rest - 0x3fau <= 6u || !fi_normal(ea) || !fi_normal(eb) || (uint32_t)(e - 1) >= 2045u) return fi_slow_mul(a, b);
+  return fi_pack((ua ^ ub) & FI_SIGN, e + 1 - small, (q >> 11) + (rest >> 10));
+}
+
+/* products by one fixed factor */
+typedef struct {
+  uint64_t sig;
+  double b;
+  fi_range range;
+  uint32_t add;
+} fi_factor;
+RRM_FN fi_factor fi_factor_of(double b) {
+  fi_factor f;
+  const uint64_t ub = rrm_bits(b);
+  const int eb = fi_exp(ub);
+  f.sig = fi_sig(ub);
+  f.b = b;
+  f.range = fi_range_of(fi_normal(eb) ? 1024 - eb : 1, fi_normal(eb) ? 3068 - eb : 0);
+  f.add = ((uint32_t)(eb - 1023) << 20) + (fi_hi(ub) & 0x80000000u);
+  return f;
+}
+RRM_FN double fi_mul_by(double a, fi_factor f) {
+  const uint64_t ua = rrm_bits(a);
+  const uint32_t ha = fi_hi(ua);
+  uint64_t q = fi_mulhi_low(fi_sig(ua), f.sig);
+  uint32_t add = (ha & 0xfff00000u) + f.add;
+  if ((int64_t)q >= 0) {
+    q += q;
+    add -= 0x00100000u;
   }
-  const uint64_t sig = hi >> 11;
-  /* the bits below the significand, the lower word as one sticky bit */
-  const uint32_t rest = ((uint32_t)hi & 0x7ffu) | (lo != 0 ? 1u : 0u);
-  const uint32_t up = rest + ((uint32_t)sig & 1u) > 0x400u ? 1u : 0u;
-  return fi_pack((ua ^ ub) & FI_SIGN, e + big, sig + up);
+  if (((uint32_t)q << 21) - (0x3fau << 21) < (7u << 21) || !fi_in_range(f.range, ha)) return fi_slow_mul(a, f.b);
+  return fi_join((q >> 11) + (((uint32_t)q >> 10) & 1u), add);
 }
 
 /* --------------------------------------------------------------- quotient -- */
@@ -118,37 +181,103 @@ RRM_FN uint64_t fi_recip64(uint64_t D) {
   return R1 + (uint64_t)((((int64_t)(int32_t)(R1 >> 33) * (int32_t)(E >> 21)) >> 41) - 2);
 }
 
-/* a / b for the divisor's bits ub (a normal number), its significand D and
- * R = fi_recip64(D) */
-RRM_FN double fi_div_by(double a, double b, uint64_t ub, uint64_t R) {
-  const uint64_t ua = rrm_bits(a);
-  const int ea = fi_exp(ua), e = ea - fi_exp(ub) + 1023;
-  const uint64_t sign = (ua ^ ub) & FI_SIGN;
-  if (!fi_normal(ea) || (uint32_t)(e - 2) >= 2045u) {
-    if ((ua << 1) == 0) return rrm_from_bits(sign); /* a zero over a normal number */
-    return RRM_DIV(a, b);
+/* quotients by one fixed divisor */
+typedef struct {
+  uint64_t R;  /* fi_recip64 of its significand */
+  double b;
+  fi_range range;
+  uint32_t add;
+} fi_divisor;
+RRM_FN fi_divisor fi_divisor_of(double b) {
+  fi_divisor d;
+  const uint64_t ub = rrm_bits(b);
+  const int eb = fi_exp(ub);
+  d.R = fi_recip64(fi_sig(ub));
+  d.b = b;
+  d.range = fi_range_of(fi_normal(eb) ? eb - 1021 : 1, fi_normal(eb) ? eb + 1023 : 0);
+  d.add = ((uint32_t)(1022 - eb) << 20) + (fi_hi(ub) & 0x80000000u);
+  return d;
+}
+/* operands out of range: a zero over a normal number is a zero, the others
+ * take the native operations (out of line: rare, and long where inlined) */
+FI_SLOW double fi_slow_div(double a, double b) {
+  const uint64_t ua = rrm_bits(a), ub = rrm_bits(b);
+  if ((ua << 1) == 0 && fi_normal(fi_exp(ub))) return rrm_from_bits((ua ^ ub) & FI_SIGN);
+  return RRM_DIV(a, b);
+}
+/* the rounded 53-bit significand of a / b for a in range; *add gets the rest
+ * of the upper word */
+RRM_FN uint64_t fi_quot(uint64_t ua, const fi_divisor* d, uint32_t* add) {
+  /* the quotient lies in [q, q + 13) after the shift */
+  uint64_t q = fi_mulhi_low(fi_sig(ua), d->R);
+  uint32_t s = (fi_hi(ua) & 0xfff00000u) + d->add;
+  const int small = (int64_t)q >= 0;
+  if (small) {
+    q += q;
+    s -= 0x00100000u;
   }
-  /* the quotient lies in [q, q + 9) after the shift */
-  uint64_t q = fi_mulhi(fi_sig(ua), R);
-  const int small = (int)(q >> 63) ^ 1;
-  q <<= small;
-  uint64_t sig = q >> 11;
-  const uint32_t rest = (uint32_t)q & 0x7ffu;
-  uint32_t up = rest >> 10;
-  if (rest - 0x3f4u < 0xcu) {
+  *add = s;
+  const uint64_t sig = q >> 11;
+  uint32_t up = ((uint32_t)q >> 10) & 1u;
+  if (((uint32_t)q << 21) - (0x3f2u << 21) < (0xeu << 21)) {
     /* just below half-way: up when A 2^(53 + small) > (2 sig + 1) D, on 53-bit
      * significands; the difference is far below 2^63 */
     const uint64_t ma = (ua & 0x000fffffffffffffull) | 0x0010000000000000ull;
-    const uint64_t mb = (ub & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    const uint64_t mb = (rrm_bits(d->b) & 0x000fffffffffffffull) | 0x0010000000000000ull;
     up = (int64_t)((ma << (53 + small)) - (2 * sig + 1) * mb) > 0 ? 1u : 0u;
   }
-  return fi_pack(sign, e - small, sig + up);
+  return sig + up;
+}
+RRM_FN double fi_div_by(double a, const fi_divisor* d) {
+  const uint64_t ua = rrm_bits(a);
+  if (!fi_in_range(d->range, fi_hi(ua))) return fi_slow_div(a, d->b);
+  uint32_t add;
+  const uint64_t sig = fi_quot(ua, d, &add);
+  return fi_join(sig, add);
 }
 
 RRM_FN double fi_div(double a, double b) {
-  const uint64_t ub = rrm_bits(b);
-  if (!fi_normal(fi_exp(ub))) return RRM_DIV(a, b);
-  return fi_div_by(a, b, ub, fi_recip64(fi_sig(ub)));
+  const fi_divisor d = fi_divisor_of(b);
+  return fi_div_by(a, &d);
+}
+
+/* f (a / b), both operations rounded: the quotient's significand goes on
+ * without being packed.  range: where both results are normal. */
+typedef struct {
+  fi_divisor d;
+  double f;
+  uint64_t sig;
+  fi_range range;
+  uint32_t add;
+} fi_scaled;
+RRM_FN fi_scaled fi_scaled_of(double f, double b) {
+  fi_scaled s;
+  const uint64_t uf = rrm_bits(f), ub = rrm_bits(b);
+  const int ef = fi_exp(uf), eb = fi_exp(ub);
+  const int ok = fi_normal(ef) && fi_normal(eb);
+  s.d = fi_divisor_of(b);
+  s.f = f;
+  s.sig = fi_sig(uf);
+  /* quotient exponent ea - eb + 1023, or one below, in [1, 2046] and in the factor's range */
+  const int lo = 1024 - ef > 1 ? 1024 - ef : 1, hi = 3068 - ef < 2046 ? 3068 - ef : 2046;
+  s.range = fi_range_of(ok ? eb - 1022 + lo : 1, ok ? eb - 1023 + hi : 0);
+  s.add = ((uint32_t)(ef - 1022) << 20) + (fi_hi(uf) & 0x80000000u);
+  return s;
+}
+FI_SLOW double fi_slow_scaled(double f, double a, double b) { return RRM_MUL(f, fi_slow_div(a, b)); }
+RRM_FN double fi_scaled_quot(double a, const fi_scaled* s) {
+  const uint64_t ua = rrm_bits(a);
+  uint32_t add;
+  const uint64_t sig = fi_quot(ua, &s->d, &add);
+  if (!fi_in_range(s->range, fi_hi(ua)) || (sig >> 53) != 0) return fi_slow_scaled(s->f, a, s->d.b);
+  uint64_t q = fi_mulhi_low(sig << 11, s->sig);
+  uint32_t add2 = add + s->add;
+  if ((int64_t)q >= 0) {
+    q += q;
+    add2 -= 0x00100000u;
+  }
+  if (((uint32_t)q << 21) - (0x3fau << 21) < (7u << 21)) return fi_slow_mul(s->f, fi_join(sig, add));
+  return fi_join((q >> 11) + (((uint32_t)q >> 10) & 1u), add2);
 }
 
 /* ------------------------------------------------------------------- root -- */

@@ -118,36 +118,23 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
 }
 
 // One-column table program on rows [r0, r1) of this block, written to Ac;
-// the column's statistics (NaN, infinite or overflowing square, non-trivial
-// tail, largest finite magnitude) merged into *cs.
+// the column's flags (NaN, infinite or overflowing square, non-trivial tail)
+// merged into *cs.
 __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len, const double* consts,
                                                   const DevData& ds, int64_t r0, int64_t r1, double* st, double* Ac,
                                                   const double* T, uint32_t* status, ColStat* cs) {
   uint32_t f = 0;
-  unsigned long long mx = 0;
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     const double v = run_row64<true>(code, len, consts, ds, r, st, nullptr, T, status);
     Ac[r] = v;
     // on the bits of |v| (non-negative doubles order as integers, NaN above)
     const unsigned long long a = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-    if (a > 0x7ff0000000000000ull) {
-      f |= kCsNaN;
-    } else if (a > 0x5ff01c2a01d98729ull) {  // above 1.35e154: infinite, or its square overflows
-      f |= kCsBig;
-    } else {
-      mx = a > mx ? a : mx;
-    }
+    if (a > 0x7ff0000000000000ull) f |= kCsNaN;
+    else if (a > 0x5ff01c2a01d98729ull) f |= kCsBig;  // above 1.35e154: infinite, or its square overflows
     if (r >= 1 && a > 0x20ca2fe76a3f9475ull) f |= kCsTail;  // above 1e-150, or not finite
   }
   f = __reduce_or_sync(0xffffffffu, f);
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long t = __shfl_xor_sync(0xffffffffu, mx, o);
-    mx = t > mx ? t : mx;
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (f) atomicOr(&cs->flags, f);
-    if (mx) atomicMax(&cs->maxabs, mx);
-  }
+  if ((threadIdx.x & 31) == 0 && f) atomicOr(&cs->flags, f);
 }
 
 }  // namespace
@@ -273,8 +260,8 @@ __device__ double make_householder_col(double* col, int64_t rows, int kk, double
     beta = __dsqrt_rn(__dadd_rn(__dmul_rn(c0, c0), tail_sq));
     if (c0 >= 0.0) beta = -beta;
     const double den = __dsub_rn(c0, beta);
-    const double rden = __drcp_rn(den);
-    for (int64_t i = kk + 1 + threadIdx.x; i < rows; i += blockDim.x) col[i] = div_by(col[i], den, rden);
+    const fi_divisor rden = fi_divisor_of(den);
+    for (int64_t i = kk + 1 + threadIdx.x; i < rows; i += blockDim.x) col[i] = fi_div_by(col[i], &rden);
     tau = __ddiv_rn(__dsub_rn(beta, c0), beta);
   }
   __syncthreads();

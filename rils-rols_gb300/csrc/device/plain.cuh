@@ -35,12 +35,15 @@ __global__ void finalize_kernel(DevBatch b, DevData ds, const int32_t* list, int
 
 __global__ void clear_results_kernel(const int32_t* list, int n, rrg_result* res, const int32_t* dcount = nullptr);
 
-// Column statistics of an FP64 table (gathered by plain_eval_kernel), for
-// deciding the column-pivoted QR's outcome on non-finite data without running it.
+// Column statistics of an FP64 table: flags gathered by plain_eval_kernel, for
+// deciding the column-pivoted QR's outcome on non-finite data without running
+// it, and the column's sums of squares in QSUM order (launch_col_sums, where
+// the chunked QR reads the column).
 struct ColStat {
-  uint32_t flags;       // kCs* bits
-  uint32_t pad;
-  unsigned long long maxabs;  // bits of the largest finite |value| (non-negative doubles order as integers)
+  uint32_t flags;   // kCs* bits
+  uint32_t ticket;  // row chunks of the sums that are done
+  double sumsq;     // over all rows
+  double tailsq;    // over the rows after the first
 };
 constexpr uint32_t kCsNaN = 1;   // a NaN value: the column's norm is NaN
 constexpr uint32_t kCsBig = 2;   // an infinite value or one whose square overflows

@@ -6,34 +6,59 @@
 // order of csrc/common/rr_sum.h.
 //
 // A candidate's rows are cut into chunks of RR_CHUNK rows.  A pass is one
-// launch over (candidate, chunk) items; an item is a 256-thread block whose
-// thread t is QSUM lane t of the chunk (its rows i with i mod 256 = t, in
-// increasing order), so the block folds its lanes into the chunk's totals.
-// The last block of a candidate to finish a pass (a ticket counter) adds the
-// chunk totals in chunk order and does the scalar work of the step (pivot
-// choice, rank rule, Householder scalars, norm down-dating) for the next pass:
+// launch over (candidate, chunk, column group) items; an item is a 256-thread
+// block whose thread t is QSUM lane t of the chunk (its rows i with
+// i mod 256 = t, in increasing order), so the block folds its lanes into the
+// chunk's totals.  The last block of a candidate to finish a pass (a ticket
+// counter) adds the chunk totals in chunk order and does the scalar work of the
+// step (pivot choice, rank rule, Householder scalars, norm down-dating):
 //
-//   init   [factors | 1 | y] copied into the working columns; the norms over
-//          rows >= 0 and the tails over rows >= 1; step 0's pivot and reflector
-//   A(kk)  the pivot tail divided by (c0 - beta) (the Householder vector v)
-//          and the dots v . a_j of the columns the reflector reaches; last
-//          block: row kk, -tmp_j, down-dating, and the pivot of step kk + 1
-//          when no norm must be recomputed
-//   B(kk)  a_j -= (tau v_i) tmp_j, and the sums of squares of updated columns
-//          step kk + 1 needs (recomputed norms over rows >= kk + 1, pivot
-//          tails over rows >= kk + 2); last block: step kk + 1's pivot and
+//   sums   once per table column, whatever the number of candidates that read
+//          it: its sum of squares over rows >= 0 and over rows >= 1, kept with
+//          the column's statistics
+//   begin  one warp per candidate: norms from those sums, step 0's pivot and
 //          reflector
+//   A(kk)  the dots v . a_j of the Householder vector v (the pivot's tail over
+//          c0 - beta) with the remaining columns; last block: row kk of R,
+//          -tmp_j, down-dating, and the pivot of step kk + 1 when no norm must
+//          be recomputed
+//   B(kk)  a_j += (tau v_i) (-tmp_j), and the sums of squares of updated
+//          columns that step kk + 1 needs (recomputed norms over rows >= kk + 1,
+//          pivot tails over rows >= kk + 2); last block: step kk + 1's pivot
+//          and reflector
 //   solve  back substitution with R and the transformed y
+//
+// What is not done: step 0 reads the table's columns, y and the column of ones
+// where they are (B(0) writes the working columns, so nothing is copied first);
+// v is not stored (both passes form it from the pivot's column, a quotient by
+// one divisor on the integer pipes, csrc/common/fp64_int.h); the last step
+// updates nothing (row kk of y is all the solve reads); and a rank cut ends the
+// factorisation, since later steps change neither the rank nor the leading
+// block that the solve reads.
 //
 // A sum over rows >= kk + 2 differs from the one over rows >= kk + 1 only in
 // the lane that owns row kk + 1, whose chain starts there: that lane forms
 // the shorter chain too, and the chunk holding row kk + 1 is folded twice.
+//
+// Bound: the FP64 pipe (one warp instruction holds it 17 to 20 cycles).  A
+// four-column candidate (three factors and the free term) takes 25 FP64
+// instructions a row (dots 10, updates 9, tails 3, its share of the column
+// sums) against 47 with the copy, a stored v and native quotients, and moves
+// about 32 columns against 51.  Measured on GB300 (QR phase, before / now): a
+// 660-candidate round at 1M rows, mostly three columns, 52.5 / 19.4 ms (13.3 ms
+// at 17 cycles for its 13 FP64 instructions a row); the re-scored candidates
+// of eight certified rounds at 1M rows 51.0 / 29.9 ms; 765 candidates at 20011
+// rows 4.02 / 2.50 ms; one candidate at 1M rows 0.59 / 0.29 ms.
+// Rows held per lane 8 (A) and 4 (B) at four resident blocks: 19.4 ms; 8 and 8
+// 19.8, 4 and 4 19.9, three resident blocks 21.6.
 #include <cfloat>
 #include <cstdint>
 
 #include "../common/error.h"
+#include "../common/fp64_int.h"
 #include "../common/rr_sum.h"
 #include "common.cuh"
+#include "plain.cuh"
 #include "qr_chunk.cuh"
 #include "qr_ops.cuh"
 #include "reduce.cuh"
@@ -43,8 +68,13 @@ namespace rrd {
 namespace {
 
 constexpr int kQC = RR_CHUNK;
-constexpr int kLaneRows = kQC / 256;
 constexpr double kDowndateThr = 1.4901161193847656e-08;  // sqrt(DBL_EPSILON)
+// rows of a lane handled together (loads in flight per column) in pass A and
+// the column sums, and in pass B
+constexpr int kRowsA = 8;
+constexpr int kRowsB = 4;
+// chunk totals staged together by a candidate's last block
+constexpr int kStage = 2048;
 
 __device__ __forceinline__ int job_count(const QrJob& j) {
   if (!j.dcount) return j.n_list;
@@ -57,46 +87,60 @@ __device__ __forceinline__ double* wcol(const QrJob& j, int t, int c, int s) {
   return j.M + (base + s) * j.ds.n_pad;
 }
 
+// Storage column s of the design [factors | 1 | y] as step 0 finds it; NULL:
+// the column of ones.
+__device__ __forceinline__ const double* design_col(const QrJob& j, int c, int k, int s) {
+  if (s == k) return j.ds.y64;
+  return s == k - 1 ? nullptr : factor_column(j.A, j.ds.n_pad, j.pc[c].a_col, s, j.colmap);
+}
+
 // chunk total of sum slot s; row nch holds the shorter-range variant
 __device__ __forceinline__ double* part_at(const QrJob& j, int t, int row, int s) {
   return j.part + ((int64_t)t * (j.nch + 1) + row) * j.max_cols + s;
 }
-
-// QSUM of the chunk totals of slot s in chunk order from 0; chunk `sp` (if
-// >= 0) contributes its variant instead
-__device__ __forceinline__ double chunk_total(const QrJob& j, int t, int s, int sp) {
-  double tot = 0.0;
-  for (int ch = 0; ch < j.nch; ++ch) tot = __dadd_rn(tot, __ldcg(part_at(j, t, ch == sp ? j.nch : ch, s)));
-  return tot;
+// R of candidate t: row kk, storage column s
+__device__ __forceinline__ double* r_at(const QrJob& j, int t, int kk, int s) {
+  return j.rmat + ((int64_t)t * j.max_cols + kk) * j.max_cols + s;
 }
 
-// Lane fold of cnt values per thread (RR256's fold: halving strides inside
-// each 32-lane group, then the eight group totals in order from 0) into
-// out[0 .. cnt) (shared).  red: 8 * CG shared doubles.
-template <int CG>
-__device__ __forceinline__ void fold_lanes(const double (&v)[CG], int cnt, double* red, double* out) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-#pragma unroll
-  for (int j = 0; j < CG; ++j)
-    if (j < cnt) {
-      const double s = warp_sum(v[j]);
-      if (l == 0) red[w * CG + j] = s;
+// Totals of sum slots [0, cnt) in chunk order from 0 into out (shared); chunk
+// `sp` (if >= 0) contributes its variant instead.  The totals are staged in
+// buf (kStage shared doubles) by the whole block, so that the ordered sums do
+// not wait on one load after the other.
+__device__ __forceinline__ void chunk_totals(const QrJob& j, int t, int cnt, int sp, double* buf, double* out) {
+  const int nch = j.nch;
+  const int per = nch <= kStage ? kStage / nch : 0;  // slots staged at once
+  if (per == 0) {
+    for (int s = threadIdx.x; s < cnt; s += blockDim.x) {
+      double tot = 0.0;
+      for (int ch = 0; ch < nch; ++ch) tot = __dadd_rn(tot, __ldcg(part_at(j, t, ch == sp ? nch : ch, s)));
+      out[s] = tot;
     }
-  __syncthreads();
-  if (threadIdx.x < cnt) {
-    double s = 0.0;
-    for (int i = 0; i < 8; ++i) s = __dadd_rn(s, red[i * CG + threadIdx.x]);
-    out[threadIdx.x] = s;
+    __syncthreads();
+    return;
   }
-  __syncthreads();
+  for (int s0 = 0; s0 < cnt; s0 += per) {
+    const int ns = cnt - s0 < per ? cnt - s0 : per;
+    for (int i = threadIdx.x; i < ns * nch; i += blockDim.x) {
+      const int s = i / nch, ch = i % nch;
+      buf[i] = __ldcg(part_at(j, t, ch == sp ? nch : ch, s0 + s));
+    }
+    __syncthreads();
+    for (int s = threadIdx.x; s < ns; s += blockDim.x) {
+      double tot = 0.0;
+      for (int ch = 0; ch < nch; ++ch) tot = __dadd_rn(tot, buf[s * nch + ch]);
+      out[s0 + s] = tot;
+    }
+    __syncthreads();
+  }
 }
 
 // After an item's chunk totals are written: true in the block that finishes
 // the candidate's pass last (every other block's writes are then visible)
-__device__ __forceinline__ bool last_block(QrState* S, int nch, int* s_flag) {
+__device__ __forceinline__ bool last_block(unsigned int* ticket, int items, int* s_flag) {
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) *s_flag = atomicAdd(&S->ticket, 1u) == (unsigned)(nch - 1) ? 1 : 0;
+  if (threadIdx.x == 0) *s_flag = atomicAdd(ticket, 1u) == (unsigned)(items - 1) ? 1 : 0;
   __syncthreads();
   const bool last = *s_flag != 0;
   if (last) __threadfence();
@@ -104,7 +148,8 @@ __device__ __forceinline__ bool last_block(QrState* S, int nch, int* s_flag) {
 }
 
 // Businger-Golub pivot of step kk (largest down-dated norm, first index on
-// ties), the rank rule of ColPivHouseholderQR.h:504-511, and the swap
+// ties), the rank rule of ColPivHouseholderQR.h:504-511, and the swap; a cut
+// ends the factorisation (size = rank)
 __device__ void select_pivot(QrState* S, int kk, double rows) {
   int big = kk;
   double bign = S->nupd[kk];
@@ -113,12 +158,14 @@ __device__ void select_pivot(QrState* S, int kk, double rows) {
       bign = S->nupd[j];
       big = j;
     }
-  if (S->nonzero == S->size && __dmul_rn(bign, bign) < __dmul_rn(S->thr_helper, rows - kk)) S->nonzero = kk;
+  if (__dmul_rn(bign, bign) < __dmul_rn(S->thr_helper, rows - kk)) {
+    S->size = kk;
+    return;
+  }
   if (big != kk) {
     double t = S->nupd[kk]; S->nupd[kk] = S->nupd[big]; S->nupd[big] = t;
     t = S->ndir[kk]; S->ndir[kk] = S->ndir[big]; S->ndir[big] = t;
-    int p = S->perm[kk]; S->perm[kk] = S->perm[big]; S->perm[big] = p;
-    p = S->pos2col[kk]; S->pos2col[kk] = S->pos2col[big]; S->pos2col[big] = p;
+    int p = S->pos2col[kk]; S->pos2col[kk] = S->pos2col[big]; S->pos2col[big] = p;
   }
 }
 
@@ -128,534 +175,456 @@ __device__ void householder_scalars(QrState* S, double c0, double tail_sq) {
     S->tau = 0.0;
     S->beta = c0;
     S->den = 1.0;
-    S->rden = 1.0;
     S->tau_zero = 1;
   } else {
     double beta = __dsqrt_rn(__dadd_rn(__dmul_rn(c0, c0), tail_sq));
     if (c0 >= 0.0) beta = -beta;
     const double den = __dsub_rn(c0, beta);
     S->den = den;
-    S->rden = __drcp_rn(den);
     S->tau = __ddiv_rn(__dsub_rn(beta, c0), beta);
     S->beta = beta;
     S->tau_zero = 0;
   }
 }
 
-// Shared per-item view of a candidate's state.
-struct ItemView {
-  int t, c, active, k, nwork, nsum, upd, tau_zero;
-  int piv;         // the pivot's storage column (step kk)
-  int fastq;       // pass B: work index of the one summed column formed during the update, or -1
-  int64_t lo, hi;  // rows of the item: [lo, hi)
-  double tau, den, rden;
-  int work[kQrMaxCols];   // storage columns the pass reads (and updates)
-  int slot[kQrMaxCols];   // per storage column: its sum slot, or -1
-  double ntmp[kQrMaxCols];
-};
+// Columns of one item.  Four: the accumulators, a column's rows and the
+// pivot's fit 64 registers (four resident blocks); a wider candidate takes
+// several items a chunk, each forming v again.
+constexpr int CG = 4;
+constexpr int kMinBlocks = 4;
 
-// Calls row(i) for the rows of this thread's lane in [lo, hi), in increasing
-// order; a full chunk needs no bounds test.
-template <class F>
-__device__ __forceinline__ void lane_rows(int64_t r0, int64_t lo, int64_t hi, F&& row) {
-  const int64_t base = r0 + threadIdx.x;
-  if (lo == r0 && hi == r0 + kQC) {
-#pragma unroll 2
-    for (int u = 0; u < kLaneRows; ++u) row(base + 256 * u);
-  } else {
-    int64_t first = base;
-    if (first < lo) first += (lo - first + 255) / 256 * 256;
-#pragma unroll 1
-    for (int64_t i = first; i < hi; i += 256) row(i);
-  }
+// Columns an item takes: CG, or fewer while the pass has less than two items
+// per block of the grid (a lone candidate at 1M rows has 62 chunks; one column
+// an item then spreads it over four times the blocks)
+__device__ __forceinline__ int cols_per_item(int64_t chunks, int width) {
+  int c = CG;
+  while (c > 1 && chunks * ((width + c - 1) / c) < 2 * (int64_t)gridDim.x) c >>= 1;
+  return c;
 }
 
-// Rows of this thread's lane in sub-chunks of kSub rows (kSubU per lane):
-// body(s0, full) for each sub-chunk of the item in order; `full` when every
-// row of the sub-chunk is in [lo, hi).
-constexpr int kSub = 2048;
-constexpr int kSubU = kSub / 256;
-template <class F>
+// Calls body(s0, full) for the lane's rows [lo, hi) of the chunk at r0 in
+// sub-chunks of U rows a lane, in order; `full`: every row of it is in range.
+template <int U, class F>
 __device__ __forceinline__ void sub_chunks(int64_t r0, int64_t lo, int64_t hi, F&& body) {
-  for (int64_t s0 = r0; s0 < r0 + kQC && s0 < hi; s0 += kSub) {
-    if (s0 + kSub <= lo) continue;
-    body(s0, s0 >= lo && s0 + kSub <= hi);
+  for (int64_t s0 = r0; s0 < r0 + kQC && s0 < hi; s0 += 256 * U) {
+    if (s0 + 256 * U <= lo) continue;
+    body(s0, s0 >= lo && s0 + 256 * U <= hi);
   }
 }
 
-// Reads the item's state into V (thread 0).  kk < 0: the copy pass.
-__device__ void load_view(ItemView& V, const QrJob& j, int t, int ch, int kk, int pass_a) {
-  QrState* S = j.state + t;
-  const int64_t rows = j.ds.n;
-  const int c = j.list[j.list_off + t];
-  V.t = t;
-  V.c = c;
-  if (kk < 0) {
-    const rrg_cand cd = j.b.cands[c];
-    const int k = j.pc[c].k;
-    V.active = cd.mode == RRG_TUNED && !(j.pc[c].pad & 1) && k >= 1;
-    if (V.active && k + 1 > j.max_cols) {
-      atomicOr(j.status, ST_TOO_LARGE);
-      V.active = 0;
-    }
-    if (!V.active && ch == 0) S->active = 0;
-    V.k = k;
-    if (V.active) {
-      V.nwork = k + 1;
-      V.nsum = k;
-      for (int s = 0; s <= k; ++s) {
-        V.work[s] = s;
-        V.slot[s] = s < k ? s : -1;
-      }
-    }
+// U rows of a column (ones when col is NULL); rows out of [lo, hi) read 0
+template <int U>
+__device__ __forceinline__ void load_rows(const double* col, int64_t i0, int64_t lo, int64_t hi, bool full,
+                                          double (&v)[U]) {
+  if (!col) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = 1.0;
+  } else if (full) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = __ldcg(col + i0 + 256 * u);
   } else {
-    V.active = S->active && kk < S->size;
-    if (V.active) {
-      const int k = S->k;
-      V.k = k;
-      V.tau = S->tau;
-      V.den = S->den;
-      V.rden = S->rden;
-      V.tau_zero = S->tau_zero;
-      V.piv = S->pos2col[kk];
-      V.upd = !S->tau_zero && rows - kk > 1;
-      int nw = 0;
-      if (V.upd) {
-        for (int p = kk + 1; p < k; ++p) V.work[nw++] = S->pos2col[p];
-        if (S->upd_y) V.work[nw++] = k;
-      }
-      if (pass_a) {
-        V.nsum = 0;
-      } else {
-        V.nsum = S->nsum;
-        for (int s = 0; s <= k; ++s) V.slot[s] = -1;
-        for (int q = 0; q < V.nsum; ++q) V.slot[S->sum_store[q]] = q;
-        V.fastq = -1;
-        if (V.upd) {
-          for (int q = 0; q < nw; ++q) {
-            V.ntmp[q] = S->ntmp[V.work[q]];
-            if (V.nsum == 1 && V.work[q] == S->sum_store[0]) V.fastq = q;
-          }
-        }
-      }
-      V.nwork = nw;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + 256 * u;
+      v[u] = i >= lo && i < hi ? __ldcg(col + i) : 0.0;
     }
   }
-  const int64_t r0 = (int64_t)ch * kQC;
-  V.lo = r0 > kk + 1 ? r0 : kk + 1;
-  V.hi = r0 + kQC < rows ? r0 + kQC : rows;
 }
 
-// ------------------------------------------------------- init and B(kk) ----
-// INIT: the copy pass (kk = -1).  Otherwise the rank-1 update of step kk and
-// the sums step kk + 1 needs.
-// Resident blocks the passes are compiled for (registers per thread <= 64K /
-// (256 x blocks)): the step passes stream columns with little register
-// state; the copy pass (run once) keeps a group's sources and sums.
-template <int CG, bool INIT = false>
-struct QrMinBlocks {
-  static constexpr int value = CG <= 8 ? (INIT ? 3 : 4) : 2;
+}  // namespace
+
+// ------------------------------------------------------------- column sums --
+__global__ void __launch_bounds__(256) col_sums_kernel(const double* T, int64_t n, int64_t n_pad, const int32_t* cols,
+                                                       int n_cols, const int32_t* dcount, ColStat* cst, double* part) {
+  __shared__ double red[8], outA[1], outB[1], buf[2 * kStage];
+  __shared__ int s_flag;
+  const int cnt = dcount ? min(*dcount, n_cols) : n_cols;
+  const int nch = (int)((n + kQC - 1) / kQC);
+  const int64_t items = (int64_t)cnt * nch;
+  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const int t = (int)(it / nch), ch = (int)(it % nch);
+    const int32_t c = cols[t];
+    const double* col = T + (int64_t)c * n_pad;
+    const int64_t r0 = (int64_t)ch * kQC, hi = r0 + kQC < n ? r0 + kQC : n;
+    const bool row0 = ch == 0 && threadIdx.x == 0;  // the lane owning row 0: also its chain without that row
+    double p = 0.0, q = 0.0;
+    sub_chunks<kRowsA>(r0, r0, hi, [&](int64_t s0, bool full) {
+      double v[kRowsA];
+      const int64_t i0 = s0 + threadIdx.x;
+      load_rows(col, i0, r0, hi, full, v);
+#pragma unroll
+      for (int u = 0; u < kRowsA; ++u)
+        if (full || i0 + 256 * u < hi) {
+          p = __fma_rn(v[u], v[u], p);
+          if (row0 && (u > 0 || s0 > 0)) q = __fma_rn(v[u], v[u], q);
+        }
+    });
+    double* pt = part + (int64_t)t * (nch + 1);
+    double va[1] = {p};
+    fold_lanes<1>(va, 1, red, outA);
+    if (ch == 0) {
+      va[0] = row0 ? q : p;
+      fold_lanes<1>(va, 1, red, outB);
+    }
+    if (threadIdx.x == 0) {
+      pt[ch] = outA[0];
+      if (ch == 0) pt[nch] = outB[0];
+    }
+    if (!last_block(&cst[c].ticket, nch, &s_flag)) continue;
+    for (int i = threadIdx.x; i <= nch && i < 2 * kStage; i += blockDim.x) buf[i] = __ldcg(pt + i);
+    __syncthreads();
+    if (threadIdx.x == 0 || threadIdx.x == 32) {
+      double tot = 0.0;
+      for (int i = 0; i < nch; ++i) {
+        const int x = threadIdx.x == 32 && i == 0 ? nch : i;
+        tot = __dadd_rn(tot, x < 2 * kStage ? buf[x] : __ldcg(pt + x));
+      }
+      if (threadIdx.x == 0) cst[c].sumsq = tot;
+      else cst[c].tailsq = tot;
+    }
+    if (threadIdx.x == 0) cst[c].ticket = 0;
+    __syncthreads();
+  }
+}
+
+namespace {
+
+// ------------------------------------------------------------------ begin --
+// One warp per candidate: norms, thresholds, step 0's pivot and reflector.
+__global__ void __launch_bounds__(128) qr_begin_kernel(QrJob j) {
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= job_count(j)) return;
+  QrState* S = j.state + t;
+  const int c = j.list[j.list_off + t];
+  const rrg_cand cd = j.b.cands[c];
+  const int k = j.pc[c].k;
+  bool active = cd.mode == RRG_TUNED && !(j.pc[c].pad & 1) && k >= 1;
+  if (active && k + 1 > j.max_cols) {
+    if (lane == 0) atomicOr(j.status, ST_TOO_LARGE);
+    active = false;
+  }
+  if (!active) {
+    if (lane == 0) S->active = 0;
+    return;
+  }
+  const double rows_d = (double)j.ds.n;
+  for (int s = lane; s <= k; s += 32) {
+    S->pos2col[s] = s;
+    if (s < k) {
+      const double sq = s == k - 1 ? rows_d : j.cst[j.colmap[j.pc[c].a_col + s]].sumsq;
+      const double nr = __dsqrt_rn(sq);
+      S->ndir[s] = nr;
+      S->nupd[s] = nr;
+    }
+  }
+  __syncwarp();
+  if (lane != 0) return;
+  S->active = 1;
+  S->k = k;
+  S->size = (int)(j.ds.n < k ? j.ds.n : k);
+  S->ticket = 0;
+  S->rec_any = 0;
+  S->nsum = 0;
+  double maxn = S->nupd[0];
+  for (int s = 1; s < k; ++s)
+    if (S->nupd[s] > maxn) maxn = S->nupd[s];
+  S->thr_helper = __ddiv_rn(__dmul_rn(__dmul_rn(maxn, DBL_EPSILON), __dmul_rn(maxn, DBL_EPSILON)), rows_d);
+  select_pivot(S, 0, rows_d);
+  if (S->size == 0) return;
+  const int ps = S->pos2col[0];
+  const double* col = design_col(j, c, k, ps);
+  const double tail = !col ? rows_d - 1.0 : j.cst[j.colmap[j.pc[c].a_col + ps]].tailsq;
+  householder_scalars(S, col ? col[0] : 1.0, j.ds.n == 1 ? 0.0 : tail);
+}
+
+// Shared per-item view: the columns of the item's group.
+struct ItemView {
+  const double* src[CG];  // NULL: ones
+  double* dst[CG];
+  double ntmp[CG];
+  int slot[CG];           // sum slot, or -1
 };
 
-template <int CG, bool INIT>
-__global__ void __launch_bounds__(256, (QrMinBlocks<CG, INIT>::value)) qr_sums_kernel(QrJob j, int kk) {
-  __shared__ ItemView V;
-  __shared__ double red[8 * CG], outA[CG], outB[CG];
-  __shared__ int s_flag;
-  __shared__ double s_norm[kQrMaxCols], s_tail[kQrMaxCols];
-  __shared__ double sbuf[kSub];  // pass B: tau v_i of a sub-chunk (lane-owned entries)
-  const int cnt = job_count(j);
-  const int64_t items = (int64_t)cnt * j.nch;
-  const int64_t rows = j.ds.n;
-  const int64_t sp_row = kk + 1;  // the row only the longer sums include
-  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-    const int t = (int)(it / j.nch), ch = (int)(it % j.nch);
-    QrState* S = j.state + t;
-    if (threadIdx.x == 0) load_view(V, j, t, ch, kk, 0);
-    __syncthreads();
-    if (!V.active) {
-      __syncthreads();
-      continue;
-    }
-    if (INIT) {
-      const int c = V.c, k = V.k;
-      const int64_t r0 = (int64_t)ch * kQC;
-      constexpr bool upd = false;
-      const bool sp_chunk = sp_row >= r0 && sp_row < r0 + kQC;
-      const bool sp_lane = sp_chunk && (int)(sp_row & 255) == (int)threadIdx.x;
-      for (int g0 = 0; g0 < V.nwork; g0 += CG) {
-        const int gc = V.nwork - g0 < CG ? V.nwork - g0 : CG;
-        double* cp[CG];
-        const double* src[CG];
-        double nt[CG], sa[CG];
-        bool sum[CG];
-        bool any_sum = false;
-  #pragma unroll
-        for (int q = 0; q < CG; ++q) {
-          const int s = q < gc ? V.work[g0 + q] : 0;
-          cp[q] = q < gc ? wcol(j, t, c, s) : nullptr;
-          sum[q] = q < gc && V.slot[s] >= 0;
-          any_sum = any_sum || sum[q];
-          nt[q] = 0.0;
-          sa[q] = 0.0;
-          src[q] = nullptr;
-          if (q < gc && s != k - 1)
-            src[q] = s < k - 1 ? factor_column(j.A, j.ds.n_pad, j.pc[c].a_col, s, j.colmap) : j.ds.y64;
-        }
-        // one row: every load first, then the arithmetic and the stores
-        auto load = [&](int64_t i, double (&a)[CG], double& tv) {
-  #pragma unroll
-          for (int q = 0; q < CG; ++q)
-            if (q < gc) a[q] = src[q] ? src[q][i] : 1.0;
-          tv = 0.0;
-        };
-        auto finish = [&](int64_t i, double (&a)[CG], double tv) {
-  #pragma unroll
-          for (int q = 0; q < CG; ++q)
-            if (q < gc) {
-              cp[q][i] = a[q];
-              if (sum[q]) sa[q] = __fma_rn(a[q], a[q], sa[q]);
-            }
-        };
-        lane_rows(r0, V.lo, V.hi, [&](int64_t i) {
-          double a[CG], tv;
-          load(i, a, tv);
-          finish(i, a, tv);
-        });
-        if (!any_sum) continue;  // uniform over the block
-        double va[CG], vb[CG];
-  #pragma unroll
-        for (int q = 0; q < CG; ++q) va[q] = sum[q] ? sa[q] : 0.0;
-        fold_lanes<CG>(va, gc, red, outA);
-        if (sp_chunk) {
-          // the lane owning row sp_row: its chain without that row
-  #pragma unroll
-          for (int q = 0; q < CG; ++q) vb[q] = va[q];
-          if (sp_lane) {
-  #pragma unroll
-            for (int q = 0; q < CG; ++q) vb[q] = 0.0;
-            for (int64_t i = sp_row + 256; i < V.hi; i += 256) {
-  #pragma unroll
-              for (int q = 0; q < CG; ++q)
-                if (sum[q]) {
-                  const double x = cp[q][i];
-                  vb[q] = __fma_rn(x, x, vb[q]);
-                }
-            }
-          }
-          fold_lanes<CG>(vb, gc, red, outB);
-        }
-        if (threadIdx.x < gc) {
-          const int sl = V.slot[V.work[g0 + threadIdx.x]];
-          if (sl >= 0) {
-            *part_at(j, t, ch, sl) = outA[threadIdx.x];
-            if (sp_chunk) *part_at(j, t, j.nch, sl) = outB[threadIdx.x];
-          }
-        }
-      }
-    } else {
-      const int c = V.c, k = V.k;
-      (void)k;
-      const int64_t r0 = (int64_t)ch * kQC;
-      const int64_t np = j.ds.n_pad;
-      double* Mb = j.M + (j.slot_cols > 0 ? (int64_t)t * j.slot_cols : j.pc[c].m_col) * np;
-      const double* vcol = Mb + (int64_t)V.piv * np;
-      const double tau = V.tau;
-      const bool sp_chunk = sp_row >= r0 && sp_row < r0 + kQC;
-      const bool sp_lane = sp_chunk && (int)(sp_row & 255) == (int)threadIdx.x;
-      const int fq = V.fastq;
-      double sf = 0.0;  // the summed column's chain, formed during the update
-      if (V.upd) {
-        // tau v_i of a sub-chunk's rows staged in shared memory (each thread
-        // reads back only its own lane's entries), then each column streamed
-        // on its own: its loads are independent of the other columns' stores
-        for (int g0 = 0; g0 < V.nwork; g0 += CG) {
-          const int gc = V.nwork - g0 < CG ? V.nwork - g0 : CG;
-          sub_chunks(r0, V.lo, V.hi, [&](int64_t s0, bool full) {
-#pragma unroll
-            for (int u = 0; u < kSubU; ++u) {
-              const int64_t i = s0 + threadIdx.x + 256 * u;
-              sbuf[threadIdx.x + 256 * u] = (full || (i >= V.lo && i < V.hi)) ? __dmul_rn(tau, vcol[i]) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < CG; ++q) {
-              if (q >= gc) break;
-              double* col = Mb + (int64_t)V.work[g0 + q] * np;
-              const double nt = V.ntmp[g0 + q];
-              const bool fsum = g0 + q == fq;
-              if (full) {
-#pragma unroll
-                for (int u = 0; u < kSubU; ++u) {
-                  const int64_t i = s0 + threadIdx.x + 256 * u;
-                  const double a = __fma_rn(sbuf[threadIdx.x + 256 * u], nt, col[i]);
-                  col[i] = a;
-                  if (fsum) sf = __fma_rn(a, a, sf);
-                }
-              } else {
-                for (int u = 0; u < kSubU; ++u) {
-                  const int64_t i = s0 + threadIdx.x + 256 * u;
-                  if (i < V.lo || i >= V.hi) continue;
-                  const double a = __fma_rn(sbuf[threadIdx.x + 256 * u], nt, col[i]);
-                  col[i] = a;
-                  if (fsum) sf = __fma_rn(a, a, sf);
-                }
-              }
-            }
-          });
-        }
-      }
-      // sums of squares of the summed columns (updated values): the one formed
-      // above, or a pass over each (a norm recomputation, an identity reflector)
-      for (int q0 = 0; q0 < V.nsum; ++q0) {
-        const double* col;
-        double pa;
-        if (fq >= 0) {
-          col = Mb + (int64_t)V.work[fq] * np;
-          pa = sf;
-        } else {
-          col = nullptr;
-          for (int s2 = 0; s2 <= V.k; ++s2)
-            if (V.slot[s2] == q0) col = Mb + (int64_t)s2 * np;
-          pa = 0.0;
-          lane_rows(r0, V.lo, V.hi, [&](int64_t i) {
-            const double x = col[i];
-            pa = __fma_rn(x, x, pa);
-          });
-        }
-        double va[1] = {pa}, vb[1];
-        fold_lanes<1>(va, 1, red, outA);
-        if (sp_chunk) {
-          // the lane owning row sp_row: its chain without that row
-          vb[0] = pa;
-          if (sp_lane) {
-            vb[0] = 0.0;
-            for (int64_t i = sp_row + 256; i < V.hi; i += 256) vb[0] = __fma_rn(col[i], col[i], vb[0]);
-          }
-          fold_lanes<1>(vb, 1, red, outB);
-        }
-        if (threadIdx.x == 0) {
-          const int sl = fq >= 0 ? 0 : q0;
-          *part_at(j, t, ch, sl) = outA[0];
-          if (sp_chunk) *part_at(j, t, j.nch, sl) = outB[0];
-        }
-        if (fq >= 0) break;
-      }
-    }
-    if (!last_block(S, j.nch, &s_flag)) continue;
-    // ---- the candidate's last block: totals, then step kk + 1's scalars
-    const int nsum = V.nsum;
-    const int sp = (int)(sp_row / kQC);
-    for (int q = threadIdx.x; q < nsum; q += blockDim.x) {
-      s_norm[q] = chunk_total(j, t, q, -1);
-      s_tail[q] = chunk_total(j, t, q, sp);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int c = V.c, k = V.k;
-      const double rows_d = (double)rows;
-      const int next = kk + 1;
-      bool choose = true;
-      if (INIT) {
-        S->active = 1;
-        S->k = k;
-        S->size = (int)(rows < k ? rows : k);
-        S->nonzero = S->size;
-        for (int s = 0; s < k; ++s) {
-          S->ndir[s] = __dsqrt_rn(s_norm[s]);
-          S->nupd[s] = S->ndir[s];
-          S->perm[s] = s;
-          S->pos2col[s] = s;
-          S->sum_store[s] = s;
-        }
-        S->pos2col[k] = k;
-        double maxn = S->nupd[0];
-        for (int s = 1; s < k; ++s)
-          if (S->nupd[s] > maxn) maxn = S->nupd[s];
-        S->thr_helper = __ddiv_rn(__dmul_rn(__dmul_rn(maxn, DBL_EPSILON), __dmul_rn(maxn, DBL_EPSILON)), rows_d);
-      } else {
-        // recomputed norms (ColPivHouseholderQR.h:566-569)
-        for (int q = 0; q < nsum; ++q)
-          if (S->sum_norm[q]) {
-            const int s = S->sum_store[q];
-            for (int p = next; p < k; ++p)
-              if (S->pos2col[p] == s) {
-                S->ndir[p] = __dsqrt_rn(s_norm[q]);
-                S->nupd[p] = S->ndir[p];
-              }
-          }
-        choose = S->rec_any != 0;
-      }
-      if (next < S->size) {
-        if (choose) {
-          select_pivot(S, next, rows_d);
-          S->upd_y = S->nonzero == S->size;
-        } else {
-          S->upd_y = S->upd_y_next;
-        }
-        const int ps = S->pos2col[next];
-        int q = 0;
-        while (q < nsum && S->sum_store[q] != ps) ++q;
-        if (q == nsum) {
-          atomicOr(j.status, ST_QR_STATE);
-          S->active = 0;
-        } else {
-          const double tail_sq = rows - next == 1 ? 0.0 : s_tail[q];
-          householder_scalars(S, __ldcg(wcol(j, t, c, ps) + next), tail_sq);
-        }
-      }
-      S->kk = next;
-      S->ticket = 0;
-    }
-    __syncthreads();
-  }
+// The whole state of a candidate between global and shared memory.
+__device__ __forceinline__ void copy_state(QrState* dst, const QrState* src) {
+  static_assert(sizeof(QrState) % 8 == 0, "copied by words");
+  const unsigned long long* s = reinterpret_cast<const unsigned long long*>(src);
+  unsigned long long* d = reinterpret_cast<unsigned long long*>(dst);
+  for (int i = threadIdx.x; i < (int)(sizeof(QrState) / 8); i += blockDim.x) d[i] = s[i];
+  __syncthreads();
 }
 
 // ------------------------------------------------------------------ A(kk) --
-template <int CG>
-__global__ void __launch_bounds__(256, QrMinBlocks<CG>::value) qr_passA_kernel(QrJob j, int kk) {
+__global__ void __launch_bounds__(256, kMinBlocks) qr_passA_kernel(QrJob j, int kk, int width) {
   __shared__ ItemView V;
   __shared__ double red[8 * CG], outA[CG];
   __shared__ int s_flag;
-  __shared__ double sbuf[kSub];  // v_i of a sub-chunk (lane-owned entries)
+  __shared__ double buf[kStage], tot[kQrMaxCols];
+  __shared__ QrState Ss;
+  __shared__ int8_t rec[kQrMaxCols];
   const int cnt = job_count(j);
-  const int64_t items = (int64_t)cnt * j.nch;
   const int64_t rows = j.ds.n;
+  const int cpi = cols_per_item((int64_t)cnt * j.nch, width);
+  const int gmax = (width + cpi - 1) / cpi;
+  const int64_t items = (int64_t)cnt * j.nch * gmax;
   for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-    const int t = (int)(it / j.nch), ch = (int)(it % j.nch);
+    const int g = (int)(it % gmax), ch = (int)(it / gmax % j.nch), t = (int)(it / ((int64_t)gmax * j.nch));
     QrState* S = j.state + t;
-    if (threadIdx.x == 0) load_view(V, j, t, ch, kk, 1);
+    if (!S->active || kk >= S->size) continue;  // uniform over the block
+    const int k = S->k, nw = k - kk, groups = (nw + cpi - 1) / cpi;
+    if (g >= groups) continue;
+    const int c = j.list[j.list_off + t];
+    const int q0 = g * cpi, gc = min(cpi, nw - q0);
+    const bool upd = !S->tau_zero && rows - kk > 1;
+    const int ps = S->pos2col[kk];
+    const double* piv = kk == 0 ? design_col(j, c, k, ps) : wcol(j, t, c, ps);
+    const fi_divisor den = fi_divisor_of(S->den);
+    if (threadIdx.x < gc) {
+      const int p = kk + 1 + q0 + threadIdx.x, s = p < k ? S->pos2col[p] : k;
+      V.src[threadIdx.x] = kk == 0 ? design_col(j, c, k, s) : wcol(j, t, c, s);
+    }
     __syncthreads();
-    if (!V.active) {
-      __syncthreads();
-      continue;
-    }
-    const int c = V.c;
-    const int64_t r0 = (int64_t)ch * kQC;
-    double* pcol = wcol(j, t, c, V.piv);
-    const double den = V.den, rden = V.rden;
-    // the Householder vector (Householder.h:83-90): the tail over c0 - beta,
-    // or zeros when the reflector is the identity
-    if (V.nwork == 0) {
-      const bool tz = V.tau_zero != 0;
-      lane_rows(r0, V.lo, V.hi, [&](int64_t i) { pcol[i] = tz ? 0.0 : div_by(pcol[i], den, rden); });
-    }
-    for (int g0 = 0; g0 < V.nwork; g0 += CG) {
-      const int gc = V.nwork - g0 < CG ? V.nwork - g0 : CG;
+    if (upd) {
+      const int64_t r0 = (int64_t)ch * kQC;
+      const int64_t lo = r0 > kk + 1 ? r0 : kk + 1, hi = r0 + kQC < rows ? r0 + kQC : rows;
       double pa[CG];
 #pragma unroll
       for (int q = 0; q < CG; ++q) pa[q] = 0.0;
-      const bool first = g0 == 0;
-      sub_chunks(r0, V.lo, V.hi, [&](int64_t s0, bool full) {
-        // the sub-chunk's v_i (divided once, by the first group) staged in
-        // shared memory; then each column's dot chain on its own
+      sub_chunks<kRowsA>(r0, lo, hi, [&](int64_t s0, bool full) {
+        const int64_t i0 = s0 + threadIdx.x;
+        double v[kRowsA], a[kRowsA];
+        load_rows(piv, i0, lo, hi, full, v);
+        load_rows(V.src[0], i0, lo, hi, full, a);
+        // the Householder vector (Householder.h:83-90): the tail over c0 - beta
 #pragma unroll
-        for (int u = 0; u < kSubU; ++u) {
-          const int64_t i = s0 + threadIdx.x + 256 * u;
-          double v = 0.0;
-          if (full || (i >= V.lo && i < V.hi)) {
-            v = pcol[i];
-            if (first) {
-              v = div_by(v, den, rden);
-              pcol[i] = v;
-            }
-          }
-          sbuf[threadIdx.x + 256 * u] = v;
-        }
+        for (int u = 0; u < kRowsA; ++u) v[u] = fi_div_by(v[u], &den);
 #pragma unroll
         for (int q = 0; q < CG; ++q) {
           if (q >= gc) break;
-          const double* col = wcol(j, t, c, V.work[g0 + q]);
+          if (q > 0) load_rows(V.src[q], i0, lo, hi, full, a);
           double acc = pa[q];
           if (full) {
 #pragma unroll
-            for (int u = 0; u < kSubU; ++u)
-              acc = __fma_rn(sbuf[threadIdx.x + 256 * u], col[s0 + threadIdx.x + 256 * u], acc);
+            for (int u = 0; u < kRowsA; ++u) acc = __fma_rn(v[u], a[u], acc);
           } else {
-            for (int u = 0; u < kSubU; ++u) {
-              const int64_t i = s0 + threadIdx.x + 256 * u;
-              if (i >= V.lo && i < V.hi) acc = __fma_rn(sbuf[threadIdx.x + 256 * u], col[i], acc);
+#pragma unroll
+            for (int u = 0; u < kRowsA; ++u) {
+              const int64_t i = i0 + 256 * u;
+              if (i >= lo && i < hi) acc = __fma_rn(v[u], a[u], acc);
             }
           }
           pa[q] = acc;
         }
       });
       fold_lanes<CG>(pa, gc, red, outA);
-      if (threadIdx.x < gc) *part_at(j, t, ch, g0 + threadIdx.x) = outA[threadIdx.x];
+      if (threadIdx.x < gc) *part_at(j, t, ch, q0 + threadIdx.x) = outA[threadIdx.x];
     }
-    if (!last_block(S, j.nch, &s_flag)) continue;
+    if (!last_block(&S->ticket, j.nch * groups, &s_flag)) continue;
     // ---- last block: row kk (Householder.h:121-126), then down-dating
-    const int nw = V.nwork;
-    const double tau = V.tau;
+    copy_state(&Ss, S);
+    if (upd) chunk_totals(j, t, nw, -1, buf, tot);
+    const int next = kk + 1;
     for (int q = threadIdx.x; q < nw; q += blockDim.x) {
-      const int s = V.work[q];
-      double* a = wcol(j, t, c, s);
-      const double w = chunk_total(j, t, q, -1);
-      const double qk = __ldcg(a + kk);
-      const double tmp = __dadd_rn(w, qk);
-      a[kk] = __dsub_rn(qk, __dmul_rn(tau, tmp));
-      S->ntmp[s] = -tmp;
+      const int p = next + q, s = p < k ? Ss.pos2col[p] : k;
+      const double* col = kk == 0 ? design_col(j, c, k, s) : wcol(j, t, c, s);
+      const double qk = col ? __ldcg(col + kk) : 1.0;
+      double a = qk;
+      if (upd) {
+        const double tmp = __dadd_rn(tot[q], qk);
+        a = __dsub_rn(qk, __dmul_rn(Ss.tau, tmp));
+        Ss.ntmp[s] = -tmp;
+      } else if (rows - kk == 1) {
+        a = __dmul_rn(qk, __dsub_rn(1.0, Ss.tau));  // a one-row tail
+      }
+      *r_at(j, t, kk, s) = a;
+      // LAWN 176 norm down-dating (ColPivHouseholderQR.h:549-572); the
+      // recomputations happen in pass B, which sums the updated columns
+      int flag = 0;
+      if (p < k && Ss.nupd[p] != 0.0) {
+        double temp = __ddiv_rn(fabs(a), Ss.nupd[p]);
+        temp = __dmul_rn(__dadd_rn(1.0, temp), __dsub_rn(1.0, temp));
+        temp = temp < 0.0 ? 0.0 : temp;
+        const double ratio = __ddiv_rn(Ss.nupd[p], Ss.ndir[p]);
+        const double temp2 = __dmul_rn(temp, __dmul_rn(ratio, ratio));
+        if (temp2 <= kDowndateThr) flag = 1;
+        else Ss.nupd[p] = __dmul_rn(Ss.nupd[p], __dsqrt_rn(temp));
+      }
+      rec[q] = (int8_t)flag;
+      Ss.slot_of[s] = -1;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      const int k = V.k;
-      if (rows - kk == 1) {
-        // a one-row tail: row kk of the other columns scaled by 1 - tau
-        for (int p = kk + 1; p < k; ++p) {
-          double* a = wcol(j, t, c, S->pos2col[p]);
-          a[kk] = __dmul_rn(__ldcg(a + kk), __dsub_rn(1.0, tau));
-        }
-        if (S->upd_y) {
-          double* a = wcol(j, t, c, k);
-          a[kk] = __dmul_rn(__ldcg(a + kk), __dsub_rn(1.0, tau));
-        }
-      }
-      pcol[kk] = S->beta;
-      // LAWN 176 norm down-dating (ColPivHouseholderQR.h:549-572); the
-      // recomputations happen in pass B, which sums the updated columns
+      *r_at(j, t, kk, ps) = Ss.beta;
       int rec_any = 0, nsum = 0;
-      for (int p = kk + 1; p < k; ++p) {
-        if (S->nupd[p] == 0.0) continue;
-        double temp = __ddiv_rn(fabs(__ldcg(wcol(j, t, c, S->pos2col[p]) + kk)), S->nupd[p]);
-        temp = __dmul_rn(__dadd_rn(1.0, temp), __dsub_rn(1.0, temp));
-        temp = temp < 0.0 ? 0.0 : temp;
-        const double ratio = __ddiv_rn(S->nupd[p], S->ndir[p]);
-        const double temp2 = __dmul_rn(temp, __dmul_rn(ratio, ratio));
-        if (temp2 <= kDowndateThr) {
-          S->sum_store[nsum] = S->pos2col[p];
-          S->sum_norm[nsum] = 1;
-          ++nsum;
-          rec_any = 1;
+      for (int q = 0; q < nw - 1; ++q) rec_any |= rec[q];
+      if (next < Ss.size) {
+        if (rec_any) {
+          // the pivot of step kk + 1 depends on the recomputed norms (and on
+          // NaN norms through the scan's running maximum): the sums of every
+          // remaining column, which a recomputation step can afford
+          for (int p = next; p < k; ++p) {
+            Ss.slot_of[Ss.pos2col[p]] = nsum;
+            Ss.sum_norm[nsum++] = rec[p - next];
+          }
         } else {
-          S->nupd[p] = __dmul_rn(S->nupd[p], __dsqrt_rn(temp));
+          select_pivot(&Ss, next, (double)rows);
+          if (next < Ss.size) {
+            Ss.slot_of[Ss.pos2col[next]] = 0;
+            Ss.sum_norm[0] = 0;
+            nsum = 1;
+          }
         }
       }
-      const int next = kk + 1;
-      if (next >= S->size) {
-        nsum = 0;  // no later step reads the norms
-      } else if (rec_any) {
-        // the pivot of step kk + 1 depends on the recomputed norms (and on
-        // NaN norms through the scan's running maximum): the tails of every
-        // remaining column, which a recomputation step can afford
-        for (int p = next; p < k; ++p) {
-          bool flagged = false;
-          for (int q = 0; q < nsum && !flagged; ++q) flagged = S->sum_store[q] == S->pos2col[p];
-          if (flagged) continue;
-          S->sum_store[nsum] = S->pos2col[p];
-          S->sum_norm[nsum] = 0;
-          ++nsum;
-        }
-      } else {
-        select_pivot(S, next, (double)rows);
-        S->upd_y_next = S->nonzero == S->size;
-        S->sum_store[0] = S->pos2col[next];
-        S->sum_norm[0] = 0;
-        nsum = 1;
-      }
-      S->rec_any = rec_any;
-      S->nsum = nsum;
-      S->ticket = 0;
+      Ss.rec_any = rec_any;
+      Ss.nsum = nsum;
+      Ss.ticket = 0;
     }
     __syncthreads();
+    copy_state(S, &Ss);
+  }
+}
+
+// ------------------------------------------------------------------ B(kk) --
+__global__ void __launch_bounds__(256, kMinBlocks) qr_passB_kernel(QrJob j, int kk, int width) {
+  __shared__ ItemView V;
+  __shared__ double red[8], outA[1], outB[1];
+  __shared__ int s_flag;
+  __shared__ double buf[kStage], s_norm[kQrMaxCols], s_tail[kQrMaxCols];
+  __shared__ QrState Ss;
+  const int cnt = job_count(j);
+  const int64_t rows = j.ds.n;
+  const int next = kk + 1;
+  const int cpi = cols_per_item((int64_t)cnt * j.nch, width);
+  const int gmax = (width + cpi - 1) / cpi;
+  const int64_t items = (int64_t)cnt * j.nch * gmax;
+  for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+    const int64_t it = items - 1 - w;  // pass A's last items first: what they read is still in L2
+    const int g = (int)(it % gmax), ch = (int)(it / gmax % j.nch), t = (int)(it / ((int64_t)gmax * j.nch));
+    QrState* S = j.state + t;
+    if (!S->active || next >= S->size) continue;  // the last step updates nothing that is read
+    const int k = S->k, nw = k - kk, groups = (nw + cpi - 1) / cpi;
+    if (g >= groups) continue;
+    const int c = j.list[j.list_off + t];
+    const int q0 = g * cpi, gc = min(cpi, nw - q0);
+    const bool upd = !S->tau_zero && rows - kk > 1;
+    const int ps = S->pos2col[kk];
+    const double* piv = kk == 0 ? design_col(j, c, k, ps) : wcol(j, t, c, ps);
+    const fi_scaled tq = fi_scaled_of(S->tau, S->den);
+    if (threadIdx.x < gc) {
+      const int p = next + q0 + threadIdx.x, s = p < k ? S->pos2col[p] : k;
+      V.dst[threadIdx.x] = wcol(j, t, c, s);
+      V.src[threadIdx.x] = kk == 0 ? design_col(j, c, k, s) : V.dst[threadIdx.x];
+      V.ntmp[threadIdx.x] = S->ntmp[s];
+      V.slot[threadIdx.x] = S->slot_of[s];
+    }
+    __syncthreads();
+    const int64_t r0 = (int64_t)ch * kQC;
+    const int64_t lo = r0 > next ? r0 : next, hi = r0 + kQC < rows ? r0 + kQC : rows;
+    const bool write = upd || kk == 0;
+    double ps2[CG];
+#pragma unroll
+    for (int q = 0; q < CG; ++q) ps2[q] = 0.0;
+    sub_chunks<kRowsB>(r0, lo, hi, [&](int64_t s0, bool full) {
+      const int64_t i0 = s0 + threadIdx.x;
+      double tv[kRowsB], a[kRowsB];
+      if (upd) load_rows(piv, i0, lo, hi, full, tv);
+      load_rows(V.src[0], i0, lo, hi, full, a);
+      if (upd) {
+#pragma unroll
+        for (int u = 0; u < kRowsB; ++u) tv[u] = fi_scaled_quot(tv[u], &tq);  // tau v_i
+      }
+#pragma unroll
+      for (int q = 0; q < CG; ++q) {
+        if (q >= gc) break;
+        double* dst = V.dst[q];
+        const double nt = V.ntmp[q];
+        const bool sum = V.slot[q] >= 0;
+        if (q > 0) load_rows(V.src[q], i0, lo, hi, full, a);
+        if (upd) {
+#pragma unroll
+          for (int u = 0; u < kRowsB; ++u) a[u] = __fma_rn(tv[u], nt, a[u]);
+        }
+        double acc = ps2[q];
+        if (full) {
+          if (write) {
+#pragma unroll
+            for (int u = 0; u < kRowsB; ++u) dst[i0 + 256 * u] = a[u];
+          }
+          if (sum) {
+#pragma unroll
+            for (int u = 0; u < kRowsB; ++u) acc = __fma_rn(a[u], a[u], acc);
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < kRowsB; ++u) {
+            const int64_t i = i0 + 256 * u;
+            if (i >= lo && i < hi) {
+              if (write) dst[i] = a[u];
+              if (sum) acc = __fma_rn(a[u], a[u], acc);
+            }
+          }
+        }
+        ps2[q] = acc;
+      }
+    });
+    // the sums' chunk totals; in the chunk holding row kk + 1 also without
+    // that row (the lane owning it forms its chain again)
+    const bool sp_chunk = next >= r0 && next < r0 + kQC;
+    const bool sp_lane = sp_chunk && (next & 255) == (int)threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < CG; ++q) {
+      if (q >= gc) break;
+      const int sl = V.slot[q];
+      if (sl < 0) continue;  // uniform
+      double va[1] = {ps2[q]};
+      fold_lanes<1>(va, 1, red, outA);
+      if (sp_chunk) {
+        if (sp_lane) {
+          va[0] = 0.0;
+          const double* col = write ? V.dst[q] : V.src[q];
+          for (int64_t i = next + 256; i < hi; i += 256) {
+            const double x = __ldcg(col + i);
+            va[0] = __fma_rn(x, x, va[0]);
+          }
+        }
+        fold_lanes<1>(va, 1, red, outB);
+      }
+      if (threadIdx.x == 0) {
+        *part_at(j, t, ch, sl) = outA[0];
+        if (sp_chunk) *part_at(j, t, j.nch, sl) = outB[0];
+      }
+    }
+    if (!last_block(&S->ticket, j.nch * groups, &s_flag)) continue;
+    // ---- the candidate's last block: totals, then step kk + 1's scalars
+    copy_state(&Ss, S);
+    const int nsum = Ss.nsum;
+    chunk_totals(j, t, nsum, -1, buf, s_norm);
+    chunk_totals(j, t, nsum, next / kQC, buf, s_tail);
+    if (threadIdx.x == 0) {
+      if (Ss.rec_any) {
+        // recomputed norms (ColPivHouseholderQR.h:566-569)
+        for (int p = next; p < k; ++p) {
+          const int q = Ss.slot_of[Ss.pos2col[p]];
+          if (q >= 0 && Ss.sum_norm[q]) {
+            Ss.ndir[p] = __dsqrt_rn(s_norm[q]);
+            Ss.nupd[p] = Ss.ndir[p];
+          }
+        }
+        select_pivot(&Ss, next, (double)rows);
+      }
+      if (next < Ss.size) {
+        const int np = Ss.pos2col[next], q = Ss.slot_of[np];
+        if (q < 0) {
+          atomicOr(j.status, ST_QR_STATE);
+          Ss.active = 0;
+        } else {
+          householder_scalars(&Ss, __ldcg(wcol(j, t, c, np) + next), rows - next == 1 ? 0.0 : s_tail[q]);
+        }
+      }
+      Ss.ticket = 0;
+    }
+    __syncthreads();
+    copy_state(S, &Ss);
   }
 }
 
@@ -667,51 +636,27 @@ __global__ void qr_solve_kernel(QrJob j) {
     if (!S->active) continue;
     const int c = j.list[j.list_off + t];
     const rrg_cand cd = j.b.cands[c];
-    const int k = S->k, r = S->nonzero, size = S->size;
+    const int k = S->k, r = S->size;
     double cvec[kQrMaxCols];
-    const double* yq = wcol(j, t, c, k);
-    for (int i = 0; i < r; ++i) cvec[i] = yq[i];
+    for (int i = 0; i < r; ++i) cvec[i] = *r_at(j, t, i, k);
     for (int kk = r - 1; kk >= 0; --kk) {
-      const double* rc = wcol(j, t, c, S->pos2col[kk]);
-      cvec[kk] = __ddiv_rn(cvec[kk], rc[kk]);
-      for (int i = 0; i < kk; ++i) cvec[i] = __dsub_rn(cvec[i], __dmul_rn(cvec[kk], rc[i]));
+      const int s = S->pos2col[kk];
+      cvec[kk] = __ddiv_rn(cvec[kk], *r_at(j, t, kk, s));
+      for (int i = 0; i < kk; ++i) cvec[i] = __dsub_rn(cvec[i], __dmul_rn(cvec[kk], *r_at(j, t, i, s)));
     }
     double* out = j.coefs + cd.coef_offset;
     for (int q = 0; q < k; ++q) out[q] = 0.0;
-    for (int i = 0; i < r; ++i) out[S->perm[i]] = cvec[i];
+    for (int i = 0; i < r; ++i) out[S->pos2col[i]] = cvec[i];
     j.res[c].rank = r;
     if (j.count_bytes) {
-      // the copy, then every remaining column (y while kk < rank) read and
-      // written once per step
-      double cols = (double)(2 * k + 1);
-      for (int kk = 0; kk < size; ++kk) cols += 2.0 * (double)((kk < r ? k + 1 : k) - kk);
+      // every remaining column read and written once per step, the pivot's
+      // and y read in the last
+      double cols = r > 0 ? 2.0 : 0.0;
+      for (int kk = 0; kk + 1 < r; ++kk) cols += 2.0 * (double)(k + 1 - kk);
       atomicAdd(reinterpret_cast<unsigned long long*>(j.status + kStatusQrBytes),
                 (unsigned long long)(cols * 8.0 * (double)j.ds.n));
     }
   }
-}
-
-template <int CG>
-bool launch_passes(const QrJob& job, int blocks, cudaStream_t st, int64_t* launches) {
-  const int steps = job.max_steps > 0 && job.max_steps < job.max_cols ? job.max_steps : job.max_cols - 1;
-  // tickets (and every other field) start at zero
-  if (cudaMemsetAsync(job.state, 0, sizeof(QrState) * (size_t)job.n_list, st) != cudaSuccess) {
-    cudaGetLastError();
-    rrc::set_error("QR state reset failed");
-    return false;
-  }
-  qr_sums_kernel<CG, true><<<blocks, 256, 0, st>>>(job, -1);
-  if (!launch_ok("QR init pass")) return false;
-  for (int kk = 0; kk < steps; ++kk) {
-    qr_passA_kernel<CG><<<blocks, 256, 0, st>>>(job, kk);
-    qr_sums_kernel<CG, false><<<blocks, 256, 0, st>>>(job, kk);
-    if (!launch_ok("QR step passes")) return false;
-  }
-  const int sb = (int)((job.n_list + 127) / 128);
-  qr_solve_kernel<<<sb < 1 ? 1 : sb, 128, 0, st>>>(job);
-  if (!launch_ok("QR solve")) return false;
-  if (launches) *launches += 2 + 2 * (int64_t)steps;
-  return true;
 }
 
 }  // namespace
@@ -719,7 +664,7 @@ bool launch_passes(const QrJob& job, int blocks, cudaStream_t st, int64_t* launc
 size_t qr_chunk_scratch_bytes(int64_t n_list, int64_t rows, int max_cols) {
   const int64_t nch = (rows + kQC - 1) / kQC;
   const size_t st = round_up(sizeof(QrState) * (size_t)n_list, 256);
-  return st + sizeof(double) * (size_t)n_list * (size_t)(nch + 1) * (size_t)max_cols;
+  return st + sizeof(double) * (size_t)n_list * (size_t)max_cols * (size_t)(nch + 1 + max_cols);
 }
 
 void qr_chunk_bind(QrJob& job, void* scratch) {
@@ -727,22 +672,13 @@ void qr_chunk_bind(QrJob& job, void* scratch) {
   const size_t st = round_up(sizeof(QrState) * (size_t)job.n_list, 256);
   job.state = static_cast<QrState*>(scratch);
   job.part = reinterpret_cast<double*>(static_cast<char*>(scratch) + st);
+  job.rmat = job.part + (size_t)job.n_list * (size_t)(job.nch + 1) * (size_t)job.max_cols;
 }
 
-int qr_chunk_blocks_per_sm(int max_cols) {
+int qr_chunk_blocks_per_sm() {
   int a = 0, b = 0;
-  cudaError_t e1, e2;
-  if (max_cols <= 5) {
-    e1 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, qr_sums_kernel<4, false>, 256, 0);
-    e2 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, qr_passA_kernel<4>, 256, 0);
-  } else if (max_cols <= 9) {
-    e1 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, qr_sums_kernel<8, false>, 256, 0);
-    e2 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, qr_passA_kernel<8>, 256, 0);
-  } else {
-    e1 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, qr_sums_kernel<16, false>, 256, 0);
-    e2 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, qr_passA_kernel<16>, 256, 0);
-  }
-  if (e1 != cudaSuccess || e2 != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, qr_passA_kernel, 256, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, qr_passB_kernel, 256, 0) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
@@ -750,18 +686,39 @@ int qr_chunk_blocks_per_sm(int max_cols) {
   return m < 1 ? 1 : m;
 }
 
-bool launch_qr_chunked(const QrJob& job, int blocks, cudaStream_t st, int64_t* launches) {
+bool launch_col_sums(const double* T, const DevData& ds, const int32_t* cols, int n_cols, const int32_t* dcount,
+                     ColStat* cst, double* part, int max_blocks, cudaStream_t st) {
+  if (n_cols <= 0) return true;
+  const int64_t items = (int64_t)n_cols * ((ds.n + kQC - 1) / kQC);
+  const int grid = (int)(items < max_blocks ? items : max_blocks);
+  col_sums_kernel<<<grid < 1 ? 1 : grid, 256, 0, st>>>(T, ds.n, ds.n_pad, cols, n_cols, dcount, cst, part);
+  return launch_ok("column sums");
+}
+
+bool launch_qr_chunked(const QrJob& job, int max_blocks, cudaStream_t st, int64_t* launches) {
   if (job.n_list <= 0) return true;
   if (job.max_cols > kQrMaxCols || job.max_cols < 2) {
     rrc::set_error("QR launch: column bound outside the kernel's range");
     return false;
   }
-  if (blocks < 1) blocks = 1;
-  // the work set of a pass: the columns after the pivot and y (at most k)
-  const int w = job.max_cols - 1;
-  if (w <= 4) return launch_passes<4>(job, blocks, st, launches);
-  if (w <= 8) return launch_passes<8>(job, blocks, st, launches);
-  return launch_passes<16>(job, blocks, st, launches);
+  const int steps = job.max_steps > 0 && job.max_steps < job.max_cols ? job.max_steps : job.max_cols - 1;
+  qr_begin_kernel<<<(job.n_list + 3) / 4, 128, 0, st>>>(job);
+  if (!launch_ok("QR begin")) return false;
+  for (int kk = 0; kk < steps; ++kk) {
+    // a candidate of k columns reaches k - kk of them (the free term and y
+    // included); at most steps - kk over the job
+    const int width = steps - kk;
+    const int64_t items = (int64_t)job.n_list * job.nch * width;
+    const int blocks = (int)(items < max_blocks ? items : max_blocks);
+    qr_passA_kernel<<<blocks < 1 ? 1 : blocks, 256, 0, st>>>(job, kk, width);
+    if (kk + 1 < steps) qr_passB_kernel<<<blocks < 1 ? 1 : blocks, 256, 0, st>>>(job, kk, width);
+    if (!launch_ok("QR step passes")) return false;
+  }
+  const int sb = (int)((job.n_list + 127) / 128);
+  qr_solve_kernel<<<sb < 1 ? 1 : sb, 128, 0, st>>>(job);
+  if (!launch_ok("QR solve")) return false;
+  if (launches) *launches += 1 + 2 * (int64_t)steps;
+  return true;
 }
 
 }  // namespace rrd

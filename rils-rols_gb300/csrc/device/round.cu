@@ -1276,7 +1276,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       const int nbx = (int)std::max<int64_t>(1, std::min<int64_t>(16, (ds->n + 32767) / 32768));
       const size_t stat_words = 2 + kFbReasons + (size_t)n_levels;
       if (!d_rlist2.reserve(sizeof(int32_t) * (cnt + 1)) || !d_fbneed.reserve(std::max(1, ncol)) ||
-          !d_fbcols.reserve(sizeof(int32_t) * (ncol + n_levels + 1)) ||
+          !d_fbcols.reserve(sizeof(int32_t) * (2 * (size_t)ncol + n_levels + 1)) ||
+          !d_cpart.reserve(sizeof(double) * std::max<size_t>(1, (size_t)ncol * (size_t)(nch + 1))) ||
           !d_fbF64.reserve(col8 * std::max(1, ncol)) || !d_fbcst.reserve(sizeof(ColStat) * std::max(1, ncol)) ||
           !d_fbgram.reserve(sizeof(double) * (size_t)cnt * nbx * (kGramCols * (kGramCols + 1) / 2)) ||
           !d_fbblist.reserve(sizeof(int32_t) * ((size_t)kQrBuckets * cnt + kQrBuckets)) ||
@@ -1290,6 +1291,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       uint8_t* need = static_cast<uint8_t*>(d_fbneed.ptr);
       int32_t* lvl_cols = static_cast<int32_t*>(d_fbcols.ptr);
       int32_t* lvl_count = lvl_cols + ncol;
+      int32_t* all_cols = lvl_count + n_levels;  // the same columns in one list, its length last
+      int32_t* all_count = all_cols + ncol;
       double* F64 = static_cast<double*>(d_fbF64.ptr);
       ColStat* cst = static_cast<ColStat*>(d_fbcst.ptr);
       double* gpart = static_cast<double*>(d_fbgram.ptr);
@@ -1351,7 +1354,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
                                pf.at<const int32_t>(d_fbpack, o_doff), pf.at<const int32_t>(d_fbpack, o_deps),
                                n_kept ? d_kept : nullptr, need, stream) ||
           !launch_rescore_levels(need, pf.at<const int32_t>(d_fbpack, o_lend), n_levels, lvl_cols, lvl_count,
-                                 stream) ||
+                                 all_cols, all_count, stream) ||
           (n_kept && !launch_lane_copy(need, d_kept, ncol, static_cast<const double*>(d_F64.ptr),
                                        static_cast<const ColStat*>(d_ccst.ptr), F64, cst, ds->n_pad, stream))) {
         cuda_ok(cudaGetLastError(), "re-scoring list launch");
@@ -1391,6 +1394,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         }
       }
       for (int32_t L = 0; L < n_levels; ++L) eval_level(L, waves);
+      if (!launch_col_sums(F64, dd, all_cols, ncol, all_count, cst, static_cast<double*>(d_cpart.ptr), 8 * sm_count,
+                           stream))
+        return RRG_E_CUDA;
       sentinel_classify_kernel<<<(cnt + 127) / 128, 128, 0, stream>>>(dev, fb_list, 0, cnt, d_pcs, d_ccol, cst,
                                                                      ds->n, coefs, res, status + kStatusSentinel,
                                                                      fb_count);
@@ -1403,7 +1409,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         return RRG_E_CUDA;
       }
       mark_end(P_PLAIN_EVAL, t0);
-      launches += n_levels + 6;
+      launches += n_levels + 7;
       // the QR of every bucket, side by side on the side streams: the chunked
       // passes over the bucket's list, qbatch[q] candidates per batch
       t0 = mark_begin();
@@ -1425,6 +1431,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
           jb.dcount = bcount + q;
           jb.A = F64;
           jb.colmap = d_ccol;
+          jb.cst = cst;
           jb.M = Mq + m_off * ds->n_pad;
           jb.slot_cols = kBucketCols[q];
           jb.coefs = coefs;
@@ -1434,7 +1441,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
           jb.max_cols = kBucketCols[q];
           jb.max_steps = bucket_wide[q] - 1;
           qr_chunk_bind(jb, static_cast<char*>(d_qrs.ptr) + q_off);
-          if (!launch_qr_chunked(jb, qr_blocks(kBucketCols[q], (int64_t)qbatch[q] * nch), sq, &launches)) {
+          if (!launch_qr_chunked(jb, qr_blocks(), sq, &launches)) {
             cuda_ok(cudaGetLastError(), "QR launch");
             return RRG_E_CUDA;
           }
@@ -1700,7 +1707,18 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       for (int s = 0; s < m; ++s) colmap.push_back(cp.fslot[lid[ft.ids[ft.cand_off[c] + s]]]);
     }
     subs.push_back({sub0, ng});
+    // the columns whose sums of squares the chunked QR starts from: the
+    // factors' among the evaluated ones (kept columns keep theirs, so they are
+    // formed wherever columns are kept)
+    const bool chunked = ds->n > RR_CHUNK;
+    std::vector<int32_t> scol;
+    if (chunked || cp.kept) {
+      for (int32_t l : cp.mprog) scol.push_back(cp.fslot[l]);
+      std::sort(scol.begin(), scol.end());
+      scol.erase(std::unique(scol.begin(), scol.end()), scol.end());
+    }
     Packer pk;
+    const size_t o_scol = pk.add(scol.data(), sizeof(int32_t) * std::max<size_t>(1, scol.size()));
     const size_t o_fcode = pk.add(fcode.data(), sizeof(uint32_t) * std::max<size_t>(1, fcode.size()));
     const size_t o_ewcol = pk.add(cp.ewcol.data(), sizeof(int32_t) * std::max<size_t>(1, cp.ewcol.size()));
     const size_t o_fc = pk.add(fc.data(), sizeof(rrg_cand) * fc.size());
@@ -1712,7 +1730,8 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     if (pst != RRG_OK) return pst;
     const size_t n_slots = (size_t)std::max<int64_t>(1, cp.arena);
     if (!d_F64.grow_keep(col8 * n_slots, d_F64.cap) || !d_M.reserve(col8 * mcols_max) ||
-        !d_ccst.grow_keep(sizeof(ColStat) * n_slots, d_ccst.cap)) {
+        !d_ccst.grow_keep(sizeof(ColStat) * n_slots, d_ccst.cap) ||
+        !d_cpart.reserve(sizeof(double) * std::max<size_t>(1, scol.size() * (size_t)(nb_res + 1)))) {
       rrc::set_error("FP64 round: table allocation failed");
       return RRG_E_OOM;
     }
@@ -1736,11 +1755,11 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     // gathered by the evaluator, then the candidates whose QR outcome is
     // certainly the all-NaN sentinel (their QR and residual work is skipped)
     ColStat* cst = static_cast<ColStat*>(d_ccst.ptr);
-    static_assert(sizeof(ColStat) == 2 * sizeof(unsigned long long), "ColStat is two words");
+    static_assert(sizeof(ColStat) == 3 * sizeof(unsigned long long), "ColStat is three words");
     if (!cp.kept)
       RRG_CUDA(cudaMemsetAsync(cst, 0, sizeof(ColStat) * (size_t)std::max(1, ne), stream));
     else if (!launch_fill_slots(pk.at<const int32_t>(d_ft64, o_ewcol), ne, reinterpret_cast<unsigned long long*>(cst),
-                                2, 0ull, stream))
+                                3, 0ull, stream))
       return RRG_E_CUDA;
     cudaEvent_t t0 = mark_begin();
     // one launch (or several of at most 65535 columns) per level; blocks per
@@ -1783,6 +1802,10 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       }
       c0 = c1;
     }
+    if (!launch_col_sums(F64, dd, pk.at<const int32_t>(d_ft64, o_scol), (int)scol.size(), nullptr, cst,
+                         static_cast<double*>(d_cpart.ptr), 8 * sm_count, stream))
+      return RRG_E_CUDA;
+    launches += scol.empty() ? 0 : 1;
     sentinel_classify_kernel<<<(ng + 127) / 128, 128, 0, stream>>>(dev, d_list, 0, ng,
                                                                    pk.at<PlainCand>(d_ft64, o_pcs), d_cmap, cst,
                                                                    ds->n, coefs, res, status + kStatusSentinel);
@@ -1821,7 +1844,6 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
         size_t off;
       };
       std::vector<QrRun> runs;
-      const bool chunked = ds->n > RR_CHUNK;
       size_t qbytes = 0;
       for (int32_t b0 = sb.first; b0 < sb.second;) {
         const int bk = bucket(list[pos + b0]);
@@ -1861,6 +1883,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
           jb.dcount = nullptr;
           jb.A = F64;
           jb.colmap = d_cmap;
+          jb.cst = cst;
           jb.M = M;
           jb.slot_cols = 0;
           jb.coefs = coefs;
@@ -1870,7 +1893,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
           jb.max_cols = r.bk;
           jb.max_steps = r.wide - 1;
           qr_chunk_bind(jb, static_cast<char*>(d_qrs.ptr) + r.off);
-          ok = launch_qr_chunked(jb, qr_blocks(r.bk, (int64_t)jb.n_list * jb.nch), s, &launches);
+          ok = launch_qr_chunked(jb, qr_blocks(), s, &launches);
         }
         if (!ok) {
           cuda_ok(cudaGetLastError(), "QR launch");

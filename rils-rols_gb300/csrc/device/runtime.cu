@@ -560,16 +560,13 @@ std::vector<DevBuf*> rrg_context::all_bufs() {
   return {&d_batch, &d_A, &d_pc, &d_partial, &d_list, &d_qrs, &d_terms, &d_fallback, &d_sse1, &d_probe,
           &d_nanrow, &d_cert_e, &d_ft, &d_ftp, &d_ft64, &d_F, &d_P, &d_Pc, &d_psum, &d_F64, &d_M,
           &d_gram, &d_rlist2, &d_fbpack, &d_fbneed, &d_fbcols, &d_fbF64, &d_fbcst, &d_fbgram, &d_fbblist,
-          &d_fbM, &d_fbctr, &d_cself, &d_cprobe, &d_cfnan, &d_ccst, &d_slots, &d_store, &d_res, &d_coefs, &d_status};
+          &d_fbM, &d_fbctr, &d_cself, &d_cprobe, &d_cfnan, &d_ccst, &d_cpart, &d_store, &d_res, &d_coefs, &d_status};
 }
 
-// Persistent grid of the chunked QR's passes for `items` candidate x chunk items.
-int rrg_context::qr_blocks(int max_cols, int64_t items) {
-  const int w = max_cols - 1;
-  const int g = w <= 4 ? 0 : (w <= 8 ? 1 : 2);
-  if (!qr_bps[g]) qr_bps[g] = qr_chunk_blocks_per_sm(max_cols);
-  const int64_t cap = (int64_t)sm_count * qr_bps[g];
-  return (int)std::max<int64_t>(1, std::min<int64_t>(cap, items));
+// Most blocks of a chunked QR pass: what is resident at once.
+int rrg_context::qr_blocks() {
+  if (!qr_bps) qr_bps = qr_chunk_blocks_per_sm();
+  return sm_count * qr_bps;
 }
 
 int64_t rrg_context::device_bytes() {

@@ -78,11 +78,11 @@ struct rrg_context {
   std::vector<rrg_cand> host_cands;
   // plain scratch
   DevBuf d_A, d_pc, d_partial, d_list;
-  // chunked-QR state and chunk totals (qr_chunk.cu); blocks per SM of its
-  // passes by column group (0: not asked yet)
+  // chunked-QR state, chunk totals and R (qr_chunk.cu); resident blocks per
+  // SM of its passes (0: not asked yet)
   DevBuf d_qrs;
-  int qr_bps[3] = {0, 0, 0};
-  int qr_blocks(int max_cols, int64_t items);
+  int qr_bps = 0;
+  int qr_blocks();
   HostBuf h_pc, h_list;
   // mixed scratch
   DevBuf d_terms, d_fallback, d_sse1, d_probe, d_nanrow, d_cert_e;
@@ -116,7 +116,7 @@ struct rrg_context {
   ColumnCache fcache, pcache;
   FactorRegistry freg;  // factor ids of the pair cache
   PairCache pairc;      // cross-pair sums kept across rounds (slots of d_psum)
-  DevBuf d_cself, d_cprobe, d_cfnan, d_ccst, d_slots;
+  DevBuf d_cself, d_cprobe, d_cfnan, d_ccst, d_cpart;
   int64_t fcache_npad = 0, pcache_npad = 0;  // the row padding the arenas' slots are sized for
   uint64_t next_uid = 0;
   int64_t last_cache_hits = 0, last_cache_evals = 0, last_cache64_hits = 0, last_cache64_evals = 0;

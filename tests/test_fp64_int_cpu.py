@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 HERE = Path(__file__).resolve().parent
-OPS = ["mul", "div", "sqrt", "lt", "eq", "sin", "cos", "log", "exp"]
+OPS = ["mul", "div", "sqrt", "lt", "eq", "sin", "cos", "log", "exp", "mul_by", "scaled", "scaled2"]
 SPECIAL = np.array([0.0, -0.0, 1.0, -1.0, 0.5, 2.0, np.inf, -np.inf, np.nan, 5e-324, -5e-324, 2.2250738585072014e-308,
                     2.225073858507201e-308, 1.7976931348623157e308, -1.7976931348623157e308, 3.0, 1.0 + 2.0**-52,
                     1.0 - 2.0**-53, 2.0 - 2.0**-52, 0.7853981633974483, np.nextafter(0.7853981633974483, 1), 1048576.0,
