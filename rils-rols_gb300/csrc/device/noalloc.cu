@@ -285,7 +285,8 @@ extern "C" rrg_status rrg_eval_plain_noalloc(const double* X_col, int64_t ld, co
   // QR launch is only visible through its return value
   if (!launch_plain_qr((int)k + 1, 1, st, db, dd, dpc, nullptr, 0, arena, arena, cf, result, status, nullptr))
     return cuda_fail("QR launch", cudaErrorLaunchFailure);
-  plain_resid_kernel<<<dim3(nb_res, 1), 256, 0, st>>>(db, dd, dpc, nullptr, 0, arena, cf, partial, nullptr);
+  if (!launch_plain_resid(db, dd, dpc, nullptr, 0, 1, arena, cf, partial, nullptr, nullptr, nb_res, st))
+    return cuda_fail("residual launch", cudaErrorLaunchFailure);
   finalize_kernel<<<1, 128, 0, st>>>(db, dd, nullptr, 0, 1, partial, nb_res, cf, result, 0u, nullptr);
   uint32_t dev_status = 0;
   if ((e = cudaGetLastError()) != cudaSuccess ||

@@ -12,6 +12,7 @@
 //   plain_resid  the rebuilt sum  sum_i c_i * f_i  with the drop / snap rules
 //                of rils_rols_cpp.cpp:488-517 and its squared residual;
 //   finalize     R2, RMSE and the NaN sentinel (rils_rols_cpp.cpp:40-49, 520-541).
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 
@@ -476,61 +477,146 @@ bool launch_plain_qr(int max_cols, int grid, cudaStream_t st, DevBatch b, DevDat
 
 
 
-// grid (ceil(n / RR_CHUNK), candidates): SSE of the rebuilt sum per chunk of
-// RR_CHUNK rows in the fixed order of csrc/common/rr_sum.h
-__global__ void __launch_bounds__(256) plain_resid_kernel(DevBatch b, DevData ds, const PlainCand* pc,
-                                                           const int32_t* list, int cand0, const double* A,
-                                                           const double* coefs, double* partial,
-                                                           const int32_t* colmap, const int32_t* dcount) {
-  if (dcount && cand0 + (int)blockIdx.y >= *dcount) return;
-  __shared__ double red[32];
-  __shared__ double cs[kMaxK];
+// SSE of the rebuilt sum per (candidate, chunk of RR_CHUNK rows) item in the
+// fixed order of csrc/common/rr_sum.h; the grid walks the items.
+//
+// Bound: the FP64 pipe.  The scaled terms' products and the squared residual
+// are formed on the integer pipes (csrc/common/fp64_int.h), so a row of m scaled
+// terms and a free term takes m + 2 FP64 additions (2 m + 4 FP64 instructions
+// before); kResidRows rows of a lane are handled together, term by term, so that
+// their loads are in flight at once.  GB300, 605 candidates at 1M rows: 10.3 ms
+// before, 6.4 now.
+// SEG = 4: blocks of 1024 threads, four to a lane, each forming a quarter of
+// the lane's squares before the lane's sum passes from one to the next: for
+// launches that leave most SMs without a block (one candidate at 1M rows has
+// 62 chunks: 0.125 ms before, 0.045 now).
+constexpr int kResidRows = 8;
+template <int SEG>
+__global__ void __launch_bounds__(256 * SEG) plain_resid_kernel(DevBatch b, DevData ds, const PlainCand* pc,
+                                                                const int32_t* list, int cand0, int n_cand,
+                                                                const double* A, const double* coefs, double* partial,
+                                                                const int32_t* colmap, const int32_t* dcount) {
+  __shared__ double red[8], lane_acc[256];
+  __shared__ fi_factor cs[kMaxK];
   __shared__ int kind[kMaxK];  // 0 skip, 1 free term, 2 bare factor, 3 scaled factor
   __shared__ const double* colp[kMaxK];
-  const int c = list ? list[cand0 + blockIdx.y] : cand0 + blockIdx.y;
-  const rrg_cand cd = b.cands[c];
-  const int nb = gridDim.x;
-  const bool tuned = cd.mode == RRG_TUNED;
-  if (tuned && (pc[c].pad & 1)) {
-    // all-NaN coefficients: every row's rebuilt sum is NaN
-    if (threadIdx.x == 0)
-      partial[(int64_t)c * nb + blockIdx.x] = blockIdx.x == 0 ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
-    return;
-  }
-  const int k = pc[c].k;
-  const int m = tuned ? k - 1 : 1;
-  if (tuned) {
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-      const double ci = coefs[cd.coef_offset + i];
-      cs[i] = ci;
-      kind[i] = fabs(ci) < kEps12 ? 0 : (i == m ? 1 : (fabs(ci - 1) < kEps12 ? 2 : 3));
+  constexpr int kSegRows = RR_CHUNK / 256 / SEG;  // rows of a lane per thread
+  static_assert(kSegRows % kResidRows == 0, "whole row groups");
+  const int lane = threadIdx.x & 255, seg = threadIdx.x >> 8;
+  const int nb = (int)((ds.n + RR_CHUNK - 1) / RR_CHUNK);
+  const int cnt = dcount ? min(max(*dcount - cand0, 0), n_cand) : n_cand;
+  const int64_t items = (int64_t)cnt * nb;
+  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const int i = (int)(it / nb), ch = (int)(it % nb);
+    const int c = list ? list[cand0 + i] : cand0 + i;
+    const rrg_cand cd = b.cands[c];
+    const bool tuned = cd.mode == RRG_TUNED;
+    if (tuned && (pc[c].pad & 1)) {
+      // all-NaN coefficients: every row's rebuilt sum is NaN
+      if (threadIdx.x == 0)
+        partial[(int64_t)c * nb + ch] = ch == 0 ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+      continue;
     }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < m; i += blockDim.x) colp[i] = factor_column(A, ds.n_pad, pc[c].a_col, i, colmap);
-  __syncthreads();
-  const int64_t r0 = (int64_t)blockIdx.x * RR_CHUNK, r1 = min(ds.n, r0 + (int64_t)RR_CHUNK);
-  double acc = 0.0;
-  for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-    double yp;
-    if (tuned) {
-      yp = 0.0;
+    const int k = tuned ? pc[c].k : 1;
+    const int m = tuned ? k - 1 : 1;
+    __syncthreads();  // the previous item's terms are no longer read
+    for (int t = threadIdx.x; t < k; t += blockDim.x) {
+      const double ci = tuned ? coefs[cd.coef_offset + t] : 1.0;
+      cs[t] = fi_factor_of(ci);
+      kind[t] = fabs(ci) < kEps12 ? 0 : (tuned && t == m ? 1 : (fabs(ci - 1) < kEps12 ? 2 : 3));
+      if (t < m) colp[t] = factor_column(A, ds.n_pad, pc[c].a_col, t, colmap);
+    }
+    __syncthreads();
+    const int64_t r0 = (int64_t)ch * RR_CHUNK;
+    const int64_t first = r0 + lane + (int64_t)seg * kSegRows * 256;
+    double acc = 0.0, sq[SEG == 1 ? kResidRows : kSegRows];
+#pragma unroll 1
+    for (int u0 = 0; u0 < kSegRows; u0 += kResidRows) {
+      const int64_t i0 = first + 256 * u0;
+      if (i0 >= ds.n) break;
+      const bool full = i0 + 256 * (kResidRows - 1) < ds.n;
+      double yp[kResidRows], e[kResidRows];
       bool have = false;
-      for (int i = 0; i < k; ++i) {
-        const int kd = kind[i];
+      for (int t = 0; t < k; ++t) {
+        const int kd = kind[t];
         if (kd == 0) continue;
-        const double term = kd == 1 ? __dmul_rn(cs[i], 1.0) : (kd == 2 ? colp[i][r] : __dmul_rn(cs[i], colp[i][r]));
-        yp = have ? __dadd_rn(yp, term) : term;
+        const fi_factor f = cs[t];
+        if (kd == 1) {
+#pragma unroll
+          for (int u = 0; u < kResidRows; ++u) yp[u] = have ? __dadd_rn(yp[u], f.b) : f.b;
+        } else {
+          const double* col = colp[t];
+          double v[kResidRows];
+#pragma unroll
+          for (int u = 0; u < kResidRows; ++u) v[u] = full || i0 + 256 * u < ds.n ? __ldg(col + i0 + 256 * u) : 0.0;
+#pragma unroll
+          for (int u = 0; u < kResidRows; ++u) {
+            const double term = kd == 2 ? v[u] : fi_mul_by(v[u], f);
+            yp[u] = have ? __dadd_rn(yp[u], term) : term;
+          }
+        }
         have = true;
       }
-    } else {
-      yp = colp[0][r];
+#pragma unroll
+      for (int u = 0; u < kResidRows; ++u) {
+        const double y = full || i0 + 256 * u < ds.n ? __ldg(ds.y64 + i0 + 256 * u) : 0.0;
+        e[u] = __dsub_rn(y, have ? yp[u] : 0.0);
+        e[u] = fi_mul(e[u], e[u]);
+      }
+      if constexpr (SEG == 1) {
+#pragma unroll
+        for (int u = 0; u < kResidRows; ++u)
+          if (full || i0 + 256 * u < ds.n) acc = __dadd_rn(acc, e[u]);
+      } else {
+        // (constant indexes keep the squares in registers)
+#pragma unroll
+        for (int g = 0; g < kSegRows; g += kResidRows)
+          if (g == u0) {
+#pragma unroll
+            for (int u = 0; u < kResidRows; ++u) sq[g + u] = e[u];
+          }
+      }
     }
-    const double e = __dsub_rn(ds.y64[r], yp);
-    acc = __dadd_rn(acc, __dmul_rn(e, e));
+    if constexpr (SEG > 1) {
+      // the lane's sum in row order: each quarter goes on from the one before
+      for (int s = 0; s < SEG; ++s) {
+        if (seg == s) {
+          acc = s ? lane_acc[lane] : 0.0;
+#pragma unroll
+          for (int u = 0; u < kSegRows; ++u)
+            if (first + 256 * u < ds.n) acc = __dadd_rn(acc, sq[u]);
+          lane_acc[lane] = acc;
+        }
+        __syncthreads();
+      }
+      acc = lane_acc[lane];
+    }
+    // the first 256 threads fold the lanes
+    const double ws = warp_sum(acc);
+    if (seg == 0 && (lane & 31) == 0) red[lane >> 5] = ws;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double s = 0.0;
+      for (int w = 0; w < 8; ++w) s = __dadd_rn(s, red[w]);
+      partial[(int64_t)c * nb + ch] = s;
+    }
   }
-  const double s = block_sum(acc, red);
-  if (threadIdx.x == 0) partial[(int64_t)c * nb + blockIdx.x] = s;
+}
+
+bool launch_plain_resid(DevBatch b, const DevData& ds, const PlainCand* pc, const int32_t* list, int cand0, int n_cand,
+                        const double* A, const double* coefs, double* partial, const int32_t* colmap,
+                        const int32_t* dcount, int sm_count, cudaStream_t st) {
+  if (n_cand <= 0) return true;
+  const int64_t items = (int64_t)n_cand * ((ds.n + RR_CHUNK - 1) / RR_CHUNK);
+  // four threads a lane while that gives every SM at most two such blocks and
+  // a lane has more rows than one thread takes together
+  if (!dcount && items <= 2 * sm_count && ds.n > 256 * kResidRows)
+    plain_resid_kernel<4><<<(int)items, 1024, 0, st>>>(b, ds, pc, list, cand0, n_cand, A, coefs, partial, colmap,
+                                                       dcount);
+  else
+    plain_resid_kernel<1><<<(int)std::min<int64_t>(items, 16 * (int64_t)sm_count), 256, 0, st>>>(
+        b, ds, pc, list, cand0, n_cand, A, coefs, partial, colmap, dcount);
+  return launch_ok("residual");
 }
 
 // one thread per candidate: R2, RMSE, sentinel, rebuilt size

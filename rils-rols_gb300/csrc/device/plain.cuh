@@ -22,11 +22,13 @@ int plain_qr_bucket(int cols);
 bool launch_plain_qr(int max_cols, int grid, cudaStream_t st, DevBatch b, DevData ds, const PlainCand* pc,
                      const int32_t* list, int cand0, const double* A, double* M, double* coefs, rrg_result* res,
                      uint32_t* status, const int32_t* colmap);
-// dcount (may be NULL): grid positions at or beyond *dcount do nothing (a
-// list whose length the device decided; the grid covers its capacity).
-__global__ void plain_resid_kernel(DevBatch b, DevData ds, const PlainCand* pc, const int32_t* list, int cand0,
-                                   const double* A, const double* coefs, double* partial, const int32_t* colmap,
-                                   const int32_t* dcount = nullptr);
+// Squared residual of the rebuilt sum of the candidates list[cand0 .. cand0 +
+// n_cand) per chunk of RR_CHUNK rows: partial[c * chunks + chunk].  dcount (may
+// be NULL): list positions at or beyond *dcount do nothing (a list whose length
+// the device decided).
+bool launch_plain_resid(DevBatch b, const DevData& ds, const PlainCand* pc, const int32_t* list, int cand0, int n_cand,
+                        const double* A, const double* coefs, double* partial, const int32_t* colmap,
+                        const int32_t* dcount, int sm_count, cudaStream_t st);
 // partial[c * nb + j]: per-candidate squared-residual partial sums; when
 // sse_direct is given and sse_direct[c] >= 0 (or NaN) it is the SSE itself.
 __global__ void finalize_kernel(DevBatch b, DevData ds, const int32_t* list, int cand0, int cand1,

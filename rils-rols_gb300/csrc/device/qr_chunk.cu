@@ -45,10 +45,10 @@
 // instructions a row (dots 10, updates 9, tails 3, its share of the column
 // sums) against 47 with the copy, a stored v and native quotients, and moves
 // about 32 columns against 51.  Measured on GB300 (QR phase, before / now): a
-// 660-candidate round at 1M rows, mostly three columns, 52.5 / 19.4 ms (13.3 ms
+// 660-candidate round at 1M rows, mostly three columns, 52.5 / 18.7 ms (13.3 ms
 // at 17 cycles for its 13 FP64 instructions a row); the re-scored candidates
-// of eight certified rounds at 1M rows 51.0 / 29.9 ms; 765 candidates at 20011
-// rows 4.02 / 2.50 ms; one candidate at 1M rows 0.59 / 0.29 ms.
+// of eight certified rounds at 1M rows 51.0 / 28.9 ms; 765 candidates at 20011
+// rows 4.02 / 2.47 ms; one candidate at 1M rows 0.59 / 0.29 ms.
 // Rows held per lane 8 (A) and 4 (B) at four resident blocks: 19.4 ms; 8 and 8
 // 19.8, 4 and 4 19.9, three resident blocks 21.6.
 #include <cfloat>
@@ -103,33 +103,33 @@ __device__ __forceinline__ double* r_at(const QrJob& j, int t, int kk, int s) {
   return j.rmat + ((int64_t)t * j.max_cols + kk) * j.max_cols + s;
 }
 
-// Totals of sum slots [0, cnt) in chunk order from 0 into out (shared); chunk
-// `sp` (if >= 0) contributes its variant instead.  The totals are staged in
-// buf (kStage shared doubles) by the whole block, so that the ordered sums do
-// not wait on one load after the other.
-__device__ __forceinline__ void chunk_totals(const QrJob& j, int t, int cnt, int sp, double* buf, double* out) {
+// Totals of sum slots [0, cnt) in chunk order from 0 into out (shared) and,
+// when sp >= 0, the totals with chunk sp's variant in its place into out_sp.
+// The totals are staged in buf (kStage shared doubles) by the whole block, and
+// a thread adds one of them up: an FP64 addition that waits for the one before
+// takes about 95 cycles, so the ordered sums run side by side.
+__device__ __forceinline__ void chunk_totals(const QrJob& j, int t, int cnt, int sp, double* buf, double* out,
+                                             double* out_sp) {
   const int nch = j.nch;
-  const int per = nch <= kStage ? kStage / nch : 0;  // slots staged at once
-  if (per == 0) {
-    for (int s = threadIdx.x; s < cnt; s += blockDim.x) {
-      double tot = 0.0;
-      for (int ch = 0; ch < nch; ++ch) tot = __dadd_rn(tot, __ldcg(part_at(j, t, ch == sp ? nch : ch, s)));
-      out[s] = tot;
+  const int per = nch + 1 <= kStage ? kStage / (nch + 1) : 0;  // slots staged at once
+  const int sums = sp >= 0 ? 2 : 1;
+  for (int s0 = 0; s0 < cnt; s0 += per > 0 ? per : cnt) {
+    const int ns = per > 0 && per < cnt - s0 ? per : cnt - s0;
+    if (per > 0) {
+      for (int i = threadIdx.x; i < ns * (nch + 1); i += blockDim.x) {
+        const int row = i % (nch + 1);
+        if (row < nch || sp >= 0) buf[i] = __ldcg(part_at(j, t, row, s0 + i / (nch + 1)));
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    return;
-  }
-  for (int s0 = 0; s0 < cnt; s0 += per) {
-    const int ns = cnt - s0 < per ? cnt - s0 : per;
-    for (int i = threadIdx.x; i < ns * nch; i += blockDim.x) {
-      const int s = i / nch, ch = i % nch;
-      buf[i] = __ldcg(part_at(j, t, ch == sp ? nch : ch, s0 + s));
-    }
-    __syncthreads();
-    for (int s = threadIdx.x; s < ns; s += blockDim.x) {
+    for (int x = threadIdx.x; x < ns * sums; x += blockDim.x) {
+      const int s = x / sums, skip = x % sums ? sp : -1;
       double tot = 0.0;
-      for (int ch = 0; ch < nch; ++ch) tot = __dadd_rn(tot, buf[s * nch + ch]);
-      out[s0 + s] = tot;
+      for (int ch = 0; ch < nch; ++ch) {
+        const int row = ch == skip ? nch : ch;
+        tot = __dadd_rn(tot, per > 0 ? buf[s * (nch + 1) + row] : __ldcg(part_at(j, t, row, s0 + s)));
+      }
+      (x % sums ? out_sp : out)[s0 + s] = tot;
     }
     __syncthreads();
   }
@@ -154,11 +154,11 @@ __device__ void select_pivot(QrState* S, int kk, double rows) {
   int big = kk;
   double bign = S->nupd[kk];
   for (int j = kk + 1; j < S->k; ++j)
-    if (S->nupd[j] > bign) {
+    if (fi_lt(bign, S->nupd[j])) {
       bign = S->nupd[j];
       big = j;
     }
-  if (__dmul_rn(bign, bign) < __dmul_rn(S->thr_helper, rows - kk)) {
+  if (fi_lt(fi_mul(bign, bign), fi_mul(S->thr_helper, rows - kk))) {
     S->size = kk;
     return;
   }
@@ -177,11 +177,11 @@ __device__ void householder_scalars(QrState* S, double c0, double tail_sq) {
     S->den = 1.0;
     S->tau_zero = 1;
   } else {
-    double beta = __dsqrt_rn(__dadd_rn(__dmul_rn(c0, c0), tail_sq));
+    double beta = fi_sqrt(__dadd_rn(fi_mul(c0, c0), tail_sq));
     if (c0 >= 0.0) beta = -beta;
     const double den = __dsub_rn(c0, beta);
     S->den = den;
-    S->tau = __ddiv_rn(__dsub_rn(beta, c0), beta);
+    S->tau = fi_div(-den, beta);
     S->beta = beta;
     S->tau_zero = 0;
   }
@@ -234,9 +234,27 @@ __device__ __forceinline__ void load_rows(const double* col, int64_t i0, int64_t
 }  // namespace
 
 // ------------------------------------------------------------- column sums --
+// A column's totals from its chunk totals pt[0 .. nch] (the last one chunk 0's
+// without row 0), by its last block.
+__device__ __forceinline__ void col_sums_finish(const double* pt, int nch, double* buf, ColStat* cs) {
+  for (int i = threadIdx.x; i <= nch && i < kStage; i += blockDim.x) buf[i] = __ldcg(pt + i);
+  __syncthreads();
+  if (threadIdx.x == 0 || threadIdx.x == 32) {
+    double tot = 0.0;
+    for (int i = 0; i < nch; ++i) {
+      const int x = threadIdx.x == 32 && i == 0 ? nch : i;
+      tot = __dadd_rn(tot, x < kStage ? buf[x] : __ldcg(pt + x));
+    }
+    if (threadIdx.x == 0) cs->sumsq = tot;
+    else cs->tailsq = tot;
+  }
+  if (threadIdx.x == 0) cs->ticket = 0;
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(256) col_sums_kernel(const double* T, int64_t n, int64_t n_pad, const int32_t* cols,
                                                        int n_cols, const int32_t* dcount, ColStat* cst, double* part) {
-  __shared__ double red[8], outA[1], outB[1], buf[2 * kStage];
+  __shared__ double red[8], outA[1], outB[1], buf[kStage];
   __shared__ int s_flag;
   const int cnt = dcount ? min(*dcount, n_cols) : n_cols;
   const int nch = (int)((n + kQC - 1) / kQC);
@@ -270,20 +288,7 @@ __global__ void __launch_bounds__(256) col_sums_kernel(const double* T, int64_t 
       pt[ch] = outA[0];
       if (ch == 0) pt[nch] = outB[0];
     }
-    if (!last_block(&cst[c].ticket, nch, &s_flag)) continue;
-    for (int i = threadIdx.x; i <= nch && i < 2 * kStage; i += blockDim.x) buf[i] = __ldcg(pt + i);
-    __syncthreads();
-    if (threadIdx.x == 0 || threadIdx.x == 32) {
-      double tot = 0.0;
-      for (int i = 0; i < nch; ++i) {
-        const int x = threadIdx.x == 32 && i == 0 ? nch : i;
-        tot = __dadd_rn(tot, x < 2 * kStage ? buf[x] : __ldcg(pt + x));
-      }
-      if (threadIdx.x == 0) cst[c].sumsq = tot;
-      else cst[c].tailsq = tot;
-    }
-    if (threadIdx.x == 0) cst[c].ticket = 0;
-    __syncthreads();
+    if (last_block(&cst[c].ticket, nch, &s_flag)) col_sums_finish(pt, nch, buf, cst + c);
   }
 }
 
@@ -354,14 +359,124 @@ __device__ __forceinline__ void copy_state(QrState* dst, const QrState* src) {
   __syncthreads();
 }
 
+// Shared memory of a candidate's last block.
+struct Finish {
+  QrState Ss;
+  double buf[kStage], tot[kQrMaxCols], tail[kQrMaxCols];
+  int8_t rec[kQrMaxCols];
+};
+
+// Pass A's scalar work, by a candidate's last block.
+__device__ void passA_finish(Finish& F, const QrJob& j, int t, int c, int kk, bool upd) {
+  // ---- last block: row kk (Householder.h:121-126), then down-dating
+  QrState* S = j.state + t;
+  copy_state(&F.Ss, S);
+  const int k = F.Ss.k, nw = k - kk, ps = F.Ss.pos2col[kk];
+  const int64_t rows = j.ds.n;
+  if (upd) chunk_totals(j, t, nw, -1, F.buf, F.tot, nullptr);
+  const int next = kk + 1;
+  for (int q = threadIdx.x; q < nw; q += blockDim.x) {
+    const int p = next + q, s = p < k ? F.Ss.pos2col[p] : k;
+    const double* col = kk == 0 ? design_col(j, c, k, s) : wcol(j, t, c, s);
+    const double qk = col ? __ldcg(col + kk) : 1.0;
+    double a = qk;
+    if (upd) {
+      const double tmp = __dadd_rn(F.tot[q], qk);
+      a = __dsub_rn(qk, fi_mul(F.Ss.tau, tmp));
+      F.Ss.ntmp[s] = -tmp;
+    } else if (rows - kk == 1) {
+      a = __dmul_rn(qk, __dsub_rn(1.0, F.Ss.tau));  // a one-row tail
+    }
+    *r_at(j, t, kk, s) = a;
+    // LAWN 176 norm down-dating (ColPivHouseholderQR.h:549-572); the
+    // recomputations happen in pass B, which sums the updated columns
+    int flag = 0;
+    if (p < k && F.Ss.nupd[p] != 0.0) {
+      const double nu = F.Ss.nupd[p];
+      double temp = fi_div(fabs(a), nu);
+      temp = fi_mul(__dadd_rn(1.0, temp), __dsub_rn(1.0, temp));
+      temp = temp < 0.0 ? 0.0 : temp;
+      const double ratio = fi_div(nu, F.Ss.ndir[p]);
+      const double temp2 = fi_mul(temp, fi_mul(ratio, ratio));
+      if (temp2 <= kDowndateThr) flag = 1;
+      else F.Ss.nupd[p] = fi_mul(nu, fi_sqrt(temp));
+    }
+    F.rec[q] = (int8_t)flag;
+    F.Ss.slot_of[s] = -1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *r_at(j, t, kk, ps) = F.Ss.beta;
+    int rec_any = 0, nsum = 0;
+    for (int q = 0; q < nw - 1; ++q) rec_any |= F.rec[q];
+    if (next < F.Ss.size) {
+      if (rec_any) {
+        // the pivot of step kk + 1 depends on the recomputed norms (and on
+        // NaN norms through the scan's running maximum): the sums of every
+        // remaining column, which a recomputation step can afford
+        for (int p = next; p < k; ++p) {
+          F.Ss.slot_of[F.Ss.pos2col[p]] = nsum;
+          F.Ss.sum_norm[nsum++] = F.rec[p - next];
+        }
+      } else {
+        select_pivot(&F.Ss, next, (double)rows);
+        if (next < F.Ss.size) {
+          F.Ss.slot_of[F.Ss.pos2col[next]] = 0;
+          F.Ss.sum_norm[0] = 0;
+          nsum = 1;
+        }
+      }
+    }
+    F.Ss.rec_any = rec_any;
+    F.Ss.nsum = nsum;
+    F.Ss.ticket = 0;
+  }
+  __syncthreads();
+  copy_state(S, &F.Ss);
+}
+
+// Pass B's.
+__device__ void passB_finish(Finish& F, const QrJob& j, int t, int c, int kk) {
+  // ---- the candidate's last block: totals, then step kk + 1's scalars
+  QrState* S = j.state + t;
+  copy_state(&F.Ss, S);
+  const int k = F.Ss.k, next = kk + 1;
+  const int64_t rows = j.ds.n;
+  const int nsum = F.Ss.nsum;
+  chunk_totals(j, t, nsum, next / kQC, F.buf, F.tot, F.tail);
+  if (threadIdx.x == 0) {
+    if (F.Ss.rec_any) {
+      // recomputed norms (ColPivHouseholderQR.h:566-569)
+      for (int p = next; p < k; ++p) {
+        const int q = F.Ss.slot_of[F.Ss.pos2col[p]];
+        if (q >= 0 && F.Ss.sum_norm[q]) {
+          F.Ss.ndir[p] = fi_sqrt(F.tot[q]);
+          F.Ss.nupd[p] = F.Ss.ndir[p];
+        }
+      }
+      select_pivot(&F.Ss, next, (double)rows);
+    }
+    if (next < F.Ss.size) {
+      const int np = F.Ss.pos2col[next], q = F.Ss.slot_of[np];
+      if (q < 0) {
+        atomicOr(j.status, ST_QR_STATE);
+        F.Ss.active = 0;
+      } else {
+        householder_scalars(&F.Ss, __ldcg(wcol(j, t, c, np) + next), rows - next == 1 ? 0.0 : F.tail[q]);
+      }
+    }
+    F.Ss.ticket = 0;
+  }
+  __syncthreads();
+  copy_state(S, &F.Ss);
+}
+
 // ------------------------------------------------------------------ A(kk) --
 __global__ void __launch_bounds__(256, kMinBlocks) qr_passA_kernel(QrJob j, int kk, int width) {
   __shared__ ItemView V;
   __shared__ double red[8 * CG], outA[CG];
   __shared__ int s_flag;
-  __shared__ double buf[kStage], tot[kQrMaxCols];
-  __shared__ QrState Ss;
-  __shared__ int8_t rec[kQrMaxCols];
+  __shared__ Finish F;
   const int cnt = job_count(j);
   const int64_t rows = j.ds.n;
   const int cpi = cols_per_item((int64_t)cnt * j.nch, width);
@@ -420,67 +535,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) qr_passA_kernel(QrJob j, int 
       if (threadIdx.x < gc) *part_at(j, t, ch, q0 + threadIdx.x) = outA[threadIdx.x];
     }
     if (!last_block(&S->ticket, j.nch * groups, &s_flag)) continue;
-    // ---- last block: row kk (Householder.h:121-126), then down-dating
-    copy_state(&Ss, S);
-    if (upd) chunk_totals(j, t, nw, -1, buf, tot);
-    const int next = kk + 1;
-    for (int q = threadIdx.x; q < nw; q += blockDim.x) {
-      const int p = next + q, s = p < k ? Ss.pos2col[p] : k;
-      const double* col = kk == 0 ? design_col(j, c, k, s) : wcol(j, t, c, s);
-      const double qk = col ? __ldcg(col + kk) : 1.0;
-      double a = qk;
-      if (upd) {
-        const double tmp = __dadd_rn(tot[q], qk);
-        a = __dsub_rn(qk, __dmul_rn(Ss.tau, tmp));
-        Ss.ntmp[s] = -tmp;
-      } else if (rows - kk == 1) {
-        a = __dmul_rn(qk, __dsub_rn(1.0, Ss.tau));  // a one-row tail
-      }
-      *r_at(j, t, kk, s) = a;
-      // LAWN 176 norm down-dating (ColPivHouseholderQR.h:549-572); the
-      // recomputations happen in pass B, which sums the updated columns
-      int flag = 0;
-      if (p < k && Ss.nupd[p] != 0.0) {
-        double temp = __ddiv_rn(fabs(a), Ss.nupd[p]);
-        temp = __dmul_rn(__dadd_rn(1.0, temp), __dsub_rn(1.0, temp));
-        temp = temp < 0.0 ? 0.0 : temp;
-        const double ratio = __ddiv_rn(Ss.nupd[p], Ss.ndir[p]);
-        const double temp2 = __dmul_rn(temp, __dmul_rn(ratio, ratio));
-        if (temp2 <= kDowndateThr) flag = 1;
-        else Ss.nupd[p] = __dmul_rn(Ss.nupd[p], __dsqrt_rn(temp));
-      }
-      rec[q] = (int8_t)flag;
-      Ss.slot_of[s] = -1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      *r_at(j, t, kk, ps) = Ss.beta;
-      int rec_any = 0, nsum = 0;
-      for (int q = 0; q < nw - 1; ++q) rec_any |= rec[q];
-      if (next < Ss.size) {
-        if (rec_any) {
-          // the pivot of step kk + 1 depends on the recomputed norms (and on
-          // NaN norms through the scan's running maximum): the sums of every
-          // remaining column, which a recomputation step can afford
-          for (int p = next; p < k; ++p) {
-            Ss.slot_of[Ss.pos2col[p]] = nsum;
-            Ss.sum_norm[nsum++] = rec[p - next];
-          }
-        } else {
-          select_pivot(&Ss, next, (double)rows);
-          if (next < Ss.size) {
-            Ss.slot_of[Ss.pos2col[next]] = 0;
-            Ss.sum_norm[0] = 0;
-            nsum = 1;
-          }
-        }
-      }
-      Ss.rec_any = rec_any;
-      Ss.nsum = nsum;
-      Ss.ticket = 0;
-    }
-    __syncthreads();
-    copy_state(S, &Ss);
+    passA_finish(F, j, t, c, kk, upd);
   }
 }
 
@@ -489,8 +544,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) qr_passB_kernel(QrJob j, int 
   __shared__ ItemView V;
   __shared__ double red[8], outA[1], outB[1];
   __shared__ int s_flag;
-  __shared__ double buf[kStage], s_norm[kQrMaxCols], s_tail[kQrMaxCols];
-  __shared__ QrState Ss;
+  __shared__ Finish F;
   const int cnt = job_count(j);
   const int64_t rows = j.ds.n;
   const int next = kk + 1;
@@ -595,36 +649,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) qr_passB_kernel(QrJob j, int 
       }
     }
     if (!last_block(&S->ticket, j.nch * groups, &s_flag)) continue;
-    // ---- the candidate's last block: totals, then step kk + 1's scalars
-    copy_state(&Ss, S);
-    const int nsum = Ss.nsum;
-    chunk_totals(j, t, nsum, -1, buf, s_norm);
-    chunk_totals(j, t, nsum, next / kQC, buf, s_tail);
-    if (threadIdx.x == 0) {
-      if (Ss.rec_any) {
-        // recomputed norms (ColPivHouseholderQR.h:566-569)
-        for (int p = next; p < k; ++p) {
-          const int q = Ss.slot_of[Ss.pos2col[p]];
-          if (q >= 0 && Ss.sum_norm[q]) {
-            Ss.ndir[p] = __dsqrt_rn(s_norm[q]);
-            Ss.nupd[p] = Ss.ndir[p];
-          }
-        }
-        select_pivot(&Ss, next, (double)rows);
-      }
-      if (next < Ss.size) {
-        const int np = Ss.pos2col[next], q = Ss.slot_of[np];
-        if (q < 0) {
-          atomicOr(j.status, ST_QR_STATE);
-          Ss.active = 0;
-        } else {
-          householder_scalars(&Ss, __ldcg(wcol(j, t, c, np) + next), rows - next == 1 ? 0.0 : s_tail[q]);
-        }
-      }
-      Ss.ticket = 0;
-    }
-    __syncthreads();
-    copy_state(S, &Ss);
+    passB_finish(F, j, t, c, kk);
   }
 }
 

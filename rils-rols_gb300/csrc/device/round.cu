@@ -1456,8 +1456,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       }
       mark_end(P_PLAIN_QR, t0);
       t0 = mark_begin();
-      plain_resid_kernel<<<dim3(nb_res, cnt), 256, 0, stream>>>(dev, dd, d_pcs, fb_list, 0, F64, coefs, sse, d_ccol,
-                                                               fb_count);
+      if (!launch_plain_resid(dev, dd, d_pcs, fb_list, 0, cnt, F64, coefs, sse, d_ccol, fb_count, sm_count, stream))
+        return RRG_E_CUDA;
       mark_end(P_PLAIN_RESID, t0);
       t0 = mark_begin();
       finalize_kernel<<<(cnt + 127) / 128, 128, 0, stream>>>(dev, dd, fb_list, 0, cnt, sse, nb_res, coefs, res,
@@ -1907,8 +1907,9 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       }
       mark_end(P_PLAIN_QR, t0);
       t0 = mark_begin();
-      plain_resid_kernel<<<dim3(nb_res, ns), 256, 0, stream>>>(dev, dd, d_pcs, d_list, sb.first, F64, coefs, partial,
-                                                               d_cmap);
+      if (!launch_plain_resid(dev, dd, d_pcs, d_list, sb.first, ns, F64, coefs, partial, d_cmap, nullptr, sm_count,
+                              stream))
+        return RRG_E_CUDA;
       mark_end(P_PLAIN_RESID, t0);
       t0 = mark_begin();
       finalize_kernel<<<(ns + 127) / 128, 128, 0, stream>>>(dev, dd, d_list, sb.first, sb.second, partial, nb_res,
