@@ -51,6 +51,7 @@ struct FacEvalArgs {
   const int2* meta;          // [f] (code offset, length)
   const int2* groups;        // [g] (first factor, count); a group's programs are contiguous
   const int32_t* wcol;       // [f] column of F (and of fnan) program f writes; NULL: column f
+  const uint8_t* stop;       // [f] 1: chunks after one with a NaN may be left out
   const float* K;            // constant pool, double-float high parts
   const float* Klo;          // low parts
   int32_t chunk;             // rows per chunk, a multiple of kFacStep
@@ -83,6 +84,8 @@ struct PairArgs {
   const int32_t* partner;    // [cross pair] factor b (pairs of a unit share a)
   float2* P;                 // [row block][n_pairs]
   int32_t n_pairs, cross0;   // pair index of cross pair 0
+  const unsigned long long* fnan;  // [column] first row with a NaN value (n or more: none)
+  int64_t n;
 };
 
 struct ResidArgs {

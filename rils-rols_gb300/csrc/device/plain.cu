@@ -120,18 +120,33 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
 
 // One-column table program on rows [r0, r1) of this block, written to Ac;
 // the column's flags (NaN, infinite or overflowing square, non-trivial tail)
-// merged into *cs.
+// merged into *cs.  stop: a column that no program reads as an operand; once
+// some block has stored a NaN at row kStopRow or later, the blocks leave off
+// (the block of row 0 after its first rows, so that rows below kStopRow are
+// all there).  2048 random trees at 100k rows, seven of eight with a NaN
+// somewhere: 78.5 ms without the stop, 23.8 with it.
 __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len, const double* consts,
                                                   const DevData& ds, int64_t r0, int64_t r1, double* st, double* Ac,
-                                                  const double* T, uint32_t* status, ColStat* cs) {
+                                                  const double* T, uint32_t* status, ColStat* cs, bool stop,
+                                                  volatile int* found) {
+  static_assert(kStopRow <= 256, "within the first rows of a block");
   uint32_t f = 0;
+  const bool skip = stop && (__ldcg(&cs->flags) & kCsStop) != 0;  // (any mix of answers in a block does)
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+    if (stop && r >= blockDim.x && (skip || (r - r0 >= blockDim.x && *found))) break;
     const double v = run_row64<true>(code, len, consts, ds, r, st, nullptr, T, status);
     Ac[r] = v;
     // on the bits of |v| (non-negative doubles order as integers, NaN above)
     const unsigned long long a = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-    if (a > 0x7ff0000000000000ull) f |= kCsNaN;
-    else if (a > 0x5ff01c2a01d98729ull) f |= kCsBig;  // above 1.35e154: infinite, or its square overflows
+    if (a > 0x7ff0000000000000ull) {
+      f |= kCsNaN;
+      if (stop && r >= kStopRow && !*found) {
+        *found = 1;
+        atomicOr(&cs->flags, kCsStop | kCsNaN | kCsTail);
+      }
+    } else if (a > 0x5ff01c2a01d98729ull) {
+      f |= kCsBig;  // above 1.35e154: infinite, or its square overflows
+    }
     if (r >= 1 && a > 0x20ca2fe76a3f9475ull) f |= kCsTail;  // above 1e-150, or not finite
   }
   f = __reduce_or_sync(0xffffffffu, f);
@@ -157,14 +172,16 @@ __global__ void __launch_bounds__(256) table_eval_list_kernel(DevBatch b, DevDat
     const int bi = (int)(w % nbc);
     const rrg_cand cd = b.cands[c];
     const int64_t r0 = ds.n * (int64_t)bi / nbc, r1 = ds.n * (int64_t)(bi + 1) / nbc;
-    const bool staged = cd.code_len <= kMaxCodeSmem;
+    const bool staged = cd.code_len < kMaxCodeSmem;
+    volatile int* found = reinterpret_cast<int*>(code_s + kMaxCodeSmem - 1);
     __syncthreads();  // the previous item's program is no longer read
+    if (threadIdx.x == 0) *found = 0;
     if (staged)
       for (int i = threadIdx.x; i < cd.code_len; i += blockDim.x) code_s[i] = b.code[cd.code_offset + i];
     __syncthreads();
     const uint32_t* code = staged ? code_s : b.code + cd.code_offset;
     eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, A + pc[c].a_col * ds.n_pad, A, status,
-                      &cst[pc[c].a_col]);
+                      &cst[pc[c].a_col], cd.reserved != 0, found);
   }
 }
 
@@ -179,14 +196,17 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
   const int64_t r0 = ds.n * (int64_t)blockIdx.x / nb, r1 = ds.n * (int64_t)(blockIdx.x + 1) / nb;
   double* st = smem + threadIdx.x;  // spill stack, RRG_MAX_STACK * blockDim.x doubles
   uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + RRG_MAX_STACK * blockDim.x);
-  const bool staged = cd.code_len <= kMaxCodeSmem;
+  const bool staged = cd.code_len < kMaxCodeSmem;
+  volatile int* found = reinterpret_cast<int*>(code_s + kMaxCodeSmem - 1);
+  if (threadIdx.x == 0) *found = 0;
   if (staged)
     for (int i = threadIdx.x; i < cd.code_len; i += blockDim.x) code_s[i] = b.code[cd.code_offset + i];
   __syncthreads();
   const uint32_t* code = staged ? code_s : b.code + cd.code_offset;
   double* Ac = A + pc[c].a_col * ds.n_pad;
   if (cst) {
-    eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, Ac, A, status, &cst[pc[c].a_col]);
+    eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, Ac, A, status, &cst[pc[c].a_col],
+                      cd.reserved != 0, found);
     return;
   }
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x)

@@ -4,7 +4,7 @@
 
 namespace rrd {
 
-constexpr int kMaxCodeSmem = 4096;  // program words staged in shared memory per block
+constexpr int kMaxCodeSmem = 4096;  // words of a block's program staging; the last one flags a NaN
 
 struct ColStat;
 // `list` (may be NULL) maps grid positions to candidates: candidate = list[cand0 + i].
@@ -49,6 +49,10 @@ struct ColStat {
 };
 constexpr uint32_t kCsNaN = 1;   // a NaN value: the column's norm is NaN
 constexpr uint32_t kCsBig = 2;   // an infinite value or one whose square overflows
+constexpr uint32_t kCsStop = 8;  // a NaN at row kStopRow or later: the remaining rows may be left out
+// From this row on a NaN decides what a factor column can do in any refit:
+// its rows up to the deepest pivot row are then all evaluated.
+constexpr int64_t kStopRow = 128;
 constexpr uint32_t kCsTail = 4;  // a row after the first with |value| > 1e-150 or non-finite
 // One thread per listed tuned candidate: where the QR's result is certain to
 // be all-NaN coefficients at full rank (the fitness sentinel), writes that

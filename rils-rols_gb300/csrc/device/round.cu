@@ -381,8 +381,9 @@ struct CachePlan {
   TableProgs ep;
   std::vector<int32_t> ewcol;
   std::vector<int32_t> ecol;     // [evaluated program] its table column
+  std::vector<uint8_t> stop;     // [evaluated program] may stop at a NaN (operand_free)
   std::vector<int32_t> fslot;    // [local factor] slot
-  std::vector<int32_t> mprog;    // local factors evaluated (not found)
+  std::vector<int32_t> mprog;    // local factors evaluated
   std::vector<int32_t> scratch;  // slots of shared columns (this sub-round only)
   int64_t hits = 0;
   int64_t arena = 0;             // slots the arena must hold
@@ -392,6 +393,25 @@ struct CachePlan {
 bool table_ref(uint32_t w) {
   const int op = (int)(w & 0xffu);
   return op == kOpLDT || op == kOpPST || (op >= RRG_OP_BIN && (((op - RRG_OP_BIN) & 7) >> 1) == kSrcT);
+}
+
+// Columns of `tp` that some program of it (of those in `run`, when given)
+// reads as an operand.  The others are read as factors only, and a factor
+// column with a NaN beyond the first rows has one possible use: it makes its
+// candidate's sums, and so its refit, NaN (or is never read, after a rank
+// cut).  Which NaN rows, and what the finite ones hold, changes no result, so
+// the evaluator leaves off such a column's remaining rows.  An operand's rows
+// all count: a comparison, a minimum or a power turns NaN into a number.
+std::vector<uint8_t> operand_columns(const TableProgs& tp, const std::vector<uint8_t>* run = nullptr) {
+  std::vector<uint8_t> op(tp.meta.size(), 0);
+  for (size_t c = 0; c < tp.meta.size(); ++c) {
+    if (run && !(*run)[c]) continue;
+    for (int pc = 0; pc < tp.meta[c].y; ++pc) {
+      const uint32_t w = tp.code[tp.meta[c].x + pc];
+      if (table_ref(w)) op[w >> 8] = 1;
+    }
+  }
+  return op;
 }
 
 // Starts a sub-round of `cc`.  When the shared columns do not fit next to
@@ -412,6 +432,8 @@ bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode
     out.ecol.resize(nc);
     for (int32_t c = 0; c < nc; ++c) out.ewcol[c] = out.ecol[c] = c;
     out.fslot = tp.fcol;
+    out.stop = operand_columns(tp);
+    for (uint8_t& v : out.stop) v = v ? 0 : 1;  // (a shared column is an operand)
     for (int32_t l = 0; l < nfl; ++l) out.mprog.push_back(l);
     out.arena = nc;
     return true;
@@ -444,11 +466,13 @@ bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode
       if (!need[c]) continue;
       for (int pc = 0; pc < tp.meta[c].y; ++pc) {
         const uint32_t w = tp.code[tp.meta[c].x + pc];
-        if (table_ref(w) && slot_of[w >> 8] < 0) need[w >> 8] = 1;
+        // an operand not kept, or kept without all its rows (then evaluated
+        // again, into the same slot)
+        if (table_ref(w) && (slot_of[w >> 8] < 0 || !cc.whole(slot_of[w >> 8]))) need[w >> 8] = 1;
       }
     }
     n_new = 0;
-    for (int32_t c = 0; c < nc; ++c) n_new += need[c] ? 1 : 0;
+    for (int32_t c = 0; c < nc; ++c) n_new += need[c] && slot_of[c] < 0 ? 1 : 0;
     return n_new <= cc.available();
   };
   if (!plan()) {
@@ -459,15 +483,18 @@ bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode
   const int32_t nc = (int32_t)tp.meta.size();
   size_t t = 0;
   for (int32_t c = 0; c < nc; ++c)
-    if (need[c]) {
+    if (need[c] && slot_of[c] < 0) {
       slot_of[c] = taken[t++];
       if (!is_fac[c]) out.scratch.push_back(slot_of[c]);
     }
+  const std::vector<uint8_t> operand = operand_columns(tp, &need);
   out.fslot.resize(nfl);
   for (int32_t l = 0; l < nfl; ++l) {
-    out.fslot[l] = slot_of[tp.fcol[l]];
-    if (fhit[l] < 0) {
-      cc.insert(prog(l), hash[l], out.fslot[l]);
+    const int32_t c = tp.fcol[l];
+    out.fslot[l] = slot_of[c];
+    if (fhit[l] < 0) cc.insert(prog(l), hash[l], out.fslot[l]);
+    if (need[c]) {
+      cc.set_whole(out.fslot[l], operand[c] != 0);
       out.mprog.push_back(l);
     }
   }
@@ -485,6 +512,7 @@ bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode
       ep.stack.push_back(tp.stack[c]);
       out.ewcol.push_back(slot_of[c]);
       out.ecol.push_back(c);
+      out.stop.push_back(operand[c] ? 0 : 1);
     }
     ep.level_end.push_back((int32_t)ep.meta.size());
   }
@@ -812,6 +840,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   const size_t o_ecode = pkt.add(ep.code.data(), sizeof(uint32_t) * std::max<size_t>(1, ep.code.size()));
   const size_t o_emeta = pkt.add(ep.meta.data(), sizeof(int2) * std::max<size_t>(1, ep.meta.size()));
   const size_t o_ewcol = pkt.add(ewcol.data(), sizeof(int32_t) * std::max<size_t>(1, ewcol.size()));
+  const size_t o_estop = pkt.add(cp.stop.data(), std::max<size_t>(1, cp.stop.size()));
   for (GroupSet& gs : gsets) {
     gs.off = pkt.add(gs.groups.data(), sizeof(int2) * gs.groups.size());
     gs.off_foff = pkt.add(gs.feat_off.data(), sizeof(int32_t) * gs.feat_off.size());
@@ -837,6 +866,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   fa.code = pkt.at<const uint32_t>(d_ftp, o_ecode);
   fa.meta = pkt.at<const int2>(d_ftp, o_emeta);
   fa.wcol = d_ewcol;
+  fa.stop = pkt.at<const uint8_t>(d_ftp, o_estop);
   fa.K = dev.consts32;
   fa.Klo = dev.consts32lo;
   fa.chunk = chunk;
@@ -1082,6 +1112,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   pa.n_pad = ds->n_pad;
   pa.partner = pk.at<const int32_t>(d_ft, o_partner);
   pa.P = Pcross;
+  pa.fnan = fnan;
+  pa.n = ds->n;
   pa.n_pairs = n_miss;
   pa.cross0 = 0;
   auto pair_all = [&](int v) {
@@ -1198,6 +1230,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       // the next round starts (which ones, the device decides: the lane's
       // marks are read back with the round's results)
       std::vector<int32_t> kept(std::max(1, ncol), -1);
+      const std::vector<uint8_t> operand = operand_columns(tp);
       const bool keep64 = cache_on && ds->n >= kCacheMinRows;
       int64_t n_kept = 0;
       if (keep64) {
@@ -1211,7 +1244,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         for (int32_t l = 0; l < nfl; ++l) {
           const FactorProg fp{lcode.data() + lmeta[l].x, lmeta[l].y, consts64};
           const int32_t sl = pcache.find(fp, fp.hash());
-          if (sl >= 0) {
+          if (sl >= 0 && (pcache.whole(sl) || !operand[tp.fcol[l]])) {
             kept[tp.fcol[l]] = sl;
             ++n_kept;
           }
@@ -1234,7 +1267,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         p.mode = RRG_UNTUNED;
         p.coef_offset = 0;
         p.stack_need = tp.stack[i];
-        p.reserved = 0;
+        p.reserved = operand[i] ? 0 : 1;  // may stop at a NaN
         fpc[i] = PlainCand{i, 0, 0, 1, 0};
         std::vector<int32_t>& cl = closure[i];
         for (int pc = 0; pc < tp.meta[i].y; ++pc) {
@@ -1488,6 +1521,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         ls.code.clear();
         ls.meta.clear();
         ls.col.clear();
+        ls.whole.clear();
         const double* pool = consts64;
         ls.consts.assign(pool, pool + std::max(0, dev.n_consts));
         for (int32_t l = 0; l < nfl; ++l) {
@@ -1495,6 +1529,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
           ls.meta.push_back(make_int2((int)ls.code.size(), lmeta[l].y));
           ls.code.insert(ls.code.end(), lcode.begin() + lmeta[l].x, lcode.begin() + lmeta[l].x + lmeta[l].y);
           ls.col.push_back(tp.fcol[l]);
+          ls.whole.push_back(operand[tp.fcol[l]]);
         }
       }
       fbstat_pending = true;
@@ -1672,7 +1707,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       p.mode = RRG_UNTUNED;
       p.coef_offset = 0;
       p.stack_need = ep.stack[i];
-      p.reserved = 0;
+      p.reserved = cp.stop[i];
       if (ep.stack[i] > RRG_MAX_STACK) {
         rrc::set_error("FP64 round: a table program exceeds the spill stack");
         return RRG_E_INVALID;
@@ -1952,7 +1987,8 @@ rrg_status rrg_context::store_lane_columns() {
   std::vector<int32_t> pairs(2 * (size_t)k);
   for (int64_t i = 0; i < k; ++i) {
     const int32_t f = fsel[i];
-    pcache.insert(FactorProg{ls.code.data() + ls.meta[f].x, ls.meta[f].y, ls.consts.data()}, hsel[i], slots[i]);
+    pcache.insert(FactorProg{ls.code.data() + ls.meta[f].x, ls.meta[f].y, ls.consts.data()}, hsel[i], slots[i],
+                  ls.whole[f] != 0);
     pairs[2 * i] = ls.col[f];
     pairs[2 * i + 1] = slots[i];
   }

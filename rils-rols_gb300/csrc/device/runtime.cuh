@@ -132,6 +132,7 @@ struct rrg_context {
     std::vector<int2> meta;
     std::vector<double> consts;
     std::vector<int32_t> col;  // the lane table column of each program
+    std::vector<uint8_t> whole;  // every row of it evaluated
   } lane_store;
   HostBuf h_fbneed, h_store;
   DevBuf d_store;

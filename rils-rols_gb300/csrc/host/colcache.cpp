@@ -145,12 +145,13 @@ bool ColumnCache::take(int64_t count, std::vector<int32_t>& out) {
   return true;
 }
 
-void ColumnCache::insert(const FactorProg& p, uint64_t h, int32_t s) {
+void ColumnCache::insert(const FactorProg& p, uint64_t h, int32_t s, bool whole) {
   Slot& sl = slot_[s];
   sl.key.clear();
   for (int i = 0; i < p.len; ++i) key_words(p.code[i], p.consts, [&](uint64_t v) { sl.key.push_back(v); });
   sl.hash = h;
   sl.held = true;
+  sl.whole = whole;
   sl.last = stamp_;
   auto it = head_.find(h);
   sl.next = it == head_.end() ? -1 : it->second;

@@ -117,7 +117,12 @@ class ColumnCache {
   // with nothing taken, when fewer are available.
   bool take(int64_t count, std::vector<int32_t>& out);
   // slot `s` (from take) now holds the column of `p` (hash h)
-  void insert(const FactorProg& p, uint64_t h, int32_t s);
+  void insert(const FactorProg& p, uint64_t h, int32_t s, bool whole = true);
+  // whether every row of the column in slot `s` was evaluated: a factor's
+  // evaluation may stop once a NaN has decided what the factor can do, and
+  // such a column serves as that factor only, not as an operand
+  bool whole(int32_t s) const { return slot_[s].whole; }
+  void set_whole(int32_t s, bool w) { slot_[s].whole = w; }
   // slots from take that hold no entry (scratch columns) back to the free list
   void give_back(const std::vector<int32_t>& s);
 
@@ -127,6 +132,7 @@ class ColumnCache {
     uint64_t hash = 0;
     int32_t next = -1;   // next slot with the same hash
     bool held = false;   // holds an entry
+    bool whole = true;   // every row evaluated
     int64_t last = -1;   // sub-round stamp of its last use
   };
   bool matches(const Slot& s, const FactorProg& p) const;
