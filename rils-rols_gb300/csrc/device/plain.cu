@@ -512,7 +512,7 @@ bool launch_plain_qr(int max_cols, int grid, cudaStream_t st, DevBatch b, DevDat
 // 62 chunks: 0.125 ms before, 0.045 now).
 constexpr int kResidRows = 8;
 template <int SEG>
-__global__ void __launch_bounds__(256 * SEG) plain_resid_kernel(DevBatch b, DevData ds, const PlainCand* pc,
+__global__ void __launch_bounds__(256 * SEG, 4 / SEG) plain_resid_kernel(DevBatch b, DevData ds, const PlainCand* pc,
                                                                 const int32_t* list, int cand0, int n_cand,
                                                                 const double* A, const double* coefs, double* partial,
                                                                 const int32_t* colmap, const int32_t* dcount) {
@@ -555,6 +555,24 @@ __global__ void __launch_bounds__(256 * SEG) plain_resid_kernel(DevBatch b, DevD
       const int64_t i0 = first + 256 * u0;
       if (i0 >= ds.n) break;
       const bool full = i0 + 256 * (kResidRows - 1) < ds.n;
+      if (SEG == 1 && !full) {
+        // the last rows one at a time (small datasets have few to a lane)
+        for (int64_t r = i0; r < ds.n; r += 256) {
+          double yp = 0.0;
+          bool have = false;
+          for (int t = 0; t < k; ++t) {
+            const int kd = kind[t];
+            if (kd == 0) continue;
+            const double v = kd == 1 ? 1.0 : __ldg(colp[t] + r);
+            const double term = kd == 1 ? cs[t].b : (kd == 2 ? v : fi_mul_by(v, cs[t]));
+            yp = have ? __dadd_rn(yp, term) : term;
+            have = true;
+          }
+          const double e = __dsub_rn(__ldg(ds.y64 + r), yp);
+          acc = __dadd_rn(acc, fi_mul(e, e));
+        }
+        break;
+      }
       double yp[kResidRows], e[kResidRows];
       bool have = false;
       for (int t = 0; t < k; ++t) {
@@ -568,7 +586,8 @@ __global__ void __launch_bounds__(256 * SEG) plain_resid_kernel(DevBatch b, DevD
           const double* col = colp[t];
           double v[kResidRows];
 #pragma unroll
-          for (int u = 0; u < kResidRows; ++u) v[u] = full || i0 + 256 * u < ds.n ? __ldg(col + i0 + 256 * u) : 0.0;
+          for (int u = 0; u < kResidRows; ++u)
+            v[u] = SEG == 1 || full || i0 + 256 * u < ds.n ? __ldg(col + i0 + 256 * u) : 0.0;
 #pragma unroll
           for (int u = 0; u < kResidRows; ++u) {
             const double term = kd == 2 ? v[u] : fi_mul_by(v[u], f);
@@ -579,14 +598,13 @@ __global__ void __launch_bounds__(256 * SEG) plain_resid_kernel(DevBatch b, DevD
       }
 #pragma unroll
       for (int u = 0; u < kResidRows; ++u) {
-        const double y = full || i0 + 256 * u < ds.n ? __ldg(ds.y64 + i0 + 256 * u) : 0.0;
+        const double y = SEG == 1 || full || i0 + 256 * u < ds.n ? __ldg(ds.y64 + i0 + 256 * u) : 0.0;
         e[u] = __dsub_rn(y, have ? yp[u] : 0.0);
         e[u] = fi_mul(e[u], e[u]);
       }
       if constexpr (SEG == 1) {
 #pragma unroll
-        for (int u = 0; u < kResidRows; ++u)
-          if (full || i0 + 256 * u < ds.n) acc = __dadd_rn(acc, e[u]);
+        for (int u = 0; u < kResidRows; ++u) acc = __dadd_rn(acc, e[u]);
       } else {
         // (constant indexes keep the squares in registers)
 #pragma unroll
