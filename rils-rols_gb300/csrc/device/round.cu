@@ -17,6 +17,7 @@
 
 #include "../common/error.h"
 #include "../common/rr_sum.h"
+#include "../host/parallel.h"
 #include "common.cuh"
 #include "ftable.cuh"
 #include "mixed.cuh"
@@ -117,52 +118,6 @@ struct PNode {
   int32_t a, b; // children
 };
 
-bool parse_program(const uint32_t* code, int len, std::vector<PNode>& nd, int32_t& root) {
-  std::vector<int32_t> st;
-  auto leaf = [&](int8_t kind, uint32_t arg) {
-    nd.push_back(PNode{kind, 0, (int32_t)arg, -1, -1});
-    return (int32_t)nd.size() - 1;
-  };
-  for (int pc = 0; pc < len; ++pc) {
-    const uint32_t w = code[pc];
-    const int op = (int)(w & 0xffu);
-    const uint32_t arg = w >> 8;
-    if (op == RRG_OP_LDV || op == RRG_OP_PSV) {
-      st.push_back(leaf(0, arg));
-    } else if (op == RRG_OP_LDC || op == RRG_OP_PSC) {
-      st.push_back(leaf(1, arg));
-    } else if (op >= RRG_OP_SIN && op <= RRG_OP_SQR) {
-      if (st.empty()) return false;
-      const int32_t x = st.back();
-      nd.push_back(PNode{3, (int8_t)op, 0, x, -1});
-      st.back() = (int32_t)nd.size() - 1;
-    } else if (op == RRG_OP_EMIT) {
-      if (st.size() != 1) return false;
-      root = st.back();
-      return true;
-    } else if (op >= RRG_OP_BIN) {
-      const int kk = op - RRG_OP_BIN;
-      const int base = kk >> 3, src = (kk & 7) >> 1, dir = kk & 1;
-      if (st.empty()) return false;
-      const int32_t tos = st.back();
-      st.pop_back();
-      int32_t other;
-      if (src == RRG_SRC_S) {
-        if (st.empty()) return false;
-        other = st.back();
-        st.pop_back();
-      } else {
-        other = leaf(src == RRG_SRC_V ? 0 : 1, arg);
-      }
-      nd.push_back(PNode{4, (int8_t)base, 0, dir == RRG_DIR_N ? other : tos, dir == RRG_DIR_N ? tos : other});
-      st.push_back((int32_t)nd.size() - 1);
-    } else {
-      return false;
-    }
-  }
-  return false;
-}
-
 bool shared_root(const PNode& n) {
   return (n.kind == 3 && (n.op == RRG_OP_SIN || n.op == RRG_OP_COS || n.op == RRG_OP_LN || n.op == RRG_OP_EXP)) ||
          (n.kind == 4 && n.op == RRG_POW);
@@ -181,29 +136,18 @@ struct TableProgs {
 struct Encoder {
   const std::vector<PNode>& nd;
   const std::vector<int32_t>& col_of;  // [node] table column, -1 when computed inline
+  const std::vector<int32_t>& deep;    // [node] spill depth when computed (not read as a leaf)
   int32_t root = -1;
-  std::vector<int32_t> memo;
   std::vector<uint32_t>* out = nullptr;
   int sp = 0, maxsp = 0;
-  Encoder(const std::vector<PNode>& n, const std::vector<int32_t>& c) : nd(n), col_of(c), memo(n.size(), -1) {}
   bool leaf(int32_t m) const { return nd[m].kind <= 1 || (m != root && col_of[m] >= 0); }
-  int need(int32_t m) {
-    if (leaf(m)) return 0;
-    if (m != root && memo[m] >= 0) return memo[m];
-    const PNode& n = nd[m];
-    int v;
-    if (n.kind == 3) {
-      v = need(n.a);
-    } else if (leaf(n.b)) {
-      v = need(n.a);
-    } else if (leaf(n.a)) {
-      v = need(n.b);
-    } else {
-      const int na = need(n.a), nb = need(n.b);
-      v = na >= nb ? std::max(na, nb + 1) : std::max(nb, na + 1);
-    }
-    if (m != root) memo[m] = v;
-    return v;
+  int need(int32_t m) const { return leaf(m) ? 0 : deep[m]; }
+  // deep of a node whose children's are known
+  int depth_of(const PNode& p) const {
+    if (p.kind <= 1) return 0;
+    if (p.kind == 3 || leaf(p.b)) return need(p.a);
+    const int na = need(p.a), nb = need(p.b);
+    return leaf(p.a) ? nb : (na >= nb ? std::max(na, nb + 1) : std::max(nb, na + 1));
   }
   void src_of(int32_t m, int& src, uint32_t& arg) const {
     if (nd[m].kind == 0) { src = RRG_SRC_V; arg = (uint32_t)nd[m].arg; }
@@ -259,79 +203,171 @@ struct Encoder {
   }
 };
 
+}  // namespace
+
+// Host arrays of build_table_programs, kept by the context: a round of 8192
+// random trees fills 20 MB of them, and fresh pages cost as much as the work.
+struct TableScratch {
+  std::vector<PNode> nd;         // nodes, children before parents; program l's from 2 * lmeta[l].x on
+  std::vector<uint64_t> hash;    // [node] of its subtree
+  std::vector<int32_t> cls;      // [node] class of a transcendental subtree, else -1
+  std::vector<uint64_t> slot;    // open addressing table: the hash's upper half and the class + 1
+  std::vector<int32_t> roots;    // the transcendental subtrees, in program order
+  std::vector<int32_t> lvl, col_of, deep;
+  void grow(size_t nodes) {
+    if (nd.size() >= nodes) return;
+    nd.resize(nodes);
+    hash.resize(nodes);
+    cls.resize(nodes);
+    lvl.resize(nodes);
+    col_of.resize(nodes);
+    deep.resize(nodes);
+  }
+};
+void TableScratchDelete::operator()(TableScratch* p) const { delete p; }
+
+namespace {
+
+// programs per host-thread slice: waking the pool costs what these take
+constexpr size_t kProgSlice = 512;
+
 // Table programs of the local factors (programs in lcode / lmeta).  A
 // transcendental subtree becomes a column of its own only when it occurs at
 // least twice (a column costs a write and a read per use); share = false
-// keeps every factor a single program.
-bool build_table_programs(const std::vector<uint32_t>& lcode, const std::vector<int2>& lmeta, const double* consts,
-                          TableProgs& tp, bool share = true) {
+// keeps every factor a single program.  The programs are parsed, and the
+// columns encoded, in slices on the host threads; which subtrees are equal is
+// decided in program order, so the columns and their order do not depend on
+// the slices.  8192 random trees (17000 columns): 31.7 ms with a hash map of
+// every node's class, 4.6 now.
+bool build_table_programs(TableScratch& ts, const std::vector<uint32_t>& lcode, const std::vector<int2>& lmeta,
+                          const double* consts, TableProgs& tp, bool share = true) {
   const int32_t nfl = (int32_t)lmeta.size();
-  std::vector<PNode> nd;
-  nd.reserve(lcode.size() + 16);
-  std::vector<int32_t> froot(nfl);
-  for (int32_t l = 0; l < nfl; ++l)
-    if (!parse_program(lcode.data() + lmeta[l].x, lmeta[l].y, nd, froot[l])) return false;
-  // structural class of every node, bottom-up (children precede parents):
-  // equal classes are equal subtrees (features by index, constants by bits)
-  struct ClassKey {
-    uint64_t arg;
-    int32_t a, b;
-    int8_t kind, op;
-    bool operator==(const ClassKey& o) const {
-      return arg == o.arg && a == o.a && b == o.b && kind == o.kind && op == o.op;
-    }
+  ts.grow(2 * lcode.size());  // (an instruction makes at most two nodes)
+  std::vector<PNode>& nd = ts.nd;
+  std::vector<uint64_t>& hash = ts.hash;
+  std::vector<int32_t>&cls = ts.cls, &lvl = ts.lvl, &col_of = ts.col_of, &deep = ts.deep, &roots = ts.roots;
+  std::vector<uint64_t>& slot = ts.slot;
+  std::vector<int32_t> froot(nfl, -1), n_nodes(nfl, 0);
+  auto bits = [&](const PNode& n) {
+    uint64_t v = (uint64_t)(uint32_t)n.arg;
+    if (n.kind == 1) std::memcpy(&v, consts + n.arg, sizeof v);
+    return v;
   };
-  struct ClassHash {
-    size_t operator()(const ClassKey& k) const {
-      uint64_t h = k.arg * 0x9e3779b97f4a7c15ull;
-      h ^= ((uint64_t)(uint32_t)k.a << 32 | (uint32_t)k.b) + 0x7f4a7c159e3779b9ull + (h << 6) + (h >> 2);
-      h ^= ((uint64_t)(uint8_t)k.kind << 8 | (uint8_t)k.op) + (h << 6) + (h >> 2);
-      return (size_t)(h ^ (h >> 29));
-    }
-  };
-  std::unordered_map<ClassKey, int32_t, ClassHash> classes;
-  classes.reserve(nd.size() + 16);
-  std::vector<int32_t> cls(nd.size());
-  for (size_t i = 0; i < nd.size(); ++i) {
-    const PNode& n = nd[i];
-    ClassKey k{0, -1, -1, n.kind, 0};
-    if (n.kind == 0) {
-      k.arg = (uint64_t)n.arg;
-    } else if (n.kind == 1) {
-      std::memcpy(&k.arg, consts + n.arg, sizeof k.arg);
-    } else {
-      k.op = n.op;
-      k.a = cls[n.a];
-      if (n.kind == 4) k.b = cls[n.b];
-    }
-    cls[i] = classes.emplace(k, (int32_t)classes.size()).first->second;
-  }
-  // occurrences of every transcendental subtree
-  std::vector<int32_t> uses(classes.size(), 0);
-  if (share)
-    for (size_t i = 0; i < nd.size(); ++i)
-      if (shared_root(nd[i])) ++uses[cls[i]];
-  // shared subtrees and their levels (1 + the deepest shared subtree inside)
-  std::vector<int32_t> aux_index(classes.size(), -1);
-  std::vector<int32_t> aux_node, aux_level, aux_of(nd.size(), -1), lvl(nd.size(), 0);
-  for (size_t i = 0; i < nd.size(); ++i) {
-    const PNode& n = nd[i];
-    int inner = 0;
-    if (n.kind >= 3) inner = std::max(inner, lvl[n.a]);
-    if (n.kind == 4) inner = std::max(inner, lvl[n.b]);
-    lvl[i] = inner;
-    if (share && shared_root(n) && uses[cls[i]] >= 2) {
-      int32_t id = aux_index[cls[i]];
-      if (id < 0) {
-        id = (int32_t)aux_node.size();
-        aux_index[cls[i]] = id;
-        aux_node.push_back((int32_t)i);
-        aux_level.push_back(inner + 1);
+  rrh::parallel_slices((size_t)nfl, kProgSlice, [&](size_t l0, size_t l1) {
+    std::vector<int32_t> st;
+    for (size_t l = l0; l < l1; ++l) {
+      const uint32_t* code = lcode.data() + lmeta[l].x;
+      const int32_t base = 2 * lmeta[l].x;
+      int32_t cnt = 0;
+      auto node = [&](int8_t kind, int8_t op, int32_t arg, int32_t x, int32_t y) {
+        const int32_t id = base + cnt++;
+        nd[id] = PNode{kind, op, arg, x, y};
+        uint64_t h = kind <= 1 ? bits(nd[id]) : hash[x] + (kind == 4 ? (hash[y] << 23 | hash[y] >> 41) : 0);
+        h = (h ^ ((uint64_t)(uint8_t)kind << 8 | (uint8_t)op)) * 0x9e3779b97f4a7c15ull;
+        h = (h ^ h >> 32) * 0xd6e8feb86659fd93ull;
+        hash[id] = h ^ h >> 29;
+        return id;
+      };
+      st.clear();
+      bool ok = true;
+      for (int pc = 0; pc < lmeta[l].y && ok; ++pc) {
+        const int op = (int)(code[pc] & 0xffu);
+        const int32_t arg = (int32_t)(code[pc] >> 8);
+        if (op == RRG_OP_LDV || op == RRG_OP_PSV) {
+          st.push_back(node(0, 0, arg, -1, -1));
+        } else if (op == RRG_OP_LDC || op == RRG_OP_PSC) {
+          st.push_back(node(1, 0, arg, -1, -1));
+        } else if (op >= RRG_OP_SIN && op <= RRG_OP_SQR) {
+          ok = !st.empty();
+          if (ok) st.back() = node(3, (int8_t)op, 0, st.back(), -1);
+        } else if (op == RRG_OP_EMIT) {
+          if (st.size() == 1) froot[l] = st.back();
+          break;
+        } else if (op >= RRG_OP_BIN) {
+          const int kk = op - RRG_OP_BIN;
+          const int op2 = kk >> 3, src = (kk & 7) >> 1, dir = kk & 1;
+          ok = st.size() >= (src == RRG_SRC_S ? 2u : 1u);
+          if (!ok) break;
+          const int32_t tos = st.back();
+          st.pop_back();
+          int32_t other;
+          if (src == RRG_SRC_S) {
+            other = st.back();
+            st.pop_back();
+          } else {
+            other = node(src == RRG_SRC_V ? 0 : 1, 0, arg, -1, -1);
+          }
+          st.push_back(node(4, (int8_t)op2, 0, dir == RRG_DIR_N ? other : tos, dir == RRG_DIR_N ? tos : other));
+        } else {
+          ok = false;
+        }
       }
-      aux_of[i] = id;
-      lvl[i] = aux_level[id];
+      n_nodes[l] = cnt;
+    }
+  });
+  for (int32_t l = 0; l < nfl; ++l)
+    if (froot[l] < 0) return false;
+  // classes of the transcendental subtrees (equal subtrees: features by
+  // index, constants by bits) with their uses: found by hash, confirmed node
+  // by node
+  std::vector<int32_t> rep, uses;  // [class] its first node, its occurrences
+  auto equal = [&](auto& self, int32_t x, int32_t y) -> bool {
+    const PNode &p = nd[x], &q = nd[y];
+    if (hash[x] != hash[y] || p.kind != q.kind || p.op != q.op) return false;
+    if (p.kind <= 1) return bits(p) == bits(q);
+    return self(self, p.a, q.a) && (p.kind == 3 || self(self, p.b, q.b));
+  };
+  if (share) {
+    size_t cap = 64;
+    while (cap < 2 * lcode.size()) cap <<= 1;
+    slot.assign(cap, 0);
+    roots.clear();
+    for (int32_t l = 0; l < nfl; ++l)
+      for (int32_t i = 2 * lmeta[l].x, e = i + n_nodes[l]; i < e; ++i) {
+        cls[i] = -1;
+        if (shared_root(nd[i])) roots.push_back(i);
+      }
+    const size_t nr = roots.size(), ahead = 16;
+    for (size_t r = 0; r < nr; ++r) {
+      if (r + ahead < nr) __builtin_prefetch(&slot[(size_t)hash[roots[r + ahead]] & (cap - 1)]);
+      const int32_t i = roots[r];
+      const uint64_t tag = hash[i] >> 32 << 32;
+      size_t q = (size_t)hash[i] & (cap - 1);
+      uint64_t v;
+      while ((v = slot[q]) != 0 && !(v >> 32 << 32 == tag && equal(equal, rep[(uint32_t)v - 1], i))) q = (q + 1) & (cap - 1);
+      if (v == 0) {
+        rep.push_back(i);
+        uses.push_back(0);
+        v = slot[q] = tag | (uint32_t)rep.size();
+      }
+      ++uses[(uint32_t)v - 1];
+      cls[i] = (int32_t)(uint32_t)v - 1;
     }
   }
+  // shared subtrees and their levels (1 + the deepest shared subtree inside);
+  // col_of holds the shared subtree's number until its column is known
+  std::vector<int32_t> aux_index(rep.size(), -1), aux_node, aux_level;
+  for (int32_t l = 0; l < nfl; ++l)
+    for (int32_t i = 2 * lmeta[l].x, e = i + n_nodes[l]; i < e; ++i) {
+      col_of[i] = -1;
+      if (!share) continue;
+      const PNode& n = nd[i];
+      int inner = 0;
+      if (n.kind >= 3) inner = lvl[n.a];
+      if (n.kind == 4) inner = std::max(inner, lvl[n.b]);
+      lvl[i] = inner;
+      if (cls[i] >= 0 && uses[cls[i]] >= 2) {
+        int32_t id = aux_index[cls[i]];
+        if (id < 0) {
+          id = (int32_t)aux_node.size();
+          aux_index[cls[i]] = id;
+          aux_node.push_back(i);
+          aux_level.push_back(inner + 1);
+        }
+        col_of[i] = id;
+        lvl[i] = aux_level[id];
+      }
+    }
   // column order: shared subtrees by level, then the factors not aliased to one
   const int n_aux = (int)aux_node.size();
   const int max_level = n_aux ? *std::max_element(aux_level.begin(), aux_level.end()) : 0;
@@ -349,25 +385,43 @@ bool build_table_programs(const std::vector<uint32_t>& lcode, const std::vector<
   tp.fcol.assign(nfl, -1);
   for (int32_t l = 0; l < nfl; ++l) {
     const int32_t r = froot[l];
-    if (aux_of[r] >= 0) {
-      tp.fcol[l] = aux_col[aux_of[r]];
+    if (col_of[r] >= 0) {
+      tp.fcol[l] = aux_col[col_of[r]];
     } else {
       tp.fcol[l] = (int32_t)col_nodes.size();
       col_nodes.push_back(r);
     }
   }
   tp.level_end.push_back((int32_t)col_nodes.size());
-  std::vector<int32_t> col_of(nd.size(), -1);
-  for (size_t i = 0; i < nd.size(); ++i)
-    if (aux_of[i] >= 0) col_of[i] = aux_col[aux_of[i]];
-  Encoder enc(nd, col_of);
+  // spill depths, then every column's code (a slice's into its own vector)
+  const size_t nc = col_nodes.size();
+  rrh::parallel_slices((size_t)nfl, kProgSlice, [&](size_t l0, size_t l1) {
+    const Encoder enc{nd, col_of, deep};
+    for (size_t l = l0; l < l1; ++l)
+      for (int32_t i = 2 * lmeta[l].x, e = i + n_nodes[l]; i < e; ++i) {
+        if (col_of[i] >= 0) col_of[i] = aux_col[col_of[i]];
+        deep[i] = enc.depth_of(nd[i]);
+      }
+  });
+  tp.meta.assign(nc, make_int2(0, 0));
+  tp.stack.assign(nc, 0);
+  std::vector<std::vector<uint32_t>> part(nc / kProgSlice + 1);
+  rrh::parallel_slices(part.size(), 1, [&](size_t s0, size_t s1) {
+    Encoder enc{nd, col_of, deep};
+    for (size_t s = s0; s < s1; ++s)
+      for (size_t c = s * kProgSlice; c < std::min(nc, (s + 1) * kProgSlice); ++c) {
+        const int off = (int)part[s].size();
+        tp.stack[c] = enc.encode(col_nodes[c], part[s]);
+        tp.meta[c] = make_int2(off, (int)part[s].size() - off);
+      }
+  });
   tp.code.clear();
-  tp.meta.assign(col_nodes.size(), make_int2(0, 0));
-  tp.stack.assign(col_nodes.size(), 0);
-  for (size_t c = 0; c < col_nodes.size(); ++c) {
+  for (size_t s = 0; s < part.size(); ++s) {
     const int off = (int)tp.code.size();
-    tp.stack[c] = enc.encode(col_nodes[c], tp.code);
-    tp.meta[c] = make_int2(off, (int)tp.code.size() - off);
+    if (s)
+      for (size_t c = s * kProgSlice; c < std::min(nc, (s + 1) * kProgSlice); ++c) tp.meta[c].x += off;
+    if (part.size() == 1) tp.code.swap(part[0]);
+    else tp.code.insert(tp.code.end(), part[s].begin(), part[s].end());
   }
   return true;
 }
@@ -420,7 +474,7 @@ std::vector<uint8_t> operand_columns(const TableProgs& tp, const std::vector<uin
 // keep = false bypasses the cache (small datasets, where evaluating a
 // column costs less than looking it up): every column is evaluated into
 // slot = its table column, and whatever the cache held is forgotten.
-bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode, const std::vector<int2>& lmeta,
+bool plan_columns(TableScratch& ts, ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode, const std::vector<int2>& lmeta,
                   const double* consts, TableProgs& tp, CachePlan& out) {
   const int32_t nfl = (int32_t)lmeta.size();
   out = CachePlan();
@@ -443,8 +497,10 @@ bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode
   std::vector<uint64_t> hash(nfl);
   std::vector<int32_t> fhit(nfl, -1);
   auto prog = [&](int32_t l) { return FactorProg{lcode.data() + lmeta[l].x, lmeta[l].y, consts}; };
+  rrh::parallel_slices((size_t)nfl, kProgSlice, [&](size_t l0, size_t l1) {
+    for (size_t l = l0; l < l1; ++l) hash[l] = prog((int32_t)l).hash();
+  });
   for (int32_t l = 0; l < nfl; ++l) {
-    hash[l] = prog(l).hash();
     fhit[l] = cc.find(prog(l), hash[l]);
     out.hits += fhit[l] >= 0 ? 1 : 0;
   }
@@ -476,7 +532,7 @@ bool plan_columns(ColumnCache& cc, bool keep, const std::vector<uint32_t>& lcode
     return n_new <= cc.available();
   };
   if (!plan()) {
-    if (!build_table_programs(lcode, lmeta, consts, tp, false) || !plan()) return false;
+    if (!build_table_programs(ts, lcode, lmeta, consts, tp, false) || !plan()) return false;
   }
   std::vector<int32_t> taken;
   if (!cc.take(n_new, taken)) return false;
@@ -548,51 +604,64 @@ void build_factor_table(const rrg_cand* cands, int32_t n_cand, const uint32_t* c
     }
     return true;
   };
-  std::unordered_map<uint64_t, int32_t> index;  // hash -> latest factor with it
-  std::vector<int32_t> next_same;               // earlier factors with the same hash
-  index.reserve((size_t)n_cand * 2 + 16);
+  // every factor's hash, length and spill depth, on the host threads
+  struct Rec {
+    uint64_t h;
+    int32_t start, len, depth;
+  };
+  std::vector<int32_t> roff((size_t)n_cand + 1, 0);
+  for (int32_t c = 0; c < n_cand; ++c) roff[c + 1] = roff[c] + cands[c].n_factors;
+  std::vector<Rec> rec(roff[n_cand]);
+  rrh::parallel_slices((size_t)n_cand, 256, [&](size_t c0, size_t c1) {
+    for (size_t c = c0; c < c1; ++c) {
+      const rrg_cand& cd = cands[c];
+      int32_t start = cd.code_offset;
+      Rec* r = rec.data() + roff[c];
+      int sp = 0, depth = 0;
+      uint64_t h = 0x9e3779b97f4a7c15ull;
+      for (int32_t pc = start; pc < cd.code_offset + cd.code_len; ++pc) {
+        const uint32_t w = code[pc];
+        const int op = (int)(w & 0xffu);
+        if (op == RRG_OP_EMIT) {
+          *r++ = Rec{h, start, pc - start, depth};
+          start = pc + 1;
+          sp = depth = 0;
+          h = 0x9e3779b97f4a7c15ull;
+          continue;
+        }
+        const uint64_t v = const_arg(op) ? (const_bits(w) ^ ((uint64_t)op << 56)) : (uint64_t)w;
+        h = (h ^ v) * 0x100000001b3ull;
+        h ^= h >> 29;
+        if (op == RRG_OP_PSV || op == RRG_OP_PSC) depth = std::max(depth, ++sp);
+        else if (op >= RRG_OP_BIN && (((op - RRG_OP_BIN) & 7) >> 1) == RRG_SRC_S) --sp;
+      }
+    }
+  });
+  // the distinct ones, in order of their first use: open addressing by hash
+  size_t cap = 64;
+  while (cap < 2 * rec.size()) cap <<= 1;
+  std::vector<int32_t> slot(cap, -1);
+  std::vector<uint64_t> fhash;
   for (int32_t c = 0; c < n_cand; ++c) {
     ft.cand_off[c] = (int32_t)ft.ids.size();
-    const rrg_cand& cd = cands[c];
-    int32_t start = cd.code_offset;
-    const int32_t end = cd.code_offset + cd.code_len;
-    int sp = 0, depth = 0;
-    uint64_t h = 0x9e3779b97f4a7c15ull;
-    for (int32_t pc = start; pc < end; ++pc) {
-      const uint32_t w = code[pc];
-      const int op = (int)(w & 0xffu);
-      if (op == RRG_OP_EMIT) {
-        const int len = pc - start;
-        auto it = index.find(h);
-        int32_t id = it == index.end() ? -1 : it->second;
-        while (id >= 0 && !(ft.meta[id].y == len + 1 && same(ft.code.data() + ft.meta[id].x, code + start, len)))
-          id = next_same[id];
-        if (id < 0) {
-          id = (int32_t)ft.meta.size();
-          next_same.push_back(it == index.end() ? -1 : it->second);
-          index[h] = id;
-          int2 mt;
-          mt.x = (int)ft.code.size();
-          mt.y = len + 1;
-          ft.code.insert(ft.code.end(), code + start, code + pc);
-          ft.code.push_back(RRG_INSN(RRG_OP_EMIT, 0));
-          ft.meta.push_back(mt);
-          ft.stack.push_back(depth);
-          ft.occ.push_back(0);
-        }
-        ft.occ[id] += 1;
-        ft.ids.push_back(id);
-        start = pc + 1;
-        sp = 0;
-        depth = 0;
-        h = 0x9e3779b97f4a7c15ull;
-        continue;
+    for (int32_t i = roff[c]; i < roff[c + 1]; ++i) {
+      const Rec& r = rec[i];
+      size_t q = (size_t)(r.h * 0x9e3779b97f4a7c15ull >> 20) & (cap - 1);
+      int32_t id;
+      while ((id = slot[q]) >= 0 && !(fhash[id] == r.h && ft.meta[id].y == r.len + 1 &&
+                                      same(ft.code.data() + ft.meta[id].x, code + r.start, r.len)))
+        q = (q + 1) & (cap - 1);
+      if (id < 0) {
+        id = slot[q] = (int32_t)ft.meta.size();
+        fhash.push_back(r.h);
+        ft.meta.push_back(make_int2((int)ft.code.size(), r.len + 1));
+        ft.code.insert(ft.code.end(), code + r.start, code + r.start + r.len);
+        ft.code.push_back(RRG_INSN(RRG_OP_EMIT, 0));
+        ft.stack.push_back(r.depth);
+        ft.occ.push_back(0);
       }
-      const uint64_t v = const_arg(op) ? (const_bits(w) ^ ((uint64_t)op << 56)) : (uint64_t)w;
-      h = (h ^ v) * 0x100000001b3ull;
-      h ^= h >> 29;
-      if (op == RRG_OP_PSV || op == RRG_OP_PSC) depth = std::max(depth, ++sp);
-      else if (op >= RRG_OP_BIN && (((op - RRG_OP_BIN) & 7) >> 1) == RRG_SRC_S) --sp;
+      ft.occ[id] += 1;
+      ft.ids.push_back(id);
     }
   }
   ft.cand_off[n_cand] = (int32_t)ft.ids.size();
@@ -691,15 +760,16 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   }
   // table columns: shared transcendental subtrees (by level), then factors
   TableProgs tp;
+  if (!tscratch) tscratch.reset(new TableScratch());
   const char* hb = static_cast<const char*>(h_batch.ptr);
   const double* consts64 = reinterpret_cast<const double*>(hb + off_d);
-  if (!build_table_programs(lcode, lmeta, consts64, tp)) {
+  if (!build_table_programs(*tscratch, lcode, lmeta, consts64, tp)) {
     rrc::set_error("mixed round: a factor program could not be parsed");
     return RRG_E_INVALID;
   }
   // shared columns on top of the factors must fit the table budget
   if ((double)tp.meta.size() * sizeof(float2) * (double)ds->n_pad > (double)table_budget_bytes)
-    build_table_programs(lcode, lmeta, consts64, tp, false);
+    build_table_programs(*tscratch, lcode, lmeta, consts64, tp, false);
   // Column cache: the factor columns an earlier round on this dataset left
   // in the arena are read again; the others, and the shared columns their
   // programs read, are evaluated into free or least recently used slots (the
@@ -715,7 +785,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   }
   fcache.bind(ds->uid);
   CachePlan cp;
-  if (!plan_columns(fcache, cache_on && ds->n >= kCacheMinRows, lcode, lmeta, consts64, tp, cp)) {
+  if (!plan_columns(*tscratch, fcache, cache_on && ds->n >= kCacheMinRows, lcode, lmeta, consts64, tp, cp)) {
     rrc::set_error("mixed round: the column cache has no room for the sub-round");
     return RRG_E_OOM;
   }
@@ -1668,8 +1738,9 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       lcode.insert(lcode.end(), ft.code.begin() + mt.x, ft.code.begin() + mt.x + mt.y);
     }
     TableProgs tp;
+    if (!tscratch) tscratch.reset(new TableScratch());
     const double* consts64 = reinterpret_cast<const double*>(hb + off_d);
-    if (!build_table_programs(lcode, lmeta, consts64, tp)) {
+    if (!build_table_programs(*tscratch, lcode, lmeta, consts64, tp)) {
       rrc::set_error("FP64 round: a factor program could not be parsed");
       return RRG_E_INVALID;
     }
@@ -1682,7 +1753,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     }
     pcache.bind(ds->uid);
     CachePlan cp;
-    if (!plan_columns(pcache, cache_on && ds->n >= kCacheMinRows, lcode, lmeta, consts64, tp, cp)) {
+    if (!plan_columns(*tscratch, pcache, cache_on && ds->n >= kCacheMinRows, lcode, lmeta, consts64, tp, cp)) {
       rrc::set_error("FP64 round: the column cache has no room for the table");
       return RRG_E_OOM;
     }

@@ -19,6 +19,7 @@
 #include "../common/error.h"
 #include "../common/df32.h"
 #include "../common/rr_sum.h"
+#include "../host/parallel.h"
 #include "common.cuh"
 #include "ftable.cuh"
 #include "mixed.cuh"
@@ -164,11 +165,29 @@ void rrg_context::mark_end(int phase, cudaEvent_t begin) {
 // Every instruction is checked on the host so that kernels never index out of
 // bounds: opcodes, feature and constant indices, factor slots, and the spill
 // depth of every program.
+static rrg_status validate_cands(const rrg_batch* b, int32_t d, int32_t c0, int32_t c1, int64_t* n_coefs_out);
 static rrg_status validate(const rrg_batch* b, int32_t d, int64_t* n_coefs_out) {
   if (!b || b->n_cand < 0 || b->n_factors < 0 || b->n_code < 0 || b->n_consts < 0) return RRG_E_INVALID;
   if (b->n_cand > 0 && (!b->cands || !b->factors || !b->code)) return RRG_E_INVALID;
+  // slices of candidates on the host threads; the first malformed candidate's
+  // status, as a sequential check gives it
+  const size_t per = 256, ns = ((size_t)b->n_cand + per - 1) / per;
+  std::vector<rrg_status> st(ns, RRG_OK);
+  std::vector<int64_t> nco(ns, 0);
+  rrh::parallel_slices(ns, 4, [&](size_t s0, size_t s1) {
+    for (size_t s = s0; s < s1; ++s)
+      st[s] = validate_cands(b, d, (int32_t)(s * per), (int32_t)std::min<size_t>(b->n_cand, (s + 1) * per), &nco[s]);
+  });
+  *n_coefs_out = 0;
+  for (size_t s = 0; s < ns; ++s) {
+    if (st[s] != RRG_OK) return st[s];
+    *n_coefs_out = std::max(*n_coefs_out, nco[s]);
+  }
+  return RRG_OK;
+}
+static rrg_status validate_cands(const rrg_batch* b, int32_t d, int32_t c0, int32_t c1, int64_t* n_coefs_out) {
   int64_t n_coefs = 0;
-  for (int32_t c = 0; c < b->n_cand; ++c) {
+  for (int32_t c = c0; c < c1; ++c) {
     const rrg_cand& cd = b->cands[c];
     if (cd.code_offset < 0 || cd.code_len < 0 || (int64_t)cd.code_offset + cd.code_len > b->n_code) return RRG_E_INVALID;
     if (cd.code_len == 0 && !(cd.mode == RRG_TUNED && cd.n_factors == 0)) return RRG_E_INVALID;

@@ -1,6 +1,7 @@
 // Context and dataset objects behind the C ABI (runtime.cu).
 #pragma once
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "../host/colcache.h"
@@ -58,6 +59,12 @@ struct FactorTable {
 void build_factor_table(const rrg_cand* cands, int32_t n_cand, const uint32_t* code, const double* consts,
                         FactorTable& ft);
 
+// Host scratch of a round's table programs (round.cu).
+struct TableScratch;
+struct TableScratchDelete {
+  void operator()(TableScratch* p) const;
+};
+
 struct rrg_context {
   int device = 0;
   int sm_count = 0;
@@ -105,6 +112,7 @@ struct rrg_context {
   cudaGraphExec_t graph_exec = nullptr;
   // factor tables
   FactorTable ft;
+  std::unique_ptr<TableScratch, TableScratchDelete> tscratch;
   HostBuf h_ft, h_ftp, h_ft64;
   DevBuf d_ft, d_ftp, d_ft64, d_F, d_P, d_Pc, d_psum, d_F64, d_M, d_gram;
   // factor columns kept across rounds of one dataset (colcache.h): the

@@ -82,8 +82,13 @@ class SlicePool {
 
 template <class F>
 void parallel_slices(size_t n, size_t min_per_slice, F&& fn) {
+  const size_t most = n / std::max<size_t>(1, min_per_slice);
+  if (most <= 1) {  // one slice: the pool is not even started
+    fn(size_t(0), n);
+    return;
+  }
   SlicePool& pool = SlicePool::get();
-  const size_t t = std::min<size_t>(pool.workers() + 1, n / std::max<size_t>(1, min_per_slice));
+  const size_t t = std::min<size_t>(pool.workers() + 1, most);
   if (t <= 1) {
     fn(size_t(0), n);
     return;
