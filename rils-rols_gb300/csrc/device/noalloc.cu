@@ -283,7 +283,7 @@ extern "C" rrg_status rrg_eval_plain_noalloc(const double* X_col, int64_t ld, co
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail("factor evaluation launch", e);
   // launch_plain_qr reads (and so clears) the launch error itself: a failed
   // QR launch is only visible through its return value
-  if (!launch_plain_qr((int)k + 1, 1, st, db, dd, dpc, nullptr, 0, arena, arena, cf, result, status, nullptr))
+  if (!launch_plain_qr((int)k + 1, 1, 1, st, db, dd, dpc, nullptr, 0, arena, arena, cf, result, status, nullptr))
     return cuda_fail("QR launch", cudaErrorLaunchFailure);
   if (!launch_plain_resid(db, dd, dpc, nullptr, 0, 1, arena, cf, partial, nullptr, nullptr, nb_res, st))
     return cuda_fail("residual launch", cudaErrorLaunchFailure);

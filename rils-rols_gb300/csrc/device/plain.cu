@@ -3,12 +3,8 @@
 //
 //   plain_eval   evaluates every factor program of a candidate on every row
 //                (node::evaluate_all, node.cpp:5-95) into the A arena;
-//   plain_qr     column-pivoted Householder least squares with the pivot,
-//                rank and norm-down-dating rules of Eigen's
-//                ColPivHouseholderQR (eigen/Eigen/src/QR/ColPivHouseholderQR.h:482-608)
-//                on [A | 1 | y], one block per candidate (small row counts
-//                and the allocation-free entry; qr_chunk.cu spreads larger
-//                ones over the GPU with the same bits);
+//   (the column-pivoted QR on [A | 1 | y] is in qr_small.cu, one block per
+//                candidate, and in qr_chunk.cu, over the GPU)
 //   plain_resid  the rebuilt sum  sum_i c_i * f_i  with the drop / snap rules
 //                of rils_rols_cpp.cpp:488-517 and its squared residual;
 //   finalize     R2, RMSE and the NaN sentinel (rils_rols_cpp.cpp:40-49, 520-541).
@@ -213,289 +209,7 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
     run_row64<false>(code, cd.code_len, b.consts, ds, r, st, Ac, A, status);
 }
 
-namespace {
-
-// QSUM (csrc/common/rr_sum.h) of term(i, acc) over rows [start, rows) by the
-// block's 256 threads, thread t being lane t: per chunk of RR_CHUNK rows the
-// lanes' chains are folded as RR256, and the chunk totals are added in order
-// from 0.  Every thread gets the total.
-template <class F>
-__device__ __forceinline__ double block_qsum(int64_t start, int64_t rows, double* red, F&& term) {
-  double total = 0.0;
-  for (int64_t c0 = start / RR_CHUNK * RR_CHUNK; c0 < rows; c0 += RR_CHUNK) {
-    const int64_t hi = c0 + RR_CHUNK < rows ? c0 + RR_CHUNK : rows;
-    double p = 0.0;
-    for (int64_t i = c0 + threadIdx.x; i < hi; i += blockDim.x)
-      if (i >= start) p = term(i, p);
-    total = __dadd_rn(total, block_sum(p, red));
-  }
-  return total;
-}
-
-// The same for cnt columns at once: term(i, part) adds row i's terms to
-// part[0 .. cnt); the totals land in tot[0 .. cnt) (shared).
-template <int KB, class F>
-__device__ __forceinline__ void block_qsum_vec(int64_t start, int64_t rows, int cnt, double* red, double* tmp,
-                                               double* tot, F&& term) {
-  for (int j = threadIdx.x; j < cnt; j += blockDim.x) tot[j] = 0.0;
-  __syncthreads();
-  for (int64_t c0 = start / RR_CHUNK * RR_CHUNK; c0 < rows; c0 += RR_CHUNK) {
-    const int64_t hi = c0 + RR_CHUNK < rows ? c0 + RR_CHUNK : rows;
-    double part[KB];
-#pragma unroll
-    for (int j = 0; j < KB; ++j) part[j] = 0.0;
-    for (int64_t i = c0 + threadIdx.x; i < hi; i += blockDim.x)
-      if (i >= start) term(i, part);
-    // element-wise block fold (warps, then the eight warp totals in order)
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int j = 0; j < KB; ++j)
-      if (j < cnt) {
-        const double v = warp_sum(part[j]);
-        if (l == 0) red[w * KB + j] = v;
-      }
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      double s = 0.0;
-      for (int i = 0; i < nw; ++i) s = __dadd_rn(s, red[i * KB + j]);
-      tot[j] = __dadd_rn(tot[j], s);
-    }
-    __syncthreads();
-  }
-  (void)tmp;
-}
-
-// Householder reflector of col[kk..rows) (Householder.h:67-96 semantics).
-// Returns tau; writes beta to col[kk] and the essential part below it.
-__device__ double make_householder_col(double* col, int64_t rows, int kk, double* red) {
-  const double tail_sq =
-      (rows - kk == 1) ? 0.0 : block_qsum(kk + 1, rows, red, [&](int64_t i, double p) { return __fma_rn(col[i], col[i], p); });
-  const double c0 = col[kk];
-  double tau, beta;
-  __syncthreads();
-  if (tail_sq <= DBL_MIN) {
-    tau = 0.0;
-    beta = c0;
-    for (int64_t i = kk + 1 + threadIdx.x; i < rows; i += blockDim.x) col[i] = 0.0;
-  } else {
-    beta = __dsqrt_rn(__dadd_rn(__dmul_rn(c0, c0), tail_sq));
-    if (c0 >= 0.0) beta = -beta;
-    const double den = __dsub_rn(c0, beta);
-    const fi_divisor rden = fi_divisor_of(den);
-    for (int64_t i = kk + 1 + threadIdx.x; i < rows; i += blockDim.x) col[i] = fi_div_by(col[i], &rden);
-    tau = __ddiv_rn(__dsub_rn(beta, c0), beta);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) col[kk] = beta;
-  __syncthreads();
-  return tau;
-}
-
-// Applies H_kk = I - tau v v^T (v = [1, colp[kk][kk+1..]]) to the columns
-// colp[c_lo..c_hi) (rows kk..rows-1).  Householder.h:116-133 semantics.
-template <int KB>
-__device__ void apply_householder_cols(double* const* colp, int64_t rows, int kk, double tau, int c_lo, int c_hi,
-                                       double* red, double* sh_tmp) {
-  const int cnt = c_hi - c_lo;
-  if (cnt <= 0) return;
-  if (rows - kk == 1) {
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      double* q = colp[c_lo + j] + kk;
-      *q = __dmul_rn(*q, __dsub_rn(1.0, tau));
-    }
-    __syncthreads();
-    return;
-  }
-  if (tau == 0.0) return;
-  const double* v = colp[kk];
-  double* cp[KB];
-#pragma unroll
-  for (int j = 0; j < KB; ++j) cp[j] = j < cnt ? colp[c_lo + j] : nullptr;
-  block_qsum_vec<KB>(kk + 1, rows, cnt, red, nullptr, sh_tmp, [&](int64_t i, double (&part)[KB]) {
-    const double vi = v[i];
-#pragma unroll
-    for (int j = 0; j < KB; ++j)
-      if (j < cnt) part[j] = __fma_rn(vi, cp[j][i], part[j]);
-  });
-  // tmp_j += Q[kk, j]; Q[kk, j] -= tau * tmp_j
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < cnt; ++j) {
-      double* q = colp[c_lo + j] + kk;
-      sh_tmp[j] = __dadd_rn(sh_tmp[j], *q);
-      *q = __dsub_rn(*q, __dmul_rn(tau, sh_tmp[j]));
-    }
-  }
-  __syncthreads();
-  double t[KB];
-#pragma unroll
-  for (int j = 0; j < KB; ++j) t[j] = j < cnt ? sh_tmp[j] : 0.0;
-  for (int64_t i = kk + 1 + threadIdx.x; i < rows; i += blockDim.x) {
-    const double tv = __dmul_rn(tau, v[i]);
-#pragma unroll
-    for (int j = 0; j < KB; ++j)
-      if (j < cnt) cp[j][i] = __fma_rn(-tv, t[j], cp[j][i]);
-  }
-  __syncthreads();
-}
-
-// One block per tuned candidate: column-pivoted QR least squares on
-// [A | 1 | y] with every sum in QSUM order (bit-identical to the chunked
-// passes of qr_chunk.cu).  KB bounds the columns (k + 1) so that per-column
-// accumulators stay in registers.  Pivoting swaps column pointers, not data.
-template <int KB>
-__global__ void __launch_bounds__(256) plain_qr_kernel_t(DevBatch b, DevData ds, const PlainCand* pc,
-                                                          const int32_t* list, int cand0, const double* A, double* M,
-                                                          double* coefs, rrg_result* res, uint32_t* status,
-                                                          const int32_t* colmap) {
-  extern __shared__ double smem[];
-  const int c = list ? list[cand0 + blockIdx.x] : cand0 + blockIdx.x;
-  const rrg_cand cd = b.cands[c];
-  if (cd.mode != RRG_TUNED || (pc[c].pad & 1)) return;  // pad bit 0: outcome already written
-  const int k = pc[c].k;
-  if (k + 1 > KB || k > kMaxK) {
-    if (threadIdx.x == 0) atomicOr(status, ST_TOO_LARGE);
-    return;
-  }
-  double* red = smem;                       // 8 * (kMaxK + 1)
-  double* sh_tmp = red + 8 * (kMaxK + 1);   // kMaxK + 1
-  double* nupd = sh_tmp + (kMaxK + 1);      // kMaxK
-  double* ndir = nupd + kMaxK;              // kMaxK
-  double* hc = ndir + kMaxK;                // kMaxK
-  int* perm = reinterpret_cast<int*>(hc + kMaxK);
-  int* misc = perm + kMaxK;                 // [0] pivot, [1] nonzero, [2..] recompute flags
-  __shared__ double* colp[KB];              // current position -> column storage
-
-  double* Q = M + pc[c].m_col * ds.n_pad;
-  const int64_t ld = ds.n_pad, rows = ds.n;
-  for (int j = threadIdx.x; j <= k; j += blockDim.x) colp[j] = Q + (int64_t)j * ld;
-  // [A | 1 | y] into the working columns
-  for (int j = 0; j <= k; ++j) {
-    double* dst = Q + (int64_t)j * ld;
-    if (j < k - 1) {
-      const double* src = factor_column(A, ds.n_pad, pc[c].a_col, j, colmap);
-      for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) dst[r] = src[r];
-    } else if (j == k - 1) {
-      for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) dst[r] = 1.0;
-    } else {
-      for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) dst[r] = ds.y64[r];
-    }
-  }
-  __syncthreads();
-  // initial column norms
-  block_qsum_vec<KB>(0, rows, k, red, nullptr, sh_tmp, [&](int64_t i, double (&part)[KB]) {
-#pragma unroll
-    for (int j = 0; j < KB; ++j)
-      if (j < k) {
-        const double q = colp[j][i];
-        part[j] = __fma_rn(q, q, part[j]);
-      }
-  });
-  const double rows_thr = (double)ds.n;
-  const int size = (int)(rows < k ? rows : k);
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < k; ++j) {
-      ndir[j] = __dsqrt_rn(sh_tmp[j]);
-      nupd[j] = ndir[j];
-      perm[j] = j;
-    }
-    misc[1] = size;
-  }
-  __syncthreads();
-  double maxn = nupd[0];
-  for (int j = 1; j < k; ++j)
-    if (nupd[j] > maxn) maxn = nupd[j];
-  const double thr_helper = __ddiv_rn(__dmul_rn(__dmul_rn(maxn, DBL_EPSILON), __dmul_rn(maxn, DBL_EPSILON)), rows_thr);
-  const double downdate_thr = 1.4901161193847656e-08;  // sqrt(DBL_EPSILON)
-
-  for (int kk = 0; kk < size; ++kk) {
-    if (threadIdx.x == 0) {
-      int big = kk;
-      double bign = nupd[kk];
-      for (int j = kk + 1; j < k; ++j)
-        if (nupd[j] > bign) {
-          bign = nupd[j];
-          big = j;
-        }
-      if (misc[1] == size && __dmul_rn(bign, bign) < __dmul_rn(thr_helper, rows_thr - kk)) misc[1] = kk;
-      misc[0] = big;
-      if (big != kk) {
-        double t = nupd[kk]; nupd[kk] = nupd[big]; nupd[big] = t;
-        t = ndir[kk]; ndir[kk] = ndir[big]; ndir[big] = t;
-        int p = perm[kk]; perm[kk] = perm[big]; perm[big] = p;
-        double* cq = colp[kk]; colp[kk] = colp[big]; colp[big] = cq;
-      }
-    }
-    __syncthreads();
-    const double tau = make_householder_col(colp[kk], rows, kk, red);
-    if (threadIdx.x == 0) hc[kk] = tau;
-    // reflector kk reaches the right-hand side only while kk < rank
-    const int c_hi = misc[1] == size ? k + 1 : k;
-    apply_householder_cols<KB>(colp, rows, kk, tau, kk + 1, c_hi, red, sh_tmp);
-    // LAWN 176 norm down-dating (ColPivHouseholderQR.h:549-572)
-    int* rec = misc + 2;
-    if (threadIdx.x == 0) {
-      for (int j = kk + 1; j < k; ++j) {
-        rec[j] = 0;
-        if (nupd[j] != 0.0) {
-          double temp = __ddiv_rn(fabs(colp[j][kk]), nupd[j]);
-          temp = __dmul_rn(__dadd_rn(1.0, temp), __dsub_rn(1.0, temp));
-          temp = temp < 0.0 ? 0.0 : temp;
-          const double ratio = __ddiv_rn(nupd[j], ndir[j]);
-          const double temp2 = __dmul_rn(temp, __dmul_rn(ratio, ratio));
-          if (temp2 <= downdate_thr) rec[j] = 1;
-          else nupd[j] = __dmul_rn(nupd[j], __dsqrt_rn(temp));
-        }
-      }
-    }
-    __syncthreads();
-    for (int j = kk + 1; j < k; ++j) {
-      if (!rec[j]) continue;  // uniform
-      const double* cj = colp[j];
-      const double s = block_qsum(kk + 1, rows, red, [&](int64_t i, double p) { return __fma_rn(cj[i], cj[i], p); });
-      if (threadIdx.x == 0) {
-        ndir[j] = __dsqrt_rn(s);
-        nupd[j] = ndir[j];
-      }
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int r = misc[1];
-    double cvec[kMaxK];
-    for (int i = 0; i < r; ++i) cvec[i] = colp[k][i];
-    for (int kk = r - 1; kk >= 0; --kk) {
-      cvec[kk] = __ddiv_rn(cvec[kk], colp[kk][kk]);
-      for (int i = 0; i < kk; ++i) cvec[i] = __dsub_rn(cvec[i], __dmul_rn(cvec[kk], colp[kk][i]));
-    }
-    double* out = coefs + cd.coef_offset;
-    for (int j = 0; j < k; ++j) out[j] = 0.0;
-    for (int i = 0; i < r; ++i) out[perm[i]] = cvec[i];
-    res[c].rank = r;
-  }
-}
-
-}  // namespace
-
 int plain_qr_bucket(int cols) { return cols <= 4 ? 4 : (cols <= 8 ? 8 : (cols <= 16 ? 16 : kMaxK + 1)); }
-
-bool launch_plain_qr(int max_cols, int grid, cudaStream_t st, DevBatch b, DevData ds, const PlainCand* pc,
-                     const int32_t* list, int cand0, const double* A, double* M, double* coefs, rrg_result* res,
-                     uint32_t* status, const int32_t* colmap) {
-  if (grid <= 0) return true;
-  const size_t sm = plain_qr_smem();
-  if (max_cols <= 4)
-    plain_qr_kernel_t<4><<<grid, 256, sm, st>>>(b, ds, pc, list, cand0, A, M, coefs, res, status, colmap);
-  else if (max_cols <= 8)
-    plain_qr_kernel_t<8><<<grid, 256, sm, st>>>(b, ds, pc, list, cand0, A, M, coefs, res, status, colmap);
-  else if (max_cols <= 16)
-    plain_qr_kernel_t<16><<<grid, 256, sm, st>>>(b, ds, pc, list, cand0, A, M, coefs, res, status, colmap);
-  else
-    plain_qr_kernel_t<kMaxK + 1><<<grid, 256, sm, st>>>(b, ds, pc, list, cand0, A, M, coefs, res, status, colmap);
-  return launch_ok("launch_plain_qr");
-}
-
-
 
 // SSE of the rebuilt sum per (candidate, chunk of RR_CHUNK rows) item in the
 // fixed order of csrc/common/rr_sum.h; the grid walks the items.
@@ -901,8 +615,5 @@ __global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt,
 }
 
 size_t plain_eval_smem() { return RRG_MAX_STACK * 256 * sizeof(double) + kMaxCodeSmem * sizeof(uint32_t); }
-size_t plain_qr_smem() {
-  return (8 * (kMaxK + 1) + (kMaxK + 1) + 3 * kMaxK) * sizeof(double) + (kMaxK + 2 + kMaxK) * sizeof(int);
-}
 
 }  // namespace rrd

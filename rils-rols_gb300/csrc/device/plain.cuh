@@ -15,13 +15,14 @@ __global__ void plain_eval_kernel(DevBatch b, DevData ds, const PlainCand* pc, c
 // colmap (may be NULL): factor column j of candidate c is column
 // colmap[pc[c].a_col + j] of A (a shared factor table) instead of
 // column pc[c].a_col + j.
-// Column bucket (register footprint) of the QR kernel for k + 1 columns.
+// Column bucket of a QR launch for k + 1 columns (its widest sets the scratch).
 int plain_qr_bucket(int cols);
 // One block per candidate of the launch (the whole factorisation in one
-// launch; QSUM order, the bits of launch_qr_chunked); max_cols bounds k + 1.
-bool launch_plain_qr(int max_cols, int grid, cudaStream_t st, DevBatch b, DevData ds, const PlainCand* pc,
-                     const int32_t* list, int cand0, const double* A, double* M, double* coefs, rrg_result* res,
-                     uint32_t* status, const int32_t* colmap);
+// launch; QSUM order, the bits of launch_qr_chunked; qr_small.cu); max_cols
+// bounds k + 1.
+bool launch_plain_qr(int max_cols, int grid, int sm_count, cudaStream_t st, DevBatch b, DevData ds,
+                     const PlainCand* pc, const int32_t* list, int cand0, const double* A, double* M, double* coefs,
+                     rrg_result* res, uint32_t* status, const int32_t* colmap);
 // Squared residual of the rebuilt sum of the candidates list[cand0 .. cand0 +
 // n_cand) per chunk of RR_CHUNK rows: partial[c * chunks + chunk].  dcount (may
 // be NULL): list positions at or beyond *dcount do nothing (a list whose length
@@ -83,6 +84,5 @@ __global__ void table_eval_list_kernel(DevBatch b, DevData ds, const PlainCand* 
                                        const int32_t* count, int max_nbc, double* A, uint32_t* status, ColStat* cst);
 
 size_t plain_eval_smem();
-size_t plain_qr_smem();
 
 }  // namespace rrd

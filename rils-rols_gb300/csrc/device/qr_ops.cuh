@@ -1,4 +1,4 @@
-// Device helpers shared by the FP64 QR kernels (plain.cu, qr_chunk.cu).
+// Device helpers shared by the FP64 QR kernels (qr_small.cu, qr_chunk.cu) and the residual (plain.cu).
 #pragma once
 #include <cstdint>
 

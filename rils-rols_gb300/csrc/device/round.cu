@@ -1680,8 +1680,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
 rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<int32_t>& list_in,
                                        uint32_t flags_or) {
   if (list_in.empty()) return RRG_OK;
-  // candidates ordered by the QR kernel's column bucket, so that each launch
-  // uses the smallest register footprint its candidates allow
+  // candidates ordered by the QR launch's column bucket, so that each launch
+  // takes the shared memory or scratch of columns its own candidates need
   auto bucket = [&](int32_t c) {
     const rrg_cand& cd = host_cands[c];
     return plain_qr_bucket(cd.mode == RRG_TUNED ? cd.n_factors + 2 : 2);
@@ -1941,7 +1941,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     for (const auto& sb : subs) {
       const int32_t ns = sb.second - sb.first;
       if (ns <= 0) continue;
-      // one factorisation per register bucket of the sub-batch, side by side
+      // one factorisation per column bucket of the sub-batch, side by side
       // on the side streams: one block per candidate while the rows fit one
       // chunk, otherwise the chunked passes over the whole GPU (same bits)
       struct QrRun {
@@ -1976,7 +1976,8 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
         if (used < kSide) RRG_CUDA(cudaStreamWaitEvent(s, fork_ev, 0));
         bool ok;
         if (!chunked) {
-          ok = launch_plain_qr(r.bk, r.b1 - r.b0, s, dev, dd, d_pcs, d_list, r.b0, F64, M, coefs, res, status, d_cmap);
+          ok = launch_plain_qr(r.wide, r.b1 - r.b0, sm_count, s, dev, dd, d_pcs, d_list, r.b0, F64, M, coefs, res,
+                               status, d_cmap);
           ++launches;
         } else {
           QrJob jb{};
