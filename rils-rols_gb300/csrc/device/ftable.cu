@@ -12,14 +12,25 @@
 //                 more occupancy than the loads it saves).
 //                 Values go to the table F in HBM (rows >= n set to 0); the
 //                 self sums  sum f*f, sum f, sum f*y  of the chunk are formed
-//                 on the way;
+//                 on the way, a warp's three folded together and the warps'
+//                 added once all programs are through.  The block waits after
+//                 every program all the same: warps that run different
+//                 programs evict one another's instructions (14.8 ms without
+//                 the wait, 13.8 with it, for 8192 random trees at 100k rows);
 //   pair_sum      block = (factor a with its partners b, row block): a's
 //                 values stay in registers, each partner column is streamed
-//                 once, sum a*b in double-float arithmetic;
+//                 once, sum a*b in double-float arithmetic, four partners'
+//                 sums folded together, whole blocks of rows without bounds
+//                 checks.  Bound by instruction issue: eight rounds at 1M rows
+//                 12.9 ms with a fold and checks for each partner, 10.6
+//                 without, 8.85 with registers for four blocks an SM (packed
+//                 pairs of FP32 operations were slower, 10.6: packing them
+//                 costs more than it saves);
 //   pair_reduce   FP64 totals of the partials, in chunk order;
 //   ftab_resid    the rebuilt sum  sum_i c_i f_i  (drop / snap rules of
 //                 rils_rols_cpp.cpp:488-517) from the table, its residual
-//                 against y and the squared residuals, all double-float.
+//                 against y and the squared residuals, all double-float (four
+//                 blocks an SM: 3.82 -> 3.56 ms over the same eight rounds).
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>
@@ -40,6 +51,20 @@ __device__ __forceinline__ dfl shfl_dfl(dfl v, int o) {
 __device__ __forceinline__ dfl warp_dfl_sum(dfl v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = dfl_add(v, shfl_dfl(v, o));
+  return v;
+}
+
+// warp_dfl_sum of four values at once, lanes exchanging halves of what is left
+// (reduce.cuh, warp_sum_many): 6 additions instead of 20, each of them
+// warp_dfl_sum's (dfl_add is symmetric).  Lanes 8 i .. 8 i + 7 return value i's.
+__device__ __forceinline__ dfl warp_dfl_sum4(dfl v0, dfl v1, dfl v2, dfl v3) {
+  const int lane = threadIdx.x & 31;
+  const bool h = (lane & 16) != 0, q = (lane & 8) != 0;
+  const dfl a = dfl_add(h ? v2 : v0, shfl_dfl(h ? v0 : v2, 16));
+  const dfl b = dfl_add(h ? v3 : v1, shfl_dfl(h ? v1 : v3, 16));
+  dfl v = dfl_add(q ? b : a, shfl_dfl(q ? a : b, 8));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v = dfl_add(v, shfl_dfl(v, o));
   return v;
 }
 
@@ -236,10 +261,11 @@ __device__ __forceinline__ bool eval_fac4(const uint32_t* code, int len, const f
 }
 
 // shared-memory layout of fac_eval
-constexpr size_t kFacRedOff = 128;                                   // [warp][6] floats
-constexpr size_t kFacSkipOff = kFacRedOff + 192;                     // [program of the group] left out
-constexpr size_t kFacCodeOff = kFacSkipOff + kFacGroupMax;
-static_assert(kFacCodeOff % 128 == 0 && kFacThreads / 32 * 6 * sizeof(float) <= 192, "layout");
+constexpr int kFacWarps = kFacThreads / 32;
+constexpr size_t kFacRedOff = 0;                                     // [program of the group][warp][3] sums
+constexpr size_t kFacSkipOff = kFacRedOff + sizeof(float2) * kFacGroupMax * kFacWarps * 3;  // [program] left out
+constexpr size_t kFacCodeOff = kFacSkipOff + (kFacGroupMax + 127) / 128 * 128;
+static_assert(kFacCodeOff % 128 == 0, "layout");
 constexpr size_t kFacStackOff = kFacCodeOff + sizeof(uint32_t) * kFacCodeSmem;
 constexpr size_t kFacXOff = kFacStackOff + sizeof(float4) * (kFacThreads / 32) * kMixedStackCap * 32 * 2;  // end
 // staged form: the copy barrier, then the staged rows (hi of every slot, lo
@@ -288,7 +314,7 @@ constexpr int kStageWaitTries = 1 << 20;  // bounded wait for the staged rows
 // R = 4 rows per thread for short, shallow programs (one dispatch per op for
 // four rows), R = 2 for the others (less spill traffic per thread).
 template <int R, bool STAGED>
-__global__ void __launch_bounds__(kFacThreads) fac_eval_kernel(const __grid_constant__ FacEvalArgs a) {
+__global__ void __launch_bounds__(kFacThreads, 3) fac_eval_kernel(const __grid_constant__ FacEvalArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int2 grp = a.groups[blockIdx.x];
@@ -296,7 +322,7 @@ __global__ void __launch_bounds__(kFacThreads) fac_eval_kernel(const __grid_cons
   const int64_t n = a.ds.n, n_pad = a.ds.n_pad;
   const int64_t row0 = (int64_t)q * a.chunk;
   const int rows = (int)min((int64_t)a.chunk, n_pad - row0);  // a multiple of 256
-  float* red = reinterpret_cast<float*>(smem + kFacRedOff);
+  float2* red = reinterpret_cast<float2*>(smem + kFacRedOff);
   uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + kFacCodeOff);
   float4* stk = reinterpret_cast<float4*>(smem + kFacStackOff);
   const float* xh = a.ds.X32 + row0;
@@ -370,7 +396,7 @@ __global__ void __launch_bounds__(kFacThreads) fac_eval_kernel(const __grid_cons
   // it only decides who does the work).  Their sums are NaN by that chunk, the
   // column's first NaN row is there, and nobody reads such a column as an
   // operand (FacEvalArgs::stop).  8192 random trees at 100k rows, where seven
-  // factors of eight hold a NaN: 58.7 ms before, 15.5 now.
+  // factors of eight hold a NaN: 58.7 ms before, 13.8 now.
   uint8_t* skip_s = smem + kFacSkipOff;
   if (tid < grp.y) {
     const int f = grp.x + tid;
@@ -383,10 +409,7 @@ __global__ void __launch_bounds__(kFacThreads) fac_eval_kernel(const __grid_cons
   float4* st = stk + (size_t)warp * kMixedStackCap * 32 * 2 + lane;
   for (int i = 0; i < grp.y; ++i) {
     const int f = grp.x + i;
-    if (skip_s[i]) {  // uniform
-      if (tid < 3) a.P[(size_t)q * a.n_pairs + 3 * (size_t)f + tid] = make_float2(0.f, 0.f);
-      continue;
-    }
+    if (skip_s[i]) continue;  // uniform
     const int64_t fw = a.wcol ? a.wcol[f] : f;  // the column it writes
     const int2 mt = a.meta[f];
     const uint32_t* code = code_s + (mt.x - base);
@@ -458,20 +481,21 @@ __global__ void __launch_bounds__(kFacThreads) fac_eval_kernel(const __grid_cons
       first = other < first ? other : first;
     }
     if (lane == 0 && first != ~0ull) atomicMin(a.fnan + fw, first);
-    const dfl s0 = warp_dfl_sum(dfl_renorm(ff)), s1 = warp_dfl_sum(dfl_renorm(fs)), s2 = warp_dfl_sum(dfl_renorm(fy));
-    if (lane == 0) {
-      float* rw = red + warp * 6;
-      rw[0] = s0.hi; rw[1] = s0.lo;
-      rw[2] = s1.hi; rw[3] = s1.lo;
-      rw[4] = s2.hi; rw[5] = s2.lo;
-    }
+    const dfl sv = warp_dfl_sum4(dfl_renorm(ff), dfl_renorm(fs), dfl_renorm(fy), dfl_make(0.f, 0.f));
+    if ((lane & 7) == 0 && lane < 24) red[(i * kFacWarps + warp) * 3 + (lane >> 3)] = make_float2(sv.hi, sv.lo);
     __syncthreads();
-    if (tid < 3) {
-      dfl s = dfl_make(0.f, 0.f);
-      for (int w = 0; w < kFacThreads / 32; ++w) s = dfl_add(s, dfl_make(red[w * 6 + 2 * tid], red[w * 6 + 2 * tid + 1]));
-      a.P[(size_t)q * a.n_pairs + 3 * (size_t)f + tid] = make_float2(s.hi, s.lo);
-    }
-    __syncthreads();
+  }
+  // the warps' sums of every program, in order
+  __syncthreads();
+  for (int t = tid; t < 3 * grp.y; t += kFacThreads) {
+    const int i = t / 3, k = t % 3;
+    dfl s = dfl_make(0.f, 0.f);
+    if (!skip_s[i])
+      for (int w = 0; w < kFacWarps; ++w) {
+        const float2 v = red[(i * kFacWarps + w) * 3 + k];
+        s = dfl_add(s, dfl_make(v.x, v.y));
+      }
+    a.P[(size_t)q * a.n_pairs + 3 * (size_t)(grp.x + i) + k] = make_float2(s.hi, s.lo);
   }
 }
 
@@ -482,67 +506,89 @@ __device__ __forceinline__ float pair_lo(float ah, float al, float bh, float bl)
   return DF_ADD(DF_FMA(ah, bh, -p), DF_ADD(DF_MUL(ah, bl), DF_MUL(al, bh)));
 }
 
-__global__ void __launch_bounds__(kPairThreads) pair_sum_kernel(PairArgs a) {
-  __shared__ float red[kPairBatch][kPairThreads / 32][2];
+// sum a*b over one block of rows for one partner column (rows a multiple of
+// 256, kPairRows unless the block is the last).  Without the non-finite
+// guards: a non-finite factor value turns the sum NaN instead of +-inf, and the
+// solve sends every candidate with a non-finite cross sum (NaN or inf alike) to
+// the FP64 path.  The product is symmetric in its operands (the exact error of
+// hi x hi, then the rounded sum of the two rounded cross products), so a pair's
+// sum is the same bits whichever factor a unit holds.
+template <bool FULL>
+__device__ __forceinline__ dfl pair_column(const float4 (&av)[kPairPerThread], const float2* fb, int rows) {
+  dfl acc = dfl_make(0.f, 0.f);
+  fb += 2 * threadIdx.x;
+#pragma unroll
+  for (int s = 0; s < kPairPerThread; ++s) {
+    if (FULL || 2 * (int)threadIdx.x + 2 * kPairThreads * s < rows) {
+      const float4 bv = *reinterpret_cast<const float4*>(fb + 2 * kPairThreads * s);
+      acc2(acc, DF_MUL(av[s].x, bv.x), pair_lo(av[s].x, av[s].y, bv.x, bv.y));
+      acc2(acc, DF_MUL(av[s].z, bv.z), pair_lo(av[s].z, av[s].w, bv.z, bv.w));
+    }
+  }
+  return dfl_renorm(acc);
+}
+
+template <bool FULL>
+__device__ __forceinline__ void pair_unit(const PairArgs& a, int4 U, int qs, int rows,
+                                          float (*red)[kPairThreads / 32][2]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int u = blockIdx.x % a.n_units;
-  const int qs = blockIdx.x / a.n_units;
-  const int4 U = a.units[u];
   const int64_t row0 = (int64_t)qs * kPairRows;
-  const int rows = (int)min((int64_t)kPairRows, a.n_pad - row0);
-  const float2* fa = a.F + (int64_t)U.x * a.n_pad + row0;
-  // a factor with a NaN makes every sum with it NaN (and its column may lack
-  // rows): such pairs are not read
-  const bool a_nan = a.fnan[U.x] < (unsigned long long)a.n;
-  const float nanf = __int_as_float(0x7fc00000);
+  const float2* F = a.F + row0;
+  const float2* fa = F + (int64_t)U.x * a.n_pad;
   float4 av[kPairPerThread];
 #pragma unroll
   for (int s = 0; s < kPairPerThread; ++s) {
     const int r = 2 * tid + 2 * kPairThreads * s;
-    av[s] = r < rows && !a_nan ? *reinterpret_cast<const float4*>(fa + r) : make_float4(0.f, 0.f, 0.f, 0.f);
+    av[s] = FULL || r < rows ? *reinterpret_cast<const float4*>(fa + r) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  const dfl zero = dfl_make(0.f, 0.f);
   for (int p0 = U.y; p0 < U.z; p0 += kPairBatch) {
     const int nb = min(kPairBatch, U.z - p0);
-    for (int j = 0; j < nb; ++j) {
-      const int32_t b = a.partner[p0 + j];
-      if (a_nan || a.fnan[b] < (unsigned long long)a.n) {  // uniform
-        if (lane == 0) {
-          red[j][warp][0] = nanf;
-          red[j][warp][1] = 0.f;
-        }
-        continue;
-      }
-      const float2* fb = a.F + (int64_t)b * a.n_pad + row0;
-      dfl acc = dfl_make(0.f, 0.f);
-#pragma unroll
-      for (int s = 0; s < kPairPerThread; ++s) {
-        const int r = 2 * tid + 2 * kPairThreads * s;
-        if (r < rows) {
-          const float4 bv = *reinterpret_cast<const float4*>(fb + r);
-          // without the non-finite guards: a non-finite factor value turns the
-          // sum NaN instead of +-inf, and the solve sends every candidate with a
-          // non-finite cross sum (NaN or inf alike) to the FP64 path.  The
-          // product is symmetric in its operands (the exact error of hi x hi,
-          // then the rounded sum of the two rounded cross products), so a
-          // pair's sum is the same bits whichever factor a unit holds
-          acc2(acc, DF_MUL(av[s].x, bv.x), pair_lo(av[s].x, av[s].y, bv.x, bv.y));
-          acc2(acc, DF_MUL(av[s].z, bv.z), pair_lo(av[s].z, av[s].w, bv.z, bv.w));
-        }
-      }
-      const dfl v = warp_dfl_sum(dfl_renorm(acc));
-      if (lane == 0) {
-        red[j][warp][0] = v.hi;
-        red[j][warp][1] = v.lo;
+    // the batch's partners, one a lane; a factor with a NaN makes every sum
+    // with it NaN (and its column may lack rows): such pairs are not read
+    int32_t mine = 0;
+    bool use = false;
+    if (lane < nb) {
+      mine = a.partner[p0 + lane];
+      use = a.fnan[mine] >= (unsigned long long)a.n;
+    }
+    const uint32_t used = __ballot_sync(0xffffffffu, use);
+    auto column = [&](int j) {
+      const int32_t b = __shfl_sync(0xffffffffu, mine, j);
+      return (used >> j) & 1u ? pair_column<FULL>(av, F + (int64_t)b * a.n_pad, rows) : zero;  // uniform
+    };
+    for (int j = 0; j < nb; j += 4) {
+      const dfl c0 = column(j), c1 = column(j + 1), c2 = column(j + 2), c3 = column(j + 3);
+      const dfl v = warp_dfl_sum4(c0, c1, c2, c3);
+      if ((lane & 7) == 0) {
+        red[j + (lane >> 3)][warp][0] = v.hi;
+        red[j + (lane >> 3)][warp][1] = v.lo;
       }
     }
     __syncthreads();
-    if (tid < nb) {
-      dfl s = dfl_make(0.f, 0.f);
+    if (tid < nb) {  // warp 0 (kPairBatch <= 32): lane tid's partner
+      dfl s = zero;
       for (int w = 0; w < kPairThreads / 32; ++w) s = dfl_add(s, dfl_make(red[tid][w][0], red[tid][w][1]));
-      a.P[(size_t)qs * a.n_pairs + a.cross0 + p0 + tid] = make_float2(s.hi, s.lo);
+      a.P[(size_t)qs * a.n_pairs + a.cross0 + p0 + tid] =
+          use ? make_float2(s.hi, s.lo) : make_float2(__int_as_float(0x7fc00000), 0.f);
     }
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kPairThreads, 4) pair_sum_kernel(PairArgs a) {
+  static_assert(kPairBatch % 4 == 0 && kPairBatch <= 32, "partners by lane, four at a time");
+  __shared__ float red[kPairBatch][kPairThreads / 32][2];
+  const int4 U = a.units[blockIdx.x % a.n_units];
+  const int qs = blockIdx.x / a.n_units;
+  const int rows = (int)min((int64_t)kPairRows, a.n_pad - (int64_t)qs * kPairRows);
+  if (a.fnan[U.x] < (unsigned long long)a.n) {
+    for (int p = U.y + (int)threadIdx.x; p < U.z; p += kPairThreads)
+      a.P[(size_t)qs * a.n_pairs + a.cross0 + p] = make_float2(__int_as_float(0x7fc00000), 0.f);
+    return;
+  }
+  if (rows == kPairRows) pair_unit<true>(a, U, qs, rows, red);
+  else pair_unit<false>(a, U, qs, rows, red);
 }
 
 // psum[p] = sum over chunks q (in order) of P[q][p], in FP64.
@@ -571,7 +617,7 @@ __device__ __forceinline__ void ftab_resid_item(const ResidArgs& a, int i, int q
 
 // Items (candidate i of list2, row block qs), i = item % n2, qs = item / n2,
 // walked by the grid in any shape: each item's partial sum is the same.
-__global__ void __launch_bounds__(kResidThreads) ftab_resid_kernel(ResidArgs a) {
+__global__ void __launch_bounds__(kResidThreads, 4) ftab_resid_kernel(ResidArgs a) {
   const int n2 = a.n2_dev ? min(*a.n2_dev, a.n2) : a.n2;
   const int64_t items = (int64_t)n2 * a.n_chunks;
   for (int64_t w = blockIdx.x; w < items; w += gridDim.x) ftab_resid_item(a, (int)(w % n2), (int)(w / n2));
