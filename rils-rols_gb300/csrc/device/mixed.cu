@@ -31,6 +31,8 @@
 namespace rrd {
 
 // ------------------------------------------------------------- probe ----
+constexpr int kProbeThreads = 512;
+
 // Scalar FP64 interpreter with the semantics of the plain path (rr_math
 // functions); the double-float one is eval_row_df (dfeval.cuh).
 template <int MM>
@@ -467,25 +469,37 @@ __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
 }
 
 
-// One warp per distinct factor: both interpreters on kProbeRows rows spread
-// evenly over the dataset (every row when n <= kProbeRows).
-__global__ void __launch_bounds__(128) fac_probe_kernel(const uint32_t* code, const int2* meta, int32_t nf,
-                                                        const double* K64, const float* K32, const float* K32lo,
-                                                        DevData ds, FacProbe* out, const int32_t* omap) {
-  const int lane = threadIdx.x & 31;
-  const int f = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (f >= nf) return;
+// One block per distinct factor: both interpreters on kProbeRows rows spread
+// evenly over the dataset (every row when n <= kProbeRows).  The squares are
+// added by one warp, lane l taking the probed rows l, l + 32, ... in order.
+// Bound by latency in small rounds and by the FP64 and integer pipes in large
+// ones.  A warp for each factor, four factors a block, left most of the GPU idle
+// in the first and mixed four programs' instructions in the second: 680 factors
+// 0.45 ms with the solve, now 0.14 (256 threads 0.15, 128 threads 0.18); 8192
+// random trees 10.0 ms, now 4.1; eight rounds at 1M rows 5.8 ms, now 2.4.
+__global__ void __launch_bounds__(kProbeThreads) fac_probe_kernel(const uint32_t* code, const int2* meta,
+                                                                  const double* K64, const float* K32,
+                                                                  const float* K32lo, DevData ds, FacProbe* out,
+                                                                  const int32_t* omap) {
+  __shared__ double val[kProbeRows];
+  __shared__ float dev_s;
+  __shared__ uint32_t flags_s, cnt_s;
+  const int f = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    dev_s = 0.f;
+    flags_s = cnt_s = 0;
+  }
+  __syncthreads();
   const int2 mt = meta[f];
   const uint32_t* fc = code + mt.x;
   const int P = ds.n < kProbeRows ? (int)ds.n : kProbeRows;
   float dev = 0.f;
-  double ss = 0.0;
-  int cnt = 0;
-  uint32_t flags = 0;
-  for (int p = lane; p < P; p += 32) {
+  uint32_t flags = 0, cnt = 0;
+  for (int p = tid; p < P; p += kProbeThreads) {
     const int64_t row = ds.n < kProbeRows ? p : ((2 * (int64_t)p + 1) * ds.n) / (2 * kProbeRows);
     double f64[1] = {0.0};
     dfl fd = dfl_make(0.f, 0.f);
+    val[p] = 0.0;  // adds nothing
     if (!probe_eval64<1>(fc, mt.y, K64, ds, row, f64) || !eval_row_df(fc, mt.y, K32, K32lo, ds, row, fd)) {
       flags |= FP_FAIL;
       continue;
@@ -498,22 +512,29 @@ __global__ void __launch_bounds__(128) fac_probe_kernel(const uint32_t* code, co
     if (n64 != n32 || (i32 && !i64) || (i64 && !i32)) flags |= FP_BAD32;
     if (!n64 && !i64 && !n32 && !i32) {
       dev = fmaxf(dev, (float)fabs(dfl_to_double(fd) - v));
-      ss = __fma_rn(v, v, ss);
+      val[p] = v;
       cnt += 1;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    flags |= __shfl_xor_sync(0xffffffffu, flags, o);
-    dev = fmaxf(dev, __shfl_xor_sync(0xffffffffu, dev, o));
-    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  flags = __reduce_or_sync(0xffffffffu, flags);
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  // deviations are not negative (or NaN, which fmaxf passes over): their bits order as integers
+  const uint32_t d = __reduce_max_sync(0xffffffffu, __float_as_uint(dev));
+  if (lane == 0) {
+    atomicOr(&flags_s, flags);
+    atomicAdd(&cnt_s, cnt);
+    atomicMax(reinterpret_cast<uint32_t*>(&dev_s), d);
   }
+  __syncthreads();
+  if (tid >= 32) return;
+  double ss = 0.0;
+  for (int p = lane; p < P; p += 32) ss = __fma_rn(val[p], val[p], ss);
+  ss = warp_sum(ss);
   if (lane == 0) {
     FacProbe r;
-    r.dev = dev;
-    r.rms = cnt > 0 ? (float)sqrt(ss / (double)cnt) : 0.f;
-    r.flags = flags | (P == ds.n ? FP_ALL_ROWS : 0u);
+    r.dev = dev_s;
+    r.rms = cnt_s > 0 ? (float)sqrt(ss / (double)cnt_s) : 0.f;
+    r.flags = flags_s | (P == ds.n ? FP_ALL_ROWS : 0u);
     out[omap ? omap[f] : f] = r;
   }
 }
@@ -588,7 +609,7 @@ __global__ void split_f32_kernel(const double* src, float* hi, float* lo, int64_
 bool launch_fac_probe(const uint32_t* code, const int2* meta, int32_t nf, const double* K64, const float* K32,
                       const float* K32lo, const DevData& ds, FacProbe* out, cudaStream_t st, const int32_t* omap) {
   if (nf <= 0) return true;
-  fac_probe_kernel<<<(nf + 3) / 4, 128, 0, st>>>(code, meta, nf, K64, K32, K32lo, ds, out, omap);
+  fac_probe_kernel<<<nf, kProbeThreads, 0, st>>>(code, meta, K64, K32, K32lo, ds, out, omap);
   return launch_ok("launch_fac_probe");
 }
 bool launch_cand_probe(const rrg_cand* cands, const int32_t* list, int32_t n_list, const int32_t* cand_fac,
