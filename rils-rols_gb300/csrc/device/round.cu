@@ -964,13 +964,23 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     fa.stage_slots = gs.slots;
     fa.gfeat = pkt.at<const int32_t>(d_ftp, gs.off_feat);
     for (size_t L = 0, g0 = 0; L < gs.level_groups.size(); ++L) {
-      const int gl = (int)g0 + gs.level_light[L];
-      fa.groups = pkt.at<const int2>(d_ftp, gs.off) + g0;
-      fa.gfeat_off = pkt.at<const int32_t>(d_ftp, gs.off_foff) + g0;
-      bool ok = launch_fac_eval(fa, gl - (int)g0, n_chunks, true, stream);
+      const int gl = (int)g0 + gs.level_light[L], ge = gs.level_groups[L];
+      // the light and the other groups of a level side by side: the last
+      // blocks of one launch leave room that the other's fill (700 factors at
+      // 100k rows 1.31 -> 1.23 ms, eight rounds at 1M rows 31.5 -> 30.6 ms)
+      const bool both = gl > (int)g0 && ge > gl;
+      cudaStream_t sh = both ? side[0] : stream;
+      bool ok = !both || (cudaEventRecord(fork_ev, stream) == cudaSuccess &&
+                          cudaStreamWaitEvent(sh, fork_ev, 0) == cudaSuccess);
       fa.groups = pkt.at<const int2>(d_ftp, gs.off) + gl;
       fa.gfeat_off = pkt.at<const int32_t>(d_ftp, gs.off_foff) + gl;
-      ok = ok && launch_fac_eval(fa, gs.level_groups[L] - gl, n_chunks, false, stream);
+      ok = ok && launch_fac_eval(fa, ge - gl, n_chunks, false, sh);
+      fa.groups = pkt.at<const int2>(d_ftp, gs.off) + g0;
+      fa.gfeat_off = pkt.at<const int32_t>(d_ftp, gs.off_foff) + g0;
+      ok = ok && launch_fac_eval(fa, gl - (int)g0, n_chunks, true, stream);
+      if (both)
+        ok = ok && cudaEventRecord(join_ev[0], sh) == cudaSuccess &&
+             cudaStreamWaitEvent(stream, join_ev[0], 0) == cudaSuccess;
       if (!ok) return false;
       launches += (gl > (int)g0) + (gs.level_groups[L] > gl);
       g0 = gs.level_groups[L];
