@@ -262,6 +262,10 @@ __global__ void __launch_bounds__(256) col_sums_kernel(const double* T, int64_t 
   for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
     const int t = (int)(it / nch), ch = (int)(it % nch);
     const int32_t c = cols[t];
+    if (cst[c].flags & kCsStop) {  // a NaN beyond row 0: not read
+      if (ch == 0 && threadIdx.x == 0) cst[c].sumsq = cst[c].tailsq = __longlong_as_double(0x7ff8000000000000ll);
+      continue;
+    }
     const double* col = T + (int64_t)c * n_pad;
     const int64_t r0 = (int64_t)ch * kQC, hi = r0 + kQC < n ? r0 + kQC : n;
     const bool row0 = ch == 0 && threadIdx.x == 0;  // the lane owning row 0: also its chain without that row

@@ -316,7 +316,7 @@ rrg_status rrg_context::run_predict(const rrg_dataset* ds) {
   RRG_CUDA(cudaMemcpyAsync(d_pc.ptr, h_pc.ptr, pc_bytes, cudaMemcpyHostToDevice, stream));
   const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(4LL * sm_count, (ds->n + 1023) / 1024));
   cudaEvent_t t0 = mark_begin();
-  plain_eval_kernel<<<dim3(nb, 1), 256, plain_eval_smem(), stream>>>(dev, dd, static_cast<const PlainCand*>(d_pc.ptr),
+  plain_eval_kernel<<<dim3(1, nb), 256, plain_eval_smem(), stream>>>(dev, dd, static_cast<const PlainCand*>(d_pc.ptr),
                                                                       nullptr, 0, static_cast<double*>(d_A.ptr),
                                                                       static_cast<uint32_t*>(d_status.ptr), nullptr);
   mark_end(P_PLAIN_EVAL, t0);
