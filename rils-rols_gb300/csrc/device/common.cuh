@@ -54,6 +54,10 @@ struct PlainCand {
 constexpr int kOpLDT = 12;   // TOS = T[arg]
 constexpr int kOpPST = 13;   // spill TOS; TOS = T[arg]
 constexpr int kSrcT = 3;     // binary operand from table column `arg`
+// Kinds of a table column (rrg_cand::reserved of its program, FacEvalArgs::kind).
+constexpr uint8_t kColWhole = 0;   // a factor that some program reads as an operand
+constexpr uint8_t kColStop = 1;    // a factor that none reads: its rows after a NaN may be left out
+constexpr uint8_t kColShared = 2;  // no factor: counts as far as the columns that read it do
 
 // word of the round's 16-word status block counting candidates whose QR outcome
 // was decided from the table's column statistics (word 0 holds the error bits)

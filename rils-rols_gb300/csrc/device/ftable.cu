@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kFacThreads, 3) fac_eval_kernel(const __grid_c
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int2 grp = a.groups[blockIdx.x];
-  const int q = blockIdx.y;
+  const int q = a.chunk0 + blockIdx.y;
   const int64_t n = a.ds.n, n_pad = a.ds.n_pad;
   const int64_t row0 = (int64_t)q * a.chunk;
   const int rows = (int)min((int64_t)a.chunk, n_pad - row0);  // a multiple of 256
@@ -395,13 +395,15 @@ __global__ void __launch_bounds__(kFacThreads, 3) fac_eval_kernel(const __grid_c
   // out here (read once per block: whether an earlier chunk's block has got to
   // it only decides who does the work).  Their sums are NaN by that chunk, the
   // column's first NaN row is there, and nobody reads such a column as an
-  // operand (FacEvalArgs::stop).  8192 random trees at 100k rows, where seven
-  // factors of eight hold a NaN: 58.7 ms before, 13.8 now.
+  // operand (FacEvalArgs::kind).  8192 random trees at 100k rows, where seven
+  // factors of eight hold a NaN: 58.7 ms before, 13.6 with it, 7.9 with the
+  // shared columns left out that no factor needs any more (FacEvalArgs::live).
   uint8_t* skip_s = smem + kFacSkipOff;
   if (tid < grp.y) {
     const int f = grp.x + tid;
-    const unsigned long long seen = __ldcg(a.fnan + (a.wcol ? a.wcol[f] : f));
-    skip_s[tid] = a.stop[f] && seen < (unsigned long long)row0 ? 1 : 0;
+    const int64_t fw = a.wcol ? a.wcol[f] : f;
+    const bool done = a.kind[f] == kColStop && __ldcg(a.fnan + fw) < (unsigned long long)row0;
+    skip_s[tid] = done || (a.live && !a.live[fw]) ? 1 : 0;
   }
   __syncthreads();
   const float2* tb = a.F + row0;

@@ -51,7 +51,9 @@ struct FacEvalArgs {
   const int2* meta;          // [f] (code offset, length)
   const int2* groups;        // [g] (first factor, count); a group's programs are contiguous
   const int32_t* wcol;       // [f] column of F (and of fnan) program f writes; NULL: column f
-  const uint8_t* stop;       // [f] 1: chunks after one with a NaN may be left out
+  const uint8_t* kind;       // [f] kCol*; kColStop: chunks after one with a NaN may be left out
+  const uint8_t* live;       // [column] 0 where nothing counts any more; NULL: all do
+  int32_t chunk0;            // this launch's first chunk
   const float* K;            // constant pool, double-float high parts
   const float* Klo;          // low parts
   int32_t chunk;             // rows per chunk, a multiple of kFacStep

@@ -279,7 +279,7 @@ extern "C" rrg_status rrg_eval_plain_noalloc(const double* X_col, int64_t ld, co
   // residual, fitness), pointed at the scratch
   const int nb_eval = (int)std::min<int64_t>(1024, std::max<int64_t>(1, (n + 1023) / 1024));
   plain_eval_kernel<<<dim3(1, nb_eval), 256, plain_eval_smem(), st>>>(db, dd, dpc, nullptr, 0, arena, status,
-                                                                       nullptr);
+                                                                       nullptr, EvalRows{0, n, nullptr});
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail("factor evaluation launch", e);
   // launch_plain_qr reads (and so clears) the launch error itself: a failed
   // QR launch is only visible through its return value

@@ -120,7 +120,8 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
 // some block has stored a NaN at row kStopRow or later, the blocks leave off
 // (the block of row 0 after its first rows, so that rows below kStopRow are
 // all there).  2048 random trees at 100k rows, seven of eight with a NaN
-// somewhere: 78.5 ms without the stop, 23.8 with it, 14.3 in pieces of 4096 rows.
+// somewhere: 78.5 ms without the stop, 23.8 with it, 14.3 in
+// pieces of 4096 rows, 7.4 with the shared columns left out that no factor needs.
 __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len, const double* consts,
                                                   const DevData& ds, int64_t r0, int64_t r1, double* st, double* Ac,
                                                   const double* T, uint32_t* status, ColStat* cs, bool stop,
@@ -155,7 +156,7 @@ __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len,
 __global__ void __launch_bounds__(256) table_eval_list_kernel(DevBatch b, DevData ds, const PlainCand* pc,
                                                                const int32_t* cols, const int32_t* count,
                                                                int min_nbc, int max_nbc, double* A, uint32_t* status,
-                                                               ColStat* cst) {
+                                                               ColStat* cst, EvalRows rows) {
   extern __shared__ double smem[];
   const int cnt = *count;
   if (cnt <= 0) return;
@@ -166,8 +167,10 @@ __global__ void __launch_bounds__(256) table_eval_list_kernel(DevBatch b, DevDat
   for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
     const int c = cols[w % cnt];
     const int bi = (int)(w / cnt);
+    if (rows.live && !rows.live[pc[c].a_col]) continue;  // uniform
     const rrg_cand cd = b.cands[c];
-    const int64_t r0 = ds.n * (int64_t)bi / nbc, r1 = ds.n * (int64_t)(bi + 1) / nbc;
+    const int64_t nr = rows.hi - rows.lo;
+    const int64_t r0 = rows.lo + nr * bi / nbc, r1 = rows.lo + nr * (bi + 1) / nbc;
     const bool staged = cd.code_len < kMaxCodeSmem;
     volatile int* found = reinterpret_cast<int*>(code_s + kMaxCodeSmem - 1);
     __syncthreads();  // the previous item's program is no longer read
@@ -177,20 +180,22 @@ __global__ void __launch_bounds__(256) table_eval_list_kernel(DevBatch b, DevDat
     __syncthreads();
     const uint32_t* code = staged ? code_s : b.code + cd.code_offset;
     eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, A + pc[c].a_col * ds.n_pad, A, status,
-                      &cst[pc[c].a_col], cd.reserved != 0, found);
+                      &cst[pc[c].a_col], cd.reserved == kColStop, found);
   }
 }
 
-// grid (candidates, nb); rows of piece i: [i*n/nb, (i+1)*n/nb).  Candidates first, so
+// grid (candidates, nb): nb pieces of the rows [rows.lo, rows.hi).  Candidates first, so
 // that a piece's NaN is known before most blocks of the later pieces start.
 __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds, const PlainCand* pc,
                                                           const int32_t* list, int cand0, double* A, uint32_t* status,
-                                                          ColStat* cst) {
+                                                          ColStat* cst, EvalRows rows) {
   extern __shared__ double smem[];
   const int c = list ? list[cand0 + blockIdx.x] : cand0 + blockIdx.x;
   const rrg_cand cd = b.cands[c];
+  if (rows.live && !rows.live[pc[c].a_col]) return;
   const int nb = gridDim.y;
-  const int64_t r0 = ds.n * (int64_t)blockIdx.y / nb, r1 = ds.n * (int64_t)(blockIdx.y + 1) / nb;
+  const int64_t nr = rows.hi - rows.lo;
+  const int64_t r0 = rows.lo + nr * blockIdx.y / nb, r1 = rows.lo + nr * (blockIdx.y + 1) / nb;
   double* st = smem + threadIdx.x;  // spill stack, RRG_MAX_STACK * blockDim.x doubles
   uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + RRG_MAX_STACK * blockDim.x);
   const bool staged = cd.code_len < kMaxCodeSmem;
@@ -203,11 +208,46 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
   double* Ac = A + pc[c].a_col * ds.n_pad;
   if (cst) {
     eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, Ac, A, status, &cst[pc[c].a_col],
-                      cd.reserved != 0, found);
+                      cd.reserved == kColStop, found);
     return;
   }
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x)
     run_row64<false>(code, cd.code_len, b.consts, ds, r, st, Ac, A, status);
+}
+
+// One block.  The columns that still count after some rows are evaluated: the
+// factors without a NaN that settles them, the operands kept as factors, and
+// what these read, level by level (latency; some 20 us for 4600 columns in 15
+// levels, against milliseconds of evaluation that it saves).
+__global__ void __launch_bounds__(1024) live_columns_kernel(LiveArgs a) {
+  auto slot_of = [&](int e) { return a.wcol ? a.wcol[e] : e; };
+  const int tid = threadIdx.x, ne = a.level_end[a.n_levels - 1];
+  for (int e = tid; e < ne; e += blockDim.x) {
+    const int s = slot_of(e);
+    bool v = a.kind[e] != kColShared && !(a.only && a.only[e] != a.only_value);
+    if (v && a.kind[e] == kColStop)
+      v = a.cst ? !(a.cst[s].flags & kCsStop) : a.fnan[s] >= (unsigned long long)a.rows;
+    a.live[s] = v ? 1 : 0;
+  }
+  __syncthreads();
+  for (int L = a.n_levels - 1; L > 0; --L) {
+    for (int e = a.level_end[L - 1] + tid; e < a.level_end[L]; e += blockDim.x) {
+      if (!a.live[slot_of(e)]) continue;
+      const int2 m = a.meta[e];
+      for (int i = 0; i < m.y; ++i) {
+        const uint32_t w = a.code[m.x + i];
+        const int op = (int)(w & 0xffu);
+        if (op == kOpLDT || op == kOpPST || (op >= RRG_OP_BIN && (((op - RRG_OP_BIN) & 7) >> 1) == kSrcT))
+          a.live[w >> 8] = 1;
+      }
+    }
+    __syncthreads();
+  }
+}
+bool launch_live_columns(const LiveArgs& a, cudaStream_t st) {
+  if (a.n_levels <= 0) return true;
+  live_columns_kernel<<<1, 1024, 0, st>>>(a);
+  return launch_ok("launch_live_columns");
 }
 
 int plain_qr_bucket(int cols) { return cols <= 4 ? 4 : (cols <= 8 ? 8 : (cols <= 16 ? 16 : kMaxK + 1)); }

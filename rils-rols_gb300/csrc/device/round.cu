@@ -435,11 +435,12 @@ struct CachePlan {
   TableProgs ep;
   std::vector<int32_t> ewcol;
   std::vector<int32_t> ecol;     // [evaluated program] its table column
-  std::vector<uint8_t> stop;     // [evaluated program] may stop at a NaN (operand_free)
+  std::vector<uint8_t> kind;     // [evaluated program] kCol*
   std::vector<int32_t> fslot;    // [local factor] slot
   std::vector<int32_t> mprog;    // local factors evaluated
   std::vector<int32_t> scratch;  // slots of shared columns (this sub-round only)
   int64_t hits = 0;
+  int64_t n_shared = 0;          // evaluated programs of kind kColShared
   int64_t arena = 0;             // slots the arena must hold
   bool kept = false;             // the cache was used (slots scattered)
 };
@@ -486,8 +487,10 @@ bool plan_columns(TableScratch& ts, ColumnCache& cc, bool keep, const std::vecto
     out.ecol.resize(nc);
     for (int32_t c = 0; c < nc; ++c) out.ewcol[c] = out.ecol[c] = c;
     out.fslot = tp.fcol;
-    out.stop = operand_columns(tp);
-    for (uint8_t& v : out.stop) v = v ? 0 : 1;  // (a shared column is an operand)
+    const std::vector<uint8_t> operand = operand_columns(tp);
+    out.kind.assign(nc, kColShared);
+    for (int32_t l = 0; l < nfl; ++l) out.kind[tp.fcol[l]] = operand[tp.fcol[l]] ? kColWhole : kColStop;
+    for (uint8_t k : out.kind) out.n_shared += k == kColShared;
     for (int32_t l = 0; l < nfl; ++l) out.mprog.push_back(l);
     out.arena = nc;
     return true;
@@ -568,7 +571,8 @@ bool plan_columns(TableScratch& ts, ColumnCache& cc, bool keep, const std::vecto
       ep.stack.push_back(tp.stack[c]);
       out.ewcol.push_back(slot_of[c]);
       out.ecol.push_back(c);
-      out.stop.push_back(operand[c] ? 0 : 1);
+      out.kind.push_back(!is_fac[c] ? kColShared : operand[c] ? kColWhole : kColStop);
+      out.n_shared += !is_fac[c];
     }
     ep.level_end.push_back((int32_t)ep.meta.size());
   }
@@ -899,7 +903,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       !d_P.reserve(sizeof(float2) * (size_t)n_chunks * std::max(1, n_self)) ||
       !d_cfnan.grow_keep(sizeof(unsigned long long) * n_slots, d_cfnan.cap) ||
       !d_cself.grow_keep(sizeof(double) * 3 * n_slots, d_cself.cap) ||
-      !d_cprobe.grow_keep(sizeof(FacProbe) * n_slots, d_cprobe.cap)) {
+      !d_cprobe.grow_keep(sizeof(FacProbe) * n_slots, d_cprobe.cap) || !d_live.reserve(n_slots)) {
     rrc::set_error("mixed round: factor table allocation failed");
     return RRG_E_OOM;
   }
@@ -910,7 +914,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   const size_t o_ecode = pkt.add(ep.code.data(), sizeof(uint32_t) * std::max<size_t>(1, ep.code.size()));
   const size_t o_emeta = pkt.add(ep.meta.data(), sizeof(int2) * std::max<size_t>(1, ep.meta.size()));
   const size_t o_ewcol = pkt.add(ewcol.data(), sizeof(int32_t) * std::max<size_t>(1, ewcol.size()));
-  const size_t o_estop = pkt.add(cp.stop.data(), std::max<size_t>(1, cp.stop.size()));
+  const size_t o_ekind = pkt.add(cp.kind.data(), std::max<size_t>(1, cp.kind.size()));
+  const size_t o_elend = pkt.add(ep.level_end.data(), sizeof(int32_t) * std::max<size_t>(1, ep.level_end.size()));
+  const size_t o_tmeta = pkt.add(tp.meta.data(), sizeof(int2) * std::max<size_t>(1, tp.meta.size()));
   for (GroupSet& gs : gsets) {
     gs.off = pkt.add(gs.groups.data(), sizeof(int2) * gs.groups.size());
     gs.off_foff = pkt.add(gs.feat_off.data(), sizeof(int32_t) * gs.feat_off.size());
@@ -936,7 +942,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   fa.code = pkt.at<const uint32_t>(d_ftp, o_ecode);
   fa.meta = pkt.at<const int2>(d_ftp, o_emeta);
   fa.wcol = d_ewcol;
-  fa.stop = pkt.at<const uint8_t>(d_ftp, o_estop);
+  fa.kind = pkt.at<const uint8_t>(d_ftp, o_ekind);
   fa.K = dev.consts32;
   fa.Klo = dev.consts32lo;
   fa.chunk = chunk;
@@ -959,7 +965,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   };
   const bool maps_ok = fac_stage_maps(fa, dd);
   // one launch per level: a level reads the columns of the levels before it
-  auto eval_all = [&](const GroupSet& gs, bool stage) {
+  auto eval_rows = [&](const GroupSet& gs, bool stage, int q0, int q1, const uint8_t* live) {
+    fa.chunk0 = q0;
+    fa.live = live;
     fa.stage = stage ? 1 : 0;
     fa.stage_slots = gs.slots;
     fa.gfeat = pkt.at<const int32_t>(d_ftp, gs.off_feat);
@@ -974,10 +982,10 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
                           cudaStreamWaitEvent(sh, fork_ev, 0) == cudaSuccess);
       fa.groups = pkt.at<const int2>(d_ftp, gs.off) + gl;
       fa.gfeat_off = pkt.at<const int32_t>(d_ftp, gs.off_foff) + gl;
-      ok = ok && launch_fac_eval(fa, ge - gl, n_chunks, false, sh);
+      ok = ok && launch_fac_eval(fa, ge - gl, q1 - q0, false, sh);
       fa.groups = pkt.at<const int2>(d_ftp, gs.off) + g0;
       fa.gfeat_off = pkt.at<const int32_t>(d_ftp, gs.off_foff) + g0;
-      ok = ok && launch_fac_eval(fa, gl - (int)g0, n_chunks, true, stream);
+      ok = ok && launch_fac_eval(fa, gl - (int)g0, q1 - q0, true, stream);
       if (both)
         ok = ok && cudaEventRecord(join_ev[0], sh) == cudaSuccess &&
              cudaStreamWaitEvent(stream, join_ev[0], 0) == cudaSuccess;
@@ -986,6 +994,24 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       g0 = gs.level_groups[L];
     }
     return true;
+  };
+  const int q_first = (int)std::max<int64_t>(1, kFirstRows / chunk);
+  const bool two_parts = n_chunks >= 4 * q_first && eval_two_parts(ds->n, cp.n_shared, ne);
+  auto eval_all = [&](const GroupSet& gs, bool stage) {
+    if (!two_parts) return eval_rows(gs, stage, 0, n_chunks, nullptr);
+    LiveArgs la{};
+    la.code = fa.code;
+    la.meta = fa.meta;
+    la.wcol = fa.wcol;
+    la.kind = fa.kind;
+    la.level_end = pkt.at<const int32_t>(d_ftp, o_elend);
+    la.n_levels = (int32_t)ep.level_end.size();
+    la.fnan = fnan;
+    la.rows = std::min<int64_t>(ds->n, (int64_t)q_first * chunk);
+    la.live = static_cast<uint8_t*>(d_live.ptr);
+    ++launches;
+    return eval_rows(gs, stage, 0, q_first, nullptr) && launch_live_columns(la, stream) &&
+           eval_rows(gs, stage, q_first, n_chunks, la.live);
   };
   int gbest = 0;  // the group set in use
   if (gtrial) {
@@ -1336,6 +1362,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       // (factor columns through cand_col)
       std::vector<rrg_cand> fc(std::max(1, ncol));
       std::vector<PlainCand> fpc(std::max(1, ncol));
+      std::vector<uint8_t> kind(std::max(1, ncol)), is_fac(std::max(1, ncol), 0);
+      for (int32_t l = 0; l < nfl; ++l) is_fac[tp.fcol[l]] = 1;
+      int64_t n_shared = 0;
       std::vector<int32_t> dep_off(ncol + 1, 0), deps;
       std::vector<std::vector<int32_t>> closure(ncol);
       for (int32_t i = 0; i < ncol; ++i) {
@@ -1347,7 +1376,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         p.mode = RRG_UNTUNED;
         p.coef_offset = 0;
         p.stack_need = tp.stack[i];
-        p.reserved = operand[i] ? 0 : 1;  // may stop at a NaN
+        kind[i] = !is_fac[i] ? kColShared : operand[i] ? kColWhole : kColStop;
+        n_shared += !is_fac[i];
+        p.reserved = kind[i];
         fpc[i] = PlainCand{i, 0, 0, 1, 0};
         std::vector<int32_t>& cl = closure[i];
         for (int pc = 0; pc < tp.meta[i].y; ++pc) {
@@ -1381,6 +1412,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       const size_t o_deps = pf.add(deps.data(), sizeof(int32_t) * std::max<size_t>(1, deps.size()));
       const size_t o_liof = pf.add(li_of.data(), sizeof(int32_t) * li_of.size());
       const size_t o_pcs = pf.add(pcs.data(), sizeof(PlainCand) * pcs.size());
+      const size_t o_kind = pf.add(kind.data(), kind.size());
       const size_t o_lend = pf.add(tp.level_end.data(), sizeof(int32_t) * tp.level_end.size());
       const size_t o_kept = pf.add(kept.data(), sizeof(int32_t) * kept.size());
       pst = pf.send(h_fbpack, d_fbpack, stream, round_seq);
@@ -1388,7 +1420,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       const int nb_res = (int)((ds->n + RR_CHUNK - 1) / RR_CHUNK);
       const int nbx = (int)std::max<int64_t>(1, std::min<int64_t>(16, (ds->n + 32767) / 32768));
       const size_t stat_words = 2 + kFbReasons + (size_t)n_levels;
-      if (!d_rlist2.reserve(sizeof(int32_t) * (cnt + 1)) || !d_fbneed.reserve(std::max(1, ncol)) ||
+      if (!d_rlist2.reserve(sizeof(int32_t) * (cnt + 1)) || !d_fbneed.reserve(std::max(1, ncol)) || !d_fblive.reserve(std::max(1, ncol)) ||
           !d_fbcols.reserve(sizeof(int32_t) * (2 * (size_t)ncol + n_levels + 1)) ||
           !d_cpart.reserve(sizeof(double) * std::max<size_t>(1, (size_t)ncol * (size_t)(nch + 1))) ||
           !d_fbF64.reserve(col8 * std::max(1, ncol)) || !d_fbcst.reserve(sizeof(ColStat) * std::max(1, ncol)) ||
@@ -1480,12 +1512,33 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       // 8192 random trees at 100k rows 20.0 ms with 4 blocks an SM, 19.0 with
       // 64; eight rounds at 1M rows 12.4 -> 11.9 ms; perturbations 0.40 -> 0.38.)
       constexpr int kLaneBlocks = 64;
-      const int max_nbc = (int)std::max<int64_t>(1, (ds->n + 1023) / 1024);
-      for (int32_t L = 0; L < n_levels; ++L) {
-        const int32_t lo = L == 0 ? 0 : tp.level_end[L - 1];
-        table_eval_list_kernel<<<kLaneBlocks * sm_count, 256, plain_eval_smem(), stream>>>(
-            fdev, dd, pf.at<const PlainCand>(d_fbpack, o_fpc), lvl_cols + lo, lvl_count + L,
-            (int)eval_pieces(ds->n), max_nbc, F64, status, cst);
+      auto eval_rows = [&](EvalRows rows) {
+        const int most = (int)std::max<int64_t>(1, (rows.hi - rows.lo + 1023) / 1024);
+        for (int32_t L = 0; L < n_levels; ++L) {
+          const int32_t lo = L == 0 ? 0 : tp.level_end[L - 1];
+          table_eval_list_kernel<<<kLaneBlocks * sm_count, 256, plain_eval_smem(), stream>>>(
+              fdev, dd, pf.at<const PlainCand>(d_fbpack, o_fpc), lvl_cols + lo, lvl_count + L,
+              (int)eval_pieces(rows.hi - rows.lo), most, F64, status, cst, rows);
+        }
+        launches += n_levels;
+      };
+      if (eval_two_parts(ds->n, n_shared, ncol)) {
+        eval_rows(EvalRows{0, kFirstRows, nullptr});
+        LiveArgs la{};
+        la.code = fdev.code;
+        la.meta = pkt.at<const int2>(d_ftp, o_tmeta);
+        la.kind = pf.at<const uint8_t>(d_fbpack, o_kind);
+        la.only = need;
+        la.only_value = kNeedEval;
+        la.level_end = pf.at<const int32_t>(d_fbpack, o_lend);
+        la.n_levels = n_levels;
+        la.cst = cst;
+        la.live = static_cast<uint8_t*>(d_fblive.ptr);
+        if (!launch_live_columns(la, stream)) return RRG_E_CUDA;
+        ++launches;
+        eval_rows(EvalRows{kFirstRows, ds->n, la.live});
+      } else {
+        eval_rows(EvalRows{0, ds->n, nullptr});
       }
       if (!launch_col_sums(F64, dd, all_cols, ncol, all_count, cst, static_cast<double*>(d_cpart.ptr), 8 * sm_count,
                            stream))
@@ -1502,7 +1555,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
         return RRG_E_CUDA;
       }
       mark_end(P_PLAIN_EVAL, t0);
-      launches += n_levels + 7;
+      launches += 7;
       // the QR of every bucket, side by side on the side streams: the chunked
       // passes over the bucket's list, qbatch[q] candidates per batch
       t0 = mark_begin();
@@ -1768,7 +1821,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       p.mode = RRG_UNTUNED;
       p.coef_offset = 0;
       p.stack_need = ep.stack[i];
-      p.reserved = cp.stop[i];
+      p.reserved = cp.kind[i];
       if (ep.stack[i] > RRG_MAX_STACK) {
         rrc::set_error("FP64 round: a table program exceeds the spill stack");
         return RRG_E_INVALID;
@@ -1817,6 +1870,9 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     const size_t o_scol = pk.add(scol.data(), sizeof(int32_t) * std::max<size_t>(1, scol.size()));
     const size_t o_fcode = pk.add(fcode.data(), sizeof(uint32_t) * std::max<size_t>(1, fcode.size()));
     const size_t o_ewcol = pk.add(cp.ewcol.data(), sizeof(int32_t) * std::max<size_t>(1, cp.ewcol.size()));
+    const size_t o_kind = pk.add(cp.kind.data(), std::max<size_t>(1, cp.kind.size()));
+    const size_t o_emeta = pk.add(ep.meta.data(), sizeof(int2) * std::max<size_t>(1, ep.meta.size()));
+    const size_t o_elend = pk.add(ep.level_end.data(), sizeof(int32_t) * std::max<size_t>(1, ep.level_end.size()));
     const size_t o_fc = pk.add(fc.data(), sizeof(rrg_cand) * fc.size());
     const size_t o_fpc = pk.add(fpc.data(), sizeof(PlainCand) * fpc.size());
     const size_t o_cmap = pk.add(colmap.data(), sizeof(int32_t) * std::max<size_t>(1, colmap.size()));
@@ -1826,7 +1882,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     if (pst != RRG_OK) return pst;
     const size_t n_slots = (size_t)std::max<int64_t>(1, cp.arena);
     if (!d_F64.grow_keep(col8 * n_slots, d_F64.cap) || !d_M.reserve(col8 * mcols_max) ||
-        !d_ccst.grow_keep(sizeof(ColStat) * n_slots, d_ccst.cap) ||
+        !d_ccst.grow_keep(sizeof(ColStat) * n_slots, d_ccst.cap) || !d_live.reserve(n_slots) ||
         !d_cpart.reserve(sizeof(double) * std::max<size_t>(1, scol.size() * (size_t)(nb_res + 1)))) {
       rrc::set_error("FP64 round: table allocation failed");
       return RRG_E_OOM;
@@ -1868,31 +1924,50 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
         widest = (size_t)ep.level_end[L] - c0;
         wave_level = L;
       }
+    auto eval_level = [&](size_t L, int wv, EvalRows rows) {
+      const int32_t c0 = L == 0 ? 0 : ep.level_end[L - 1], nl = ep.level_end[L] - c0;
+      if (nl <= 0) return;
+      const int64_t nr = rows.hi - rows.lo;
+      const int64_t fill = std::min<int64_t>(((int64_t)wv * sm_count + nl - 1) / nl, (nr + 1023) / 1024);
+      const int nb = (int)std::min<int64_t>(65535, std::max(eval_pieces(nr), fill));
+      plain_eval_kernel<<<dim3(nl, nb), 256, plain_eval_smem(), stream>>>(
+          fdev, dd, pk.at<const PlainCand>(d_ft64, o_fpc), nullptr, c0, F64, status, cst, rows);
+      ++launches;
+    };
+    const EvalRows every{0, ds->n, nullptr};
+    EvalRows rest = every;
+    if (!wave_trial && eval_two_parts(ds->n, cp.n_shared, ne)) {
+      for (size_t L = 0; L < ep.level_end.size(); ++L) eval_level(L, waves, EvalRows{0, kFirstRows, nullptr});
+      LiveArgs la{};
+      la.code = fdev.code;
+      la.meta = pk.at<const int2>(d_ft64, o_emeta);
+      la.wcol = pk.at<const int32_t>(d_ft64, o_ewcol);
+      la.kind = pk.at<const uint8_t>(d_ft64, o_kind);
+      la.level_end = pk.at<const int32_t>(d_ft64, o_elend);
+      la.n_levels = (int32_t)ep.level_end.size();
+      la.cst = cst;
+      la.live = static_cast<uint8_t*>(d_live.ptr);
+      if (!launch_live_columns(la, stream)) return RRG_E_CUDA;
+      ++launches;
+      rest = EvalRows{kFirstRows, ds->n, la.live};
+    }
     for (size_t L = 0, c0 = 0; L < ep.level_end.size(); ++L) {
       const int32_t c1 = ep.level_end[L];
       const int32_t nl = c1 - (int32_t)c0;
-      auto eval_level = [&](int wv) {
-        if (nl <= 0) return;
-        const int64_t fill = std::min<int64_t>(((int64_t)wv * sm_count + nl - 1) / nl, (ds->n + 1023) / 1024);
-        const int nb = (int)std::min<int64_t>(65535, std::max(eval_pieces(ds->n), fill));
-        plain_eval_kernel<<<dim3(nl, nb), 256, plain_eval_smem(), stream>>>(
-            fdev, dd, pk.at<const PlainCand>(d_ft64, o_fpc), nullptr, (int32_t)c0, F64, status, cst);
-        ++launches;
-      };
       if (wave_trial && !capturing && L == wave_level && (int64_t)nl * ds->n >= kTuneMinWork) {
         // re-evaluating a level rewrites the same columns: time every shape
         int vals[4];
         float ms[4];
         const int nv = tune_variants(TK_EVAL_WAVES, 0, vals);
         for (int v = 0; v < nv; ++v) {
-          rrg_status ts = time_trial([&] { eval_level(vals[v]); }, ms[v]);
+          rrg_status ts = time_trial([&] { eval_level(L, vals[v], every); }, ms[v]);
           if (ts != RRG_OK) return ts;
         }
         tune_store(TK_EVAL_WAVES, 0, ds->n, vals, ms, nv);
         wave_trial = false;
         waves = tune_pick(TK_EVAL_WAVES, 0, ds->n, &wave_trial);
       } else {
-        eval_level(waves);
+        eval_level(L, waves, rest);
       }
       c0 = c1;
     }

@@ -318,7 +318,8 @@ rrg_status rrg_context::run_predict(const rrg_dataset* ds) {
   cudaEvent_t t0 = mark_begin();
   plain_eval_kernel<<<dim3(1, nb), 256, plain_eval_smem(), stream>>>(dev, dd, static_cast<const PlainCand*>(d_pc.ptr),
                                                                       nullptr, 0, static_cast<double*>(d_A.ptr),
-                                                                      static_cast<uint32_t*>(d_status.ptr), nullptr);
+                                                                      static_cast<uint32_t*>(d_status.ptr), nullptr,
+                                                                      EvalRows{0, ds->n, nullptr});
   mark_end(P_PLAIN_EVAL, t0);
   ++launches;
   RRG_CUDA(cudaGetLastError());
@@ -578,7 +579,7 @@ rrg_status rrg_context::wait(int32_t timeout_ms) {
 std::vector<DevBuf*> rrg_context::all_bufs() {
   return {&d_batch, &d_A, &d_pc, &d_partial, &d_list, &d_qrs, &d_terms, &d_fallback, &d_sse1, &d_probe,
           &d_nanrow, &d_cert_e, &d_ft, &d_ftp, &d_ft64, &d_F, &d_P, &d_Pc, &d_psum, &d_F64, &d_M,
-          &d_gram, &d_rlist2, &d_fbpack, &d_fbneed, &d_fbcols, &d_fbF64, &d_fbcst, &d_fbgram, &d_fbblist,
+          &d_gram, &d_rlist2, &d_fbpack, &d_fbneed, &d_fblive, &d_live, &d_fbcols, &d_fbF64, &d_fbcst, &d_fbgram, &d_fbblist,
           &d_fbM, &d_fbctr, &d_cself, &d_cprobe, &d_cfnan, &d_ccst, &d_cpart, &d_store, &d_res, &d_coefs, &d_status};
 }
 

@@ -96,7 +96,7 @@ struct rrg_context {
   HostBuf h_mlist, h_fallback;
   // device-decided second half of a mixed round (residual-pass list, FP64
   // re-scoring lane): its buffers, and the read-back of its statistics
-  DevBuf d_rlist2, d_fbpack, d_fbneed, d_fbcols, d_fbF64, d_fbcst, d_fbgram, d_fbblist, d_fbM, d_fbctr;
+  DevBuf d_rlist2, d_fbpack, d_fbneed, d_fblive, d_live, d_fbcols, d_fbF64, d_fbcst, d_fbgram, d_fbblist, d_fbM, d_fbctr;
   HostBuf h_fbpack, h_fbstat;
   bool fbstat_pending = false;
   int32_t fbstat_levels = 0;
