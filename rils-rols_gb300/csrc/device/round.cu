@@ -817,6 +817,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   // own program (not by the shared columns its table program happens to
   // read in this sub-round): a factor's sums are then the same bits in every
   // round, kept or evaluated again.
+  constexpr int kFirstGroup = 4;
   std::vector<uint8_t> elight(ne);
   {
     std::vector<int32_t> fac_of(ncol, -1);
@@ -888,8 +889,6 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   int gvals[4] = {tune_pick(TK_FAC_GROUP, 0, ds->n, &gtrial), 0, 0, 0};
   gtrial = gtrial && !capturing && (int64_t)ne * ds->n >= kTuneMinWork;
   const int ngv = gtrial ? tune_variants(TK_FAC_GROUP, 0, gvals) : 1;
-  std::vector<GroupSet> gsets(ngv);
-  for (int v = 0; v < ngv; ++v) build_groups(std::min(gvals[v], kFacGroupMax), gsets[v]);
   // row chunks of fac_chunk(d) rows (the self sums' partials are per chunk);
   // pair sums and the residual pass use kPairRows blocks
   const int32_t n_self = 3 * ne;
@@ -898,6 +897,14 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   const int64_t n_chunks64 = (ds->n_pad + chunk - 1) / chunk;
   const int n_chunks = (int)n_chunks64;
   const int n_super = pair_row_blocks(ds->n_pad);
+  const int q_first = (int)std::max<int64_t>(1, kFirstRows / chunk);
+  const bool two_parts = n_chunks >= 4 * q_first && eval_two_parts(ds->n, cp.n_shared, ne);
+  // the group sets, and one for the first rows alone: one chunk of them leaves
+  // the blocks to the groups, so these are small (8192 random trees at 100k
+  // rows, 15 levels: 7.9 ms of evaluation with groups of 64, 6.5 with 4)
+  std::vector<GroupSet> gsets(ngv + (two_parts ? 1 : 0));
+  for (int v = 0; v < ngv; ++v) build_groups(std::min(gvals[v], kFacGroupMax), gsets[v]);
+  if (two_parts) build_groups(kFirstGroup, gsets[ngv]);
   const size_t n_slots = (size_t)std::max<int64_t>(1, cp.arena);
   if (!d_F.grow_keep(col_bytes * n_slots, d_F.cap) ||
       !d_P.reserve(sizeof(float2) * (size_t)n_chunks * std::max(1, n_self)) ||
@@ -995,8 +1002,6 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     }
     return true;
   };
-  const int q_first = (int)std::max<int64_t>(1, kFirstRows / chunk);
-  const bool two_parts = n_chunks >= 4 * q_first && eval_two_parts(ds->n, cp.n_shared, ne);
   auto eval_all = [&](const GroupSet& gs, bool stage) {
     if (!two_parts) return eval_rows(gs, stage, 0, n_chunks, nullptr);
     LiveArgs la{};
@@ -1010,7 +1015,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     la.rows = std::min<int64_t>(ds->n, (int64_t)q_first * chunk);
     la.live = static_cast<uint8_t*>(d_live.ptr);
     ++launches;
-    return eval_rows(gs, stage, 0, q_first, nullptr) && launch_live_columns(la, stream) &&
+    return eval_rows(gsets[ngv], false, 0, q_first, nullptr) && launch_live_columns(la, stream) &&
            eval_rows(gs, stage, q_first, n_chunks, la.live);
   };
   int gbest = 0;  // the group set in use
