@@ -470,6 +470,21 @@ __global__ void clear_results_kernel(const int32_t* list, int n, rrg_result* res
   if (i < n && !(dcount && i >= *dcount)) res[list[i]] = rrg_result{};
 }
 
+// Those, and the statistics of the columns about to be evaluated: one launch.
+__global__ void table_begin_kernel(const int32_t* list, int n, rrg_result* res, const int32_t* slots, int n_slots,
+                                   ColStat* cst) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) res[list[i]] = rrg_result{};
+  if (i < n_slots) cst[slots[i]] = ColStat{};
+}
+bool launch_table_begin(const int32_t* list, int n, rrg_result* res, const int32_t* slots, int n_slots, ColStat* cst,
+                        cudaStream_t st) {
+  const int m = n > n_slots ? n : n_slots;
+  if (m <= 0) return true;
+  table_begin_kernel<<<(m + 255) / 256, 256, 0, st>>>(list, n, res, slots, n_slots, cst);
+  return launch_ok("table_begin");
+}
+
 // The outcome of the column-pivoted QR (ColPivHouseholderQR.h:482-608, as
 // restated by the oracle) on [f_0 .. f_{m-1}, 1] when its first pivot has a
 // non-finite norm.  Pivot selection keeps the first maximum under '>', so a
@@ -484,45 +499,49 @@ __global__ void clear_results_kernel(const int32_t* list, int n, rrg_result* res
 // coefficients are NaN at full rank.  A finite first pivot can leave a column
 // with an exactly zero norm that a later step cuts, so NaN columns further
 // on are left to the QR.
-__global__ void sentinel_classify_kernel(DevBatch b, const int32_t* list, int cand0, int cnt, PlainCand* pc,
-                                         const int32_t* colmap, const ColStat* cs, int64_t rows, double* coefs,
-                                         rrg_result* res, uint32_t* decided, const int32_t* dcount) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt || (dcount && cand0 + i >= *dcount)) return;
-  const int c = list[cand0 + i];
+constexpr int kGramCols = 9;  // finite columns (the free term included) of the certificate below; wider: the QR
+constexpr int kGramE = kGramCols * (kGramCols + 1) / 2;
+// Returns the candidate's PlainCand::pad: 1 decided (written), 2 for nan_gram, else 0.
+__device__ __forceinline__ int classify_candidate(const DevBatch& b, int c, const PlainCand& p, const int32_t* colmap,
+                                                  const ColStat* cs, int64_t rows, double* coefs, rrg_result* res,
+                                                  uint32_t* decided) {
   const rrg_cand cd = b.cands[c];
-  if (cd.mode != RRG_TUNED) return;
-  const int k = pc[c].k;
-  const int m = k - 1;
-  if (m < 1 || rows < (int64_t)k + 2) return;
-  bool tails = true, inf_norm = false, nan0 = false;
+  const int k = p.k, m = k - 1;
+  if (cd.mode != RRG_TUNED || m < 1 || rows < (int64_t)k + 2) return 0;
+  bool tails = true, inf_norm = false, nan0 = false, any_nan = false;
+  int nf = 0;
   for (int j = 0; j < m; ++j) {
-    const ColStat st = cs[colmap[pc[c].a_col + j]];
-    if (!(st.flags & kCsTail)) tails = false;
-    if (st.flags & kCsNaN) {
+    const uint32_t f = cs[colmap[p.a_col + j]].flags;
+    if (!(f & kCsTail)) tails = false;
+    if (f & kCsNaN) {
+      any_nan = true;
       if (j == 0) nan0 = true;
-    } else if (st.flags & kCsBig) {
-      inf_norm = true;
+    } else {
+      ++nf;
+      if (f & kCsBig) inf_norm = true;
     }
   }
-  if (!tails) return;
+  if (!tails) return 0;
   if (nan0 || inf_norm) {
     double* out = coefs + cd.coef_offset;
     for (int j = 0; j < k; ++j) out[j] = __longlong_as_double(0x7ff8000000000000ll);
     res[c].rank = k;
-    pc[c].pad = 1;
     atomicAdd(decided, 1u);
-    return;
+    return 1;
   }
   // a NaN column further right: left to nan_gram_* (bit 1), which decides it
   // when the finite columns are well conditioned
-  int nf = 0;
-  bool any_nan = false;
-  for (int j = 0; j < m; ++j) {
-    if (cs[colmap[pc[c].a_col + j]].flags & kCsNaN) any_nan = true;
-    else ++nf;
-  }
-  if (any_nan && nf + 1 <= kGramCols) pc[c].pad = 2;
+  return any_nan && nf + 1 <= kGramCols ? 2 : 0;
+}
+
+__global__ void sentinel_classify_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc,
+                                         const int32_t* colmap, const ColStat* cs, int64_t rows, double* coefs,
+                                         rrg_result* res, uint32_t* decided, const int32_t* dcount) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cnt || (dcount && i >= *dcount)) return;
+  const int c = list[i];
+  const int pad = classify_candidate(b, c, pc[c], colmap, cs, rows, coefs, res, decided);
+  if (pad) pc[c].pad = pad;
 }
 
 // A NaN column at position q >= 1, column 0 finite, no infinite norm, every
@@ -539,8 +558,6 @@ __global__ void sentinel_classify_kernel(DevBatch b, const int32_t* list, int ca
 // and a remaining norm that far above it cannot be rounded down to it).
 // nan_gram_kernel forms their FP64 Gram matrix (a certificate: any summation
 // order), nan_gram_decide_kernel factors it.
-constexpr int kGramE = kGramCols * (kGramCols + 1) / 2;
-
 __device__ __forceinline__ int gram_finite_cols(const PlainCand& p, const int32_t* colmap, const ColStat* cs,
                                                 const double* T, int64_t n_pad, const double* (&colp)[kGramCols]) {
   const int m = p.k - 1;
@@ -552,23 +569,18 @@ __device__ __forceinline__ int gram_finite_cols(const PlainCand& p, const int32_
   return nf;
 }
 
-__global__ void __launch_bounds__(256) nan_gram_kernel(const int32_t* list, int cnt, const PlainCand* pc,
-                                                       const int32_t* colmap, const ColStat* cs, const double* T,
-                                                       int64_t n, int64_t n_pad, double* gpart,
-                                                       const int32_t* dcount) {
-  __shared__ double red[8][kGramE];
-  const int i = blockIdx.y;
-  if (i >= cnt || (dcount && i >= *dcount)) return;
-  const int c = list[i];
-  const PlainCand p = pc[c];
-  if (!(p.pad & 2)) return;
+// The Gram entries of the candidate's finite columns over rows [r0, r1), by a
+// block of 256 threads, into out (K columns: the leading K (K + 1) / 2 used by
+// the factorisation are formed, the others are 0).
+__device__ __forceinline__ void gram_block(const PlainCand& p, const int32_t* colmap, const ColStat* cs,
+                                           const double* T, int64_t n_pad, int64_t r0, int64_t r1,
+                                           double (*red)[kGramE], double* out) {
   const double* colp[kGramCols];
   const int nf = gram_finite_cols(p, colmap, cs, T, n_pad, colp);
   const int K = nf + 1;  // the free term last
   double part[kGramE];
 #pragma unroll
   for (int e = 0; e < kGramE; ++e) part[e] = 0.0;
-  const int64_t r0 = n * (int64_t)blockIdx.x / gridDim.x, r1 = n * (int64_t)(blockIdx.x + 1) / gridDim.x;
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     double v[kGramCols];
 #pragma unroll
@@ -581,36 +593,49 @@ __global__ void __launch_bounds__(256) nan_gram_kernel(const int32_t* list, int 
         if (bb < K) part[e] = fma(v[a], v[bb], part[e]);
   }
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  int e = 0;
 #pragma unroll
-  for (int e = 0; e < kGramE; ++e) {
-    const double t = warp_sum(part[e]);
-    if (l == 0) red[w][e] = t;
-  }
+  for (int a = 0; a < kGramCols; ++a)
+#pragma unroll
+    for (int bb = a; bb < kGramCols; ++bb, ++e) {
+      const double t = bb < K ? warp_sum(part[e]) : 0.0;  // uniform
+      if (l == 0) red[w][e] = t;
+    }
   __syncthreads();
-  for (int e = threadIdx.x; e < kGramE; e += blockDim.x) {
+  for (int i = threadIdx.x; i < kGramE; i += blockDim.x) {
     double t = 0.0;
-    for (int ww = 0; ww < 8; ++ww) t += red[ww][e];
-    gpart[((int64_t)i * gridDim.x + blockIdx.x) * kGramE + e] = t;
+    for (int ww = 0; ww < 8; ++ww) t += red[ww][i];
+    out[i] = t;
   }
 }
 
-__global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc, const int32_t* colmap,
-                                       const ColStat* cs, int nbx, const double* gpart, double* coefs,
-                                       rrg_result* res, uint32_t* decided, const int32_t* dcount) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) nan_gram_kernel(const int32_t* list, int cnt, const PlainCand* pc,
+                                                       const int32_t* colmap, const ColStat* cs, const double* T,
+                                                       int64_t n, int64_t n_pad, double* gpart,
+                                                       const int32_t* dcount) {
+  __shared__ double red[8][kGramE];
+  const int i = blockIdx.x;
   if (i >= cnt || (dcount && i >= *dcount)) return;
-  const int c = list[i];
-  if (!(pc[c].pad & 2)) return;
-  const int k = pc[c].k, m = k - 1;
+  const PlainCand p = pc[list[i]];
+  if (!(p.pad & 2)) return;
+  gram_block(p, colmap, cs, T, n_pad, n * (int64_t)blockIdx.y / gridDim.y, n * (int64_t)(blockIdx.y + 1) / gridDim.y,
+             red, gpart + ((int64_t)i * gridDim.y + blockIdx.y) * kGramE);
+}
+
+// Whether the certificate of nan_gram holds for candidate p, from the nbx
+// partial Gram matrices at gp.
+__device__ __forceinline__ bool gram_certifies(const PlainCand& p, const int32_t* colmap, const ColStat* cs, int nbx,
+                                               const double* gp) {
+  const int m = p.k - 1;
   int nf = 0;
-  for (int j = 0; j < m; ++j) nf += (cs[colmap[pc[c].a_col + j]].flags & kCsNaN) ? 0 : 1;
+  for (int j = 0; j < m; ++j) nf += (cs[colmap[p.a_col + j]].flags & kCsNaN) ? 0 : 1;
   const int K = nf + 1;
   double G[kGramCols][kGramCols];
   for (int a = 0, e = 0; a < kGramCols; ++a)
     for (int bb = a; bb < kGramCols; ++bb, ++e) {
       double t = 0.0;
       if (bb < K)
-        for (int x = 0; x < nbx; ++x) t += gpart[((int64_t)i * nbx + x) * kGramE + e];
+        for (int x = 0; x < nbx; ++x) t += gp[(int64_t)x * kGramE + e];
       G[a][bb] = t;
       G[bb][a] = t;
     }
@@ -644,15 +669,82 @@ __global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt,
         G[bb][a] = G[a][bb];
       }
   }
+  return ok;
+}
+
+__device__ __forceinline__ void settle_candidate(const DevBatch& b, int c, PlainCand* pc, bool ok, double* coefs,
+                                                 rrg_result* res, uint32_t* decided) {
   if (!ok) {
     pc[c].pad = 0;
     return;
   }
+  const int k = pc[c].k;
   double* out = coefs + b.cands[c].coef_offset;
   for (int j = 0; j < k; ++j) out[j] = __longlong_as_double(0x7ff8000000000000ll);
   res[c].rank = k;
   pc[c].pad = 1;
   atomicAdd(decided, 1u);
+}
+
+__global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc, const int32_t* colmap,
+                                       const ColStat* cs, int nbx, const double* gpart, double* coefs,
+                                       rrg_result* res, uint32_t* decided, const int32_t* dcount) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cnt || (dcount && i >= *dcount)) return;
+  const int c = list[i];
+  if (!(pc[c].pad & 2)) return;
+  settle_candidate(b, c, pc, gram_certifies(pc[c], colmap, cs, nbx, gpart + (int64_t)i * nbx * kGramE), coefs, res,
+                   decided);
+}
+
+// The three above for one candidate a block.
+__global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc,
+                                                         const int32_t* colmap, const ColStat* cs, const double* T,
+                                                         int64_t n, int64_t n_pad, double* coefs, rrg_result* res,
+                                                         uint32_t* decided, const int32_t* dcount) {
+  __shared__ double red[8][kGramE], g[kGramE];
+  __shared__ int pad;
+  if (dcount && (int)blockIdx.x >= *dcount) return;
+  const int c = list[blockIdx.x];
+  const PlainCand p = pc[c];
+  if (threadIdx.x == 0) {
+    pad = classify_candidate(b, c, p, colmap, cs, n, coefs, res, decided);
+    if (pad == 1) pc[c].pad = 1;
+  }
+  __syncthreads();
+  if (pad != 2) return;
+  gram_block(p, colmap, cs, T, n_pad, 0, n, red, g);
+  __syncthreads();
+  if (threadIdx.x == 0) settle_candidate(b, c, pc, gram_certifies(p, colmap, cs, 1, g), coefs, res, decided);
+}
+
+constexpr int64_t kGramRows = 32768;  // rows a block
+static int nan_gram_blocks(int64_t n) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(16, (n + kGramRows - 1) / kGramRows));
+}
+size_t nan_gram_bytes(int64_t n, int cnt) {
+  const int nbx = nan_gram_blocks(n);
+  return nbx == 1 ? 1 : sizeof(double) * (size_t)cnt * nbx * kGramE;
+}
+bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list, int cnt, PlainCand* pc,
+                       const int32_t* colmap, const ColStat* cs, const double* T, double* gpart, double* coefs,
+                       rrg_result* res, uint32_t* decided, const int32_t* dcount, cudaStream_t st, int64_t* launches) {
+  if (cnt <= 0) return true;
+  const int nbx = nan_gram_blocks(ds.n);
+  // One block's rows a candidate: one launch instead of three (LONE).
+  if (nbx == 1) {
+    nan_settle_kernel<<<cnt, 256, 0, st>>>(b, list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad, coefs, res, decided,
+                                           dcount);
+    *launches += 1;
+    return launch_ok("nan_settle");
+  }
+  sentinel_classify_kernel<<<(cnt + 127) / 128, 128, 0, st>>>(b, list, cnt, pc, colmap, cs, ds.n, coefs, res, decided,
+                                                              dcount);
+  nan_gram_kernel<<<dim3(cnt, nbx), 256, 0, st>>>(list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad, gpart, dcount);
+  nan_gram_decide_kernel<<<(cnt + 127) / 128, 128, 0, st>>>(b, list, cnt, pc, colmap, cs, nbx, gpart, coefs, res,
+                                                            decided, dcount);
+  *launches += 3;
+  return launch_ok("nan_gram");
 }
 
 size_t plain_eval_smem() { return RRG_MAX_STACK * 256 * sizeof(double) + kMaxCodeSmem * sizeof(uint32_t); }

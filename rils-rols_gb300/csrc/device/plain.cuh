@@ -97,26 +97,17 @@ constexpr uint32_t kCsStop = 8;  // a NaN at row kStopRow or later: the remainin
 // its rows up to the deepest pivot row are then all evaluated.
 constexpr int64_t kStopRow = 128;
 constexpr uint32_t kCsTail = 4;  // a row after the first with |value| > 1e-150 or non-finite
-// One thread per listed tuned candidate: where the QR's result is certain to
-// be all-NaN coefficients at full rank (the fitness sentinel), writes that
-// result, sets pc[c].pad = 1 (the QR and residual kernels skip it) and
-// counts it in *decided.
-// Finite columns (the free term included) of the Gram certificate for a NaN
-// column beyond column 0; wider candidates are left to the QR.
-constexpr int kGramCols = 9;
-// grid (row blocks, listed candidates): per-block FP64 Gram sums of the finite
-// columns of the candidates sentinel_classify_kernel marked (pad bit 1)
-__global__ void nan_gram_kernel(const int32_t* list, int cnt, const PlainCand* pc, const int32_t* colmap,
-                                const ColStat* cs, const double* T, int64_t n, int64_t n_pad, double* gpart,
-                                const int32_t* dcount = nullptr);
-// one thread per listed candidate: a well-conditioned Gram decides the
-// all-NaN outcome (written, pad = 1); otherwise pad = 0 and the QR runs
-__global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc, const int32_t* colmap,
-                                       const ColStat* cs, int nbx, const double* gpart, double* coefs,
-                                       rrg_result* res, uint32_t* decided, const int32_t* dcount = nullptr);
-__global__ void sentinel_classify_kernel(DevBatch b, const int32_t* list, int cand0, int cnt, PlainCand* pc,
-                                         const int32_t* colmap, const ColStat* cs, int64_t rows, double* coefs,
-                                         rrg_result* res, uint32_t* decided, const int32_t* dcount = nullptr);
+// The listed tuned candidates whose QR result is certain to be all-NaN
+// coefficients at full rank (the fitness sentinel): that result is written,
+// pc[c].pad = 1 (the QR and residual kernels skip it) and *decided counts it.
+// gpart: nan_gram_bytes(n, cnt) bytes.  dcount as above.
+size_t nan_gram_bytes(int64_t n, int cnt);
+bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list, int cnt, PlainCand* pc,
+                       const int32_t* colmap, const ColStat* cs, const double* T, double* gpart, double* coefs,
+                       rrg_result* res, uint32_t* decided, const int32_t* dcount, cudaStream_t st, int64_t* launches);
+// Before a table's evaluation: the listed results and the columns' statistics to zero.
+bool launch_table_begin(const int32_t* list, int n, rrg_result* res, const int32_t* slots, int n_slots, ColStat* cst,
+                        cudaStream_t st);
 // Table columns listed in cols[0 .. *count) (one-column programs, pc[c].a_col
 // = the column), with their column statistics into cst: a persistent grid of
 // any size walks (column, row block) items, each column split into

@@ -1423,13 +1423,12 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       pst = pf.send(h_fbpack, d_fbpack, stream, round_seq);
       if (pst != RRG_OK) return pst;
       const int nb_res = (int)((ds->n + RR_CHUNK - 1) / RR_CHUNK);
-      const int nbx = (int)std::max<int64_t>(1, std::min<int64_t>(16, (ds->n + 32767) / 32768));
       const size_t stat_words = 2 + kFbReasons + (size_t)n_levels;
       if (!d_rlist2.reserve(sizeof(int32_t) * (cnt + 1)) || !d_fbneed.reserve(std::max(1, ncol)) || !d_fblive.reserve(std::max(1, ncol)) ||
           !d_fbcols.reserve(sizeof(int32_t) * (2 * (size_t)ncol + n_levels + 1)) ||
           !d_cpart.reserve(sizeof(double) * std::max<size_t>(1, (size_t)ncol * (size_t)(nch + 1))) ||
           !d_fbF64.reserve(col8 * std::max(1, ncol)) || !d_fbcst.reserve(sizeof(ColStat) * std::max(1, ncol)) ||
-          !d_fbgram.reserve(sizeof(double) * (size_t)cnt * nbx * (kGramCols * (kGramCols + 1) / 2)) ||
+          !d_fbgram.reserve(nan_gram_bytes(ds->n, cnt)) ||
           !d_fbblist.reserve(sizeof(int32_t) * ((size_t)kQrBuckets * cnt + kQrBuckets)) ||
           !d_fbM.reserve(col8 * std::max<size_t>(1, m_cols)) || !d_qrs.reserve(std::max<size_t>(256, q_bytes)) ||
           !h_fbstat.reserve(sizeof(int32_t) * stat_words)) {
@@ -1548,19 +1547,15 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       if (!launch_col_sums(F64, dd, all_cols, ncol, all_count, cst, static_cast<double*>(d_cpart.ptr), 8 * sm_count,
                            stream))
         return RRG_E_CUDA;
-      sentinel_classify_kernel<<<(cnt + 127) / 128, 128, 0, stream>>>(dev, fb_list, 0, cnt, d_pcs, d_ccol, cst,
-                                                                     ds->n, coefs, res, status + kStatusSentinel,
-                                                                     fb_count);
-      nan_gram_kernel<<<dim3(nbx, cnt), 256, 0, stream>>>(fb_list, cnt, d_pcs, d_ccol, cst, F64, ds->n, ds->n_pad,
-                                                          gpart, fb_count);
-      nan_gram_decide_kernel<<<(cnt + 127) / 128, 128, 0, stream>>>(dev, fb_list, cnt, d_pcs, d_ccol, cst, nbx, gpart,
-                                                                    coefs, res, status + kStatusSentinel, fb_count);
+      if (!launch_nan_settle(dev, dd, fb_list, cnt, d_pcs, d_ccol, cst, F64, gpart, coefs, res,
+                             status + kStatusSentinel, fb_count, stream, &launches))
+        return RRG_E_CUDA;
       if (!launch_rescore_buckets(dev.cands, fallback, cnt, d_pcs, blist, bcount, stream)) {
         cuda_ok(cudaGetLastError(), "re-scoring bucket launch");
         return RRG_E_CUDA;
       }
       mark_end(P_PLAIN_EVAL, t0);
-      launches += 7;
+      launches += 4;
       // the QR of every bucket, side by side on the side streams: the chunked
       // passes over the bucket's list, qbatch[q] candidates per batch
       t0 = mark_begin();
@@ -1901,7 +1896,6 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     rrg_result* res = static_cast<rrg_result*>(d_res.ptr);
     uint32_t* status = static_cast<uint32_t*>(d_status.ptr);
     double* partial = static_cast<double*>(d_partial.ptr);
-    clear_results_kernel<<<(ng + 255) / 256, 256, 0, stream>>>(d_list, ng, res);
     // distinct factors, FP64, the plain evaluator (bit-identical values)
     DevBatch fdev = dev;
     fdev.cands = pk.at<const rrg_cand>(d_ft64, o_fc);
@@ -1912,11 +1906,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     // gathered by the evaluator, then the candidates whose QR outcome is
     // certainly the all-NaN sentinel (their QR and residual work is skipped)
     ColStat* cst = static_cast<ColStat*>(d_ccst.ptr);
-    static_assert(sizeof(ColStat) == 3 * sizeof(unsigned long long), "ColStat is three words");
-    if (!cp.kept)
-      RRG_CUDA(cudaMemsetAsync(cst, 0, sizeof(ColStat) * (size_t)std::max(1, ne), stream));
-    else if (!launch_fill_slots(pk.at<const int32_t>(d_ft64, o_ewcol), ne, reinterpret_cast<unsigned long long*>(cst),
-                                3, 0ull, stream))
+    if (!launch_table_begin(d_list, ng, res, pk.at<const int32_t>(d_ft64, o_ewcol), ne, cst, stream))
       return RRG_E_CUDA;
     cudaEvent_t t0 = mark_begin();
     // one launch (or several of at most 65535 columns) per level; blocks per
@@ -1980,32 +1970,18 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
                          static_cast<double*>(d_cpart.ptr), 8 * sm_count, stream))
       return RRG_E_CUDA;
     launches += scol.empty() ? 0 : 1;
-    sentinel_classify_kernel<<<(ng + 127) / 128, 128, 0, stream>>>(dev, d_list, 0, ng,
-                                                                   pk.at<PlainCand>(d_ft64, o_pcs), d_cmap, cst,
-                                                                   ds->n, coefs, res, status + kStatusSentinel);
-    {
-      // NaN columns beyond column 0: the Gram certificate of the finite columns
-      const int nbx = (int)std::max<int64_t>(1, std::min<int64_t>(16, (ds->n + 32767) / 32768));
-      const size_t gbytes = sizeof(double) * (size_t)ng * nbx * (kGramCols * (kGramCols + 1) / 2);
-      if (!d_gram.reserve(gbytes)) {
-        rrc::set_error("FP64 round: scratch allocation failed");
-        return RRG_E_OOM;
-      }
-      double* gpart = static_cast<double*>(d_gram.ptr);
-      for (int32_t g0 = 0; g0 < ng; g0 += 65535) {
-        const int32_t gn = std::min<int32_t>(65535, ng - g0);
-        nan_gram_kernel<<<dim3(nbx, gn), 256, 0, stream>>>(d_list + g0, gn, d_pcs, d_cmap, cst, F64, ds->n,
-                                                           ds->n_pad, gpart + (size_t)g0 * nbx *
-                                                                                  (kGramCols * (kGramCols + 1) / 2));
-      }
-      nan_gram_decide_kernel<<<(ng + 127) / 128, 128, 0, stream>>>(dev, d_list, ng, pk.at<PlainCand>(d_ft64, o_pcs),
-                                                                   d_cmap, cst, nbx, gpart, coefs, res,
-                                                                   status + kStatusSentinel);
-      launches += 2;
+    // NaN columns beyond column 0: the Gram certificate of the finite columns
+    if (!d_gram.reserve(nan_gram_bytes(ds->n, ng))) {
+      rrc::set_error("FP64 round: scratch allocation failed");
+      return RRG_E_OOM;
     }
+    if (!launch_nan_settle(dev, dd, d_list, ng, pk.at<PlainCand>(d_ft64, o_pcs), d_cmap, cst, F64,
+                           static_cast<double*>(d_gram.ptr), coefs, res, status + kStatusSentinel, nullptr, stream,
+                           &launches))
+      return RRG_E_CUDA;
     mark_end(P_PLAIN_EVAL, t0);
     phase_bytes[P_PLAIN_EVAL] += (double)ds->n * 8.0 * (double)(ds->d + ne);
-    launches += 2;
+    launches += 1;
     for (const auto& sb : subs) {
       const int32_t ns = sb.second - sb.first;
       if (ns <= 0) continue;
@@ -2037,11 +2013,12 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
         return RRG_E_OOM;
       }
       t0 = mark_begin();
-      RRG_CUDA(cudaEventRecord(fork_ev, stream));
+      const bool lone = runs.size() == 1;  // nothing to run beside it: no fork, no join
+      if (!lone) RRG_CUDA(cudaEventRecord(fork_ev, stream));
       int used = 0;
       for (const QrRun& r : runs) {
-        cudaStream_t s = side[used % kSide];
-        if (used < kSide) RRG_CUDA(cudaStreamWaitEvent(s, fork_ev, 0));
+        cudaStream_t s = lone ? stream : side[used % kSide];
+        if (!lone && used < kSide) RRG_CUDA(cudaStreamWaitEvent(s, fork_ev, 0));
         bool ok;
         if (!chunked) {
           ok = launch_plain_qr(r.wide, r.b1 - r.b0, sm_count, s, dev, dd, d_pcs, d_list, r.b0, F64, M, coefs, res,
@@ -2076,7 +2053,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
         }
         ++used;
       }
-      for (int i = 0; i < std::min(used, (int)kSide); ++i) {
+      for (int i = 0; !lone && i < std::min(used, (int)kSide); ++i) {
         RRG_CUDA(cudaEventRecord(join_ev[i], side[i]));
         RRG_CUDA(cudaStreamWaitEvent(stream, join_ev[i], 0));
       }
