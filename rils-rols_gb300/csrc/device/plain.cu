@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
                                                           const int32_t* list, int cand0, double* A, uint32_t* status,
                                                           ColStat* cst, EvalRows rows) {
   extern __shared__ double smem[];
+  after_previous();
   const int c = list ? list[cand0 + blockIdx.x] : cand0 + blockIdx.x;
   const rrg_cand cd = b.cands[c];
   if (rows.live && !rows.live[pc[c].a_col]) return;
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(256 * SEG, 4 / SEG) plain_resid_kernel(DevBatc
                                                                 const int32_t* list, int cand0, int n_cand,
                                                                 const double* A, const double* coefs, double* partial,
                                                                 const int32_t* colmap, const int32_t* dcount) {
+  after_previous();
   __shared__ double red[8], lane_acc[256];
   __shared__ fi_factor cs[kMaxK];
   __shared__ int kind[kMaxK];  // 0 skip, 1 free term, 2 bare factor, 3 scaled factor
@@ -398,7 +400,7 @@ __global__ void __launch_bounds__(256 * SEG, 4 / SEG) plain_resid_kernel(DevBatc
 
 bool launch_plain_resid(DevBatch b, const DevData& ds, const PlainCand* pc, const int32_t* list, int cand0, int n_cand,
                         const double* A, const double* coefs, double* partial, const int32_t* colmap,
-                        const int32_t* dcount, int sm_count, cudaStream_t st) {
+                        const int32_t* dcount, int sm_count, cudaStream_t st, bool chained) {
   if (n_cand <= 0) return true;
   const int64_t items = (int64_t)n_cand * ((ds.n + RR_CHUNK - 1) / RR_CHUNK);
   // four threads a lane while that gives every SM at most two such blocks and
@@ -407,8 +409,8 @@ bool launch_plain_resid(DevBatch b, const DevData& ds, const PlainCand* pc, cons
     plain_resid_kernel<4><<<(int)items, 1024, 0, st>>>(b, ds, pc, list, cand0, n_cand, A, coefs, partial, colmap,
                                                        dcount);
   else
-    plain_resid_kernel<1><<<(int)std::min<int64_t>(items, 16 * (int64_t)sm_count), 256, 0, st>>>(
-        b, ds, pc, list, cand0, n_cand, A, coefs, partial, colmap, dcount);
+    launch_next(chained, plain_resid_kernel<1>, dim3((unsigned)std::min<int64_t>(items, 16 * (int64_t)sm_count)), 256,
+                0, st, b, ds, pc, list, cand0, n_cand, A, coefs, partial, colmap, dcount);
   return launch_ok("residual");
 }
 
@@ -416,6 +418,7 @@ bool launch_plain_resid(DevBatch b, const DevData& ds, const PlainCand* pc, cons
 __global__ void finalize_kernel(DevBatch b, DevData ds, const int32_t* list, int cand0, int cand1,
                                 const double* partial, int nb, const double* coefs, rrg_result* res,
                                 uint32_t flags_or, const double* sse_direct, const int32_t* dcount) {
+  after_previous();
   const int i = cand0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cand1 || (dcount && i >= *dcount)) return;
   const int c = list ? list[i] : i;
@@ -704,6 +707,7 @@ __global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32
                                                          uint32_t* decided, const int32_t* dcount) {
   __shared__ double red[8][kGramE], g[kGramE];
   __shared__ int pad;
+  after_previous();
   if (dcount && (int)blockIdx.x >= *dcount) return;
   const int c = list[blockIdx.x];
   const PlainCand p = pc[c];
@@ -735,10 +739,10 @@ bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list
   // of 150 rows is launches and latency: with this, one launch to begin a table
   // instead of two and no fork to a side stream for one QR launch, 106 -> 91 us.
   if (nbx == 1) {
-    nan_settle_kernel<<<cnt, 256, 0, st>>>(b, list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad, coefs, res, decided,
-                                           dcount);
     *launches += 1;
-    return launch_ok("nan_settle");
+    return launch_next(true, nan_settle_kernel, dim3(cnt), 256, 0, st, b, list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad,
+                       coefs, res, decided, dcount) &&
+           launch_ok("nan_settle");
   }
   sentinel_classify_kernel<<<(cnt + 127) / 128, 128, 0, st>>>(b, list, cnt, pc, colmap, cs, ds.n, coefs, res, decided,
                                                               dcount);

@@ -59,19 +59,21 @@ __global__ void plain_eval_kernel(DevBatch b, DevData ds, const PlainCand* pc, c
 // column pc[c].a_col + j.
 // Column bucket of a QR launch for k + 1 columns (its widest sets the scratch).
 int plain_qr_bucket(int cols);
-// One block per candidate of the launch (the whole factorisation in one
+// chained: as launch_next.  One block per candidate of the launch (the whole factorisation in one
 // launch; QSUM order, the bits of launch_qr_chunked; qr_small.cu); max_cols
 // bounds k + 1.
 bool launch_plain_qr(int max_cols, int grid, int sm_count, cudaStream_t st, DevBatch b, DevData ds,
                      const PlainCand* pc, const int32_t* list, int cand0, const double* A, double* M, double* coefs,
-                     rrg_result* res, uint32_t* status, const int32_t* colmap);
+                     rrg_result* res, uint32_t* status, const int32_t* colmap,
+                     bool chained = false);
 // Squared residual of the rebuilt sum of the candidates list[cand0 .. cand0 +
 // n_cand) per chunk of RR_CHUNK rows: partial[c * chunks + chunk].  dcount (may
 // be NULL): list positions at or beyond *dcount do nothing (a list whose length
 // the device decided).
 bool launch_plain_resid(DevBatch b, const DevData& ds, const PlainCand* pc, const int32_t* list, int cand0, int n_cand,
                         const double* A, const double* coefs, double* partial, const int32_t* colmap,
-                        const int32_t* dcount, int sm_count, cudaStream_t st);
+                        const int32_t* dcount, int sm_count, cudaStream_t st,
+                        bool chained = false);
 // partial[c * nb + j]: per-candidate squared-residual partial sums; when
 // sse_direct is given and sse_direct[c] >= 0 (or NaN) it is the SSE itself.
 __global__ void finalize_kernel(DevBatch b, DevData ds, const int32_t* list, int cand0, int cand1,

@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(32 * W, kWarpsSm / W)
     qr_small_kernel(DevBatch b, DevData ds, const PlainCand* pc, const int32_t* list, int cand0, const double* A,
                     double* M, double* coefs, rrg_result* res, uint32_t* status, const int32_t* colmap, int mc) {
   constexpr int G = 8 / W;
+  after_previous();
   using Row = typename std::conditional<SMEM, int, int64_t>::type;  // a column in shared memory has few rows
   extern __shared__ double smem[];
   const int c = list ? list[cand0 + blockIdx.x] : cand0 + blockIdx.x;
@@ -297,20 +298,20 @@ __global__ void __launch_bounds__(32 * W, kWarpsSm / W)
 template <int W, bool SMEM>
 bool launch_w(size_t smem, int mc, int grid, cudaStream_t st, DevBatch b, DevData ds, const PlainCand* pc,
               const int32_t* list, int cand0, const double* A, double* M, double* coefs, rrg_result* res,
-              uint32_t* status, const int32_t* colmap) {
+              uint32_t* status, const int32_t* colmap, bool chained) {
   if (smem > 48 * 1024 && cudaFuncSetAttribute(qr_small_kernel<W, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)kSmemMax) != cudaSuccess)
     return false;
-  qr_small_kernel<W, SMEM>
-      <<<grid, 32 * W, smem, st>>>(b, ds, pc, list, cand0, A, M, coefs, res, status, colmap, mc);
-  return launch_ok("launch_plain_qr");
+  return launch_next(chained, qr_small_kernel<W, SMEM>, dim3(grid), 32 * W, smem, st, b, ds, pc, list, cand0, A, M, coefs, res,
+                     status, colmap, mc) &&
+         launch_ok("launch_plain_qr");
 }
 
 }  // namespace
 
 bool launch_plain_qr(int max_cols, int grid, int sm_count, cudaStream_t st, DevBatch b, DevData ds,
                      const PlainCand* pc, const int32_t* list, int cand0, const double* A, double* M, double* coefs,
-                     rrg_result* res, uint32_t* status, const int32_t* colmap) {
+                     rrg_result* res, uint32_t* status, const int32_t* colmap, bool chained) {
   if (grid <= 0) return true;
   // Working columns in shared memory where one block's fit.  Then as few warps
   // a candidate as still give every SM 8 warps, counted over the launch: warps
@@ -328,7 +329,8 @@ bool launch_plain_qr(int max_cols, int grid, int sm_count, cudaStream_t st, DevB
     W *= 2;
   }
   const size_t sm = bytes(W, in_smem);
-#define RRD_QR(W_, S_) launch_w<W_, S_>(sm, max_cols, grid, st, b, ds, pc, list, cand0, A, M, coefs, res, status, colmap)
+#define RRD_QR(W_, S_) \
+  launch_w<W_, S_>(sm, max_cols, grid, st, b, ds, pc, list, cand0, A, M, coefs, res, status, colmap, chained)
   if (!in_smem) return RRD_QR(8, false);
   switch (W) {
     case 1: return RRD_QR(1, true);

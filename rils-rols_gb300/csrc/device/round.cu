@@ -1925,8 +1925,8 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       const int64_t nr = rows.hi - rows.lo;
       const int64_t fill = std::min<int64_t>(((int64_t)wv * sm_count + nl - 1) / nl, (nr + 1023) / 1024);
       const int nb = (int)std::min<int64_t>(65535, std::max(eval_pieces(nr), fill));
-      plain_eval_kernel<<<dim3(nl, nb), 256, plain_eval_smem(), stream>>>(
-          fdev, dd, pk.at<const PlainCand>(d_ft64, o_fpc), nullptr, c0, F64, status, cst, rows);
+      launch_next(true, plain_eval_kernel, dim3(nl, nb), 256, plain_eval_smem(), stream, fdev, dd,
+                  pk.at<const PlainCand>(d_ft64, o_fpc), nullptr, c0, F64, status, cst, rows);
       ++launches;
     };
     const EvalRows every{0, ds->n, nullptr};
@@ -2022,7 +2022,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
         bool ok;
         if (!chunked) {
           ok = launch_plain_qr(r.wide, r.b1 - r.b0, sm_count, s, dev, dd, d_pcs, d_list, r.b0, F64, M, coefs, res,
-                               status, d_cmap);
+                               status, d_cmap, lone);
           ++launches;
         } else {
           QrJob jb{};
@@ -2060,12 +2060,12 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       mark_end(P_PLAIN_QR, t0);
       t0 = mark_begin();
       if (!launch_plain_resid(dev, dd, d_pcs, d_list, sb.first, ns, F64, coefs, partial, d_cmap, nullptr, sm_count,
-                              stream))
+                              stream, lone))
         return RRG_E_CUDA;
       mark_end(P_PLAIN_RESID, t0);
       t0 = mark_begin();
-      finalize_kernel<<<(ns + 127) / 128, 128, 0, stream>>>(dev, dd, d_list, sb.first, sb.second, partial, nb_res,
-                                                            coefs, res, flags_or, nullptr);
+      launch_next(true, finalize_kernel, dim3((ns + 127) / 128), 128, 0, stream, dev, dd, d_list, sb.first, sb.second,
+                  partial, nb_res, coefs, res, flags_or, nullptr, nullptr);
       mark_end(P_FINAL, t0);
       launches += 3;
     }
