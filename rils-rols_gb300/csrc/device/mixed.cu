@@ -113,6 +113,79 @@ __device__ double cert_fitness_bound(double sse, double E, double n_d, double ss
   return rl + rr;
 }
 
+constexpr int kSolveK = kMixedMaxM + 1;
+// shared memory of one warp's solve
+struct SolveSmem {
+  double ent[GramSize<kMixedMaxM>::E];
+  double G[kSolveK][kSolveK], L[kSolveK][kSolveK];
+  double b[kSolveK], d0[kSolveK], z[kSolveK], coef[kSolveK], root[kSolveK], t[2][kSolveK * kSolveK];
+  int32_t piv[kSolveK];
+};
+// One copy each of a quotient and a root: a lone candidate's solve is bound by
+// fetching its instructions.
+static __device__ __noinline__ double one_div(double a, double b) { return fi_div(a, b); }
+static __device__ __noinline__ double one_sqrt(double a) { return fi_sqrt(a); }
+// squared-norm ratio to the largest column below which the reference's
+// rank cut (eps^2 ~ 5e-32) cannot be ruled out
+constexpr double kCutAbs = 1e-24;
+
+// Symmetric pivoted Cholesky of the leading k x k of S.L, by one warp (pivot =
+// largest remaining diagonal, i.e. the largest remaining column norm of the
+// design, as column-pivoted QR picks).  A pivot is cut when it is small against
+// its own column's norm (the Gram sums cannot resolve it) or so small against
+// the largest column that the reference's QR, whose cut is at eps^2 of the
+// largest squared norm, may cut it; a badly scaled but independent column is
+// kept.  Returns the rank, and the smallest pivot against its column's norm.
+__device__ int warp_cholesky(SolveSmem& S, int k, double tol, double maxd, double& min_ratio) {
+  const int lane = threadIdx.x & 31;
+  if (lane < k) {
+    S.d0[lane] = S.L[lane][lane];
+    S.piv[lane] = lane;
+  }
+  __syncwarp();
+  min_ratio = 1.0;
+#pragma unroll 1
+  for (int s = 0; s < k; ++s) {
+    int p = s;
+#pragma unroll 1
+    for (int j = s + 1; j < k; ++j)
+      if (fi_lt(S.L[p][p], S.L[j][j])) p = j;
+    const double dp = S.L[p][p], dq = S.d0[S.piv[p]];
+    if (!(dp > tol * dq) || !(dp > kCutAbs * maxd)) return s;
+    __syncwarp();
+    if (p != s) {
+      if (lane < k) {
+        const double v = S.L[s][lane];
+        S.L[s][lane] = S.L[p][lane];
+        S.L[p][lane] = v;
+      }
+      __syncwarp();
+      if (lane < k) {
+        const double v = S.L[lane][s];
+        S.L[lane][s] = S.L[lane][p];
+        S.L[lane][p] = v;
+      }
+      if (lane == 0) {
+        const int32_t v = S.piv[s];
+        S.piv[s] = S.piv[p];
+        S.piv[p] = v;
+      }
+      __syncwarp();
+    }
+    min_ratio = fmin(min_ratio, one_div(dp, dq));
+    const double lss = one_sqrt(dp);
+    if (lane >= s && lane < k) S.L[lane][s] = lane == s ? lss : one_div(S.L[lane][s], lss);
+    __syncwarp();
+    const int r = k - s - 1;
+    for (int e = lane; e < r * r; e += 32) {
+      const int i = s + 1 + e / r, j = s + 1 + e % r;
+      if (j <= i) S.L[i][j] = S.L[j][i] = __fma_rn(-S.L[i][s], S.L[j][s], S.L[i][j]);
+    }
+    __syncwarp();
+  }
+  return k;
+}
+
 // One warp per candidate: its Gram entries are gathered from the round's
 // pair sums (FP64 totals of the double-float partials of the factor table);
 // tuned candidates get a symmetric-pivoted Cholesky solve with one
@@ -120,35 +193,37 @@ __device__ double cert_fitness_bound(double sse, double E, double n_d, double ss
 //     SSE = y'y - 2 c'b + c'Gc      (c: coefficients after the drop / snap rules)
 // when its bound  u * (y'y + 2|c|'|b| + |c|'|G||c|)  is below pass2_tol * SSE;
 // otherwise it is flagged for the residual pass.
+// The lanes share the work: entries, rows and bounds one or a few to a lane,
+// chains only where the order of a sum asks for one, quotients and roots on the
+// integer pipes (fp64_int.h).  One candidate of three factors: 62 us with one
+// lane doing all of it, 49 so, 30 with one copy each of quotient and root; eight
+// rounds at 1M rows, with the probe: 2.39 -> 2.01 ms.
 // Entry layout per candidate (mmax = kMixedMaxM): G_ij for i <= j < mmax,
 // then sum f_i, then sum f_i * y; pair index -1 reads 0.
 __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
-  __shared__ double red[4][GramSize<kMixedMaxM>::E];
+  __shared__ SolveSmem smem[4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int li = blockIdx.x * 4 + warp;
   if (li >= a.n_list) return;
+  SolveSmem& S = smem[warp];
   const int mmax = kMixedMaxM;
   const int Gn = mmax * (mmax + 1) / 2, E = Gn + 2 * mmax;
   const int32_t* po = a.pair_of + (size_t)li * E;
   for (int e = lane; e < E; e += 32) {
     const int32_t p = po[e];
-    red[warp][e] = p >= 0 ? a.psum[p] : (p <= -2 ? a.pself[-2 - (int64_t)p] : 0.0);
+    S.ent[e] = p >= 0 ? a.psum[p] : (p <= -2 ? a.pself[-2 - (int64_t)p] : 0.0);
   }
   __syncwarp();
-  if (lane != 0) return;
   const int c = a.list[li];
   const rrg_cand cd = a.b.cands[c];
-  const double* ent = red[warp];
+  const double* ent = S.ent;
   const double yy = a.ds.yy;
   // Relative accuracy of the double-float Gram sums with respect to the sums
   // of the absolute values of their terms: about 5u^2 per product and 3u^2
   // per double-float addition (u = 2^-24) over at most ~90 sequential
   // additions per sum, plus the FP64 sum of the chunk partials: about 4e-13.
   const double kU = 1e-12;
-  // squared-norm ratio to the largest column below which the reference's
-  // rank cut (eps^2 ~ 5e-32) cannot be ruled out
-  const double kCutAbs = 1e-24;
-  auto queue_fallback = [&](int why) {
+  auto queue_fallback = [&](int why) {  // lane 0
     const int slot = atomicAdd(a.fallback, 1);
     if (slot < a.fallback_cap) a.fallback[1 + slot] = c;
     if (a.reasons) atomicAdd(a.reasons + why, 1u);
@@ -161,6 +236,7 @@ __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
   const double safety = pr.all_rows ? 1.5 : 8.0;
   auto ferr = [&](int i) { return safety * (double)pr.dev[i] + 1e-12 * (double)pr.rms[i]; };
   if (cd.mode != RRG_TUNED) {
+    if (lane != 0) return;
     // yp = f: SSE = y'y - 2 f'y + f'f
     const double ff = ent[0], fs = ent[Gn], fy = ent[Gn + mmax];
     const bool nan = ff != ff || fs != fs || fy != fy;
@@ -168,6 +244,7 @@ __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
     uint32_t confirmed = pr.nan64;
     if (nan && !(confirmed & 1u) && a.nanrow && a.nanrow[c] >= 0 && a.nanrow[c] < a.ds.n) {
       double f64[kMixedMaxM];
+#pragma unroll 1
       for (int i = 0; i < kMixedMaxM; ++i) f64[i] = 0.0;
       if (probe_eval64<kMixedMaxM>(a.b.code + cd.code_offset, cd.code_len, a.b.consts, a.ds, a.nanrow[c], f64) &&
           f64[0] != f64[0])
@@ -202,47 +279,48 @@ __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
     return;
   }
   const int m = cd.n_factors, k = m + 1;
-  double G[kMixedMaxM + 1][kMixedMaxM + 1], L[kMixedMaxM + 1][kMixedMaxM + 1], bvec[kMixedMaxM + 1];
-  int e = 0;
-  for (int i = 0; i < mmax; ++i)
-    for (int j = i; j < mmax; ++j, ++e)
-      if (i < m && j < m) G[i][j] = G[j][i] = ent[e];
-  for (int i = 0; i < m; ++i) {
-    G[i][m] = G[m][i] = ent[Gn + i];
-    bvec[i] = ent[Gn + mmax + i];
+  for (int e = lane; e < k * k; e += 32) {
+    const int i = e / k, j = e % k, lo = i < j ? i : j, hi = i < j ? j : i;
+    S.G[i][j] = lo == m ? (double)a.ds.n
+                        : hi == m ? ent[Gn + lo] : ent[lo * mmax - lo * (lo - 1) / 2 + hi - lo];
   }
-  G[m][m] = (double)a.ds.n;
-  bvec[m] = a.ds.ysum;
+  if (lane < k) S.b[lane] = lane < m ? ent[Gn + mmax + lane] : a.ds.ysum;
+  __syncwarp();
   // Non-finite sums: NaN (a domain error in some factor) gives NaN
   // coefficients and so the fitness sentinel, as the reference's QR does;
   // +-inf without NaN (FP32 exponent overflow) is re-solved by the FP64 path.
-  bool has_nan = false, has_inf = false;
-  for (int i = 0; i < k; ++i) {
-    for (int j = 0; j < k; ++j) {
-      has_nan |= G[i][j] != G[i][j];
-      has_inf |= fabs(G[i][j]) > DBL_MAX;
-    }
-    has_nan |= bvec[i] != bvec[i];
-    has_inf |= fabs(bvec[i]) > DBL_MAX;
+  bool nan_l = false, inf_l = false;
+  for (int e = lane; e < k * k + k; e += 32) {
+    const double v = e < k * k ? S.G[e / k][e % k] : S.b[e - k * k];
+    nan_l |= v != v;
+    inf_l |= fabs(v) > DBL_MAX;
   }
+  const bool has_nan = __any_sync(0xffffffffu, nan_l), has_inf = __any_sync(0xffffffffu, inf_l);
   // factors whose own sums are NaN (a domain error on some row); the cross
   // sums of a NaN factor are NaN for every partner, so only the diagonal,
   // the factor sum and the factor-y sum identify it
-  uint32_t nanmask = 0, infmask = 0;
-  for (int i = 0; i < m; ++i) {
-    const double d = G[i][i], sf = G[i][m], sy = bvec[i];
-    if (d != d || sf != sf || sy != sy) nanmask |= 1u << i;
-    else if (fabs(d) > DBL_MAX || fabs(sf) > DBL_MAX || fabs(sy) > DBL_MAX) infmask |= 1u << i;
+  bool fnan_l = false, finf_l = false;
+  if (lane < m) {
+    const double d = S.G[lane][lane], sf = S.G[lane][m], sy = S.b[lane];
+    fnan_l = d != d || sf != sf || sy != sy;
+    finf_l = !fnan_l && (fabs(d) > DBL_MAX || fabs(sf) > DBL_MAX || fabs(sy) > DBL_MAX);
   }
-  const uint32_t fullmask = (m >= 32) ? 0xffffffffu : ((1u << m) - 1u);
+  uint32_t nanmask = __ballot_sync(0xffffffffu, fnan_l);
+  const uint32_t infmask = __ballot_sync(0xffffffffu, finf_l);
+  const uint32_t fullmask = (1u << m) - 1u;  // m <= kMixedMaxM
   uint32_t confirmed = pr.nan64;
   if ((nanmask & ~confirmed) && a.nanrow && a.nanrow[c] >= 0 && a.nanrow[c] < a.ds.n) {
     // table NaN outside the probe rows: evaluate the first such row in FP64
-    double f64[kMixedMaxM];
-    for (int i = 0; i < kMixedMaxM; ++i) f64[i] = 0.0;
-    if (probe_eval64<kMixedMaxM>(a.b.code + cd.code_offset, cd.code_len, a.b.consts, a.ds, a.nanrow[c], f64))
-      for (int i = 0; i < m; ++i)
-        if (f64[i] != f64[i]) confirmed |= 1u << i;
+    if (lane == 0) {
+      double f64[kMixedMaxM];
+#pragma unroll 1
+      for (int i = 0; i < kMixedMaxM; ++i) f64[i] = 0.0;
+      if (probe_eval64<kMixedMaxM>(a.b.code + cd.code_offset, cd.code_len, a.b.consts, a.ds, a.nanrow[c], f64))
+#pragma unroll 1
+        for (int i = 0; i < m; ++i)
+          if (f64[i] != f64[i]) confirmed |= 1u << i;
+    }
+    confirmed = __shfl_sync(0xffffffffu, confirmed, 0);
   }
   nanmask |= pr.nan64 & fullmask;
   if (pr.bad32 || pr.inf64 || infmask || (nanmask & ~confirmed) ||
@@ -250,149 +328,96 @@ __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
     // the table broke down where FP64 did not, FP64 overflow, FP32 exponent
     // overflow, a table NaN the FP64 probe does not confirm, or a non-finite sum outside
     // the factor columns: the FP64 path scores it
-    queue_fallback(pr.bad32 ? FB_PROBE_NONFINITE
-                            : (pr.inf64 ? FB_FP64_INF : (infmask ? FB_FP32_OVERFLOW : FB_OTHER_NAN)));
-    a.sse1[c] = -1.0;
-    a.pass2[c] = 0;
-    a.res[c].rank = 0;
+    if (lane == 0) {
+      queue_fallback(pr.bad32 ? FB_PROBE_NONFINITE
+                              : (pr.inf64 ? FB_FP64_INF : (infmask ? FB_FP32_OVERFLOW : FB_OTHER_NAN)));
+      a.sse1[c] = -1.0;
+      a.pass2[c] = 0;
+      a.res[c].rank = 0;
+    }
     return;
   }
+  double* out = a.coefs + cd.coef_offset;
   if (nanmask) {
     // A NaN factor column makes the reference's QR return NaN coefficients
     // (the sentinel) unless a rank cut among the other columns happens before
     // the QR reaches it.  Full, well-conditioned rank of the other columns
-    // rules that out; otherwise the FP64 path decides.
-    int idx[kMixedMaxM + 1], kk2 = 0;
-    for (int i = 0; i < k; ++i)
-      if (i == m || !((nanmask >> i) & 1u)) idx[kk2++] = i;
-    double H[kMixedMaxM + 1][kMixedMaxM + 1], hd0[kMixedMaxM + 1];
-    int hp[kMixedMaxM + 1];
-    for (int i = 0; i < kk2; ++i) {
-      for (int j = 0; j < kk2; ++j) H[i][j] = G[idx[i]][idx[j]];
-      hd0[i] = H[i][i];
-      hp[i] = i;
+    // rules that out (well away from a cut: 1e-6 of the column's own norm);
+    // otherwise the FP64 path decides.
+    const uint32_t use = (fullmask & ~nanmask) | (1u << m);
+    const int kk = __popc(use);
+    if (lane < kk) S.piv[lane] = __fns(use, 0, lane + 1);
+    __syncwarp();
+    for (int e = lane; e < kk * kk; e += 32) S.L[e / kk][e % kk] = S.G[S.piv[e / kk]][S.piv[e % kk]];
+    __syncwarp();
+    double hmax = 0.0, mr;
+#pragma unroll 1
+    for (int i = 0; i < kk; ++i) hmax = fmax(hmax, S.L[i][i]);
+    const bool full = warp_cholesky(S, kk, 1e-6, hmax, mr) == kk;
+    if (lane < k) out[lane] = __longlong_as_double(0x7ff8000000000000ll);
+    if (lane == 0) {
+      if (!full) queue_fallback(FB_NAN_RANK);
+      a.sse1[c] = full ? __longlong_as_double(0x7ff8000000000000ll) : -1.0;
+      a.pass2[c] = 0;
+      a.res[c].rank = 0;
     }
-    bool full = true;
-    double hmax = 0.0;
-    for (int i = 0; i < kk2; ++i) hmax = fmax(hmax, H[i][i]);
-    for (int s2 = 0; s2 < kk2 && full; ++s2) {
-      int p = s2;
-      for (int j = s2 + 1; j < kk2; ++j)
-        if (H[j][j] > H[p][p]) p = j;
-      // well away from a cut: relative to the column's own norm and to the largest
-      if (!(H[p][p] > 1e-6 * hd0[hp[p]]) || !(H[p][p] > kCutAbs * hmax)) {
-        full = false;
-        break;
-      }
-      if (p != s2) {
-        for (int j = 0; j < kk2; ++j) { const double t2 = H[s2][j]; H[s2][j] = H[p][j]; H[p][j] = t2; }
-        for (int j = 0; j < kk2; ++j) { const double t2 = H[j][s2]; H[j][s2] = H[j][p]; H[j][p] = t2; }
-        const int t3 = hp[s2]; hp[s2] = hp[p]; hp[p] = t3;
-      }
-      const double l = sqrt(H[s2][s2]);
-      for (int i = s2 + 1; i < kk2; ++i) H[i][s2] /= l;
-      for (int i = s2 + 1; i < kk2; ++i)
-        for (int j = s2 + 1; j <= i; ++j) {
-          H[i][j] -= H[i][s2] * H[j][s2];
-          H[j][i] = H[i][j];
-        }
-    }
-    double* out = a.coefs + cd.coef_offset;
-    for (int i = 0; i < k; ++i) out[i] = __longlong_as_double(0x7ff8000000000000ll);
-    if (full) {
-      a.sse1[c] = __longlong_as_double(0x7ff8000000000000ll);
-    } else {
-      queue_fallback(FB_NAN_RANK);
-      a.sse1[c] = -1.0;
-    }
-    a.pass2[c] = 0;
-    a.res[c].rank = 0;
     return;
   }
-  // symmetric pivoted Cholesky (pivot = largest remaining diagonal, i.e. the
-  // largest remaining column norm of the design, as column-pivoted QR picks)
-  int piv[kMixedMaxM + 1];
-  double d0[kMixedMaxM + 1];
-  double maxd = 0.0;
-  for (int i = 0; i < k; ++i) {
-    piv[i] = i;
-    d0[i] = G[i][i];
-    if (G[i][i] > maxd) maxd = G[i][i];
-    for (int j = 0; j < k; ++j) L[i][j] = G[i][j];
+  // (every sum is finite from here on)
+  for (int e = lane; e < k * k; e += 32) S.L[e / k][e % k] = S.G[e / k][e % k];
+  if (lane < k) {
+    S.root[lane] = one_sqrt(fabs(S.G[lane][lane]));
+    S.coef[lane] = 0.0;
   }
-  int rank = k;
-  double min_ratio = 1.0;
-  const bool finite = !has_nan && !has_inf;
-  for (int s2 = 0; s2 < k && finite; ++s2) {
-    int p = s2;
-    for (int j = s2 + 1; j < k; ++j)
-      if (L[j][j] > L[p][p]) p = j;
-    const double dp = L[p][p];
-    // A pivot is cut when it is small against its own column's norm (the
-    // Gram sums cannot resolve it) or so small against the largest column
-    // that the reference's QR, whose cut is at eps^2 of the largest squared
-    // norm, may cut it.  A badly scaled but independent column is kept.
-    if (!(dp > a.rank_tol * d0[piv[p]]) || !(dp > kCutAbs * maxd)) {
-      rank = s2;
-      break;
+  __syncwarp();
+  double maxd = 0.0, min_ratio;
+#pragma unroll 1
+  for (int i = 0; i < k; ++i) maxd = fmax(maxd, S.G[i][i]);
+  const int rank = warp_cholesky(S, k, a.rank_tol, maxd, min_ratio);
+  // solve L L^T z = P b on the leading `rank` block, then one refinement step
+  const int pl = lane < rank ? S.piv[lane] : 0;
+  double rhs = lane < rank ? S.b[pl] : 0.0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2 && rank > 0; ++pass) {
+    double v = rhs;  // forward: lane i's row, its terms in the order of the columns
+#pragma unroll 1
+    for (int j = 0; j < rank; ++j) {
+      if (lane == j) v = one_div(v, S.L[j][j]);
+      const double zj = __shfl_sync(0xffffffffu, v, j);
+      if (lane > j && lane < rank) v = __fma_rn(-S.L[lane][j], zj, v);
     }
-    if (p != s2) {
-      for (int j = 0; j < k; ++j) { const double t2 = L[s2][j]; L[s2][j] = L[p][j]; L[p][j] = t2; }
-      for (int j = 0; j < k; ++j) { const double t2 = L[j][s2]; L[j][s2] = L[j][p]; L[j][p] = t2; }
-      const int t3 = piv[s2]; piv[s2] = piv[p]; piv[p] = t3;
+    if (lane < rank) S.z[lane] = v;
+    __syncwarp();
+#pragma unroll 1
+    for (int i = rank - 1; i >= 0; --i) {
+      double w = S.z[i];
+#pragma unroll 1
+      for (int j = i + 1; j < rank; ++j) w = __fma_rn(-S.L[j][i], S.z[j], w);
+      w = one_div(w, S.L[i][i]);
+      __syncwarp();
+      if (lane == 0) S.z[i] = w;
+      __syncwarp();
     }
-    const double ratio = dp / d0[piv[s2]];
-    if (ratio < min_ratio) min_ratio = ratio;
-    const double lss = sqrt(dp);
-    L[s2][s2] = lss;
-    for (int i = s2 + 1; i < k; ++i) L[i][s2] = L[i][s2] / lss;
-    for (int i = s2 + 1; i < k; ++i)
-      for (int j = s2 + 1; j <= i; ++j) {
-        L[i][j] = L[i][j] - L[i][s2] * L[j][s2];
-        L[j][i] = L[i][j];
-      }
-  }
-  double coef[kMixedMaxM + 1];
-  for (int i = 0; i < k; ++i) coef[i] = 0.0;
-  uint32_t flags = 0;
-  if (!finite) {
-    for (int i = 0; i < k; ++i) coef[i] = __longlong_as_double(0x7ff8000000000000ll);
-    rank = 0;
-  } else if (rank > 0) {
-    // solve L L^T z = P b on the leading `rank` block, then one refinement step
-    double z[kMixedMaxM + 1], rhs[kMixedMaxM + 1];
-    for (int i = 0; i < rank; ++i) rhs[i] = bvec[piv[i]];
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int i = 0; i < rank; ++i) {
-        double v = rhs[i];
-        for (int j = 0; j < i; ++j) v -= L[i][j] * z[j];
-        z[i] = v / L[i][i];
-      }
-      for (int i = rank - 1; i >= 0; --i) {
-        double v = z[i];
-        for (int j = i + 1; j < rank; ++j) v -= L[j][i] * z[j];
-        z[i] = v / L[i][i];
-      }
-      for (int i = 0; i < rank; ++i) coef[piv[i]] += z[i];
-      if (pass == 0) {
-        for (int i = 0; i < rank; ++i) {
-          const int pi = piv[i];
-          double v = bvec[pi];
-          for (int j = 0; j < k; ++j) v -= G[pi][j] * coef[j];
-          rhs[i] = v;
-        }
-      }
+    if (lane < rank) S.coef[pl] = S.coef[pl] + S.z[lane];
+    __syncwarp();
+    if (pass == 0 && lane < rank) {
+      double w = S.b[pl];
+#pragma unroll 1
+      for (int j = 0; j < k; ++j) w = __fma_rn(-S.G[pl][j], S.coef[j], w);
+      rhs = w;
     }
   }
-  if (rank < k) flags |= RRG_F_RANK_DEFICIENT;
+  const uint32_t flags = rank < k ? RRG_F_RANK_DEFICIENT : 0u;
   // Decisions the FP64 path must take itself: a rank cut (the reference's
   // rule works at eps^2 of the column norms), ill-conditioning, and
   // coefficients inside the ambiguity band of the drop (|c| < 1e-12) and
   // snap (|c - 1| < 1e-12) rules of the rebuilt tree.
   int why = -1;
-  if (!finite) why = FB_OTHER_NAN;
-  else if (rank < k && a.certify) why = FB_RANK;
+  if (rank < k && a.certify) why = FB_RANK;
   else if (rank == k && min_ratio < a.fallback_tol) why = FB_ILL_COND;
+  const double ci = lane < k ? S.coef[lane] : 0.0;
+  const double fe = lane < m ? ferr(lane) : 0.0;
+  const double ryy = one_sqrt(yy);
   if (why < 0 && a.certify) {
     // Coefficient error of the Gram solve: with relative errors u of the
     // Gram entries (the sums, kU, and the table's evaluation, ferr / rms of
@@ -401,61 +426,71 @@ __global__ void __launch_bounds__(128) mixed_solve_kernel(SolveArgs a) {
     //   |dc_i| <= u (|y| + sum_j |c_j| |f_j|) sqrt(k) / (lam |f_i|),  lam = min_ratio / k.
     // The drop (|c| < 1e-12) and snap (|c - 1| < 1e-12) rules of the rebuilt
     // tree are left to the FP64 path when c lies within 8 |dc_i| of them.
-    double u = kU, M = sqrt(yy);
-    for (int i = 0; i < k; ++i) {
-      M += fabs(coef[i]) * sqrt(fabs(G[i][i]));
-      if (i < m) u = fmax(u, ferr(i) / fmax((double)pr.rms[i], 1e-300));
+    double M = ryy;
+#pragma unroll 1
+    for (int i = 0; i < k; ++i) M = __fma_rn(fabs(S.coef[i]), S.root[i], M);
+    double u = lane < m ? fmax(kU, one_div(fe, fmax((double)pr.rms[lane], 1e-300))) : kU;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) u = fmax(u, __shfl_xor_sync(0xffffffffu, u, o));
+    const double lam = one_div(fmax(min_ratio, 1e-300), (double)k);
+    bool snap = false, drop = false;
+    if (lane < k) {
+      const double dc = one_div(8.0 * u * M * one_sqrt((double)k), lam * fmax(S.root[lane], 1e-300));
+      snap = lane < m && !(fabs(fabs(ci - 1.0) - kEps12) > dc);
+      drop = !snap && !(fabs(fabs(ci) - kEps12) > dc);
     }
-    const double lam = fmax(min_ratio, 1e-300) / k;
-    for (int i = 0; i < k && why < 0; ++i) {
-      const double ci = coef[i];
-      const double dc = 8.0 * u * M * sqrt((double)k) / (lam * fmax(sqrt(fabs(G[i][i])), 1e-300));
-      if (i < m && !(fabs(fabs(ci - 1.0) - kEps12) > dc)) why = FB_SNAP;
-      else if (!(fabs(fabs(ci) - kEps12) > dc)) why = FB_DROP;
-    }
+    const uint32_t sm = __ballot_sync(0xffffffffu, snap), any = sm | __ballot_sync(0xffffffffu, drop);
+    if (any) why = (sm >> (__ffs(any) - 1)) & 1u ? FB_SNAP : FB_DROP;
   }
-  double* out = a.coefs + cd.coef_offset;
-  MixedTerm& tm = a.terms[c];
-  double ceff[kMixedMaxM + 1];
+  const int kind = fabs(ci) < kEps12 ? 0 : (lane == m ? 1 : (fabs(ci - 1) < kEps12 ? 2 : 3));
+  const double ceff = kind == 0 ? 0.0 : (kind == 2 ? 1.0 : ci);
+  if (lane < k) {
+    MixedTerm& tm = a.terms[c];
+    out[lane] = ci;
+    tm.hi[lane] = (float)ci;
+    tm.lo[lane] = (float)(ci - (double)(float)ci);
+    tm.kind[lane] = (int8_t)kind;
+    S.z[lane] = ceff;
+  }
+  __syncwarp();
+  // mag bounds the sums of |terms| behind every entry used (Cauchy-Schwarz:
+  // sum |f_i f_j| <= sqrt(G_ii G_jj), sum |f_i y| <= sqrt(G_ii y'y))
+  for (int e = lane; e < k * k; e += 32) {
+    const double cc = S.z[e / k] * S.z[e % k];
+    S.t[0][e] = cc;
+    S.t[1][e] = fabs(cc) * S.root[e / k];
+  }
+  __syncwarp();
+  if (lane > 1) return;
+  // lane 0: y'y - 2 c'b + c'Gc; lane 1: mag
+  double lin = 0.0, quad = 0.0, mag = yy;
+#pragma unroll 1
   for (int i = 0; i < k; ++i) {
-    out[i] = coef[i];
-    const double ci = coef[i];
-    tm.hi[i] = (float)ci;
-    tm.lo[i] = (float)(ci - (double)tm.hi[i]);
-    const int kind = fabs(ci) < kEps12 ? 0 : (i == m ? 1 : (fabs(ci - 1) < kEps12 ? 2 : 3));
-    tm.kind[i] = (int8_t)kind;
-    ceff[i] = kind == 0 ? 0.0 : (kind == 2 ? 1.0 : ci);
+    if (lane == 0) {
+      lin = __fma_rn(S.z[i], S.b[i], lin);
+#pragma unroll 1
+      for (int j = 0; j < k; ++j) quad = __fma_rn(S.t[0][i * k + j], S.G[i][j], quad);
+    } else {
+      mag = __fma_rn(2.0 * fabs(S.z[i]) * S.root[i], ryy, mag);
+#pragma unroll 1
+      for (int j = 0; j < k; ++j) mag = __fma_rn(S.t[1][i * k + j], S.root[j], mag);
+    }
   }
-  double sse;
+  mag = __shfl_sync(0x3u, mag, 1);
+  double err = 0.0;  // per-row error of the rebuilt sum
+#pragma unroll 1
+  for (int i = 0; i < m; ++i) err = __fma_rn(fabs(S.z[i]), ferr(i), err);
+  if (lane != 0) return;
+  double sse = yy - 2.0 * lin + quad;
   uint8_t p2 = 0;
-  if (has_nan || !finite) {
-    sse = has_nan ? __longlong_as_double(0x7ff8000000000000ll) : -1.0;
-  } else {
-    // mag bounds the sums of |terms| behind every entry used (Cauchy-Schwarz:
-    // sum |f_i f_j| <= sqrt(G_ii G_jj), sum |f_i y| <= sqrt(G_ii y'y))
-    double lin = 0.0, quad = 0.0, mag = yy;
-    for (int i = 0; i < k; ++i) {
-      const double si = sqrt(fabs(G[i][i]));
-      lin += ceff[i] * bvec[i];
-      mag += 2.0 * fabs(ceff[i]) * si * sqrt(yy);
-      for (int j = 0; j < k; ++j) {
-        quad += ceff[i] * ceff[j] * G[i][j];
-        mag += fabs(ceff[i] * ceff[j]) * si * sqrt(fabs(G[j][j]));
-      }
-    }
-    sse = yy - 2.0 * lin + quad;
-    double E = 0.0;
-    for (int i = 0; i < m; ++i) E += fabs(ceff[i]) * ferr(i);
-    if (why < 0 && !(sse > 0.0 && kU * mag <= a.pass2_tol * sse)) {
-      // the residual pass gives the SSE; certified rounds check it after
-      p2 = 1;
-      if (a.certify) a.cert_e[c] = E;
-    } else if (why < 0 && a.certify && cert_bound(sse, E) > a.cert_tol) {
-      why = FB_CERT;
-    }
+  if (why < 0 && !(sse > 0.0 && kU * mag <= a.pass2_tol * sse)) {
+    // the residual pass gives the SSE; certified rounds check it after
+    p2 = 1;
+    if (a.certify) a.cert_e[c] = err;
+  } else if (why < 0 && a.certify && cert_bound(sse, err) > a.cert_tol) {
+    why = FB_CERT;
   }
-  const bool fallback = why >= 0;
-  if (fallback) {
+  if (why >= 0) {
     queue_fallback(why);
     p2 = 0;
     sse = -1.0;

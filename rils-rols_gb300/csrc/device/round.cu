@@ -903,7 +903,10 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   // the blocks to the groups, so these are small (8192 random trees at 100k
   // rows, 15 levels: 7.9 ms of evaluation with groups of 64, 6.5 with 4)
   std::vector<GroupSet> gsets(ngv + (two_parts ? 1 : 0));
-  for (int v = 0; v < ngv; ++v) build_groups(std::min(gvals[v], kFacGroupMax), gsets[v]);
+  // no larger than leaves every SM four blocks (a lone candidate of three
+  // factors at 50k rows: 42 us in one group, 24 in two)
+  const int gcap = (int)std::min<int64_t>(kFacGroupMax, std::max<int64_t>(1, (int64_t)ne * n_chunks / (4 * sm_count)));
+  for (int v = 0; v < ngv; ++v) build_groups(std::min(gvals[v], gcap), gsets[v]);
   if (two_parts) build_groups(kFirstGroup, gsets[ngv]);
   const size_t n_slots = (size_t)std::max<int64_t>(1, cp.arena);
   if (!d_F.grow_keep(col_bytes * n_slots, d_F.cap) ||
