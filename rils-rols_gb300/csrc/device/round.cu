@@ -917,9 +917,22 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     rrc::set_error("mixed round: factor table allocation failed");
     return RRG_E_OOM;
   }
+  // probe programs: the factors evaluated in this sub-round (their records
+  // go to their slots)
+  std::vector<uint32_t> pcode;
+  std::vector<int2> pmeta;
+  std::vector<int32_t> pslot;
+  for (int32_t l : mprog) {
+    pmeta.push_back(make_int2((int)pcode.size(), lmeta[l].y));
+    pcode.insert(pcode.end(), lcode.begin() + lmeta[l].x, lcode.begin() + lmeta[l].x + lmeta[l].y);
+    pslot.push_back(fslot[l]);
+  }
   // the table programs go up first and the evaluator starts; the host builds
   // the pair map while it runs
   Packer pkt;
+  const size_t o_code = pkt.add(pcode.data(), sizeof(uint32_t) * std::max<size_t>(1, pcode.size()));
+  const size_t o_meta = pkt.add(pmeta.data(), sizeof(int2) * std::max<size_t>(1, pmeta.size()));
+  const size_t o_pslot = pkt.add(pslot.data(), sizeof(int32_t) * std::max<size_t>(1, pslot.size()));
   const size_t o_tcode = pkt.add(tp.code.data(), sizeof(uint32_t) * tp.code.size());
   const size_t o_ecode = pkt.add(ep.code.data(), sizeof(uint32_t) * std::max<size_t>(1, ep.code.size()));
   const size_t o_emeta = pkt.add(ep.meta.data(), sizeof(int2) * std::max<size_t>(1, ep.meta.size()));
@@ -1021,6 +1034,19 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     return eval_rows(gsets[ngv], false, 0, q_first, nullptr) && launch_live_columns(la, stream) &&
            eval_rows(gs, stage, q_first, n_chunks, la.live);
   };
+  // The probe needs nothing of the table and runs beside the evaluation (a lone
+  // candidate at 50k rows 137 -> 117 us, eight rounds at 1M rows 91.0 -> 90.0 ms;
+  // rounds that fill the GPU take the same time as one after the other).  After
+  // the trials, which time the evaluation alone.
+  auto probe = [&] {
+    return cudaEventRecord(fork_ev, stream) == cudaSuccess && cudaStreamWaitEvent(side[1], fork_ev, 0) == cudaSuccess &&
+           launch_fac_probe(pkt.at<const uint32_t>(d_ftp, o_code), pkt.at<const int2>(d_ftp, o_meta),
+                            (int32_t)mprog.size(), dev.consts, dev.consts32, dev.consts32lo, dd, cprobe, side[1],
+                            pkt.at<const int32_t>(d_ftp, o_pslot)) &&
+           cudaEventRecord(join_ev[1], side[1]) == cudaSuccess;
+  };
+  const bool trial = gtrial || (strial && !capturing);
+  if (!trial && !probe()) return RRG_E_CUDA;
   int gbest = 0;  // the group set in use
   if (gtrial) {
     // the first round of this row class: every group size timed on the
@@ -1052,6 +1078,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   } else if (!gtrial && !eval_all(gsets[0], stage_pick && stage_ok)) {
     return RRG_E_CUDA;
   }
+  if (trial && !probe()) return RRG_E_CUDA;
   // Pair map: self pairs by slot (entries -2 - p into the slots' self
   // sums); cross pairs oriented so that `a` is the rarer factor (its
   // partners are then the widely shared ones, hot in L2) and kept across
@@ -1177,20 +1204,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     rrc::set_error("mixed round: factor table allocation failed");
     return RRG_E_OOM;
   }
-  // probe programs: the factors evaluated in this sub-round (their records
-  // go to their slots)
-  std::vector<uint32_t> pcode;
-  std::vector<int2> pmeta;
-  std::vector<int32_t> pslot;
-  for (int32_t l : mprog) {
-    pmeta.push_back(make_int2((int)pcode.size(), lmeta[l].y));
-    pcode.insert(pcode.end(), lcode.begin() + lmeta[l].x, lcode.begin() + lmeta[l].x + lmeta[l].y);
-    pslot.push_back(fslot[l]);
-  }
   Packer pk;
-  const size_t o_code = pk.add(pcode.data(), sizeof(uint32_t) * std::max<size_t>(1, pcode.size()));
-  const size_t o_meta = pk.add(pmeta.data(), sizeof(int2) * std::max<size_t>(1, pmeta.size()));
-  const size_t o_pslot = pk.add(pslot.data(), sizeof(int32_t) * std::max<size_t>(1, pslot.size()));
   const size_t o_ccol = pk.add(cand_col.data(), sizeof(int32_t) * cand_col.size());
   const size_t o_cslot = pk.add(cand_slot.data(), sizeof(int32_t) * cand_slot.size());
   std::vector<size_t> o_units(npv);
@@ -1203,8 +1217,6 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   const size_t o_list2 = pk.add(nullptr, sizeof(int32_t) * cnt);  // filled after the solve
   pst = pk.send(h_ft, d_ft, stream, round_seq);
   if (pst != RRG_OK) return pst;
-  const uint32_t* d_code = pk.at<const uint32_t>(d_ft, o_code);
-  const int2* d_meta = pk.at<const int2>(d_ft, o_meta);
   const int32_t* d_list = pk.at<const int32_t>(d_ft, o_list);
   const int32_t* d_cfac = pk.at<const int32_t>(d_ft, o_cfac);
   int32_t* d_list2 = pk.at<int32_t>(d_ft, o_list2);
@@ -1252,11 +1264,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   mark_end(P_PAIRS, t0);
   phase_bytes[P_PAIRS] += (double)ds->n * 8.0 * (double)nfl;
   t0 = mark_begin();
-  if (!launch_pair_reduce(Pself, n_self, n_chunks, 0, n_self, cself, stream, d_ewcol) ||
-      !launch_pair_reduce(Pcross, n_miss, n_super, 0, n_miss, psum, stream, nullptr,
-                          pk.at<const int32_t>(d_ft, o_omap)) ||
-      !launch_fac_probe(d_code, d_meta, (int32_t)mprog.size(), dev.consts, dev.consts32, dev.consts32lo, dd, cprobe,
-                        stream, pk.at<const int32_t>(d_ft, o_pslot)) ||
+  RRG_CUDA(cudaStreamWaitEvent(stream, join_ev[1], 0));  // the probe
+  if (!launch_pair_reduce({Pself, n_self, n_chunks, cself, d_ewcol},
+                          {Pcross, n_miss, n_super, psum, pk.at<const int32_t>(d_ft, o_omap)}, stream) ||
       !launch_cand_probe(dev.cands, d_list, cnt, d_cfac, nullptr, cprobe, fnan,
                          static_cast<ProbeOut*>(d_probe.ptr), static_cast<int64_t*>(d_nanrow.ptr), stream)) {
     cuda_ok(cudaGetLastError(), "mixed round launch");
@@ -1291,7 +1301,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     return RRG_E_CUDA;
   }
   mark_end(P_SOLVE, t0);
-  launches += 7;
+  launches += 6;
   if (async && cnt <= 65535) {
     // ------------------------------------------------------------------
     // Second half decided on the device: no read-back before the results.
