@@ -537,16 +537,6 @@ __device__ __forceinline__ int classify_candidate(const DevBatch& b, int c, cons
   return any_nan && nf + 1 <= kGramCols ? 2 : 0;
 }
 
-__global__ void sentinel_classify_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc,
-                                         const int32_t* colmap, const ColStat* cs, int64_t rows, double* coefs,
-                                         rrg_result* res, uint32_t* decided, const int32_t* dcount) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt || (dcount && i >= *dcount)) return;
-  const int c = list[i];
-  const int pad = classify_candidate(b, c, pc[c], colmap, cs, rows, coefs, res, decided);
-  if (pad) pc[c].pad = pad;
-}
-
 // A NaN column at position q >= 1, column 0 finite, no infinite norm, every
 // tail non-trivial: step 0 pivots on a finite column (NaN norms never win the
 // '>' scan unless they head the remaining columns) with tau != 0, which turns
@@ -572,11 +562,12 @@ __device__ __forceinline__ int gram_finite_cols(const PlainCand& p, const int32_
   return nf;
 }
 
-// The Gram entries of the candidate's finite columns over rows [r0, r1), by a
-// block of 256 threads, into out (K columns: the leading K (K + 1) / 2 used by
-// the factorisation are formed, the others are 0).
+// The Gram entries of the candidate's finite columns over `steps` runs of 256
+// rows, run i from row_of(i) (rows at or beyond `end` are left out), by a block
+// of 256 threads, into out.
+template <class RowOf>
 __device__ __forceinline__ void gram_block(const PlainCand& p, const int32_t* colmap, const ColStat* cs,
-                                           const double* T, int64_t n_pad, int64_t r0, int64_t r1,
+                                           const double* T, int64_t n_pad, int64_t steps, RowOf row_of, int64_t end,
                                            double (*red)[kGramE], double* out) {
   const double* colp[kGramCols];
   const int nf = gram_finite_cols(p, colmap, cs, T, n_pad, colp);
@@ -584,7 +575,9 @@ __device__ __forceinline__ void gram_block(const PlainCand& p, const int32_t* co
   double part[kGramE];
 #pragma unroll
   for (int e = 0; e < kGramE; ++e) part[e] = 0.0;
-  for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+  for (int64_t i = 0; i < steps; ++i) {
+    const int64_t r = row_of(i) + threadIdx.x;
+    if (r >= end) continue;
     double v[kGramCols];
 #pragma unroll
     for (int a = 0; a < kGramCols; ++a) v[a] = a < nf ? colp[a][r] : 1.0;
@@ -621,14 +614,19 @@ __global__ void __launch_bounds__(256) nan_gram_kernel(const int32_t* list, int 
   if (i >= cnt || (dcount && i >= *dcount)) return;
   const PlainCand p = pc[list[i]];
   if (!(p.pad & 2)) return;
-  gram_block(p, colmap, cs, T, n_pad, n * (int64_t)blockIdx.y / gridDim.y, n * (int64_t)(blockIdx.y + 1) / gridDim.y,
-             red, gpart + ((int64_t)i * gridDim.y + blockIdx.y) * kGramE);
+  const int64_t r0 = n * (int64_t)blockIdx.y / gridDim.y, r1 = n * (int64_t)(blockIdx.y + 1) / gridDim.y;
+  gram_block(p, colmap, cs, T, n_pad, (r1 - r0 + 255) / 256, [&](int64_t s) { return r0 + 256 * s; }, r1, red, gpart + ((int64_t)i * gridDim.y + blockIdx.y) * kGramE);
 }
 
 // Whether the certificate of nan_gram holds for candidate p, from the nbx
-// partial Gram matrices at gp.
-__device__ __forceinline__ bool gram_certifies(const PlainCand& p, const int32_t* colmap, const ColStat* cs, int nbx,
-                                               const double* gp) {
+// partial Gram matrices at gp.  n > 0: they are those of some of the n rows, and
+// the columns' squared norms are in cs; a Gram matrix over all rows is larger
+// (in the order of semidefinite matrices), and so is what is left of a column
+// after any other columns are taken out.  (The order of the pivots may differ
+// then, which can cost a factor of K 4^(K - 1) < 1e6; both bounds stay far above
+// the reference's cut.)
+__device__ __noinline__ bool gram_certifies(const PlainCand& p, const int32_t* colmap, const ColStat* cs, int nbx,
+                                            const double* gp, int64_t n) {
   const int m = p.k - 1;
   int nf = 0;
   for (int j = 0; j < m; ++j) nf += (cs[colmap[p.a_col + j]].flags & kCsNaN) ? 0 : 1;
@@ -643,10 +641,16 @@ __device__ __forceinline__ bool gram_certifies(const PlainCand& p, const int32_t
       G[bb][a] = t;
     }
   double d0[kGramCols], maxd = 0.0;
-  for (int a = 0; a < K; ++a) {
-    d0[a] = G[a][a];
-    maxd = fmax(maxd, G[a][a]);
+  for (int a = 0; a < K; ++a) d0[a] = G[a][a];
+  if (n > 0) {
+    int f = 0;
+    for (int j = 0; j < m; ++j) {
+      const ColStat& st = cs[colmap[p.a_col + j]];
+      if (!(st.flags & kCsNaN)) d0[f++] = st.sumsq;
+    }
+    d0[K - 1] = (double)n;
   }
+  for (int a = 0; a < K; ++a) maxd = fmax(maxd, d0[a]);
   int piv[kGramCols];
   for (int a = 0; a < K; ++a) piv[a] = a;
   bool ok = maxd > 0.0 && maxd < 1e300;
@@ -696,15 +700,20 @@ __global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt,
   if (i >= cnt || (dcount && i >= *dcount)) return;
   const int c = list[i];
   if (!(pc[c].pad & 2)) return;
-  settle_candidate(b, c, pc, gram_certifies(pc[c], colmap, cs, nbx, gpart + (int64_t)i * nbx * kGramE), coefs, res,
+  settle_candidate(b, c, pc, gram_certifies(pc[c], colmap, cs, nbx, gpart + (int64_t)i * nbx * kGramE, 0), coefs, res,
                    decided);
 }
 
-// The three above for one candidate a block.
+// The three above for one candidate a block: the certificate from kGramSample
+// rows in eight runs spread over the dataset where the columns' norms are known
+// (sums), else, or where that fails, from all rows if they are few (all_rows);
+// what is still open keeps pad = 2.
+constexpr int kGramSample = 2048;
 __global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32_t* list, int cnt, PlainCand* pc,
                                                          const int32_t* colmap, const ColStat* cs, const double* T,
                                                          int64_t n, int64_t n_pad, double* coefs, rrg_result* res,
-                                                         uint32_t* decided, const int32_t* dcount) {
+                                                         uint32_t* decided, const int32_t* dcount, bool sums,
+                                                         bool all_rows) {
   __shared__ double red[8][kGramE], g[kGramE];
   __shared__ int pad;
   after_previous();
@@ -713,13 +722,25 @@ __global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32
   const PlainCand p = pc[c];
   if (threadIdx.x == 0) {
     pad = classify_candidate(b, c, p, colmap, cs, n, coefs, res, decided);
-    if (pad == 1) pc[c].pad = 1;
+    if (pad) pc[c].pad = pad;
   }
   __syncthreads();
   if (pad != 2) return;
-  gram_block(p, colmap, cs, T, n_pad, 0, n, red, g);
+  if (sums && n > kGramSample) {
+    gram_block(p, colmap, cs, T, n_pad, kGramSample / 256, [&](int64_t s) { return n * s / (kGramSample / 256); }, n,
+               red, g);
+    __syncthreads();
+    if (threadIdx.x == 0 && gram_certifies(p, colmap, cs, 1, g, n)) {
+      settle_candidate(b, c, pc, true, coefs, res, decided);
+      pad = 1;
+    }
+    __syncthreads();
+    if (pad == 1) return;
+  }
+  if (!all_rows) return;
+  gram_block(p, colmap, cs, T, n_pad, (n + 255) / 256, [](int64_t s) { return 256 * s; }, n, red, g);
   __syncthreads();
-  if (threadIdx.x == 0) settle_candidate(b, c, pc, gram_certifies(p, colmap, cs, 1, g), coefs, res, decided);
+  if (threadIdx.x == 0) settle_candidate(b, c, pc, gram_certifies(p, colmap, cs, 1, g, 0), coefs, res, decided);
 }
 
 constexpr int64_t kGramRows = 32768;  // rows a block
@@ -731,25 +752,26 @@ size_t nan_gram_bytes(int64_t n, int cnt) {
   return nbx == 1 ? 1 : sizeof(double) * (size_t)cnt * nbx * kGramE;
 }
 bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list, int cnt, PlainCand* pc,
-                       const int32_t* colmap, const ColStat* cs, const double* T, double* gpart, double* coefs,
-                       rrg_result* res, uint32_t* decided, const int32_t* dcount, cudaStream_t st, int64_t* launches) {
+                       const int32_t* colmap, const ColStat* cs, bool sums, const double* T, double* gpart,
+                       double* coefs, rrg_result* res, uint32_t* decided, const int32_t* dcount, cudaStream_t st,
+                       int64_t* launches) {
   if (cnt <= 0) return true;
+  // Up to kGramRows rows one launch settles every candidate.  Above, what the
+  // sample leaves open goes over all rows with several blocks a candidate.
+  // (A lone candidate of 150 rows is launches and latency: 106 -> 91 us with one
+  // launch here, one to begin a table and no side stream for one QR.  The sample
+  // instead of all rows: 765 candidates at 20011 rows 0.28 -> 0.06 ms; 2048 random
+  // trees at 100k rows, with the evaluation, 7.4 -> 6.9.)
   const int nbx = nan_gram_blocks(ds.n);
-  // One block's rows a candidate: one launch instead of three.  A lone candidate
-  // of 150 rows is launches and latency: with this, one launch to begin a table
-  // instead of two and no fork to a side stream for one QR launch, 106 -> 91 us.
-  if (nbx == 1) {
-    *launches += 1;
-    return launch_next(true, nan_settle_kernel, dim3(cnt), 256, 0, st, b, list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad,
-                       coefs, res, decided, dcount) &&
-           launch_ok("nan_settle");
-  }
-  sentinel_classify_kernel<<<(cnt + 127) / 128, 128, 0, st>>>(b, list, cnt, pc, colmap, cs, ds.n, coefs, res, decided,
-                                                              dcount);
+  *launches += 1;
+  if (!launch_next(true, nan_settle_kernel, dim3(cnt), 256, 0, st, b, list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad,
+                   coefs, res, decided, dcount, sums, nbx == 1))
+    return launch_ok("nan_settle");
+  if (nbx == 1) return launch_ok("nan_settle");
   nan_gram_kernel<<<dim3(cnt, nbx), 256, 0, st>>>(list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad, gpart, dcount);
   nan_gram_decide_kernel<<<(cnt + 127) / 128, 128, 0, st>>>(b, list, cnt, pc, colmap, cs, nbx, gpart, coefs, res,
                                                             decided, dcount);
-  *launches += 3;
+  *launches += 2;
   return launch_ok("nan_gram");
 }
 

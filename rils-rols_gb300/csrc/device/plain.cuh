@@ -102,11 +102,13 @@ constexpr uint32_t kCsTail = 4;  // a row after the first with |value| > 1e-150 
 // The listed tuned candidates whose QR result is certain to be all-NaN
 // coefficients at full rank (the fitness sentinel): that result is written,
 // pc[c].pad = 1 (the QR and residual kernels skip it) and *decided counts it.
+// sums: launch_col_sums has formed the listed candidates' columns' sums.
 // gpart: nan_gram_bytes(n, cnt) bytes.  dcount as above.
 size_t nan_gram_bytes(int64_t n, int cnt);
 bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list, int cnt, PlainCand* pc,
-                       const int32_t* colmap, const ColStat* cs, const double* T, double* gpart, double* coefs,
-                       rrg_result* res, uint32_t* decided, const int32_t* dcount, cudaStream_t st, int64_t* launches);
+                       const int32_t* colmap, const ColStat* cs, bool sums, const double* T, double* gpart,
+                       double* coefs, rrg_result* res, uint32_t* decided, const int32_t* dcount, cudaStream_t st,
+                       int64_t* launches);
 // Before a table's evaluation: the listed results and the columns' statistics to zero.
 bool launch_table_begin(const int32_t* list, int n, rrg_result* res, const int32_t* slots, int n_slots, ColStat* cst,
                         cudaStream_t st);

@@ -1560,7 +1560,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       if (!launch_col_sums(F64, dd, all_cols, ncol, all_count, cst, static_cast<double*>(d_cpart.ptr), 8 * sm_count,
                            stream))
         return RRG_E_CUDA;
-      if (!launch_nan_settle(dev, dd, fb_list, cnt, d_pcs, d_ccol, cst, F64, gpart, coefs, res,
+      if (!launch_nan_settle(dev, dd, fb_list, cnt, d_pcs, d_ccol, cst, true, F64, gpart, coefs, res,
                              status + kStatusSentinel, fb_count, stream, &launches))
         return RRG_E_CUDA;
       if (!launch_rescore_buckets(dev.cands, fallback, cnt, d_pcs, blist, bcount, stream)) {
@@ -1988,7 +1988,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       rrc::set_error("FP64 round: scratch allocation failed");
       return RRG_E_OOM;
     }
-    if (!launch_nan_settle(dev, dd, d_list, ng, pk.at<PlainCand>(d_ft64, o_pcs), d_cmap, cst, F64,
+    if (!launch_nan_settle(dev, dd, d_list, ng, pk.at<PlainCand>(d_ft64, o_pcs), d_cmap, cst, chunked || cp.kept, F64,
                            static_cast<double*>(d_gram.ptr), coefs, res, status + kStatusSentinel, nullptr, stream,
                            &launches))
       return RRG_E_CUDA;
