@@ -31,8 +31,9 @@ constexpr int kMaxK = RRG_MAX_TERMS;
 // forms (rr_math_split.h): the kernel is bound by the FP64 pipe (an
 // instruction holds it for 16 cycles), so what leaves it is what is saved.
 // GB300, ms of the FP64 evaluation phase with native operations / now: 2048
-// random trees at 100k rows 105.1 / 78.5, a 660-candidate local-search round
-// at 1M rows 23.2 / 17.4.  The results are the same bits.
+// random trees at 100k rows 105.1 / 78.5 (all their rows; fewer are evaluated
+// now, see EvalRows), a 660-candidate local-search round at 1M rows 23.2 / 17.4
+// (12.8 with the pieces and six blocks an SM).  The results are the same bits.
 __device__ __forceinline__ double bin64(int base, double a, double b) {
   switch (base) {
     case RRG_ADD: return __dadd_rn(a, b);
@@ -55,7 +56,8 @@ __device__ __forceinline__ double bin64(int base, double a, double b) {
 // columns of T (same rows, column stride n_pad).
 template <bool ONE>
 __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const double* consts, const DevData& ds,
-                                            int64_t row, double* st, double* out, const double* T, uint32_t* status) {
+                                            int64_t row, double* st, int levels, double* out, const double* T,
+                                            uint32_t* status) {
   double tos = 0.0;
   int sp = 0;
   const int stride = blockDim.x;
@@ -67,12 +69,12 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
       case RRG_OP_LDV: tos = ds.X64[(int64_t)arg * ds.n_pad + row]; break;
       case RRG_OP_LDC: tos = consts[arg]; break;
       case RRG_OP_PSV:
-        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return tos; }
+        if (sp >= levels) { atomicOr(status, ST_STACK); return tos; }
         st[sp++ * stride] = tos;
         tos = ds.X64[(int64_t)arg * ds.n_pad + row];
         break;
       case RRG_OP_PSC:
-        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return tos; }
+        if (sp >= levels) { atomicOr(status, ST_STACK); return tos; }
         st[sp++ * stride] = tos;
         tos = consts[arg];
         break;
@@ -84,7 +86,7 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
       case RRG_OP_SQR: tos = fi_mul(tos, tos); break;
       case kOpLDT: tos = T[(int64_t)arg * ds.n_pad + row]; break;
       case kOpPST:
-        if (sp >= RRG_MAX_STACK) { atomicOr(status, ST_STACK); return tos; }
+        if (sp >= levels) { atomicOr(status, ST_STACK); return tos; }
         st[sp++ * stride] = tos;
         tos = T[(int64_t)arg * ds.n_pad + row];
         break;
@@ -123,7 +125,7 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
 // somewhere: 78.5 ms without the stop, 23.8 with it, 14.3 in
 // pieces of 4096 rows, 7.4 with the shared columns left out that no factor needs.
 __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len, const double* consts,
-                                                  const DevData& ds, int64_t r0, int64_t r1, double* st, double* Ac,
+                                                  const DevData& ds, int64_t r0, int64_t r1, double* st, int levels, double* Ac,
                                                   const double* T, uint32_t* status, ColStat* cs, bool stop,
                                                   volatile int* found) {
   static_assert(kStopRow <= 256, "within the first rows of a block");
@@ -131,7 +133,7 @@ __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len,
   const bool skip = stop && (__ldcg(&cs->flags) & kCsStop) != 0;  // (any mix of answers in a block does)
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     if (stop && r >= blockDim.x && (skip || (r - r0 >= blockDim.x && *found))) break;
-    const double v = run_row64<true>(code, len, consts, ds, r, st, nullptr, T, status);
+    const double v = run_row64<true>(code, len, consts, ds, r, st, levels, nullptr, T, status);
     Ac[r] = v;
     // on the bits of |v| (non-negative doubles order as integers, NaN above)
     const unsigned long long a = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(256) table_eval_list_kernel(DevBatch b, DevDat
   const int nbc = max(min_nbc, min(max_nbc, (int)((gridDim.x + cnt - 1) / cnt)));
   const int64_t items = (int64_t)cnt * nbc;
   double* st = smem + threadIdx.x;
-  uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + RRG_MAX_STACK * blockDim.x);
+  uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + rows.levels * blockDim.x);
   for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
     const int c = cols[w % cnt];
     const int bi = (int)(w / cnt);
@@ -171,15 +173,15 @@ __global__ void __launch_bounds__(256) table_eval_list_kernel(DevBatch b, DevDat
     const rrg_cand cd = b.cands[c];
     const int64_t nr = rows.hi - rows.lo;
     const int64_t r0 = rows.lo + nr * bi / nbc, r1 = rows.lo + nr * (bi + 1) / nbc;
-    const bool staged = cd.code_len < kMaxCodeSmem;
-    volatile int* found = reinterpret_cast<int*>(code_s + kMaxCodeSmem - 1);
+    const bool staged = cd.code_len < rows.words;
+    volatile int* found = reinterpret_cast<int*>(code_s + rows.words - 1);
     __syncthreads();  // the previous item's program is no longer read
     if (threadIdx.x == 0) *found = 0;
     if (staged)
       for (int i = threadIdx.x; i < cd.code_len; i += blockDim.x) code_s[i] = b.code[cd.code_offset + i];
     __syncthreads();
     const uint32_t* code = staged ? code_s : b.code + cd.code_offset;
-    eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, A + pc[c].a_col * ds.n_pad, A, status,
+    eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, rows.levels, A + pc[c].a_col * ds.n_pad, A, status,
                       &cst[pc[c].a_col], cd.reserved == kColStop, found);
   }
 }
@@ -197,10 +199,10 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
   const int nb = gridDim.y;
   const int64_t nr = rows.hi - rows.lo;
   const int64_t r0 = rows.lo + nr * blockIdx.y / nb, r1 = rows.lo + nr * (blockIdx.y + 1) / nb;
-  double* st = smem + threadIdx.x;  // spill stack, RRG_MAX_STACK * blockDim.x doubles
-  uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + RRG_MAX_STACK * blockDim.x);
-  const bool staged = cd.code_len < kMaxCodeSmem;
-  volatile int* found = reinterpret_cast<int*>(code_s + kMaxCodeSmem - 1);
+  double* st = smem + threadIdx.x;  // spill stack, rows.levels * blockDim.x doubles
+  uint32_t* code_s = reinterpret_cast<uint32_t*>(smem + rows.levels * blockDim.x);
+  const bool staged = cd.code_len < rows.words;
+  volatile int* found = reinterpret_cast<int*>(code_s + rows.words - 1);
   if (threadIdx.x == 0) *found = 0;
   if (staged)
     for (int i = threadIdx.x; i < cd.code_len; i += blockDim.x) code_s[i] = b.code[cd.code_offset + i];
@@ -208,12 +210,12 @@ __global__ void __launch_bounds__(256) plain_eval_kernel(DevBatch b, DevData ds,
   const uint32_t* code = staged ? code_s : b.code + cd.code_offset;
   double* Ac = A + pc[c].a_col * ds.n_pad;
   if (cst) {
-    eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, Ac, A, status, &cst[pc[c].a_col],
+    eval_column_stats(code, cd.code_len, b.consts, ds, r0, r1, st, rows.levels, Ac, A, status, &cst[pc[c].a_col],
                       cd.reserved == kColStop, found);
     return;
   }
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x)
-    run_row64<false>(code, cd.code_len, b.consts, ds, r, st, Ac, A, status);
+    run_row64<false>(code, cd.code_len, b.consts, ds, r, st, rows.levels, Ac, A, status);
 }
 
 // One block.  The columns that still count after some rows are evaluated: the
@@ -775,6 +777,8 @@ bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list
   return launch_ok("nan_gram");
 }
 
-size_t plain_eval_smem() { return RRG_MAX_STACK * 256 * sizeof(double) + kMaxCodeSmem * sizeof(uint32_t); }
+size_t plain_eval_smem(int levels, int words) {
+  return (size_t)levels * 256 * sizeof(double) + (size_t)words * sizeof(uint32_t);
+}
 
 }  // namespace rrd

@@ -18,6 +18,8 @@ inline int64_t eval_pieces(int64_t n) { return n <= kEvalRows ? 1 : (n + kEvalRo
 struct EvalRows {
   int64_t lo, hi;
   const uint8_t* live;
+  // the launch's shared memory: spill levels, words of program staging
+  int32_t levels = RRG_MAX_STACK, words = kMaxCodeSmem;
 };
 // Shared columns, most of a batch of unlike trees, count only as long as a
 // factor that reads them does.  So where there are many, the first kFirstRows
@@ -121,6 +123,6 @@ __global__ void table_eval_list_kernel(DevBatch b, DevData ds, const PlainCand* 
                                        const int32_t* count, int min_nbc, int max_nbc, double* A, uint32_t* status,
                                        ColStat* cst, EvalRows rows);
 
-size_t plain_eval_smem();
+size_t plain_eval_smem(int levels = RRG_MAX_STACK, int words = kMaxCodeSmem);
 
 }  // namespace rrd
