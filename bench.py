@@ -629,7 +629,7 @@ PHASE_KERNELS = {
     "factor_eval": "fac_eval_kernel (double-float factor table)",
     "pair_sums": "pair_sum_kernel",
     "fp64_eval": "plain_eval_kernel (FP64 table)",
-    "fp64_qr": "qr_passA_kernel + qr_sums_kernel (column-pivoted QR, FP64, chunked passes over the GPU)",
+    "fp64_qr": "qr_passA_kernel + qr_passB_kernel (column-pivoted QR, FP64, chunked passes over the GPU)",
 }
 
 

@@ -469,16 +469,12 @@ rrg_status rrg_context::enqueue_round(rrg_dataset* ds, const rrg_batch* b, int32
   if (st != RRG_OK) return st;
   st = stage_batch(b);
   if (st != RRG_OK) return st;
-  const size_t res_bytes = sizeof(rrg_result) * std::max(1, b->n_cand);
-  const size_t coef_bytes = sizeof(double) * std::max<int64_t>(1, n_coefs);
-  if (!d_res.reserve(res_bytes) || !d_coefs.reserve(coef_bytes) || !d_status.reserve(64) ||
-      !h_res.reserve(res_bytes) || !h_coefs.reserve(coef_bytes) || !h_status.reserve(64)) {
+  size_t out_bytes = 0;
+  if (!reserve_out((size_t)std::max(1, b->n_cand), (size_t)std::max<int64_t>(1, n_coefs), out_bytes)) {
     rrc::set_error("cannot reserve result buffers");
     return RRG_E_OOM;
   }
-  RRG_CUDA(cudaMemsetAsync(d_res.ptr, 0, res_bytes, stream));
-  RRG_CUDA(cudaMemsetAsync(d_coefs.ptr, 0, coef_bytes, stream));
-  RRG_CUDA(cudaMemsetAsync(d_status.ptr, 0, 64, stream));
+  RRG_CUDA(cudaMemsetAsync(d_out.ptr, 0, out_bytes, stream));
   // distinct factor programs, and candidates with identical factor lists
   // (same programs, same order, same mode) scored once
   build_factor_table(host_cands.data(), b->n_cand, b->code, b->consts, ft);
@@ -497,10 +493,25 @@ rrg_status rrg_context::enqueue_round(rrg_dataset* ds, const rrg_batch* b, int32
     st = run_mixed(ds, reps, precision == RRG_MIXED_CERTIFIED);
   }
   if (st != RRG_OK) return st;
-  RRG_CUDA(cudaMemcpyAsync(h_res.ptr, d_res.ptr, res_bytes, cudaMemcpyDeviceToHost, stream));
-  RRG_CUDA(cudaMemcpyAsync(h_coefs.ptr, d_coefs.ptr, coef_bytes, cudaMemcpyDeviceToHost, stream));
-  RRG_CUDA(cudaMemcpyAsync(h_status.ptr, d_status.ptr, 64, cudaMemcpyDeviceToHost, stream));
+  RRG_CUDA(cudaMemcpyAsync(h_out.ptr, d_out.ptr, out_bytes, cudaMemcpyDeviceToHost, stream));
   return RRG_OK;
+}
+
+bool rrg_context::reserve_out(size_t n_res, size_t n_coefs, size_t& bytes) {
+  constexpr size_t kStatusBytes = 64;
+  static_assert(sizeof(rrg_result) % sizeof(double) == 0, "coefficients follow the results");
+  const size_t o_coefs = kStatusBytes + sizeof(rrg_result) * n_res;
+  bytes = o_coefs + sizeof(double) * n_coefs;
+  if (!d_out.reserve(bytes) || !h_out.reserve(bytes)) return false;
+  char* d = static_cast<char*>(d_out.ptr);
+  char* h = static_cast<char*>(h_out.ptr);
+  d_status.ptr = d;
+  d_res.ptr = d + kStatusBytes;
+  d_coefs.ptr = d + o_coefs;
+  h_status.ptr = h;
+  h_res.ptr = h + kStatusBytes;
+  h_coefs.ptr = h + o_coefs;
+  return true;
 }
 
 rrg_status rrg_context::wait(int32_t timeout_ms) {
@@ -580,7 +591,7 @@ std::vector<DevBuf*> rrg_context::all_bufs() {
   return {&d_batch, &d_A, &d_pc, &d_partial, &d_list, &d_qrs, &d_terms, &d_fallback, &d_sse1, &d_probe,
           &d_nanrow, &d_cert_e, &d_ft, &d_ftp, &d_ft64, &d_F, &d_P, &d_Pc, &d_psum, &d_F64, &d_M,
           &d_gram, &d_rlist2, &d_fbpack, &d_fbneed, &d_fblive, &d_live, &d_fbcols, &d_fbF64, &d_fbcst, &d_fbgram, &d_fbblist,
-          &d_fbM, &d_fbctr, &d_cself, &d_cprobe, &d_cfnan, &d_ccst, &d_cpart, &d_store, &d_res, &d_coefs, &d_status};
+          &d_fbM, &d_fbctr, &d_cself, &d_cprobe, &d_cfnan, &d_ccst, &d_cpart, &d_store, &d_out};
 }
 
 // Most blocks of a chunked QR pass: what is resident at once.
@@ -635,9 +646,7 @@ rrg_context::~rrg_context() {
   h_ftp.release();
   h_ft64.release();
   h_batch.release();
-  h_res.release();
-  h_coefs.release();
-  h_status.release();
+  h_out.release();
   h_pc.release();
   for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
   if (done) cudaEventDestroy(done);
@@ -906,7 +915,8 @@ rrg_status rrg_predict(rrg_dataset* ds, const rrg_batch* batch, double* values) 
   ++ctx->round_seq;
   st = ctx->stage_batch(&one);
   if (st != RRG_OK) return st;
-  if (!ctx->d_status.reserve(64) || !ctx->h_status.reserve(64)) return RRG_E_OOM;
+  size_t out_bytes = 0;
+  if (!ctx->reserve_out(0, 0, out_bytes)) return RRG_E_OOM;
   RRG_CUDA(cudaMemsetAsync(ctx->d_status.ptr, 0, 64, ctx->stream));
   st = ctx->run_predict(ds);
   if (st != RRG_OK) return st;
