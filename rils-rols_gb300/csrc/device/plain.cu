@@ -620,15 +620,16 @@ __global__ void __launch_bounds__(256) nan_gram_kernel(const int32_t* list, int 
   gram_block(p, colmap, cs, T, n_pad, (r1 - r0 + 255) / 256, [&](int64_t s) { return r0 + 256 * s; }, r1, red, gpart + ((int64_t)i * gridDim.y + blockIdx.y) * kGramE);
 }
 
-// Whether the certificate of nan_gram holds for candidate p, from the nbx
-// partial Gram matrices at gp.  n > 0: they are those of some of the n rows, and
+// Whether the certificate of nan_gram holds for candidate p (1; 0 not; -1 not,
+// and a column all but depends on the others, as twice the same factor does),
+// from the nbx partial Gram matrices at gp.  n > 0: they are those of some of the n rows, and
 // the columns' squared norms are in cs; a Gram matrix over all rows is larger
 // (in the order of semidefinite matrices), and so is what is left of a column
 // after any other columns are taken out.  (The order of the pivots may differ
 // then, which can cost a factor of K 4^(K - 1) < 1e6; both bounds stay far above
 // the reference's cut.)
-__device__ __noinline__ bool gram_certifies(const PlainCand& p, const int32_t* colmap, const ColStat* cs, int nbx,
-                                            const double* gp, int64_t n) {
+__device__ __noinline__ int gram_certifies(const PlainCand& p, const int32_t* colmap, const ColStat* cs, int nbx,
+                                           const double* gp, int64_t n) {
   const int m = p.k - 1;
   int nf = 0;
   for (int j = 0; j < m; ++j) nf += (cs[colmap[p.a_col + j]].flags & kCsNaN) ? 0 : 1;
@@ -642,8 +643,8 @@ __device__ __noinline__ bool gram_certifies(const PlainCand& p, const int32_t* c
       G[a][bb] = t;
       G[bb][a] = t;
     }
-  double d0[kGramCols], maxd = 0.0;
-  for (int a = 0; a < K; ++a) d0[a] = G[a][a];
+  double d0[kGramCols], g0[kGramCols], maxd = 0.0;
+  for (int a = 0; a < K; ++a) d0[a] = g0[a] = G[a][a];
   if (n > 0) {
     int f = 0;
     for (int j = 0; j < m; ++j) {
@@ -655,16 +656,13 @@ __device__ __noinline__ bool gram_certifies(const PlainCand& p, const int32_t* c
   for (int a = 0; a < K; ++a) maxd = fmax(maxd, d0[a]);
   int piv[kGramCols];
   for (int a = 0; a < K; ++a) piv[a] = a;
-  bool ok = maxd > 0.0 && maxd < 1e300;
-  for (int s2 = 0; s2 < K && ok; ++s2) {
+  if (!(maxd > 0.0 && maxd < 1e300)) return 0;
+  for (int s2 = 0; s2 < K; ++s2) {
     int q = s2;
     for (int j = s2 + 1; j < K; ++j)
       if (G[j][j] > G[q][q]) q = j;
     const double dp = G[q][q];
-    if (!(dp > 1e-8 * d0[piv[q]]) || !(dp > 1e-24 * maxd)) {
-      ok = false;
-      break;
-    }
+    if (!(dp > 1e-8 * d0[piv[q]]) || !(dp > 1e-24 * maxd)) return dp < 1e-13 * g0[piv[q]] ? -1 : 0;
     if (q != s2) {
       for (int j = 0; j < K; ++j) { const double t = G[s2][j]; G[s2][j] = G[q][j]; G[q][j] = t; }
       for (int j = 0; j < K; ++j) { const double t = G[j][s2]; G[j][s2] = G[j][q]; G[j][q] = t; }
@@ -678,7 +676,7 @@ __device__ __noinline__ bool gram_certifies(const PlainCand& p, const int32_t* c
         G[bb][a] = G[a][bb];
       }
   }
-  return ok;
+  return 1;
 }
 
 __device__ __forceinline__ void settle_candidate(const DevBatch& b, int c, PlainCand* pc, bool ok, double* coefs,
@@ -702,8 +700,8 @@ __global__ void nan_gram_decide_kernel(DevBatch b, const int32_t* list, int cnt,
   if (i >= cnt || (dcount && i >= *dcount)) return;
   const int c = list[i];
   if (!(pc[c].pad & 2)) return;
-  settle_candidate(b, c, pc, gram_certifies(pc[c], colmap, cs, nbx, gpart + (int64_t)i * nbx * kGramE, 0), coefs, res,
-                   decided);
+  settle_candidate(b, c, pc, gram_certifies(pc[c], colmap, cs, nbx, gpart + (int64_t)i * nbx * kGramE, 0) > 0, coefs,
+                   res, decided);
 }
 
 // The three above for one candidate a block: the certificate from kGramSample
@@ -732,9 +730,12 @@ __global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32
     gram_block(p, colmap, cs, T, n_pad, kGramSample / 256, [&](int64_t s) { return n * s / (kGramSample / 256); }, n,
                red, g);
     __syncthreads();
-    if (threadIdx.x == 0 && gram_certifies(p, colmap, cs, 1, g, n)) {
-      settle_candidate(b, c, pc, true, coefs, res, decided);
-      pad = 1;
+    if (threadIdx.x == 0) {
+      const int r = gram_certifies(p, colmap, cs, 1, g, n);
+      // dependent on the sample: most likely on all rows, and the QR's to find
+      // (8192 random trees' re-scoring, with its evaluation, 14.8 -> 13.9 ms)
+      if (r) settle_candidate(b, c, pc, r > 0, coefs, res, decided);
+      pad = r ? 1 : 2;
     }
     __syncthreads();
     if (pad == 1) return;
@@ -742,7 +743,7 @@ __global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32
   if (!all_rows) return;
   gram_block(p, colmap, cs, T, n_pad, (n + 255) / 256, [](int64_t s) { return 256 * s; }, n, red, g);
   __syncthreads();
-  if (threadIdx.x == 0) settle_candidate(b, c, pc, gram_certifies(p, colmap, cs, 1, g, 0), coefs, res, decided);
+  if (threadIdx.x == 0) settle_candidate(b, c, pc, gram_certifies(p, colmap, cs, 1, g, 0) > 0, coefs, res, decided);
 }
 
 constexpr int64_t kGramRows = 32768;  // rows a block
