@@ -392,6 +392,7 @@ rrg_status rrg_context::submit(rrg_dataset* ds, const rrg_batch* b, int32_t prec
     // (storing them may grow the cache's arena, which a capture refuses)
     const rrg_status sst = store_lane_columns();
     if (sst != RRG_OK) {
+      drain();
       clear_caches();
       return sst;
     }
@@ -432,6 +433,7 @@ rrg_status rrg_context::submit(rrg_dataset* ds, const rrg_batch* b, int32_t prec
     st = enqueue_round(ds, b, precision, n_coefs);
   }
   if (st != RRG_OK) {
+    drain();
     clear_caches();  // a round that failed part-way may have left slots unwritten
     return st;
   }
@@ -442,6 +444,17 @@ rrg_status rrg_context::submit(rrg_dataset* ds, const rrg_batch* b, int32_t prec
   out_n = b->n_cand;
   out_ncoef = n_coefs;
   return RRG_OK;
+}
+
+// Waits for what a round that failed part-way had queued.  It may have left a
+// side stream that the context stream does not wait for (the probe, a group of
+// factors, a QR bucket), and these read the round's uploads and the dataset's
+// columns; the next round reuses the uploads and their pinned buffers, and the
+// caller may destroy the dataset.
+void rrg_context::drain() {
+  for (cudaStream_t s : side) cudaStreamSynchronize(s);
+  cudaStreamSynchronize(stream);
+  cudaGetLastError();
 }
 
 // The device work of one round on the context stream: batch upload, the
@@ -866,7 +879,7 @@ rrg_status rrg_dataset_destroy(rrg_dataset* ds) {
     cudaSetDevice(ctx->device);
     if (ctx->in_flight) cudaEventSynchronize(ctx->done);
     // freed behind the context stream's queued work (every round of this
-    // dataset ran on that stream or joined it)
+    // dataset ran on that stream or joined it, or failed and was waited for)
     release_dataset_memory(ds, ctx->stream);
     // its kept columns go with it
     if (ctx->fcache.uid() == ds->uid) ctx->fcache.bind(0);
