@@ -309,11 +309,13 @@ bool build_table_programs(TableScratch& ts, const std::vector<uint32_t>& lcode, 
     if (froot[l] < 0) return false;
   // classes of the transcendental subtrees (equal subtrees: features by
   // index, constants by bits) with their uses: found by hash, confirmed node
-  // by node
+  // by node down to the transcendental subtrees inside, whose classes are known
+  // (inner ones come first): every node is compared once, however deep they nest
   std::vector<int32_t> rep, uses;  // [class] its first node, its occurrences
   auto equal = [&](auto& self, int32_t x, int32_t y) -> bool {
     const PNode &p = nd[x], &q = nd[y];
     if (hash[x] != hash[y] || p.kind != q.kind || p.op != q.op) return false;
+    if (cls[x] >= 0 && cls[y] >= 0) return cls[x] == cls[y];  // nested subtrees have theirs already
     if (p.kind <= 1) return bits(p) == bits(q);
     return self(self, p.a, q.a) && (p.kind == 3 || self(self, p.b, q.b));
   };
