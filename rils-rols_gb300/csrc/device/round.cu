@@ -989,6 +989,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
            fac_eval_smem_staged(chunk, gs.slots) <= (size_t)227 * 1024;
   };
   const bool maps_ok = fac_stage_maps(fa, dd);
+  strial = strial && !capturing && (int64_t)ne * ds->n >= kTuneMinWork;
   // one launch per level: a level reads the columns of the levels before it
   auto eval_rows = [&](const GroupSet& gs, bool stage, int q0, int q1, const uint8_t* live) {
     fa.chunk0 = q0;
@@ -1038,8 +1039,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   };
   // The probe needs nothing of the table and runs beside the evaluation (a lone
   // candidate at 50k rows 137 -> 117 us, eight rounds at 1M rows 91.0 -> 90.0 ms;
-  // rounds that fill the GPU take the same time as one after the other).  After
-  // the trials, which time the evaluation alone.
+  // rounds that fill the GPU take the same time as one after the other).  In a
+  // round with a trial it comes after, so that the evaluation is timed alone.
   auto probe = [&] {
     return cudaEventRecord(fork_ev, stream) == cudaSuccess && cudaStreamWaitEvent(side[1], fork_ev, 0) == cudaSuccess &&
            launch_fac_probe(pkt.at<const uint32_t>(d_ftp, o_code), pkt.at<const int2>(d_ftp, o_meta),
@@ -1047,7 +1048,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
                             pkt.at<const int32_t>(d_ftp, o_pslot)) &&
            cudaEventRecord(join_ev[1], side[1]) == cudaSuccess;
   };
-  const bool trial = gtrial || (strial && !capturing);
+  const bool trial = gtrial || (strial && maps_ok && can_stage(gsets[0]));
   if (!trial && !probe()) return RRG_E_CUDA;
   int gbest = 0;  // the group set in use
   if (gtrial) {
@@ -1065,7 +1066,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     tune_store(TK_FAC_GROUP, 0, ds->n, gvals, ms, ngv);
   }
   const bool stage_ok = maps_ok && can_stage(gsets[gbest]);
-  if (strial && !capturing && stage_ok && (int64_t)ne * ds->n >= kTuneMinWork) {
+  if (strial && stage_ok) {
     // the first round of this feature count: reading X from global memory
     // and staging it, both timed on the real launches
     int vals[2] = {1, 2};
