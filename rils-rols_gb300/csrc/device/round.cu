@@ -956,10 +956,11 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   FacProbe* cprobe = static_cast<FacProbe*>(d_cprobe.ptr);
   uint32_t* status = static_cast<uint32_t*>(d_status.ptr);
   const int32_t* d_ewcol = pkt.at<const int32_t>(d_ftp, o_ewcol);
-  if (!cp.kept)
-    RRG_CUDA(cudaMemsetAsync(fnan, 0x7f, sizeof(unsigned long long) * std::max(1, ne), stream));
-  else if (!launch_fill_slots(d_ewcol, ne, fnan, 1, 0x7f7f7f7f7f7f7f7full, stream))
-    return RRG_E_CUDA;
+  auto clear_nan = [&] {
+    return cp.kept ? launch_fill_slots(d_ewcol, ne, fnan, 1, 0x7f7f7f7f7f7f7f7full, stream)
+                   : cuda_ok(cudaMemsetAsync(fnan, 0x7f, sizeof(unsigned long long) * std::max(1, ne), stream), "NaN marks");
+  };
+  if (!clear_nan()) return RRG_E_CUDA;
 
   cudaEvent_t t0 = mark_begin();
   FacEvalArgs fa;
@@ -1053,12 +1054,13 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   int gbest = 0;  // the group set in use
   if (gtrial) {
     // the first round of this row class: every group size timed on the
-    // real launches (a repeat rewrites the same columns and sums)
+    // real launches (a repeat rewrites the same columns and sums, from clear
+    // NaN marks as the first: a mark leaves rows out)
     float ms[4];
     for (int v = 0; v < ngv; ++v) {
-      bool ok = true;
+      bool ok = clear_nan();
       const bool st = stage_pick && maps_ok && can_stage(gsets[v]);
-      const rrg_status ts = time_trial([&] { ok = eval_all(gsets[v], st); }, ms[v]);
+      const rrg_status ts = time_trial([&] { ok = ok && eval_all(gsets[v], st); }, ms[v]);
       if (!ok) return RRG_E_CUDA;
       if (ts != RRG_OK) return ts;
       if (ms[v] < ms[gbest]) gbest = v;
@@ -1072,8 +1074,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     int vals[2] = {1, 2};
     float ms[2];
     for (int v = 0; v < 2; ++v) {
-      bool ok = true;
-      const rrg_status ts = time_trial([&] { ok = eval_all(gsets[gbest], vals[v] == 2); }, ms[v]);
+      bool ok = clear_nan();
+      const rrg_status ts = time_trial([&] { ok = ok && eval_all(gsets[gbest], vals[v] == 2); }, ms[v]);
       if (!ok) return RRG_E_CUDA;
       if (ts != RRG_OK) return ts;
     }
@@ -1984,11 +1986,14 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       const int32_t c1 = ep.level_end[L];
       const int32_t nl = c1 - (int32_t)c0;
       if (wave_trial && !capturing && L == wave_level && (int64_t)nl * ds->n >= kTuneMinWork) {
-        // re-evaluating a level rewrites the same columns: time every shape
+        // re-evaluating a level rewrites the same columns, from clear statistics
+        // as the first time (a NaN found leaves rows out): time every shape
         int vals[4];
         float ms[4];
         const int nv = tune_variants(TK_EVAL_WAVES, 0, vals);
         for (int v = 0; v < nv; ++v) {
+          if (!launch_table_begin(nullptr, 0, res, pk.at<const int32_t>(d_ft64, o_ewcol) + c0, nl, cst, stream))
+            return RRG_E_CUDA;
           rrg_status ts = time_trial([&] { eval_level(L, vals[v], every); }, ms[v]);
           if (ts != RRG_OK) return ts;
         }
