@@ -1253,7 +1253,9 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     return launch_pair_sum(pa, n_super, stream);
   };
   if (ptrial) {
-    // every unit size timed on the real launch (a repeat rewrites the same sums)
+    // every unit size timed on the real launch (a repeat rewrites the same sums),
+    // none of them beside the probe
+    RRG_CUDA(cudaStreamWaitEvent(stream, join_ev[1], 0));
     float ms[4];
     for (int v = 0; v < npv; ++v) {
       bool ok = true;
