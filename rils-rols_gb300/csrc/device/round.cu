@@ -1937,16 +1937,31 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     if (!launch_table_begin(d_list, ng, res, pk.at<const int32_t>(d_ft64, o_ewcol), ne, cst, stream))
       return RRG_E_CUDA;
     cudaEvent_t t0 = mark_begin();
-    // one launch (or several of at most 65535 columns) per level; blocks per
-    // column from the tuner's SM waves (any value gives the same columns)
+    // one launch per level: all columns of it, each in pieces of rows, at least
+    // eval_pieces and, where a level has few columns, as many as give the tuner's
+    // SM waves (any number gives the same columns)
     bool wave_trial = false;
     int waves = tune_pick(TK_EVAL_WAVES, 0, ds->n, &wave_trial);
-    size_t wave_level = 0;  // a trial times the widest level
-    for (size_t L = 0, c0 = 0, widest = 0; L < ep.level_end.size(); c0 = ep.level_end[L++])
+    size_t wave_level = 0, widest = 0;  // a trial times the widest level
+    for (size_t L = 0, c0 = 0; L < ep.level_end.size(); c0 = ep.level_end[L++])
       if ((size_t)ep.level_end[L] - c0 > widest) {
         widest = (size_t)ep.level_end[L] - c0;
         wave_level = L;
       }
+    auto pieces = [&](int64_t nl, int wv, int64_t nr) {
+      const int64_t fill = std::min<int64_t>((wv * (int64_t)sm_count + nl - 1) / nl, (nr + 1023) / 1024);
+      return (int)std::min<int64_t>(65535, std::max(eval_pieces(nr), fill));
+    };
+    int wvals[4];
+    const int nwv = tune_variants(TK_EVAL_WAVES, 0, wvals);
+    if (wave_trial) {
+      // no trial where the rows decide and every shape is the same launch (from
+      // 16 SMs / eval_pieces columns on: 25 at 400k rows), nor in a capture
+      bool differ = false;
+      for (int v = 1; v < nwv && widest > 0; ++v)
+        differ |= pieces((int64_t)widest, wvals[v], ds->n) != pieces((int64_t)widest, wvals[0], ds->n);
+      wave_trial = differ && !capturing && (int64_t)widest * ds->n >= kTuneMinWork;
+    }
     // shared memory for what the programs need, not for what they may: six
     // blocks an SM instead of four (627 columns of 1M rows 14.7 -> 12.8 ms)
     int32_t levels = 1, words = 64;
@@ -1960,9 +1975,7 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
       if (nl <= 0) return;
       rows.levels = levels;
       rows.words = words;
-      const int64_t nr = rows.hi - rows.lo;
-      const int64_t fill = std::min<int64_t>(((int64_t)wv * sm_count + nl - 1) / nl, (nr + 1023) / 1024);
-      const int nb = (int)std::min<int64_t>(65535, std::max(eval_pieces(nr), fill));
+      const int nb = pieces(nl, wv, rows.hi - rows.lo);
       launch_next(true, plain_eval_kernel, dim3(nl, nb), 256, plain_eval_smem(levels, words), stream, fdev, dd,
                   pk.at<const PlainCand>(d_ft64, o_fpc), nullptr, c0, F64, status, cst, rows);
       ++launches;
@@ -1987,19 +2000,17 @@ rrg_status rrg_context::run_fp64_table(const rrg_dataset* ds, const std::vector<
     for (size_t L = 0, c0 = 0; L < ep.level_end.size(); ++L) {
       const int32_t c1 = ep.level_end[L];
       const int32_t nl = c1 - (int32_t)c0;
-      if (wave_trial && !capturing && L == wave_level && (int64_t)nl * ds->n >= kTuneMinWork) {
+      if (wave_trial && L == wave_level) {
         // re-evaluating a level rewrites the same columns, from clear statistics
         // as the first time (a NaN found leaves rows out): time every shape
-        int vals[4];
         float ms[4];
-        const int nv = tune_variants(TK_EVAL_WAVES, 0, vals);
-        for (int v = 0; v < nv; ++v) {
+        for (int v = 0; v < nwv; ++v) {
           if (!launch_table_begin(nullptr, 0, res, pk.at<const int32_t>(d_ft64, o_ewcol) + c0, nl, cst, stream))
             return RRG_E_CUDA;
-          rrg_status ts = time_trial([&] { eval_level(L, vals[v], every); }, ms[v]);
+          rrg_status ts = time_trial([&] { eval_level(L, wvals[v], every); }, ms[v]);
           if (ts != RRG_OK) return ts;
         }
-        tune_store(TK_EVAL_WAVES, 0, ds->n, vals, ms, nv);
+        tune_store(TK_EVAL_WAVES, 0, ds->n, wvals, ms, nwv);
         wave_trial = false;
         waves = tune_pick(TK_EVAL_WAVES, 0, ds->n, &wave_trial);
       } else {
