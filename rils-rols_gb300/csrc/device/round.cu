@@ -890,7 +890,6 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   bool gtrial = false;
   int gvals[4] = {tune_pick(TK_FAC_GROUP, 0, ds->n, &gtrial), 0, 0, 0};
   gtrial = gtrial && !capturing && (int64_t)ne * ds->n >= kTuneMinWork;
-  const int ngv = gtrial ? tune_variants(TK_FAC_GROUP, 0, gvals) : 1;
   // row chunks of fac_chunk(d) rows (the self sums' partials are per chunk);
   // pair sums and the residual pass use kPairRows blocks
   const int32_t n_self = 3 * ne;
@@ -904,12 +903,31 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   // the group sets, and one for the first rows alone: one chunk of them leaves
   // the blocks to the groups, so these are small (8192 random trees at 100k
   // rows, 15 levels: 7.9 ms of evaluation with groups of 64, 6.5 with 4)
-  std::vector<GroupSet> gsets(ngv + (two_parts ? 1 : 0));
-  // no larger than leaves every SM four blocks (a lone candidate of three
-  // factors at 50k rows: 42 us in one group, 24 in two)
-  const int gcap = (int)std::min<int64_t>(kFacGroupMax, std::max<int64_t>(1, (int64_t)ne * n_chunks / (4 * sm_count)));
-  for (int v = 0; v < ngv; ++v) build_groups(std::min(gvals[v], gcap), gsets[v]);
-  if (two_parts) build_groups(kFirstGroup, gsets[ngv]);
+  std::vector<GroupSet> gsets;
+  if (gtrial) {
+    // a trial times the sizes as they are, for the rounds of this row class that
+    // fill the GPU with them; sizes that give the same groups are not timed
+    const int nv = tune_variants(TK_FAC_GROUP, 0, gvals);
+    gsets.resize(nv);
+    gtrial = false;
+    for (int v = 0; v < nv; ++v) {
+      build_groups(std::min(gvals[v], kFacGroupMax), gsets[v]);
+      gtrial |= !std::equal(gsets[v].groups.begin(), gsets[v].groups.end(), gsets[0].groups.begin(),
+                            gsets[0].groups.end(), [](int2 a, int2 b) { return a.x == b.x && a.y == b.y; });
+    }
+  }
+  if (!gtrial) {
+    // no larger than leaves every SM four blocks (a lone candidate of three
+    // factors at 50k rows: 42 us in one group, 24 in two)
+    const int64_t gcap = std::max<int64_t>(1, (int64_t)ne * n_chunks / (4 * sm_count));
+    gsets.assign(1, GroupSet());
+    build_groups((int)std::min<int64_t>({gvals[0], kFacGroupMax, gcap}), gsets[0]);
+  }
+  const int ngv = (int)gsets.size();
+  if (two_parts) {
+    gsets.emplace_back();
+    build_groups(kFirstGroup, gsets[ngv]);
+  }
   const size_t n_slots = (size_t)std::max<int64_t>(1, cp.arena);
   if (!d_F.grow_keep(col_bytes * n_slots, d_F.cap) ||
       !d_P.reserve(sizeof(float2) * (size_t)n_chunks * std::max(1, n_self)) ||

@@ -1,10 +1,11 @@
 """No trial of shapes that are the same launch: nothing is timed or stored, and the
 round takes its usual form.  Wide levels of FP64 columns run in pieces that the rows
-decide, whatever the tuner's waves."""
+decide, whatever the tuner's waves; groups of factors are timed in the sizes that a round
+large enough for them would use."""
 import numpy as np
 import pytest
 
-from rils_rols_gb300.fitness import PLAIN, Context, encode, tune_mode, tune_report, tune_reset
+from rils_rols_gb300.fitness import CERTIFIED, MIXED, PLAIN, Context, encode, tune_mode, tune_report, tune_reset
 
 pytestmark = pytest.mark.gpu
 N, D = 100_000, 4
@@ -45,3 +46,23 @@ def test_wide_level_of_fp64_columns(ds):
     assert np.array_equal(out["loss"], ref["loss"]) and np.array_equal(out["rmse"], ref["rmse"])
     # a narrow level of the same rows is timed
     assert knobs(ds, encode(factors(12), tuned=True), PLAIN)[2] == {"eval_waves"}
+
+
+@pytest.mark.parametrize("prec", [MIXED, CERTIFIED])
+def test_factor_groups(ds, prec):
+    b = encode(factors(14), tuned=True)  # at most 16 factors: one group in every size
+    tune_mode(False)
+    ref = ds.evaluate(b, prec)
+    out, _, rep = knobs(ds, b, prec)
+    assert "fac_group" not in rep
+    assert np.array_equal(out["loss"], ref["loss"]) and np.array_equal(out["rmse"], ref["rmse"])
+    # the sizes differ from 17 factors on, though 48 are few for 16 to a block
+    b = encode(factors(48), tuned=True)
+    tune_mode(False)
+    ref = ds.evaluate(b, prec)
+    out, _, rep = knobs(ds, b, prec)
+    assert "fac_group" in rep
+    e = next(e for e in tune_report() if e["knob"] == "fac_group")
+    # 48 factors in one block take longer than in three; as one and the same launch they would not
+    assert set(e["ms"]) == {64, 32, 16} and e["ms"][64] > 1.3 * e["ms"][16], e
+    assert np.array_equal(out["loss"], ref["loss"]) and np.array_equal(out["rmse"], ref["rmse"])
