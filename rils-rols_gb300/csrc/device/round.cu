@@ -2159,26 +2159,34 @@ rrg_status rrg_context::store_lane_columns() {
   pcache.begin();
   std::vector<int32_t> fsel;
   std::vector<uint64_t> hsel;
+  std::vector<int32_t> pairs;  // (lane column, slot)
   for (size_t f = 0; f < ls.col.size(); ++f) {
     if (need[ls.col[f]] != kNeedEval) continue;
     const FactorProg fp{ls.code.data() + ls.meta[f].x, ls.meta[f].y, ls.consts.data()};
     const uint64_t h = fp.hash();
-    if (pcache.find(fp, h) >= 0) continue;  // stored meanwhile
+    const int32_t s = pcache.find(fp, h);
+    if (s >= 0) {
+      // there already; a column kept in part gives way to a whole one, or every
+      // round that reads it as an operand would evaluate it again
+      if (ls.whole[f] && !pcache.whole(s)) {
+        pcache.set_whole(s, true);
+        pairs.insert(pairs.end(), {ls.col[f], s});
+      }
+      continue;
+    }
     fsel.push_back((int32_t)f);
     hsel.push_back(h);
   }
   const int64_t k = std::min<int64_t>((int64_t)fsel.size(), pcache.available());
-  if (k <= 0) return RRG_OK;
   std::vector<int32_t> slots;
-  if (!pcache.take(k, slots)) return RRG_OK;
-  std::vector<int32_t> pairs(2 * (size_t)k);
-  for (int64_t i = 0; i < k; ++i) {
-    const int32_t f = fsel[i];
-    pcache.insert(FactorProg{ls.code.data() + ls.meta[f].x, ls.meta[f].y, ls.consts.data()}, hsel[i], slots[i],
-                  ls.whole[f] != 0);
-    pairs[2 * i] = ls.col[f];
-    pairs[2 * i + 1] = slots[i];
-  }
+  if (k > 0 && pcache.take(k, slots))
+    for (int64_t i = 0; i < k; ++i) {
+      const int32_t f = fsel[i];
+      pcache.insert(FactorProg{ls.code.data() + ls.meta[f].x, ls.meta[f].y, ls.consts.data()}, hsel[i], slots[i],
+                    ls.whole[f] != 0);
+      pairs.insert(pairs.end(), {ls.col[f], slots[i]});
+    }
+  if (pairs.empty()) return RRG_OK;
   const size_t col8 = sizeof(double) * (size_t)ls.n_pad;
   const size_t n_slots = (size_t)pcache.size();
   if (!d_F64.grow_keep(col8 * n_slots, d_F64.cap) || !d_ccst.grow_keep(sizeof(ColStat) * n_slots, d_ccst.cap) ||
@@ -2188,9 +2196,9 @@ rrg_status rrg_context::store_lane_columns() {
   }
   std::memcpy(h_store.ptr, pairs.data(), sizeof(int32_t) * pairs.size());
   RRG_CUDA(cudaMemcpyAsync(d_store.ptr, h_store.ptr, sizeof(int32_t) * pairs.size(), cudaMemcpyHostToDevice, stream));
-  if (!launch_cache_store(static_cast<const int32_t*>(d_store.ptr), (int32_t)k, static_cast<const double*>(d_fbF64.ptr),
-                          static_cast<const ColStat*>(d_fbcst.ptr), static_cast<double*>(d_F64.ptr),
-                          static_cast<ColStat*>(d_ccst.ptr), ls.n_pad, stream))
+  if (!launch_cache_store(static_cast<const int32_t*>(d_store.ptr), (int32_t)(pairs.size() / 2),
+                          static_cast<const double*>(d_fbF64.ptr), static_cast<const ColStat*>(d_fbcst.ptr),
+                          static_cast<double*>(d_F64.ptr), static_cast<ColStat*>(d_ccst.ptr), ls.n_pad, stream))
     return RRG_E_CUDA;
   ++launches;
   return RRG_OK;
