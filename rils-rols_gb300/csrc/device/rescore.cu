@@ -67,12 +67,13 @@ __global__ void rescore_mark_kernel(const rrg_cand* cands, const int32_t* fb, in
   }
 }
 
-__global__ void __launch_bounds__(kScanThreads) rescore_levels_kernel(const uint8_t* need, const int32_t* level_end,
-                                                                      int32_t n_levels, int32_t* cols, int32_t* count,
-                                                                      int32_t* all, int32_t* all_count) {
+__global__ void __launch_bounds__(kScanThreads) rescore_levels_kernel(const uint8_t* need, const uint8_t* kind,
+                                                                      const int32_t* level_end, int32_t n_levels,
+                                                                      int32_t* cols, int32_t* count, int32_t* fac,
+                                                                      int32_t* fac_count) {
   __shared__ int warp_tot[kScanThreads / 32];
   __shared__ int total;
-  int whole = 0;
+  int n_fac = 0;
   for (int L = 0; L < n_levels; ++L) {
     const int32_t lo = L == 0 ? 0 : level_end[L - 1], hi = level_end[L];
     int base = 0;
@@ -80,16 +81,16 @@ __global__ void __launch_bounds__(kScanThreads) rescore_levels_kernel(const uint
       const int32_t col = c0 + (int32_t)threadIdx.x;
       const int flag = col < hi && need[col] == kNeedEval ? 1 : 0;
       const int pos = block_prefix(flag, warp_tot, &total);
-      if (flag) {
-        cols[lo + base + pos] = col;
-        all[whole + base + pos] = col;
-      }
+      if (flag) cols[lo + base + pos] = col;
       base += total;
+      const int is_fac = flag && kind[col] != kColShared ? 1 : 0;
+      const int fpos = block_prefix(is_fac, warp_tot, &total);
+      if (is_fac) fac[n_fac + fpos] = col;
+      n_fac += total;
     }
     if (threadIdx.x == 0) count[L] = base;
-    whole += base;
   }
-  if (threadIdx.x == 0) *all_count = whole;
+  if (threadIdx.x == 0) *fac_count = n_fac;
 }
 
 __global__ void rescore_buckets_kernel(const rrg_cand* cands, const int32_t* fb, int32_t cap, const PlainCand* pc,
@@ -166,10 +167,10 @@ bool launch_rescore_mark(const rrg_cand* cands, const int32_t* fb, int32_t cap, 
   return launch_ok("launch_rescore_mark");
 }
 
-bool launch_rescore_levels(const uint8_t* need, const int32_t* level_end, int32_t n_levels, int32_t* cols,
-                           int32_t* count, int32_t* all, int32_t* all_count, cudaStream_t st) {
+bool launch_rescore_levels(const uint8_t* need, const uint8_t* kind, const int32_t* level_end, int32_t n_levels,
+                           int32_t* cols, int32_t* count, int32_t* fac, int32_t* fac_count, cudaStream_t st) {
   if (n_levels <= 0) return true;
-  rescore_levels_kernel<<<1, kScanThreads, 0, st>>>(need, level_end, n_levels, cols, count, all, all_count);
+  rescore_levels_kernel<<<1, kScanThreads, 0, st>>>(need, kind, level_end, n_levels, cols, count, fac, fac_count);
   return launch_ok("launch_rescore_levels");
 }
 

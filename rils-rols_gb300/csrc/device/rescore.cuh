@@ -36,10 +36,11 @@ bool launch_cache_store(const int32_t* pairs, int32_t n_pairs, const double* tab
                         double* arena, ColStat* arena_cs, int64_t n_pad, cudaStream_t st);
 
 // Per level L (columns [level_end[L - 1], level_end[L])): the kNeedEval columns
-// in ascending order at cols[level_end[L - 1] ..], their count in count[L];
-// all levels' in one list at all[0 .. *all_count).  One block.
-bool launch_rescore_levels(const uint8_t* need, const int32_t* level_end, int32_t n_levels, int32_t* cols,
-                           int32_t* count, int32_t* all, int32_t* all_count, cudaStream_t st);
+// in ascending order at cols[level_end[L - 1] ..], their count in count[L].  The
+// factors among them (kind, kCol*), of all levels, at fac[0 .. *fac_count).
+// One block.
+bool launch_rescore_levels(const uint8_t* need, const uint8_t* kind, const int32_t* level_end, int32_t n_levels,
+                           int32_t* cols, int32_t* count, int32_t* fac, int32_t* fac_count, cudaStream_t st);
 
 // The tuned candidates of fb[1 .. 1 + fb[0]) whose QR still runs (pc[c].pad
 // bit 0 clear) by column bucket: bucket q's candidates at blist[q * cap ..],

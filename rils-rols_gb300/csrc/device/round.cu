@@ -1478,8 +1478,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       uint8_t* need = static_cast<uint8_t*>(d_fbneed.ptr);
       int32_t* lvl_cols = static_cast<int32_t*>(d_fbcols.ptr);
       int32_t* lvl_count = lvl_cols + ncol;
-      int32_t* all_cols = lvl_count + n_levels;  // the same columns in one list, its length last
-      int32_t* all_count = all_cols + ncol;
+      int32_t* fac_cols = lvl_count + n_levels;  // the factors among them in one list, its length last
+      int32_t* fac_count = fac_cols + ncol;
       double* F64 = static_cast<double*>(d_fbF64.ptr);
       ColStat* cst = static_cast<ColStat*>(d_fbcst.ptr);
       double* gpart = static_cast<double*>(d_fbgram.ptr);
@@ -1540,8 +1540,8 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       if (!launch_rescore_mark(dev.cands, fallback, cnt, pf.at<const int32_t>(d_fbpack, o_liof), d_ccol,
                                pf.at<const int32_t>(d_fbpack, o_doff), pf.at<const int32_t>(d_fbpack, o_deps),
                                n_kept ? d_kept : nullptr, need, stream) ||
-          !launch_rescore_levels(need, pf.at<const int32_t>(d_fbpack, o_lend), n_levels, lvl_cols, lvl_count,
-                                 all_cols, all_count, stream) ||
+          !launch_rescore_levels(need, pf.at<const uint8_t>(d_fbpack, o_kind), pf.at<const int32_t>(d_fbpack, o_lend),
+                                 n_levels, lvl_cols, lvl_count, fac_cols, fac_count, stream) ||
           (n_kept && !launch_lane_copy(need, d_kept, ncol, static_cast<const double*>(d_F64.ptr),
                                        static_cast<const ColStat*>(d_ccst.ptr), F64, cst, ds->n_pad, stream))) {
         cuda_ok(cudaGetLastError(), "re-scoring list launch");
@@ -1590,7 +1590,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
       } else {
         eval_rows(EvalRows{0, ds->n, nullptr});
       }
-      if (!launch_col_sums(F64, dd, all_cols, ncol, all_count, cst, static_cast<double*>(d_cpart.ptr), 8 * sm_count,
+      if (!launch_col_sums(F64, dd, fac_cols, ncol, fac_count, cst, static_cast<double*>(d_cpart.ptr), 8 * sm_count,
                            stream))
         return RRG_E_CUDA;
       if (!launch_nan_settle(dev, dd, fb_list, cnt, d_pcs, d_ccol, cst, true, F64, gpart, coefs, res,
