@@ -625,9 +625,13 @@ __global__ void __launch_bounds__(256) nan_gram_kernel(const int32_t* list, int 
 // from the nbx partial Gram matrices at gp.  n > 0: they are those of some of the n rows, and
 // the columns' squared norms are in cs; a Gram matrix over all rows is larger
 // (in the order of semidefinite matrices), and so is what is left of a column
-// after any other columns are taken out.  (The order of the pivots may differ
-// then, which can cost a factor of K 4^(K - 1) < 1e6; both bounds stay far above
-// the reference's cut.)
+// after any other columns are taken out.  The QR may take the pivots in another
+// order then.  What any order leaves of a column is at least the sample matrix's
+// smallest eigenvalue, and pivoted elimination's smallest pivot is at most
+// K 4^(K - 1) times that; so the pivots have to be that much above the bound of
+// the all-rows form, 1e-24 of the largest squared norm, which then holds in the
+// QR's order too: what is left of a column is at least 1e-12 of the largest norm
+// and of its own, far above rounding (2^-53) and above the cut (2^-52).
 __device__ __noinline__ int gram_certifies(const PlainCand& p, const int32_t* colmap, const ColStat* cs, int nbx,
                                            const double* gp, int64_t n) {
   const int m = p.k - 1;
@@ -643,7 +647,7 @@ __device__ __noinline__ int gram_certifies(const PlainCand& p, const int32_t* co
       G[a][bb] = t;
       G[bb][a] = t;
     }
-  double d0[kGramCols], g0[kGramCols], maxd = 0.0;
+  double d0[kGramCols], g0[kGramCols], maxd = 0.0, floor = 1e-24;
   for (int a = 0; a < K; ++a) d0[a] = g0[a] = G[a][a];
   if (n > 0) {
     int f = 0;
@@ -652,6 +656,7 @@ __device__ __noinline__ int gram_certifies(const PlainCand& p, const int32_t* co
       if (!(st.flags & kCsNaN)) d0[f++] = st.sumsq;
     }
     d0[K - 1] = (double)n;
+    floor *= ldexp((double)K, 2 * (K - 1));
   }
   for (int a = 0; a < K; ++a) maxd = fmax(maxd, d0[a]);
   int piv[kGramCols];
@@ -662,7 +667,7 @@ __device__ __noinline__ int gram_certifies(const PlainCand& p, const int32_t* co
     for (int j = s2 + 1; j < K; ++j)
       if (G[j][j] > G[q][q]) q = j;
     const double dp = G[q][q];
-    if (!(dp > 1e-8 * d0[piv[q]]) || !(dp > 1e-24 * maxd)) return dp < 1e-13 * g0[piv[q]] ? -1 : 0;
+    if (!(dp > 1e-8 * d0[piv[q]]) || !(dp > floor * maxd)) return dp < 1e-13 * g0[piv[q]] ? -1 : 0;
     if (q != s2) {
       for (int j = 0; j < K; ++j) { const double t = G[s2][j]; G[s2][j] = G[q][j]; G[q][j] = t; }
       for (int j = 0; j < K; ++j) { const double t = G[j][s2]; G[j][s2] = G[j][q]; G[j][q] = t; }
