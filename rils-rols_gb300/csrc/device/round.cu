@@ -1056,19 +1056,18 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     return eval_rows(gsets[ngv], false, 0, q_first, nullptr) && launch_live_columns(la, stream) &&
            eval_rows(gs, stage, q_first, n_chunks, la.live);
   };
-  // The probe needs nothing of the table and runs beside the evaluation (a lone
-  // candidate at 50k rows 137 -> 117 us, eight rounds at 1M rows 91.0 -> 90.0 ms;
-  // rounds that fill the GPU take the same time as one after the other).  In a
-  // round with a trial it comes after, so that the evaluation is timed alone.
-  auto probe = [&] {
-    return cudaEventRecord(fork_ev, stream) == cudaSuccess && cudaStreamWaitEvent(side[1], fork_ev, 0) == cudaSuccess &&
-           launch_fac_probe(pkt.at<const uint32_t>(d_ftp, o_code), pkt.at<const int2>(d_ftp, o_meta),
-                            (int32_t)mprog.size(), dev.consts, dev.consts32, dev.consts32lo, dd, cprobe, side[1],
-                            pkt.at<const int32_t>(d_ftp, o_pslot)) &&
-           cudaEventRecord(join_ev[1], side[1]) == cudaSuccess;
+  // The probe needs nothing of the table and runs beside the evaluation, but is
+  // launched after it: the evaluation's blocks come first and the probe's fill
+  // what they leave (one candidate of a long factor at 50k rows 261 us with the
+  // probe in series, 177 beside; of a short one 122, 106, and 114 where the probe
+  // is launched first, which also costs eight rounds at 1M rows 0.3 of 93 ms).
+  // In a round with a trial it waits for that too, so that the evaluation is
+  // timed alone.
+  auto probe_from_here = [&] {
+    return cudaEventRecord(fork_ev, stream) == cudaSuccess && cudaStreamWaitEvent(side[1], fork_ev, 0) == cudaSuccess;
   };
   const bool trial = gtrial || (strial && maps_ok && can_stage(gsets[0]));
-  if (!trial && !probe()) return RRG_E_CUDA;
+  if (!trial && !probe_from_here()) return RRG_E_CUDA;
   int gbest = 0;  // the group set in use
   if (gtrial) {
     // the first round of this row class: every group size timed on the
@@ -1101,7 +1100,12 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
   } else if (!gtrial && !eval_all(gsets[0], stage_pick && stage_ok)) {
     return RRG_E_CUDA;
   }
-  if (trial && !probe()) return RRG_E_CUDA;
+  if ((trial && !probe_from_here()) ||
+      !launch_fac_probe(pkt.at<const uint32_t>(d_ftp, o_code), pkt.at<const int2>(d_ftp, o_meta),
+                        (int32_t)mprog.size(), dev.consts, dev.consts32, dev.consts32lo, dd, cprobe, side[1],
+                        pkt.at<const int32_t>(d_ftp, o_pslot)) ||
+      cudaEventRecord(join_ev[1], side[1]) != cudaSuccess)
+    return RRG_E_CUDA;
   // Pair map: self pairs by slot (entries -2 - p into the slots' self
   // sums); cross pairs oriented so that `a` is the rarer factor (its
   // partners are then the widely shared ones, hot in L2) and kept across
