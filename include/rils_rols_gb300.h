@@ -350,8 +350,8 @@ int32_t rrg_last_round_bytes(const rrg_context* ctx, double* bytes, int32_t n);
  * feature count d, 1..64).  Knobs 0 and 5 (the warps per CTA of an earlier
  * cluster QR) are retired: the QR's passes have one shape.  With
  * RRG_TUNE_ON (the default) the first launch of a (knob, bucket, row class
- * floor(log2 n)) that carries enough work is timed in every shape, and the
- * fastest is kept for the process (and in the file named by the environment
+ * floor(log2 n)) that carries enough work, and whose evaluator shapes are not one
+ * and the same launch there, is timed in every shape, and the fastest is kept for the process (and in the file named by the environment
  * variable RRG_TUNE_CACHE, when set); RRG_TUNE_OFF uses the built-in shapes.
  * No counterpart in the reference. */
 #define RRG_TUNE_OFF 0

@@ -76,7 +76,7 @@ struct DevData {
 struct PlainCand {
   int64_t a_col;   // first column of its factor values in the A arena (n_pad doubles per column)
   int64_t m_col;   // first column of its QR working copy (k+1 columns)
-  int64_t s_off;   // offset of its stacked R blocks (TSQR only)
+  int64_t s_off;   // unused (0)
   int32_t k;       // OLS columns (factors + free term); 1 when untuned
   int32_t pad;
 };

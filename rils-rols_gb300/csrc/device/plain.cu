@@ -30,10 +30,9 @@ constexpr int kMaxK = RRG_MAX_TERMS;
 // pipes (csrc/common/fp64_int.h) and the elementary functions in their split
 // forms (rr_math_split.h): the kernel is bound by the FP64 pipe (an
 // instruction holds it for 16 cycles), so what leaves it is what is saved.
-// GB300, ms of the FP64 evaluation phase with native operations / now: 2048
-// random trees at 100k rows 105.1 / 78.5 (all their rows; fewer are evaluated
-// now, see EvalRows), a 660-candidate local-search round at 1M rows 23.2 / 17.4
-// (12.8 with the pieces and six blocks an SM).  The results are the same bits.
+// GB300, the FP64 evaluation of a 660-candidate local-search round at 1M rows with
+// native operations / with these, all else alike: 23.2 / 17.4 ms (12.8 with the
+// pieces of eval_pieces and shared memory by need).  The results are the same bits.
 __device__ __forceinline__ double bin64(int base, double a, double b) {
   switch (base) {
     case RRG_ADD: return __dadd_rn(a, b);
@@ -122,8 +121,8 @@ __device__ __forceinline__ double run_row64(const uint32_t* code, int len, const
 // some block has stored a NaN at row kStopRow or later, the blocks leave off
 // (the block of row 0 after its first rows, so that rows below kStopRow are
 // all there).  2048 random trees at 100k rows, seven of eight with a NaN
-// somewhere: 78.5 ms without the stop, 23.8 with it, 14.3 in
-// pieces of 4096 rows, 7.4 with the shared columns left out that no factor needs.
+// somewhere: with the pieces (eval_pieces) and the shared columns left out that no
+// factor needs (eval_two_parts) 6.9 ms, where all their rows took 78.5.
 __device__ __forceinline__ void eval_column_stats(const uint32_t* code, int len, const double* consts,
                                                   const DevData& ds, int64_t r0, int64_t r1, double* st, int levels, double* Ac,
                                                   const double* T, uint32_t* status, ColStat* cs, bool stop,
@@ -738,7 +737,8 @@ __global__ void __launch_bounds__(256) nan_settle_kernel(DevBatch b, const int32
     if (threadIdx.x == 0) {
       const int r = gram_certifies(p, colmap, cs, 1, g, n);
       // dependent on the sample: most likely on all rows, and the QR's to find
-      // (8192 random trees' re-scoring, with its evaluation, 14.8 -> 13.9 ms)
+      // (8192 random trees' re-scoring with its evaluation 13.9 ms, 14.8 with the
+      // Gram matrix of all rows for these)
       if (r) settle_candidate(b, c, pc, r > 0, coefs, res, decided);
       pad = r ? 1 : 2;
     }
@@ -766,10 +766,9 @@ bool launch_nan_settle(const DevBatch& b, const DevData& ds, const int32_t* list
   if (cnt <= 0) return true;
   // Up to kGramRows rows one launch settles every candidate.  Above, what the
   // sample leaves open goes over all rows with several blocks a candidate.
-  // (A lone candidate of 150 rows is launches and latency: 106 -> 91 us with one
-  // launch here, one to begin a table and no side stream for one QR.  The sample
-  // instead of all rows: 765 candidates at 20011 rows 0.28 -> 0.06 ms; 2048 random
-  // trees at 100k rows, with the evaluation, 7.4 -> 6.9.)
+  // (A lone candidate of 150 rows is launches and latency.  The sample, against all
+  // rows at once: 765 candidates at 20011 rows 0.06 against 0.28 ms; 2048 random
+  // trees at 100k rows, with the evaluation, 6.9 against 7.4.)
   const int nbx = nan_gram_blocks(ds.n);
   *launches += 1;
   if (!launch_next(true, nan_settle_kernel, dim3(cnt), 256, 0, st, b, list, cnt, pc, colmap, cs, T, ds.n, ds.n_pad,

@@ -26,8 +26,8 @@ struct EvalRows {
 // rows of all levels are evaluated first, live_columns_kernel finds what still
 // counts, and the other rows of the other columns are left out.  (They are
 // nobody's: a shared column lives for one round.)  2048 random trees at 100k rows,
-// 2100 shared columns: FP64 evaluation 14.3 -> 7.4 ms (8.0 with 4096 first rows,
-// 8.4 with 8192); 8192 trees: double-float 13.6 -> 6.5 ms, re-scoring 18.9 -> 14.8.
+// 2100 shared columns: FP64 evaluation 7.4 ms, in one part 14.3 (8.0 with 4096
+// first rows, 8.4 with 8192); 8192 trees: double-float 6.5, in one part 13.6.
 // Where few columns are shared, or the work is below about 2 ms, the second pass
 // over the levels could cost more than it saves.
 constexpr int64_t kFirstRows = 1024;

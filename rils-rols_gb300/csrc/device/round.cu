@@ -61,7 +61,8 @@ int64_t fp64_cache_slots(size_t scratch_bytes, int64_t n_pad) {
 }
 // rows from which rounds keep their columns: below, evaluating a column
 // costs less than the bookkeeping of finding it (a 569-row classifier
-// search ran 0.46 ms per round slower with the cache)
+// search ran 0.46 ms per round slower with the cache on an earlier build; now a
+// first round of 1000 unlike trees, which finds nothing, 0.5 ms at 8192 rows)
 constexpr int64_t kCacheMinRows = 8192;
 
 bool const_arg(int op) {
@@ -1337,7 +1338,7 @@ rrg_status rrg_context::mixed_subround(const rrg_dataset* ds, const int32_t* lis
     // The residual-pass list is compacted from the solve's flags; the FP64
     // re-scoring lane evaluates, from the round's own table programs, only
     // the columns its candidates read, decides the certain sentinels, and
-    // factorises the rest with the list form of the cluster QR.  Every value
+    // factorises the rest with the list form of the chunked QR.  Every value
     // is computed by the same arithmetic as the host-driven path.
     // ------------------------------------------------------------------
     const size_t col8 = sizeof(double) * (size_t)ds->n_pad;

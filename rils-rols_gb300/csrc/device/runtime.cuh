@@ -177,9 +177,11 @@ struct rrg_context {
   // certified bound on the relative fitness error of a mixed result; larger
   // bounds are re-scored by the FP64 path
   double cert_tol = 5e-7;
-  // datasets with fewer rows run mixed-precision rounds in FP64 (at 569 rows
-  // a 600-candidate round takes 1.4 ms in FP64 against 3.0 ms mixed; the
-  // mixed form wins from about 7000 rows)
+  // datasets with fewer rows run mixed-precision rounds in FP64.  FP64 / certified
+  // ms of a round: 1760 neighbours of a model at 569 rows 0.92 / 1.49, 2000 1.57 /
+  // 1.53, 8192 3.30 / 2.13; 1000 unlike trees at 569 rows 1.92 / 2.87, 8192 4.00 /
+  // 5.58, 50000 8.35 / 8.29: neighbourhoods would gain from about 2000 rows on,
+  // unlike trees lose up to 50000
   int64_t mixed_min_rows = 8192;
   // optional per-phase device timing (CUDA events on the context stream)
   bool timing = false;
