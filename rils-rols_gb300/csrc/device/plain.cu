@@ -655,7 +655,7 @@ __device__ __noinline__ int gram_certifies(const PlainCand& p, const int32_t* co
       if (!(st.flags & kCsNaN)) d0[f++] = st.sumsq;
     }
     d0[K - 1] = (double)n;
-    floor *= ldexp((double)K, 2 * (K - 1));
+    floor *= (double)(K << 2 * (K - 1));
   }
   for (int a = 0; a < K; ++a) maxd = fmax(maxd, d0[a]);
   int piv[kGramCols];
